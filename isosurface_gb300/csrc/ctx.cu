@@ -230,6 +230,11 @@ void classify(iso_program* p) {
         p->kind = PK_SPHERE_SET_HARD;
         p->set_at = arg(set_pc);
         p->set_n = (uint32_t)p->consts[p->set_at];
+    } else if (set_pc != SIZE_MAX) {
+        p->smooth_set = true;
+        p->set_at = arg(set_pc);
+        p->set_n = (uint32_t)p->consts[p->set_at];
+        p->set_k = p->consts[p->set_at + 2];
     }
     // [DOMAIN] TRANSLATE prim POP (TRANSLATE prim POP UNION)* [POP]: a left
     // fold of hard unions over translated primitives, compiled to a flat list
@@ -630,7 +635,7 @@ iso_status iso_program_create(iso_ctx* ctx, const uint8_t* bytes, size_t len, is
     auto at16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t o_ops = 0, o_consts = at16(o_ops + 4 * p->ops.size()), o_jump = at16(o_consts + 4 * nk);
     const size_t o_set = at16(o_jump + 4 * p->jump.size());
-    const size_t set_bytes = p->kind == PK_SPHERE_SET_HARD ? 16ull * p->set_n : 0;
+    const size_t set_bytes = p->kind == PK_SPHERE_SET_HARD || p->smooth_set ? 16ull * p->set_n : 0;
     const size_t o_prims = at16(o_set + set_bytes), total = at16(o_prims + 4 * p->prims.size());
     std::vector<unsigned char> staged(total, 0);
     std::memcpy(staged.data() + o_ops, p->ops.data(), 4 * p->ops.size());

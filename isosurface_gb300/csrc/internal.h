@@ -167,10 +167,13 @@ struct iso_program {
     uint32_t* d_ops = nullptr;
     float* d_consts = nullptr;
     int32_t* d_jump = nullptr;
-    float* d_set = nullptr;  // PK_SPHERE_SET_HARD: n float4 spheres, 16-byte aligned
+    float* d_set = nullptr;  // PK_SPHERE_SET_HARD or smooth_set: n float4 spheres, 16-byte aligned
     int kind = iso::PK_GENERIC;
     bool has_normal = true;
-    // PK_SPHERE_SET_HARD
+    // PK_SPHERE_SET_HARD or smooth_set (a PK_GENERIC program that is one smooth
+    // sphere set, optionally behind a domain map)
+    bool smooth_set = false;
+    float set_k = 0.0f;  // smooth_set: the smooth minimum's width
     bool has_domain = false;
     float domain[6] = {0, 0, 0, 0, 0, 0};
     uint32_t set_at = 0, set_n = 0;

@@ -2,9 +2,10 @@
 // (src/traversal/primal_grid.rs:44-70) as kernels that write the f32 field
 // and, with warp ballots, the packed sign bits (bit set iff !(v > 0),
 // classify_corners, marching_cubes_impl.rs:26-37) that the marching-cubes
-// passes classify from.  launch_sample_grid picks one of three samplers:
+// passes classify from.  launch_sample_grid picks one of four samplers:
 // for the extractors (near_only) on a hard union of spheres, the per-tile
-// sphere culling below; on another program with a Lipschitz bound and a
+// sphere culling below, on a smooth union the per-box sphere lists of
+// smooth_set.cuh; on another program with a Lipschitz bound and a
 // lattice of at least one tile per SM, the culled sampler of bricks_core.cuh
 // (compiled for the program by jit.cu when it can be, else interpreted);
 // otherwise every point (field_warp): for a full field with the program's
@@ -22,6 +23,7 @@
 #include "bricks.cuh"
 #include "internal.h"
 #include "vm.cuh"
+#include "smooth_set.cuh"
 
 namespace iso {
 namespace {
@@ -589,12 +591,17 @@ iso_status launch_sample_grid(iso_ctx* ctx, const iso_program* prog, uint32_t nx
                               float* field, uint64_t pitch, uint32_t* bits, bool near_only, uint32_t zoff,
                               float reach_steps) {
     const uint32_t W = words_per_row(nx);
+    const bool smooth = near_only && smooth_culled(prog, nx, ny, nz);
     // the culled sampler (bricks.cuh) for the extractors on general
     // programs; hard sphere unions have their own culling below
-    const bool bricks = near_only && prog->lip > 0.0f && 4 * W <= BRICK_MAX &&
+    const bool bricks = near_only && !smooth && prog->lip > 0.0f && 4 * W <= BRICK_MAX &&
                         brick_tiles(W, ny, nz) >= (uint64_t)ctx->sms && brick_tiles(W, ny, nz) < (1ull << 22) &&
                         !(prog->kind == PK_SPHERE_SET_HARD && prog->set_n <= 8192);
-    if (bricks) {
+    if (smooth) {
+        iso_status s = launch_smooth_set(
+            ctx, prog, brick_lattice(prog, nx, ny, nz, inv, field, pitch, bits, W, zoff, reach_steps));
+        if (s != ISO_OK) return s;
+    } else if (bricks) {
         // values only where marching cubes can read them (bricks.cuh): tiles
         // of 4 layers x up to 32 rows, one block each, then the mixed
         // sub-bricks over a persistent grid.  A grid with fewer tiles than
