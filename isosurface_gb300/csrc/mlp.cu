@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -50,93 +51,218 @@ __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-
 __host__ __device__ __forceinline__ float freq(int j) { return 3.14159265358979f * exp2f((float)(7 * j) / 15.0f); }
 
 // ------------------------------------------------------------ fp32 GEMM ---
-// C[M x N] (ldc) (+)= op(A)[M x K] * op(B)[K x N], element (i,k) of op(A) at
-// A[i*sa0 + k*sa1], element (k,j) of op(B) at B[k*sb0 + j*sb1].  64x64 tiles,
-// 256 threads, 4x4 per thread.  Split-K over gridDim.z accumulates with
-// atomicAdd (accumulate must be set then).  bias (nullable) is added per column
-// by the z == 0 slice.
-constexpr int TM = 64, TN = 64, TK = 16;
+// C[M x N] = A[M x K] * B[K x N] in fp32 FMAs, packed two rows to an
+// instruction (fma.rn.f32x2: the FMA pipe's full rate from half of the issue
+// slots, which leaves room for the shared-memory loads).  256 threads as 16 x
+// 16, BM = 16 TM, BN = 16 TN, K steps of 8 by asynchronous copies, three steps
+// ahead (through registers, ptxas sank the loads to where they were stored:
+// 59 % of the FMA pipe, mostly waiting for them).
+//   A_K: element (i, k) of A at A[i * lda + k], else at A[k * lda + i]
+//   B_K: element (k, j) of B at B[j * ldb + k], else at B[k * ldb + j]
+// M and K may be any numbers (M a multiple of 4 where A is not K-contiguous);
+// N, lda and ldb are multiples of 4, the pointers are 16-byte
+// aligned.
+//   EPI_FORWARD   C = acc + bias[j] and C2 = softplus(C)
+//   EPI_BACKWARD  C = acc * sigmoid(Z[i][j]), and colsum[j] += its column sums
+//   EPI_WEIGHTS   C += acc by atomics, K split over gridDim.z
+// 65536 x 256 x 256 (8.6 GFLOP) on the GB300, whose FMA pipe reaches 77
+// TFLOP/s: 0.17 ms as the weights' product (50 TFLOP/s, bound by the packed
+// FMAs' register reads: 67 % of the pipe), 0.19 ms with either elementwise
+// epilogue.  64 x 64 tiles with scalar loads and 4 x 4 per thread took 0.59
+// and 0.67 ms, and 0.05-0.13 ms more for the elementwise passes, column sums
+// and copies that the epilogues replace.  Scalar FMAs in the same tiles: 0.17
+// and 0.21 ms.
+enum Epilogue { EPI_FORWARD, EPI_BACKWARD, EPI_WEIGHTS };
+constexpr int TK = 8;
+constexpr int STAGES = 4;  // K steps of shared memory, three of them in flight
 
-__global__ void __launch_bounds__(256) sgemm(int M, int N, int K, const float* __restrict__ A, int64_t sa0,
-                                             int64_t sa1, const float* __restrict__ B, int64_t sb0, int64_t sb1,
-                                             float* __restrict__ C, int64_t ldc, const float* __restrict__ bias,
-                                             int accumulate) {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int i0 = blockIdx.y * TM, j0 = blockIdx.x * TN;
-    const int kslices = gridDim.z;
-    const int kper = ((K + kslices - 1) / kslices + TK - 1) / TK * TK;
-    const int kbeg = blockIdx.z * kper, kend = min(K, kbeg + kper);
-    float acc[4][4] = {};
-    for (int k0 = kbeg; k0 < kend; k0 += TK) {
-        for (int t = threadIdx.x; t < TK * TM; t += 256) {
-            const int kk = t / TM, ii = t % TM;
-            const int gi = i0 + ii, gk = k0 + kk;
-            As[kk][ii] = (gi < M && gk < kend) ? A[(int64_t)gi * sa0 + (int64_t)gk * sa1] : 0.0f;
+struct GemmArgs {
+    int M, N, K;
+    const float* A;
+    const float* B;
+    int lda, ldb;
+    float* C;
+    int ldc;
+    const float* bias;  // EPI_FORWARD
+    float* C2;          // EPI_FORWARD
+    const float* Z;     // EPI_BACKWARD, laid out as C
+    float* colsum;      // EPI_BACKWARD
+};
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// Asynchronous copy of one operand's tile, E rows (or columns) x TK, to
+// s[k][e]; KC says whether k is its contiguous index (4 bytes at a time then,
+// transposing; 16 otherwise).  Entries past the limits are zero.
+template <int E, bool KC>
+__device__ __forceinline__ void copy_tile(float (*s)[E + 4], const float* __restrict__ p, int ld, int e0, int elim,
+                                          int k0, int klim) {
+    if (KC) {
+#pragma unroll
+        for (int i = 0; i < E * TK / 256; ++i) {
+            const int k = threadIdx.x % TK, e = threadIdx.x / TK + (256 / TK) * i;
+            const bool in = e0 + e < elim && k0 + k < klim;
+            const float* src = in ? p + (int64_t)(e0 + e) * ld + k0 + k : p;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(&s[k][e])),
+                         "l"(src), "r"(in ? 4 : 0));
         }
-        for (int t = threadIdx.x; t < TK * TN; t += 256) {
-            const int kk = t / TN, jj = t % TN;
-            const int gj = j0 + jj, gk = k0 + kk;
-            Bs[kk][jj] = (gj < N && gk < kend) ? B[(int64_t)gk * sb0 + (int64_t)gj * sb1] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[kk][ty * 4 + r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx * 4 + c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
-        }
-        __syncthreads();
+    } else if (threadIdx.x < E * TK / 4) {
+        const int k = threadIdx.x / (E / 4), e = 4 * (threadIdx.x % (E / 4));
+        const bool in = e0 + e < elim && k0 + k < klim;
+        const float* src = in ? p + (int64_t)(k0 + k) * ld + e0 + e : p;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(&s[k][e])),
+                     "l"(src), "r"(in ? 16 : 0));
     }
+}
+
+template <int TM, int TN, bool A_K, bool B_K, int EPI>
+__global__ void __launch_bounds__(256, 2) gemm_f32(GemmArgs G) {
+    constexpr int BM = 16 * TM, BN = 16 * TN;
+    __shared__ __align__(16) float As[STAGES][TK][BM + 4];
+    __shared__ __align__(16) float Bs[STAGES][TK][BN + 4];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
+    int kbeg = 0, kend = G.K;
+    if (EPI == EPI_WEIGHTS) {
+        const int per = ((G.K + (int)gridDim.z - 1) / (int)gridDim.z + TK - 1) / TK * TK;
+        kbeg = min(G.K, (int)blockIdx.z * per);
+        kend = min(G.K, kbeg + per);
+    }
+    uint64_t acc[TM / 2][TN] = {};  // pairs of rows
+    const int steps = (kend - kbeg + TK - 1) / TK;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            copy_tile<BM, A_K>(As[step % STAGES], G.A, G.lda, i0, G.M, kbeg + step * TK, kend);
+            copy_tile<BN, B_K>(Bs[step % STAGES], G.B, G.ldb, j0, G.N, kbeg + step * TK, kend);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int step = 0; step < STAGES - 1; ++step) fetch(step);
+    for (int step = 0; step < steps; ++step) {
+        const int buf = step % STAGES;
+        // this step's copies have landed, and every thread is done with the
+        // step before, whose buffer the next copies take
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();
+        fetch(step + STAGES - 1);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int gi = i0 + ty * 4 + r;
-        if (gi >= M) continue;
+        for (int k = 0; k < TK; ++k) {
+            // rows ty*4.. (and BM/2 + ty*4..), columns tx*4.. (and BN/2 + tx*4..)
+            uint64_t a[TM / 2], b[TN];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int gj = j0 + tx * 4 + c;
-            if (gj >= N) continue;
-            float v = acc[r][c];
-            if (bias && blockIdx.z == 0) v += bias[gj];
-            float* dst = C + (int64_t)gi * ldc + gj;
-            if (accumulate) atomicAdd(dst, v);
-            else *dst = v;
+            for (int h = 0; h < TM / 4; ++h) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&As[buf][k][h * (BM / 2) + ty * 4]);
+                a[2 * h] = q.x;
+                a[2 * h + 1] = q.y;
+            }
+#pragma unroll
+            for (int h = 0; h < TN / 4; ++h) {
+                const float4 q = *reinterpret_cast<const float4*>(&Bs[buf][k][h * (BN / 2) + tx * 4]);
+                b[4 * h] = pack2(q.x, q.x);
+                b[4 * h + 1] = pack2(q.y, q.y);
+                b[4 * h + 2] = pack2(q.z, q.z);
+                b[4 * h + 3] = pack2(q.w, q.w);
+            }
+#pragma unroll
+            for (int r = 0; r < TM / 2; ++r)
+#pragma unroll
+                for (int c = 0; c < TN; ++c) acc[r][c] = fma2(a[r], b[c], acc[r][c]);
+        }
+    }
+    float col[TN] = {};
+#pragma unroll
+    for (int r = 0; r < TM; ++r) {
+        const int gi = i0 + (r / 4) * (BM / 2) + ty * 4 + r % 4;
+        if (gi >= G.M) continue;
+#pragma unroll
+        for (int h = 0; h < TN / 4; ++h) {
+            const int gj = j0 + h * (BN / 2) + tx * 4;
+            if (gj >= G.N) continue;
+            float v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float2 two = unpack2(acc[r / 2][4 * h + c]);
+                v[c] = r % 2 ? two.y : two.x;
+            }
+            const int64_t at = (int64_t)gi * G.ldc + gj;
+            if (EPI == EPI_FORWARD) {
+                const float4 bb = __ldg(reinterpret_cast<const float4*>(G.bias + gj));
+                const float4 z = make_float4(v[0] + bb.x, v[1] + bb.y, v[2] + bb.z, v[3] + bb.w);
+                *reinterpret_cast<float4*>(G.C + at) = z;
+                *reinterpret_cast<float4*>(G.C2 + at) =
+                    make_float4(softplus(z.x), softplus(z.y), softplus(z.z), softplus(z.w));
+            } else if (EPI == EPI_BACKWARD) {
+                const float4 z = __ldg(reinterpret_cast<const float4*>(G.Z + at));
+                const float4 d = make_float4(v[0] * sigmoid(z.x), v[1] * sigmoid(z.y), v[2] * sigmoid(z.z),
+                                             v[3] * sigmoid(z.w));
+                *reinterpret_cast<float4*>(G.C + at) = d;
+                col[4 * h] += d.x;
+                col[4 * h + 1] += d.y;
+                col[4 * h + 2] += d.z;
+                col[4 * h + 3] += d.w;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) atomicAdd(G.C + at + c, v[c]);
+            }
+        }
+    }
+    if (EPI == EPI_BACKWARD) {
+        // column sums of the tile: over the 16 thread rows in shared memory
+        __syncthreads();  // the last step's tile is used
+        float(*s_col)[BN] = reinterpret_cast<float(*)[BN]>(&Bs[0][0][0]);
+#pragma unroll
+        for (int c = 0; c < TN; ++c) s_col[ty][(c / 4) * (BN / 2) + tx * 4 + c % 4] = col[c];
+        __syncthreads();
+        for (int j = threadIdx.x; j < BN && j0 + j < G.N; j += 256) {
+            float sum = 0.0f;
+            for (int r = 0; r < 16; ++r) sum += s_col[r][j];
+            atomicAdd(G.colsum + j0 + j, sum);
         }
     }
 }
 
-void gemm(cudaStream_t s, int M, int N, int K, const float* A, int64_t sa0, int64_t sa1, const float* B, int64_t sb0,
-          int64_t sb1, float* C, int64_t ldc, const float* bias, bool accumulate, int ksplit = 1) {
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, ksplit);
-    sgemm<<<grid, 256, 0, s>>>(M, N, K, A, sa0, sa1, B, sb0, sb1, C, ldc, bias, accumulate ? 1 : 0);
+// 128 x 128 tiles once they give every SM one (n x 256 outputs: n >= 64 per
+// SM), else 64 x 64 ones, four times as many blocks
+template <bool A_K, bool B_K, int EPI>
+void gemm(cudaStream_t s, int sms, const GemmArgs& G) {
+    if (EPI != EPI_WEIGHTS && (int64_t)((G.M + 127) / 128) * ((G.N + 127) / 128) < sms)
+        gemm_f32<4, 4, A_K, B_K, EPI><<<dim3((G.N + 63) / 64, (G.M + 63) / 64), 256, 0, s>>>(G);
+    else if (EPI != EPI_WEIGHTS)
+        gemm_f32<8, 8, A_K, B_K, EPI><<<dim3((G.N + 127) / 128, (G.M + 127) / 128), 256, 0, s>>>(G);
+    else {
+        // K = the points: slices of at least 64, two blocks per SM
+        const int tiles = ((G.N + 127) / 128) * ((G.M + 127) / 128);
+        const int slices = std::max(1, std::min(2 * sms / tiles, (G.K + 63) / 64));
+        gemm_f32<8, 8, A_K, B_K, EPI><<<dim3((G.N + 127) / 128, (G.M + 127) / 128, slices), 256, 0, s>>>(G);
+    }
 }
 
 // ------------------------------------------------------- elementwise kernels ---
+// one thread per frequency: its sine and cosine
 __global__ void fourier(const float* pts, uint32_t n, float* out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * FF) return;
-    const uint32_t p = i / FF, f = i % FF;
-    const uint32_t a = f / 32, j = (f % 32) / 2;
-    const float x = freq(j) * pts[3 * p + a];
-    out[i] = (f & 1) ? cosf(x) : sinf(x);
-}
-
-__global__ void act_softplus(const float* z, float* a, uint64_t n) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = softplus(z[i]);
-}
-
-// dz = da * sigmoid(z), in place on da
-__global__ void act_backward(const float* z, float* da, uint64_t n) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) da[i] *= sigmoid(z[i]);
+    if (i >= n * (FF / 2)) return;
+    const uint32_t p = i / (FF / 2), f = i % (FF / 2);
+    const float x = freq(f % 16) * pts[3 * p + f / 16];
+    float sn, cs;
+    sincosf(x, &sn, &cs);
+    reinterpret_cast<float2*>(out)[i] = make_float2(sn, cs);
 }
 
 // y[p] = a[p] . w + b; warp per point
@@ -153,35 +279,54 @@ __global__ void out_forward(const float* a, uint32_t n, const float* w, const fl
 // Truncated L1: e = y - t inside the band |t| < d; where the target is
 // saturated (t >= d or t <= -d) only a prediction on the band's side of +-d
 // is penalised (e = min(y - d, 0) or max(y + d, 0)).  loss = mean |e|,
-// dy = sign(e) / n; the loss accumulates into *loss.
-__global__ void loss_l1(const float* y, const float* t, uint32_t n, float clampd, float* dy, float* loss) {
+// dy = sign(e) / n; the loss accumulates into *loss and the sum of dy (the
+// output bias' gradient) into *dsum.
+__global__ void loss_l1(const float* y, const float* t, uint32_t n, float clampd, float* dy, float* loss,
+                        float* dsum) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
+    float l = 0.0f, g = 0.0f;
     if (i < n) {
         const float ti = t[i], yi = y[i];
         const float d = (ti >= clampd) ? fminf(yi - clampd, 0.0f) : (ti <= -clampd) ? fmaxf(yi + clampd, 0.0f) : yi - ti;
         l = fabsf(d);
-        dy[i] = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f)) / (float)n;
+        g = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f)) / (float)n;
+        dy[i] = g;
     }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l / (float)n);
+    for (int o = 16; o > 0; o >>= 1) {
+        l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
+        g += __shfl_xor_sync(0xFFFFFFFFu, g, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(loss, l / (float)n);
+        atomicAdd(dsum, g);
+    }
 }
 
-// da[p][k] = dy[p] * w[k]
-__global__ void out_backward_act(const float* dy, const float* w, uint32_t n, float* da) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (uint64_t)n * HID) da[i] = dy[i / HID] * w[i % HID];
-}
-
-// column sums: out[j] += sum_p m[p][j]  (block per 256 columns chunk of rows)
-__global__ void colsum(const float* m, uint32_t n, uint32_t cols, float* out) {
-    const uint32_t j = threadIdx.x;
-    if (j >= cols) return;
-    const uint32_t rows_per = (n + gridDim.x - 1) / gridDim.x;
-    const uint32_t r0 = blockIdx.x * rows_per, r1 = min(n, r0 + rows_per);
-    float s = 0.0f;
-    for (uint32_t r = r0; r < r1; ++r) s += m[(size_t)r * cols + j];
-    atomicAdd(out + j, s);
+// The backward pass of the output layer in one read of the last layer's z
+// and a (thread = column, a range of points per block):
+//   dz[p][k] = dy[p] w[k] sigmoid(z[p][k]), its column sums into gb, and
+//   gw[k] += sum_p dy[p] a[p][k]
+__global__ void __launch_bounds__(HID) out_backward(const float* __restrict__ dy, const float* __restrict__ w,
+                                                    const float* __restrict__ z, const float* __restrict__ a,
+                                                    uint32_t n, float* __restrict__ dz, float* gw, float* gb) {
+    const uint32_t k = threadIdx.x;
+    const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
+    const uint32_t p0 = blockIdx.x * per, p1 = min(n, p0 + per);
+    const float wk = w[k];
+    float sw = 0.0f, sb = 0.0f;
+#pragma unroll 4
+    for (uint32_t p = p0; p < p1; ++p) {
+        const float g = __ldg(dy + p);
+        const size_t at = (size_t)p * HID + k;
+        const float d = g * wk * sigmoid(z[at]);
+        dz[at] = d;
+        sb += d;
+        sw += g * a[at];
+    }
+    if (p0 < p1) {
+        atomicAdd(gw + k, sw);
+        atomicAdd(gb + k, sb);
+    }
 }
 
 __global__ void adam(float* p, const float* g, float* m, float* v, uint64_t n, float lr, float b1, float b2,
@@ -249,14 +394,18 @@ using namespace iso::mlp;
 namespace {
 
 struct Views {
-    float *pts, *ff, *z[NLAYERS], *a[NLAYERS], *y, *t, *dy, *da, *db_scratch, *loss;
+    float *pts, *ff, *z[NLAYERS], *a[NLAYERS], *y, *t, *dy, *d[2], *loss;
 };
+
+// each piece starts on a 256-byte boundary (the GEMMs load 16 bytes at once)
+inline size_t piece(size_t floats) { return (floats + 63) & ~(size_t)63; }
 
 iso_status ensure_work(iso_mlp* net, uint32_t n) {
     if (n <= net->cap && net->work) return ISO_OK;
     if (net->work) cudaFree(net->work);
     net->work = nullptr;
-    const size_t floats = (size_t)n * (3 + FF + 2 * NLAYERS * HID + 3 + 2 * HID) + 1024;
+    const size_t floats = piece(3 * (size_t)n) + piece(FF * (size_t)n) + (2 * NLAYERS + 2) * piece(HID * (size_t)n) +
+                          3 * piece(n) + 1024;
     cudaError_t e = cudaMalloc(&net->work, floats * 4);
     if (e != cudaSuccess) return cuda_fail(net->ctx, e, "mlp work");
     net->work_bytes = floats * 4;
@@ -268,15 +417,20 @@ Views views(iso_mlp* net) {
     Views w;
     float* p = net->work;
     const size_t n = net->cap;
-    w.pts = p; p += 3 * n;
-    w.ff = p; p += FF * n;
-    for (int l = 0; l < NLAYERS; ++l) { w.z[l] = p; p += HID * n; }
-    for (int l = 0; l < NLAYERS; ++l) { w.a[l] = p; p += HID * n; }
-    w.y = p; p += n;
-    w.t = p; p += n;
-    w.dy = p; p += n;
-    w.da = p; p += HID * n;
-    w.db_scratch = p; p += HID * n;
+    auto take = [&](size_t floats) {
+        float* at = p;
+        p += piece(floats);
+        return at;
+    };
+    w.pts = take(3 * n);
+    w.ff = take(FF * n);
+    for (int l = 0; l < NLAYERS; ++l) w.z[l] = take(HID * n);
+    for (int l = 0; l < NLAYERS; ++l) w.a[l] = take(HID * n);
+    w.y = take(n);
+    w.t = take(n);
+    w.dy = take(n);
+    w.d[0] = take(HID * n);
+    w.d[1] = take(HID * n);
     w.loss = p;
     return w;
 }
@@ -287,20 +441,17 @@ inline unsigned blocks(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) /
 void forward(iso_mlp* net, const Views& w, uint32_t n) {
     cudaStream_t s = net->ctx->stream;
     const float* P = net->params;
-    fourier<<<blocks((uint64_t)n * FF, 256), 256, 0, s>>>(w.pts, n, w.ff);
-    const float* in = w.ff;
-    int in_dim = FF;
+    fourier<<<blocks((uint64_t)n * (FF / 2), 256), 256, 0, s>>>(w.pts, n, w.ff);
     for (int l = 0; l < NLAYERS; ++l) {
-        const float* W = P + weight_offset(l);
-        const float* b = P + bias_offset(l);
-        // z = in [n x in_dim] * W^T [in_dim x HID] + b
-        gemm(s, n, HID, in_dim, in, in_dim, 1, W, 1, in_dim, w.z[l], HID, b, false);
-        act_softplus<<<blocks((uint64_t)n * HID, 256), 256, 0, s>>>(w.z[l], w.a[l], (uint64_t)n * HID);
-        in = w.a[l];
-        in_dim = HID;
+        // z = in [n x in_dim] * W^T [in_dim x HID] + b, a = softplus(z)
+        const int in_dim = l ? HID : FF;
+        GemmArgs g{(int)n, HID, in_dim, l ? w.a[l - 1] : w.ff, P + weight_offset(l), in_dim, in_dim, w.z[l], HID};
+        g.bias = P + bias_offset(l);
+        g.C2 = w.a[l];
+        gemm<true, true, EPI_FORWARD>(s, net->ctx->sms, g);
     }
     out_forward<<<blocks(n, 8), 256, 0, s>>>(w.a[NLAYERS - 1], n, P + OUT_W, P + OUT_B, w.y);
-    net->ctx->launches += 2 + 2 * NLAYERS;
+    net->ctx->launches += 2 + NLAYERS;
 }
 
 // grads (zeroed first) of the loss over n points with targets w.t; *loss
@@ -310,26 +461,28 @@ void backward(iso_mlp* net, const Views& w, uint32_t n, float clampd) {
     float* G = net->grads;
     cudaMemsetAsync(G, 0, NPARAMS * 4, s);
     cudaMemsetAsync(w.loss, 0, 4, s);
-    loss_l1<<<blocks(n, 256), 256, 0, s>>>(w.y, w.t, n, clampd, w.dy, w.loss);
-    // output layer
-    gemm(s, 1, HID, n, w.dy, 1, 1, w.a[NLAYERS - 1], HID, 1, G + OUT_W, HID, nullptr, true, 64);
-    colsum<<<64, 32, 0, s>>>(w.dy, n, 1, G + OUT_B);
-    out_backward_act<<<blocks((uint64_t)n * HID, 256), 256, 0, s>>>(w.dy, P + OUT_W, n, w.da);
-    for (int l = NLAYERS - 1; l >= 0; --l) {
-        act_backward<<<blocks((uint64_t)n * HID, 256), 256, 0, s>>>(w.z[l], w.da, (uint64_t)n * HID);
-        const float* in = l ? w.a[l - 1] : w.ff;
+    loss_l1<<<blocks(n, 256), 256, 0, s>>>(w.y, w.t, n, clampd, w.dy, w.loss, G + OUT_B);
+    // dz of the last layer and the output layer's gradients
+    const int last = NLAYERS - 1;
+    float *dz = w.d[0], *below = w.d[1];
+    out_backward<<<std::min<unsigned>(blocks(n, 16), 4 * (unsigned)net->ctx->sms), HID, 0, s>>>(
+        w.dy, P + OUT_W, w.z[last], w.a[last], n, dz, G + OUT_W, G + bias_offset(last));
+    for (int l = last; l >= 0; --l) {
         const int in_dim = l ? HID : FF;
         // dW = dz^T [HID x n] * in [n x in_dim]
-        gemm(s, HID, in_dim, n, w.da, 1, HID, in, in_dim, 1, G + weight_offset(l), in_dim, nullptr, true, 64);
-        colsum<<<64, HID, 0, s>>>(w.da, n, HID, G + bias_offset(l));
+        gemm<false, false, EPI_WEIGHTS>(s, net->ctx->sms,
+                                        GemmArgs{HID, in_dim, (int)n, dz, l ? w.a[l - 1] : w.ff, HID, in_dim,
+                                                 G + weight_offset(l), in_dim});
         if (l > 0) {
-            // d in = dz [n x HID] * W [HID x in_dim]
-            gemm(s, n, in_dim, HID, w.da, HID, 1, P + weight_offset(l), in_dim, 1, w.db_scratch, in_dim, nullptr,
-                 false);
-            cudaMemcpyAsync(w.da, w.db_scratch, (size_t)n * in_dim * 4, cudaMemcpyDeviceToDevice, s);
+            // dz of the layer below = (dz [n x HID] * W [HID x HID]) sigmoid(z), and its bias' gradient
+            GemmArgs g{(int)n, HID, HID, dz, P + weight_offset(l), HID, HID, below, HID};
+            g.Z = w.z[l - 1];
+            g.colsum = G + bias_offset(l - 1);
+            gemm<true, false, EPI_BACKWARD>(s, net->ctx->sms, g);
+            std::swap(dz, below);
         }
     }
-    net->ctx->launches += 4 + 5 * NLAYERS;
+    net->ctx->launches += 2 + 2 * NLAYERS - 1;
 }
 
 }  // namespace
