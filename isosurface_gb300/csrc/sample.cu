@@ -327,20 +327,42 @@ __global__ void __launch_bounds__(256) sample_sphere_set(SetArgs A) {
     sample_column(A, s_keep, s_keep + A.n, nk, px, py, x, y, z0, z1, valid, lane, blockIdx.x);
 }
 
-// Sign bits of a caller-supplied field (one warp per 32-point chunk of a row).
-__global__ void __launch_bounds__(256) sign_bits(const float* field, uint32_t nx, uint32_t ny, uint32_t nz,
-                                                 uint64_t pitch, uint32_t* bits, uint32_t W) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t gw = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (gw >= (uint64_t)W * ny * nz) return;
-    const uint32_t w = (uint32_t)(gw % W);
-    const uint64_t row = gw / W;
-    const uint32_t x = 32 * w + lane;
-    bool inside = false;
-    if (x < nx) inside = !(__ldg(field + row * pitch + x) > 0.0f);
-    uint32_t b = __ballot_sync(FULL, inside);
-    if (lane == 0) bits[row * W + w] = b;
+// Sign bits of a caller-supplied field: a warp takes SIGN_WORDS consecutive
+// words of the packed rows, 32 samples each (any pitch: 4-byte loads, one
+// whole line per word), all loaded before the first is used, so that enough
+// bytes are in flight to run at the memory's rate; lane j stores word j.
+// 401 x 401 x 301 (194 MB): 0.058 ms (3.3 TB/s), against 0.156 ms with one
+// word per warp.
+constexpr int SIGN_WORDS = 16;
+
+__global__ void __launch_bounds__(256) sign_bits(const float* __restrict__ field, uint32_t nx, uint64_t words,
+                                                 uint64_t pitch, uint32_t* __restrict__ bits, uint32_t W) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t first = ((uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * SIGN_WORDS;
+    if (first >= words) return;
+    uint64_t row = first / W;
+    uint32_t w = (uint32_t)(first - row * W);
+    const float* at = field + row * pitch;
+    float v[SIGN_WORDS];
+#pragma unroll
+    for (int j = 0; j < SIGN_WORDS; ++j) {
+        const uint32_t x = 32 * w + lane;
+        v[j] = first + j < words && x < nx ? __ldg(at + x) : 1.0f;  // outside past the row's end
+        if (++w == W) {
+            w = 0;
+            at += pitch;
+        }
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < SIGN_WORDS; ++j) {
+        const uint32_t b = __ballot_sync(FULL, !(v[j] > 0.0f));
+        if (lane == j) mine = b;
+    }
+    if (lane < SIGN_WORDS && first + lane < words) bits[first + lane] = mine;
 }
+
+inline unsigned sign_blocks(uint64_t words) { return (unsigned)((words + 8 * SIGN_WORDS - 1) / (8 * SIGN_WORDS)); }
 
 __global__ void sample_points(ProgView pv, const float* pts, uint64_t n, float* vals, float* normals) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -696,9 +718,9 @@ iso_status launch_sample_grid(iso_ctx* ctx, const iso_program* prog, uint32_t nx
 iso_status launch_sign_bits(iso_ctx* ctx, const float* field, uint32_t nx, uint32_t ny, uint32_t nz, uint64_t pitch,
                             uint32_t* bits) {
     const uint32_t W = words_per_row(nx);
-    uint64_t warps = (uint64_t)W * ny * nz;
+    const uint64_t words = (uint64_t)W * ny * nz;
     StageTimer timer(ctx, ISO_STAGE_SIGNS);
-    sign_bits<<<(unsigned)((warps + 7) / 8), 256, 0, ctx->stream>>>(field, nx, ny, nz, pitch, bits, W);
+    sign_bits<<<sign_blocks(words), 256, 0, ctx->stream>>>(field, nx, words, pitch, bits, W);
     ctx->launches++;
     return check_launch(ctx, "sign_bits");
 }
@@ -706,8 +728,8 @@ iso_status launch_sign_bits(iso_ctx* ctx, const float* field, uint32_t nx, uint3
 cudaError_t launch_sign_bits_on(cudaStream_t stream, const float* field, uint32_t nx, uint32_t ny, uint32_t nz,
                                 uint64_t pitch, uint32_t* bits) {
     const uint32_t W = words_per_row(nx);
-    uint64_t warps = (uint64_t)W * ny * nz;
-    sign_bits<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(field, nx, ny, nz, pitch, bits, W);
+    const uint64_t words = (uint64_t)W * ny * nz;
+    sign_bits<<<sign_blocks(words), 256, 0, stream>>>(field, nx, words, pitch, bits, W);
     return cudaGetLastError();
 }
 
