@@ -112,7 +112,8 @@ class ClockSampler:
 # counts only for the sources it was taken from
 # every source of the translation units that hold the extraction's kernels
 TRAFFIC_SOURCES = ["isosurface_gb300/csrc/" + f for f in
-                   ("mc.cu", "mc_chunk.cuh", "mc_tables.h", "sample.cu", "bricks.cuh", "bricks_core.cuh", "vm.cuh",
+                   ("mc.cu", "mc_chunk.cuh", "mc_cells.cuh", "mc_tables.h", "sample.cu", "smooth_set.cuh", "bricks.cuh",
+                    "bricks_core.cuh", "vm.cuh",
                     "vm_math.cuh", "internal.h")] + ["include/isosurface_gpu.h"]
 
 
@@ -752,7 +753,7 @@ def main():
     peak, peak_kind = peaks()
     achieved = algo / (extract_ms / 1e3) / 1e9
     traffic, traffic_note = measured_traffic()
-    roofline = {"bound": "hbm", "kernel": "extraction (mc_chunk_count, mc_range_scan, mc_cell_emit, mc_resolve_ids)",
+    roofline = {"bound": "hbm", "kernel": "extraction (mc_cell_count, mc_cell_scan, mc_cell_emit, mc_resolve_ids)",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": traffic, "traffic_source": traffic_note, "algorithmic_bytes": algo,
                 "ms_per_launch": extract_ms,

@@ -39,7 +39,7 @@ UNITS = {
     "emc.cu": ["-fmad=false"],
     "jit.cu": ["-fmad=false"],
 }
-HEADERS = ["internal.h", "vm.cuh", "vm_math.cuh", "bricks.cuh", "bricks_core.cuh", "smooth_set.cuh", "mc_tables.h", "mc_chunk.cuh",
+HEADERS = ["internal.h", "vm.cuh", "vm_math.cuh", "bricks.cuh", "bricks_core.cuh", "smooth_set.cuh", "mc_tables.h", "mc_chunk.cuh", "mc_cells.cuh",
            "qef.cuh", "qef_planes.cuh", "dc_core.cuh", "mlp.h", "emc.cuh", "emc_tables.h"]
 # sources the library compiles again at run time, for one program at a time
 # (jit.cu): embedded as string literals in _build/jit_sources.inc

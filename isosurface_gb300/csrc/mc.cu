@@ -14,15 +14,16 @@
 //   cell's triangles -- checked when the tables are generated), so each cell
 //   knows which of its crossing edges it "owns": interior cells own the three
 //   edges at their far corner; cells on the x=0 / y=0 / z=0 faces own more.
-// * Extractions with a context use the chunk passes of mc_chunk.cuh (a chunk
-//   is 32 cells of a row): mc_chunk_count classifies every cell from packed
-//   sign bits and counts triangles and owned vertices per 32-chunk segment
-//   (or per chunk for the block emit), mc_range_scan turns the totals into
-//   offsets, and mc_cell_emit writes the vertices, records each owned
-//   vertex's id in a dense per-edge map and writes the triangles as map keys,
-//   which mc_resolve_ids turns into vertex ids.  Dual lattices, chunk batches
-//   and grids whose edge count exceeds 32 bits use mc_block_emit instead,
-//   which finds each owner's id from per-chunk prefixes in shared memory.
+// * Extractions with a context use the cell passes of mc_cells.cuh:
+//   mc_cell_count classifies every cell from packed sign bits and counts
+//   triangles and owned vertices per segment (32 chunks; a chunk is 32 cells
+//   of a row), mc_cell_scan turns the counts into offsets and lists the
+//   segments with active cells, and mc_cell_emit writes those segments'
+//   vertices, records each owned vertex's id in a dense per-edge map and
+//   writes the triangles as map keys, which mc_resolve_ids turns into vertex
+//   ids.  Chunk batches and grids whose edge count exceeds 32 bits use the
+//   passes of mc_chunk.cuh, whose mc_block_emit finds each owner's id from
+//   per-chunk prefixes in shared memory.
 // * The allocation-free entry point (iso_mc_extract_field_noalloc) keeps the
 //   row passes below: mc_count_scan classifies every cell and scans, per
 //   x-row of cells, the triangle count and the owned-vertex count with a
@@ -43,6 +44,7 @@
 #include <cstring>
 
 #include "internal.h"
+#include "vm_math.cuh"
 #define ISO_TABLE static __device__ const
 #include "mc_tables.h"
 
@@ -538,6 +540,7 @@ __device__ __forceinline__ uint32_t owned_count(const Corners& q, uint32_t sel, 
 }
 
 #include "mc_chunk.cuh"
+#include "mc_cells.cuh"
 
 __global__ void mc_cases_kernel(const uint32_t* bits, uint32_t W, uint32_t nx, uint32_t ny, uint32_t nz,
                                 uint8_t* out) {
@@ -637,75 +640,96 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     const uint32_t CW = (ncx + 31) / 32;
     const uint64_t chunks = (uint64_t)CW * (L.ny - 1) * (L.nz - 1);
     if (chunks >= 0xFFFFFFF0ull) return fail(ctx, ISO_ERR_TOO_LARGE, "grid too large");
+    const bool keys = (flags & ISO_FLAG_KEYS) != 0;
+    // the cell passes with the dense edge -> vertex map (4 B per lattice edge)
+    // when the edge indices fit 32 bits; otherwise the block emit resolves
+    // owners itself
+    const uint64_t nedges = 3ull * L.nx * L.ny * L.nz;
+    const bool cells = nedges < (1ull << 32);
+    const Grid grid = make_grid(L, 0);
     const uint32_t nranges = (uint32_t)((chunks + RANGE - 1) / RANGE);
+    const uint64_t nsegs = (uint64_t)grid.SL * (L.nz - 1);
+    const uint32_t nblocks = (uint32_t)((nsegs + SCAN_BLOCK_SEGS - 1) / SCAN_BLOCK_SEGS);
     const size_t smem = block_emit_smem(CW);
     if (smem > 220 * 1024) return fail(ctx, ISO_ERR_INVALID_ARG, "rows too long for the emit pass");
     iso_status s;
-    // per-chunk prefixes (block emit) or per-segment records (cell emit)
-    if ((s = ensure(ctx, ctx->rowtri, 8 * (chunks + 1))) != ISO_OK) return s;
-    const uint32_t nblocks = (nranges + 7) / 8;  // counting blocks of 8 ranges
-    if ((s = ensure(ctx, ctx->scan, 16 * (size_t)nranges + 64 + sizeof(Grid) + 256 + 16 * ((size_t)nblocks + 1) + 256)) !=
-        ISO_OK)
-        return s;
-    const bool keys = (flags & ISO_FLAG_KEYS) != 0;
+    // list entries per emitting warp: several pool their cells into full
+    // rounds of 32, while that leaves about four waves of warps (a warp's
+    // chain of loads takes a few us whatever its cells)
+    const uint32_t group = (uint32_t)std::min<uint64_t>(
+        4, std::max<uint64_t>(1, nsegs / (128 * (uint64_t)std::max(ctx->sms, 1))));
+    // cell passes: per segment its counts, active chunks and list entry (and
+    // the padding of each scan block's part); block emit: per-chunk prefixes
+    const size_t masks_at = (8 * (size_t)nsegs + 255) & ~(size_t)255;
+    const size_t list_at = (masks_at + 4 * (size_t)nsegs + 255) & ~(size_t)255;
+    const size_t seg_bytes = list_at + 16 * ((size_t)nsegs + group * (size_t)nblocks);
+    if ((s = ensure(ctx, ctx->rowtri, cells ? seg_bytes : 8 * (chunks + 1))) != ISO_OK) return s;
+    const size_t scan_bytes = cells ? 8 * (size_t)nblocks : 16 * (size_t)nranges + 64 + sizeof(Grid) + 256;
+    if ((s = ensure(ctx, ctx->scan, scan_bytes + 256)) != ISO_OK) return s;
     // a first extraction starts from a modest guess; later ones reuse what grew
     if ((s = ensure(ctx, ctx->mesh_v, 12 * (size_t)65536)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->mesh_i, 12 * (size_t)131072)) != ISO_OK) return s;
     if (keys && (s = ensure(ctx, ctx->mesh_k, 16 * (size_t)65536)) != ISO_OK) return s;
-    // the dense edge -> vertex map (4 B per lattice edge) when the edge
-    // indices fit 32 bits; otherwise the block emit resolves owners itself
-    const uint64_t nedges = 3ull * L.nx * L.ny * L.nz;
-    const bool edge_map = nedges < (1ull << 32) && L.positions == nullptr;
-    if (edge_map && (s = ensure(ctx, ctx->edges, 4 * nedges)) != ISO_OK) return s;
-    uint2* local = (uint2*)ctx->rowtri.p;
-    uint2* rangeagg = (uint2*)ctx->scan.p;
-    uint2* rangepre = rangeagg + nranges;
-    uint64_t* totals = (uint64_t*)(rangepre + nranges + 2);
-    Grid* d_grid = (Grid*)(((uintptr_t)(totals + 4) + 255) & ~(uintptr_t)255);
-    uint2* blockagg = (uint2*)(((uintptr_t)(d_grid + 1) + 255) & ~(uintptr_t)255);  // segment mode
-    uint2* blockpre = blockagg + nblocks;
-    cudaError_t e = emit_smem_attribute(smem);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "emit smem attribute");
+    if (cells && (s = ensure(ctx, ctx->edges, 4 * nedges)) != ISO_OK) return s;
+    uint64_t* totals = (uint64_t*)ctx->scan.p;  // then, 64 bytes on, the control words, then the scan's arrays
+    uint32_t* ctrl = (uint32_t*)(totals + 8);
+    char* arrays = (char*)ctx->scan.p + 128;
     // only the cell emit delivers to host buffers
-    ctx->host_out.armed = edge_map && ctx->host_out.v && ctx->host_out.i;
-    // the cell emit reads one record per 32-chunk segment; the block emit
-    // needs every chunk's prefix
-    const uint32_t nsegs = (uint32_t)((chunks + 31) / 32);
-    uint4* segs = edge_map ? (uint4*)ctx->rowtri.p : nullptr;
-    write_grid<<<1, 1, 0, ctx->stream>>>(d_grid, make_grid(L, 0));
-    {
+    ctx->host_out.armed = cells && ctx->host_out.v && ctx->host_out.i;
+    cudaError_t e = cudaSuccess;
+    CellArgs ca{};
+    uint2 *local = (uint2*)ctx->rowtri.p, *rangeagg = (uint2*)arrays, *rangepre = rangeagg + nranges;
+    Grid* d_grid = nullptr;
+    if (cells) {
+        ca.grid = grid;
+        ca.nsegs = (uint32_t)nsegs;
+        // layers per counting warp: long runs share the sign words between
+        // layers; short ones keep the warps many (a step is one round trip to
+        // memory) and their ends even
+        ca.run = (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, nsegs / (160 * (uint64_t)std::max(ctx->sms, 1))));
+        ca.ntasks = grid.SL * ((L.nz - 1 + ca.run - 1) / ca.run);
+        ca.segs = (uint2*)ctx->rowtri.p;
+        ca.masks = (uint32_t*)((char*)ctx->rowtri.p + masks_at);
+        ca.list = (uint4*)((char*)ctx->rowtri.p + list_at);
+        ca.blocks = (uint2*)arrays;
+        ca.nblocks = nblocks;
+        ca.group = group;
+        ca.ctrl = ctrl;
+        ca.totals = totals;
+        ca.err = ctx->d_err;
+        // chained with programmatic dependent launch: each kernel's blocks
+        // are resident when its predecessor finishes, and wait for it on the device
         StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
-        ChunkCountArgs ca{d_grid, nullptr, (uint32_t)chunks, edge_map ? nullptr : local, rangeagg, segs, blockagg};
-        if (edge_map) {
-            // range prefixes inside blocks of 8 ranges; one scan over the block totals
-            // chained with programmatic dependent launch: each kernel starts
-            // while its predecessor finishes and waits for it on the device
-            e = launch_pdl(mc_chunk_count<true>, dim3(nblocks), dim3(256), 0, ctx->stream, ca);
-            if (e == cudaSuccess)
-                e = launch_pdl(mc_range_scan, dim3(1), dim3(1024), 0, ctx->stream, (const uint2*)blockagg, nblocks,
-                               blockpre, totals, (uint2*)nullptr, (uint32_t)chunks, ctx->d_err);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "count launch");
-        } else {
-            mc_chunk_count<false><<<nblocks, 256, 0, ctx->stream>>>(ca);
-            mc_range_scan<<<1, 1024, 0, ctx->stream>>>(rangeagg, nranges, rangepre, totals, local, (uint32_t)chunks,
-                                                       ctx->d_err);
-        }
+        e = launch_pdl(mc_cell_count<false>, dim3((ca.ntasks + 7) / 8), dim3(256), 0, ctx->stream, ca);
+        if (e == cudaSuccess) e = launch_pdl(mc_cell_scan, dim3(nblocks), dim3(512), 0, ctx->stream, ca);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "count launch");
+        ctx->launches += 2;
+    } else {
+        if ((e = emit_smem_attribute(smem)) != cudaSuccess) return cuda_fail(ctx, e, "emit smem attribute");
+        d_grid = (Grid*)(((uintptr_t)(rangepre + nranges + 2) + 255) & ~(uintptr_t)255);
+        write_grid<<<1, 1, 0, ctx->stream>>>(d_grid, grid);
+        StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
+        mc_chunk_count<<<(nranges + 7) / 8, 256, 0, ctx->stream>>>(
+            ChunkCountArgs{d_grid, nullptr, (uint32_t)chunks, local, rangeagg});
+        mc_range_scan<<<1, 1024, 0, ctx->stream>>>(rangeagg, nranges, rangepre, totals, local, (uint32_t)chunks,
+                                                   ctx->d_err);
+        ctx->launches += 3;
     }
-    ctx->launches += 3;
-    if ((s = check_launch(ctx, "mc_chunk_count")) != ISO_OK) return s;
+    if ((s = check_launch(ctx, "mc count")) != ISO_OK) return s;
     auto emit = [&]() -> iso_status {
         uint64_t cap_v = ctx->mesh_v.bytes / 12, cap_t = ctx->mesh_i.bytes / 12;
         if (keys) cap_v = std::min<uint64_t>(cap_v, ctx->mesh_k.bytes / 16);
         const iso_ctx::HostOut& H = ctx->host_out;
-        ChunkEmitArgs ea{d_grid, nullptr, (uint32_t)chunks, local, edge_map ? rangeagg : rangepre,
-                         (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p, keys ? (uint64_t*)ctx->mesh_k.p : nullptr,
-                         cap_v, cap_t, ctx->d_err, (uint32_t*)ctx->edges.p, H.v, H.i, H.cap_v, H.cap_t, totals,
-                         blockpre};
+        uint64_t* out_k = keys ? (uint64_t*)ctx->mesh_k.p : nullptr;
         {
             StageTimer timer(ctx, ISO_STAGE_EMIT);
-            if (edge_map) {
-                cudaError_t le = launch_pdl(mc_cell_emit, dim3((nsegs + 8 * EMIT_SEGS - 1) / (8 * EMIT_SEGS)),
-                                            dim3(256), 0, ctx->stream, ea, (const uint4*)segs, nsegs);
+            if (cells) {
+                const CellEmitArgs ea{ca, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p, out_k, cap_v, cap_t,
+                                      (uint32_t*)ctx->edges.p, H.v, H.cap_v, H.cap_t};
+                // persistent: five blocks of 256 threads per SM, or a warp for every group the list could hold
+                const uint64_t groups = nsegs / group + nblocks;
+                const uint64_t blocks = std::min<uint64_t>((groups + 7) / 8, 5ull * (uint64_t)std::max(ctx->sms, 1));
+                cudaError_t le = launch_pdl(mc_cell_emit<false>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, ea);
                 if (le == cudaSuccess)
                     le = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream,
                                     (uint32_t*)ctx->mesh_i.p, (const uint64_t*)totals, cap_t,
@@ -713,6 +737,8 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
                 if (le != cudaSuccess) return cuda_fail(ctx, le, "emit launch");
                 ctx->launches++;
             } else {
+                const ChunkEmitArgs ea{d_grid, nullptr, (uint32_t)chunks, local, rangepre, (float*)ctx->mesh_v.p,
+                                       (uint32_t*)ctx->mesh_i.p, out_k, cap_v, cap_t, ctx->d_err};
                 mc_block_emit<<<(unsigned)((chunks + 255) / 256), 256, smem, ctx->stream>>>(ea, CW);
             }
         }
@@ -738,6 +764,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     if (err || grow) {
         // out of room (the counts are exact): again into buffers of that size
         e = cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ctrl + 1, 0, 4, ctx->stream);  // the emit's queue starts over
         if (e != cudaSuccess) return cuda_fail(ctx, e, "clear error flags");
         if ((s = ensure(ctx, ctx->mesh_v, 12 * std::max<uint64_t>(nv, 1))) != ISO_OK) return s;
         if ((s = ensure(ctx, ctx->mesh_i, 12 * std::max<uint64_t>(nt, 1))) != ISO_OK) return s;
@@ -970,10 +997,10 @@ iso_status mc_extract_grids(iso_ctx* ctx, const void* d_grids, uint32_t ngrids, 
     uint2* rangeagg = local + ((chunks + 1 + 31) & ~31u);
     uint2* rangepre = rangeagg + nranges;
     const Grid* grids = (const Grid*)d_grids;
-    ChunkCountArgs ca{grids, d_range_grid, chunks, local, rangeagg, nullptr, nullptr};
+    ChunkCountArgs ca{grids, d_range_grid, chunks, local, rangeagg};
     {
         StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
-        mc_chunk_count<false><<<(nranges + 1 + 7) / 8, 256, 0, ctx->stream>>>(ca);
+        mc_chunk_count<<<(nranges + 1 + 7) / 8, 256, 0, ctx->stream>>>(ca);
         mc_range_scan<<<1, 1024, 0, ctx->stream>>>(rangeagg, nranges, rangepre, totals, local, chunks, ctx->d_err);
     }
     ctx->launches += 2;
@@ -994,9 +1021,7 @@ iso_status mc_extract_grids(iso_ctx* ctx, const void* d_grids, uint32_t ngrids, 
     const size_t smem = block_emit_smem(max_cw);
     cudaError_t e = emit_smem_attribute(smem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "emit smem attribute");
-    // the block emit: no edge map, no delivery to host buffers, no block prefixes
-    ChunkEmitArgs ea{grids,   d_range_grid, chunks,  local, rangepre, out_v,   out_i,  nullptr, cap_v,
-                     cap_t,   ctx->d_err,   nullptr, nullptr, nullptr, 0,       0,      totals,  nullptr};
+    ChunkEmitArgs ea{grids, d_range_grid, chunks, local, rangepre, out_v, out_i, nullptr, cap_v, cap_t, ctx->d_err};
     {
         StageTimer timer(ctx, ISO_STAGE_EMIT);
         mc_block_emit<<<nranges, 256, smem, ctx->stream>>>(ea, max_cw);

@@ -1,4 +1,7 @@
-// Chunked marching-cubes passes (included by mc.cu inside iso::{anonymous}).
+// Chunked marching-cubes passes (included by mc.cu inside iso::{anonymous}):
+// the lattice record that every pass takes, the passes of the block emit
+// (lattices and batches whose edge maps do not fit a 32-bit key space; the
+// others take the cell passes of mc_cells.cuh) and mc_resolve_ids.
 //
 // A chunk is 32 consecutive cells of a row (x = 32c .. 32c+31); inside a
 // grid, chunk id = row * CW + c with CW = ceil((nx-1)/32), which is the
@@ -7,18 +10,13 @@
 // funnel shifts, so activity and owned-vertex counts cost a few dozen bit
 // operations per 32 cells.
 //
-// Offsets come in two forms.  Chunk mode (the block emit): pass 1 gives every
-// chunk its exclusive prefix inside its range of 256 chunks plus each range's
-// total; a one-block scan turns range totals into range offsets; chunk base =
-// range offset + in-range prefix.  Several grids can be processed by one
-// launch in this mode: each grid's chunks occupy a run of whole ranges of a
-// global chunk index space, range_grid maps a range to its grid (a null map
-// means one grid), and vertex indices are written relative to the grid's
-// first vertex, so each grid gets its own mesh.  Segment mode (the cell emit,
-// one grid): pass 1 writes one record per 32-chunk segment (prefix inside
-// its range, own counts), each range's prefix inside its block of 8 ranges
-// and each block's totals; the one-block scan runs over the block totals;
-// segment base = block offset + in-block range prefix + in-range prefix.
+// Offsets: pass 1 gives every chunk its exclusive prefix inside its range of
+// 256 chunks plus each range's total; a one-block scan turns range totals
+// into range offsets; chunk base = range offset + in-range prefix.  Several
+// grids can be processed by one launch: each grid's chunks occupy a run of
+// whole ranges of a global chunk index space, range_grid maps a range to its
+// grid (a null map means one grid), and vertex indices are written relative
+// to the grid's first vertex, so each grid gets its own mesh.
 // Corners, load_corners, case_at, chunk_valid, active_cells and owned_count
 // are defined in mc.cu above the include.
 
@@ -48,9 +46,13 @@ struct Grid {
     uint32_t zoff;     // lattice z of layer 0 (a slab of a larger grid): positions and keys use z + zoff
     uint32_t chunk0;   // first global chunk id (a multiple of RANGE)
     uint32_t nchunks;  // CW * (ny-1) * (nz-1)
+    // the cell passes: chunks per cell layer, segments of 32 chunks per layer,
+    // first global segment, first key of its edges in the edge map
+    uint32_t S, SL, seg0, edge0;
+    FastDiv div_sl;
 };
 
-inline Grid make_grid(const Lattice& L, uint32_t chunk0) {
+inline Grid make_grid(const Lattice& L, uint32_t chunk0, uint32_t seg0 = 0, uint32_t edge0 = 0) {
     Grid g;
     g.bits = L.bits;
     g.values = L.values;
@@ -67,6 +69,11 @@ inline Grid make_grid(const Lattice& L, uint32_t chunk0) {
     g.zoff = L.zoff;
     g.chunk0 = chunk0;
     g.nchunks = g.CW * (L.ny - 1) * (L.nz - 1);
+    g.S = g.CW * (L.ny - 1);
+    g.SL = (g.S + 31) / 32;
+    g.seg0 = seg0;
+    g.edge0 = edge0;
+    g.div_sl = make_fastdiv(g.SL);
     return g;
 }
 
@@ -78,64 +85,28 @@ struct ChunkCountArgs {
     const Grid* grids;
     const uint32_t* range_grid;
     uint32_t chunks;   // global (padded) chunk count
-    uint2* local;      // chunk mode: chunks + 1 (vertex, triangle) exclusive prefixes inside the range
+    uint2* local;      // chunks + 1 (vertex, triangle) exclusive prefixes inside the range
     uint2* rangeagg;   // per range: (vertices, triangles)
-    uint4* segs;       // segment mode: per 32 chunks (first vertex, first triangle) inside the range,
-                       // (vertices, triangles); rangeagg then holds each range's prefix inside
-                       // its block of 8 ranges and blockagg each block's totals
-    uint2* blockagg;
 };
 
-// Segments of 32 chunks per warp in mc_cell_emit: a segment (two cell rows at
-// 513^3) holds a dozen or two active cells, so a warp takes several and hands
-// out their active cells together.
-constexpr int EMIT_SEGS = 2;
-constexpr int EMIT_CH = 32 * EMIT_SEGS;  // chunks per warp
-
-// N chunks of a warp in shared memory: corner words (padded to 9 words, so
-// that lanes reading different chunks hit different banks), active-cell masks
-// and the exclusive prefix of their counts in chunk order.
-template <int N>
-struct ChunkStage {
-    uint32_t q[N][9];
-    uint32_t act[N];
-    uint32_t excl[N];
-    // the chunk holding active cell number kk (kk < the chunks' total): the
-    // last one whose prefix is <= kk
-    __device__ __forceinline__ uint32_t find(uint32_t kk) const {
-        uint32_t j = 0;
-#pragma unroll
-        for (uint32_t step = N / 2; step > 0; step >>= 1)
-            if (excl[j + step] <= kk) j += step;
-        return j;
-    }
-};
-using EmitChunks = ChunkStage<EMIT_CH>;
-
-// Pass 1: per-chunk (SEG = false) or per-segment (32 chunks, SEG = true)
-// counts and in-range prefixes.  One warp per range of 256 chunks, 32 per
+// Pass 1: per-chunk counts and in-range prefixes.  One warp per range of 256 chunks, 32 per
 // round (no barrier); the next round's corner words are loaded while this
 // round is counted, so the loads' latency overlaps the counting.
 #ifndef ISO_COUNT_BLOCKS
 #define ISO_COUNT_BLOCKS 4  // resident blocks per SM the register budget is sized for (64 registers)
 #endif
-template <bool SEG>
 __global__ void __launch_bounds__(256, ISO_COUNT_BLOCKS) mc_chunk_count(ChunkCountArgs A) {
     __shared__ uint8_t s_ntri[256];
     __shared__ uint16_t s_owned[8];
-    __shared__ uint32_t s_tri[8][32];  // chunk mode, per warp: triangles of each of the round's chunks
-    __shared__ ChunkStage<SEG ? 64 : 2> s_pair[8];  // segment mode, per warp: two rounds of chunks
+    __shared__ uint32_t s_tri[8][32];  // per warp: triangles of each of the round's chunks
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_wait();     // the grid record and the sign bits
-    pdl_trigger();
     s_ntri[threadIdx.x] = iso_tri_count[threadIdx.x];
     if (threadIdx.x < 8) s_owned[threadIdx.x] = iso_owned_mask[threadIdx.x];
     __syncthreads();
     const uint32_t range = blockIdx.x * 8 + (threadIdx.x >> 5);
-    const bool live = range * RANGE <= A.chunks;  // warp-uniform
-    if (!SEG && !live) return;
+    if (range * RANGE > A.chunks) return;  // warp-uniform
     uint32_t agg_t = 0, agg_v = 0;
-    if (live) {
+    {
         const Grid g = A.grids[grid_of_range(A.range_grid, min(range, A.chunks / RANGE - (A.chunks % RANGE == 0)))];
         const uint32_t ncx = g.nx - 1;
         // corner words of chunk ch (zeros outside the grid)
@@ -158,7 +129,6 @@ __global__ void __launch_bounds__(256, ISO_COUNT_BLOCKS) mc_chunk_count(ChunkCou
         };
         uint32_t ny_, nz_, nc_;
         bool nin;
-        uint32_t pair_total = 0, vr_first = 0;  // segment mode
         Corners qn = fetch(range * RANGE + lane, ny_, nz_, nc_, nin);
         for (int r = 0; r < RANGE_ROUNDS; ++r) {
             const uint32_t ch = range * RANGE + r * 32 + lane;
@@ -178,61 +148,6 @@ __global__ void __launch_bounds__(256, ISO_COUNT_BLOCKS) mc_chunk_count(ChunkCou
                     const int cls = (y == 0 ? 2 : 0) | (z == 0 ? 4 : 0);
                     v = owned_count(q, act, s_owned[cls], s_owned[cls | 1], c == 0 ? 1u : 0u);
                 }
-            }
-            if constexpr (SEG) {
-                // two rounds (two segments) at a time: the chunks go to shared
-                // memory, and the pair's active cells are handed out one per
-                // lane in chunk order, their triangles summed per segment
-                const uint32_t h = r & 1;
-                ChunkStage<64>& P = s_pair[warp];
-                uint32_t vr = 0;
-                if (__any_sync(FULL, act != 0)) {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) P.q[32 * h + lane][k] = q.k[k];
-                    P.act[32 * h + lane] = act;
-                    const uint32_t n = __popc(act);
-                    const uint32_t incl = warp_incl_scan(n, lane);
-                    P.excl[32 * h + lane] = pair_total + incl - n;
-                    pair_total += __shfl_sync(FULL, incl, 31);
-                    vr = __reduce_add_sync(FULL, v);
-                } else {
-                    // no active cell in the round (most rounds): no corners to
-                    // stage, no counts to scan (v is 0 without active cells);
-                    // the chunk lookup never lands on a chunk without any
-                    P.act[32 * h + lane] = 0;
-                    P.excl[32 * h + lane] = pair_total;
-                }
-                if (h == 0) {
-                    vr_first = vr;
-                    continue;
-                }
-                __syncwarp();
-                uint32_t t0 = 0, t1 = 0;
-                for (uint32_t b0 = 0; b0 < pair_total; b0 += 32) {
-                    const uint32_t kk = b0 + lane;
-                    if (kk < pair_total) {
-                        const uint32_t j = P.find(kk);
-                        Corners cq;
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) cq.k[k] = P.q[j][k];
-                        const uint32_t t = s_ntri[case_at(cq, __fns(P.act[j], 0, (int)(kk - P.excl[j]) + 1))];
-                        if (j < 32)
-                            t0 += t;
-                        else
-                            t1 += t;
-                    }
-                }
-                const uint32_t tr0 = __reduce_add_sync(FULL, t0), tr1 = __reduce_add_sync(FULL, t1);
-                const uint32_t first = ch - lane - 32;  // the pair's first chunk
-                if (lane == 0 && first < A.chunks) A.segs[first / 32] = make_uint4(agg_v, agg_t, vr_first, tr0);
-                agg_v += vr_first;
-                agg_t += tr0;
-                if (lane == 0 && first + 32 < A.chunks) A.segs[first / 32 + 1] = make_uint4(agg_v, agg_t, vr, tr1);
-                agg_v += vr;
-                agg_t += tr1;
-                pair_total = 0;
-                __syncwarp();  // the pair's chunks are read before the next pair overwrites them
-                continue;
             }
             // triangles: the round's active cells one per lane (in chunk order),
             // their counts summed back per chunk in shared memory
@@ -268,31 +183,13 @@ __global__ void __launch_bounds__(256, ISO_COUNT_BLOCKS) mc_chunk_count(ChunkCou
             agg_v += __shfl_sync(FULL, vi, 31);
         }
     }
-    if (!SEG) {
-        if (lane == 0 && range * RANGE < A.chunks) A.rangeagg[range] = make_uint2(agg_v, agg_t);
-        return;
-    }
-    // segment mode: each range's exclusive prefix inside the block's eight
-    // ranges, and the block's totals (scanned across blocks by mc_range_scan)
-    __shared__ uint2 s_agg[8];
-    if (lane == 0) s_agg[warp] = range * RANGE < A.chunks ? make_uint2(agg_v, agg_t) : make_uint2(0, 0);
-    __syncthreads();
-    if (threadIdx.x < 8) {  // thread w: range blockIdx.x * 8 + w
-        const uint32_t r = blockIdx.x * 8 + threadIdx.x;
-        uint2 pre = make_uint2(0, 0);
-        for (uint32_t w = 0; w < threadIdx.x; ++w) {
-            pre.x += s_agg[w].x;
-            pre.y += s_agg[w].y;
-        }
-        if (r * RANGE < A.chunks) A.rangeagg[r] = pre;
-        if (threadIdx.x == 7) A.blockagg[blockIdx.x] = make_uint2(pre.x + s_agg[7].x, pre.y + s_agg[7].y);
-    }
+    if (lane == 0 && range * RANGE < A.chunks) A.rangeagg[range] = make_uint2(agg_v, agg_t);
 }
 
 // Exclusive scan of the range totals (one block).  Each thread holds
 // SCAN_ITEMS consecutive ranges per pass (all loaded before any is used), so
 // 8K ranges take one pass of one block scan.  rangepre[nr] and totals
-// receive the grand totals; local[chunks] (chunk mode) is cleared when
+// receive the grand totals; local[chunks] is cleared when
 // `chunks` starts a range that no warp counted.
 constexpr int SCAN_ITEMS = 8;
 
@@ -300,8 +197,6 @@ __global__ void __launch_bounds__(1024) mc_range_scan(const uint2* rangeagg, uin
                                                       uint64_t* totals, uint2* local, uint32_t chunks, uint32_t* err) {
     __shared__ uint64_t s_wv[32], s_wt[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_wait();     // the counting pass's totals
-    pdl_trigger();
     uint64_t carry_t = 0, carry_v = 0;
     for (uint32_t base = 0; base < nr; base += 1024 * SCAN_ITEMS) {
         const uint32_t i0 = base + threadIdx.x * SCAN_ITEMS;
@@ -358,7 +253,7 @@ __global__ void __launch_bounds__(1024) mc_range_scan(const uint2* rangeagg, uin
         totals[0] = carry_t;
         totals[1] = carry_v;
         rangepre[nr] = make_uint2((uint32_t)carry_v, (uint32_t)carry_t);
-        if (local && chunks % RANGE == 0) local[chunks] = make_uint2(0, 0);
+        if (chunks % RANGE == 0) local[chunks] = make_uint2(0, 0);
     }
 }
 
@@ -373,17 +268,6 @@ struct ChunkEmitArgs {
     uint64_t* out_k;
     uint64_t cap_v, cap_t;
     uint32_t* err;
-    uint32_t* edge_id;  // mc_cell_emit: vertex id per lattice edge, keyed by (upper end point * 3 + axis)
-    // mc_cell_emit / mc_resolve_ids: page-locked host buffers (device-side
-    // pointers, null: none) that also receive the mesh when all of it fits
-    // both them and the device buffers (`totals` = triangles, vertices)
-    float* host_v;
-    uint32_t* host_i;
-    uint64_t host_cap_v, host_cap_t;
-    const uint64_t* totals;
-    // mc_cell_emit: rangepre holds each range's prefix inside its block of 8
-    // ranges, blockpre each block's exclusive prefix
-    const uint2* blockpre;
 };
 
 // whether this launch copies the mesh to the host buffers
@@ -642,239 +526,6 @@ __global__ void __launch_bounds__(256) mc_block_emit(ChunkEmitArgs A, uint32_t m
         }
         vcarry += vtot;
         tcarry += ttot;
-    }
-}
-
-// One vertex on lattice edge (pa, pb) with values (fa, fb): the crossing
-// point (Signed::find_crossing_point, distance.rs:64-69), its optional lattice
-// edge key (lower end point * 3 + axis), and its grid-local id in the edge map
-// under ``key``.
-__device__ __forceinline__ void put_vertex(const ChunkEmitArgs& A, const Grid& g, float fa, float fb, float pax,
-                                           float pay, float paz, float pbx, float pby, float pbz, uint32_t vid,
-                                           uint32_t key, uint32_t grid_v0, uint32_t lx, uint32_t ly, uint32_t lz,
-                                           uint32_t ax) {
-    const float delta = fb - fa;
-    const float tt = (delta == 0.0f) ? 0.5f : -fa / delta;
-    const float omt = 1.0f - tt;
-    if (vid < A.cap_v) {
-        A.out_v[3 * (size_t)vid + 0] = pax * omt + pbx * tt;
-        A.out_v[3 * (size_t)vid + 1] = pay * omt + pby * tt;
-        A.out_v[3 * (size_t)vid + 2] = paz * omt + pbz * tt;
-        if (A.out_k) {
-            A.out_k[2 * (size_t)vid] = (((uint64_t)(lz + g.zoff) * g.ny + ly) * g.nx + lx) * 3 + ax;
-            A.out_k[2 * (size_t)vid + 1] = 0;
-        }
-    } else {
-        atomicOr(A.err, DERR_CAPACITY);
-    }
-    A.edge_id[key] = vid - grid_v0;
-}
-
-// Active cell number kk (in chunk order) of the warp's chunks starting at
-// grid chunk rc; every lane calls it, have = kk < total.
-struct SegCell {
-    uint32_t x, y, z, cs, nown, nt;
-    int cls;
-    bool have;
-    uint4 pk;  // interior cells: the case's packed entry (iso_case_pack)
-};
-
-__device__ __forceinline__ SegCell seg_cell(const Grid& g, uint32_t rc, uint32_t kk, uint32_t total,
-                                            const EmitChunks& S) {
-    SegCell c{0, 0, 0, 0, 0, 0, 0, kk < total, make_uint4(0, 0, 0, 0)};
-    if (!c.have) return c;
-    const uint32_t j = S.find(kk);
-    Corners cq;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) cq.k[k] = S.q[j][k];
-    const uint32_t i = __fns(S.act[j], 0, (int)(kk - S.excl[j]) + 1);
-    const uint32_t cch = rc + j;
-    const uint32_t row = fdiv(cch, g.div_cw);
-    c.z = fdiv(row, g.div_ncy);
-    c.y = row - c.z * (g.ny - 1);
-    c.x = 32 * (cch - row * g.CW) + i;
-    c.cs = case_at(cq, i);
-    c.cls = (c.x == 0 ? 1 : 0) | (c.y == 0 ? 2 : 0) | (c.z == 0 ? 4 : 0);
-    if (c.cls == 0) {
-        c.pk = __ldg(reinterpret_cast<const uint4*>(&iso_case_pack[c.cs]));
-        c.nown = __popc(c.pk.z & 0x460u);  // owned edges 5, 6, 10
-        c.nt = (c.pk.z >> 12) & 7u;
-    } else {
-        c.nown = __popc((uint32_t)__ldg(&iso_edge_mask[c.cs]) & __ldg(&iso_owned_mask[c.cls]));
-        c.nt = __ldg(&iso_tri_count[c.cs]);
-    }
-    return c;
-}
-
-// The vertices and triangles of one round of cells (every lane calls it).
-// koff (lane e < 12): the edge-map key of cell edge e relative to 3 * (corner
-// 0's lattice point).
-__device__ __forceinline__ void emit_cells(const ChunkEmitArgs& A, const Grid& g, const SegCell& c, uint32_t vstart,
-                                           uint32_t tstart, uint32_t koff, uint32_t grid_v0) {
-    uint32_t own = 0, cell = 0;
-    uint64_t tedges = 0;
-    if (c.have) {
-        cell = (c.z * g.ny + c.y) * g.nx + c.x;  // lattice point of corner 0
-        if (c.cls == 0) {
-            own = c.pk.z & 0x460u;
-            tedges = ((uint64_t)c.pk.y << 32) | c.pk.x;
-        } else {
-            own = (uint32_t)__ldg(&iso_edge_mask[c.cs]) & __ldg(&iso_owned_mask[c.cls]);
-            tedges = __ldg(&iso_tri_edges[c.cs]);
-        }
-    }
-    if (own) {
-        // owned edges: this cell creates their vertices, numbered by
-        // first use in the cell's visit order (rank table)
-        if (c.cls == 0) {
-            // interior cell: its owned edges are among 5, 6 and 10, the
-            // three edges ending at corner 6 = (x+1, y+1, z+1); all their
-            // values are loaded before any vertex is formed
-            const float* v6 = g.values + ((size_t)(c.z + 1) * g.ny + (c.y + 1)) * g.pitch + (c.x + 1);
-            const bool e5 = (own >> 5) & 1u, e6 = (own >> 6) & 1u, e10 = (own >> 10) & 1u;
-            const float f6 = __ldg(v6);
-            const float f5 = e5 ? __ldg(v6 - g.pitch) : 0.0f;                    // corner 5
-            const float f7 = e6 ? __ldg(v6 - 1) : 0.0f;                          // corner 7
-            const float f2 = e10 ? __ldg(v6 - (size_t)g.ny * g.pitch) : 0.0f;    // corner 2
-            const float X0 = (float)c.x * g.inv, X1 = (float)(c.x + 1) * g.inv;
-            const float Y0 = (float)c.y * g.inv, Y1 = (float)(c.y + 1) * g.inv;
-            const float Z0 = (float)(c.z + g.zoff) * g.inv, Z1 = (float)(c.z + 1 + g.zoff) * g.inv;
-            const uint32_t k6 = 3 * (cell + g.nx * (g.ny + 1) + 1);  // corner 6's key base
-            if (e5)  // corners 5 -> 6, y axis
-                put_vertex(A, g, f5, f6, X1, Y0, Z1, X1, Y1, Z1, vstart + (c.pk.z >> 16 & 15u), k6 + 1, grid_v0,
-                           c.x + 1, c.y, c.z + 1, 1);
-            if (e6)  // corners 6 -> 7, x axis
-                put_vertex(A, g, f6, f7, X1, Y1, Z1, X0, Y1, Z1, vstart + (c.pk.z >> 20 & 15u), k6 + 0, grid_v0,
-                           c.x, c.y + 1, c.z + 1, 0);
-            if (e10)  // corners 2 -> 6, z axis
-                put_vertex(A, g, f2, f6, X1, Y1, Z0, X1, Y1, Z1, vstart + (c.pk.z >> 24 & 15u), k6 + 2, grid_v0,
-                           c.x + 1, c.y + 1, c.z, 2);
-        } else {
-            const uint64_t rk = __ldg(&iso_owned_rank[c.cls][c.cs]);
-            for (uint32_t m = own; m; m &= m - 1) {
-                const uint32_t e = __ffs(m) - 1;
-                const uint32_t ax = __ldg(&g_edge_axis[e]);
-                const uint32_t lx = c.x + __ldg(&g_edge_lo[e][0]), ly = c.y + __ldg(&g_edge_lo[e][1]),
-                               lz = c.z + __ldg(&g_edge_lo[e][2]);
-                const uint32_t hx = lx + (ax == 0), hy = ly + (ax == 1), hz = lz + (ax == 2);
-                const uint32_t u = __ldg(&iso_edge_connection[e][0]), v = __ldg(&iso_edge_connection[e][1]);
-                const uint32_t ux = c.x + __ldg(&iso_corners[u][0]), uy = c.y + __ldg(&iso_corners[u][1]),
-                               uz = c.z + __ldg(&iso_corners[u][2]);
-                const uint32_t vx = c.x + __ldg(&iso_corners[v][0]), vy = c.y + __ldg(&iso_corners[v][1]),
-                               vz = c.z + __ldg(&iso_corners[v][2]);
-                const float fa = __ldg(g.values + ((size_t)uz * g.ny + uy) * g.pitch + ux);
-                const float fb = __ldg(g.values + ((size_t)vz * g.ny + vy) * g.pitch + vx);
-                put_vertex(A, g, fa, fb, (float)ux * g.inv, (float)uy * g.inv, (float)(uz + g.zoff) * g.inv,
-                           (float)vx * g.inv, (float)vy * g.inv, (float)(vz + g.zoff) * g.inv,
-                           vstart + (uint32_t)(rk >> (4 * e) & 15u), ((hz * g.ny + hy) * g.nx + hx) * 3 + ax,
-                           grid_v0, lx, ly, lz, ax);
-            }
-        }
-    }
-    // triangles (march_cube, marching_cubes_impl.rs:102-117) as edge-map
-    // keys, resolved to vertex ids once every owner has written its ids
-    const bool tfit = (uint64_t)tstart + c.nt <= A.cap_t;
-    if (c.have && !tfit) atomicOr(A.err, DERR_CAPACITY);
-    const uint32_t kmax = __reduce_max_sync(FULL, 3 * c.nt);
-    for (uint32_t k = 0; k < kmax; ++k) {
-        const uint32_t ko = __shfl_sync(FULL, koff, (uint32_t)(tedges >> (4 * k)) & 15u);
-        if (k < 3 * c.nt && tfit) A.out_i[3 * (size_t)tstart + k] = 3 * cell + ko;
-    }
-}
-
-// Pass 2, cell-parallel, for one lattice given by values alone (no explicit
-// sample positions) whose edge count fits 32 bits.  Warp = EMIT_SEGS
-// consecutive segments of 32 chunks, whose first vertex and triangle come
-// from pass 1's segment records.  Lane = chunk, once per segment: corner
-// words and active cells, staged in shared memory with their count prefix.
-// The chunks' active cells are then handed out 32 at a time in chunk order
-// (lane = cell: the owning chunk by a binary search over the prefix, the bit
-// by __fns), so lanes stay busy however the active cells are spread.  A
-// cell's own offsets are the warp's base plus a running warp scan of
-// owned-vertex and triangle counts in cell order (the reference's emission
-// order).  Every owned vertex records its id in a dense per-lattice-edge map,
-// and triangles are written as map keys; mc_resolve_ids then replaces each
-// key by the id its owner recorded (the map needs no initialisation: every
-// crossing edge has an owner, and only crossing edges are referenced).  Keys
-// are 3 * (upper end point) + axis, so the (at most three) edges an interior
-// cell owns, which all end at its corner 6, share one 12-byte slot.
-__global__ void __launch_bounds__(256, 5) mc_cell_emit(ChunkEmitArgs A, const uint4* segs, uint32_t nsegs) {
-    __shared__ EmitChunks s_ch[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    pdl_trigger();
-    const uint32_t seg0 = (blockIdx.x * 8 + warp) * EMIT_SEGS;  // the warp's first segment
-    if (seg0 >= nsegs) return;
-    // the staging below reads only the sign bits and the grid record, which
-    // the counting pass's predecessors wrote: it overlaps the counting pass
-    const Grid g = A.grids[0];
-    const uint32_t rc = seg0 * 32, c_end = min(rc + (uint32_t)EMIT_CH, g.nchunks);
-    EmitChunks& S = s_ch[warp];
-    // lane = chunk, EMIT_SEGS times: corner bit-vectors, active cells, prefix
-    uint32_t total = 0;
-#pragma unroll
-    for (int h = 0; h < EMIT_SEGS; ++h) {
-        const uint32_t ch = rc + 32 * h + lane;
-        Corners q;
-        uint32_t act = 0;
-        if (ch < c_end) {
-            const uint32_t row = fdiv(ch, g.div_cw);
-            const uint32_t cc = ch - row * g.CW;
-            const uint32_t z = fdiv(row, g.div_ncy);
-            q = load_corners(g.bits, g.W, g.ny, row - z * (g.ny - 1), z, cc);
-            act = active_cells(q, chunk_valid(cc, g.nx - 1));
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) q.k[k] = 0;
-        }
-        if (__any_sync(FULL, act != 0)) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) S.q[32 * h + lane][k] = q.k[k];
-            S.act[32 * h + lane] = act;
-            const uint32_t n = __popc(act);
-            const uint32_t incl = warp_incl_scan(n, lane);
-            S.excl[32 * h + lane] = total + incl - n;
-            total += __shfl_sync(FULL, incl, 31);
-        } else {
-            // no active cell in the segment: nothing to stage (the chunk
-            // lookup never lands on a chunk without active cells)
-            S.act[32 * h + lane] = 0;
-            S.excl[32 * h + lane] = total;
-        }
-    }
-    if (total == 0) return;  // no active cell: no vertex, no triangle
-    pdl_wait();              // the counts and their scan
-    // records: (first vertex, first triangle) in the range, (vertices, triangles)
-    const uint4 sr = __ldg(&segs[seg0]);
-    uint32_t nv_w = sr.z;
-#pragma unroll
-    for (int h = 1; h < EMIT_SEGS; ++h)
-        if (seg0 + h < nsegs) nv_w += __ldg(&segs[seg0 + h]).z;
-    const uint32_t range = seg0 / (RANGE / 32);  // EMIT_SEGS divides the 8 segments of a range
-    const uint2 rin = __ldg(&A.rangepre[range]), rb = __ldg(&A.blockpre[range / 8]);
-    const uint32_t vbase = rb.x + rin.x + sr.x, tbase = rb.y + rin.y + sr.y;
-    __syncwarp();
-    uint32_t koff = 0;
-    if (lane < 12) {
-        const uint32_t ax = __ldg(&g_edge_axis[lane]);
-        const uint32_t hx = __ldg(&g_edge_lo[lane][0]) + (ax == 0), hy = __ldg(&g_edge_lo[lane][1]) + (ax == 1),
-                       hz = __ldg(&g_edge_lo[lane][2]) + (ax == 2);
-        koff = 3 * (hx + g.nx * (hy + g.ny * hz)) + ax;
-    }
-    uint32_t vcarry = vbase, tcarry = tbase;  // global offsets of the next cell's outputs
-    for (uint32_t b0 = 0; b0 < total; b0 += 32) {
-        const SegCell c = seg_cell(g, rc, b0 + lane, total, S);
-        const uint32_t vi = warp_incl_scan(c.nown, lane), ti = warp_incl_scan(c.nt, lane);
-        const uint32_t vstart = vcarry + vi - c.nown, tstart = tcarry + ti - c.nt;
-        vcarry += __shfl_sync(FULL, vi, 31);
-        tcarry += __shfl_sync(FULL, ti, 31);
-        emit_cells(A, g, c, vstart, tstart, koff, 0u);
-    }
-    if (mesh_to_host(A.host_v, A.totals, A.host_cap_v, A.host_cap_t, A.cap_v, A.cap_t)) {
-        // the segments' vertices, just written by this warp, in whole lines
-        // to the host (the warp's own stores are ordered before its reads)
-        __syncwarp();
-        const size_t f0 = 3 * (size_t)vbase, f1 = f0 + 3 * (size_t)nv_w;
-        for (size_t f = f0 + lane; f < f1; f += 32) A.host_v[f] = __ldcg(A.out_v + f);
     }
 }
 

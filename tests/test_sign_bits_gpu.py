@@ -13,7 +13,7 @@ from isosurface_gb300.surrogate import case_disagreement
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,nz,pad", [(2, 2, 0), (31, 3, 0), (32, 5, 1), (33, 4, 0), (65, 9, 3), (257, 3, 2)])
+@pytest.mark.parametrize("nx,nz,pad", [(2, 2, 0), (31, 3, 0), (32, 5, 1), (33, 4, 0), (65, 9, 3), (257, 3, 2), (545, 2, 1), (1000, 2, 0)])
 def test_every_sign_is_read(ctx, nx, nz, pad):
     import torch
     r = np.random.default_rng(nx)
