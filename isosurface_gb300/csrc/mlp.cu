@@ -63,7 +63,7 @@ __host__ __device__ __forceinline__ float freq(int j) { return 3.14159265358979f
 // N, lda and ldb are multiples of 4, the pointers are 16-byte
 // aligned.
 //   EPI_FORWARD   C = acc + bias[j] and C2 = softplus(C)
-//   EPI_BACKWARD  C = acc * sigmoid(Z[i][j]), and colsum[j] += its column sums
+//   EPI_BACKWARD  C = acc * sigmoid(Z[i][j]), and colsum[tile row][j] = the tile's column sums
 //   EPI_WEIGHTS   C += acc by atomics, K split over gridDim.z
 // 65536 x 256 x 256 (8.6 GFLOP) on the GB300, whose FMA pipe reaches 77
 // TFLOP/s: 0.17 ms as the weights' product (50 TFLOP/s, bound by the packed
@@ -232,25 +232,29 @@ __global__ void __launch_bounds__(256, 2) gemm_f32(GemmArgs G) {
         for (int j = threadIdx.x; j < BN && j0 + j < G.N; j += 256) {
             float sum = 0.0f;
             for (int r = 0; r < 16; ++r) sum += s_col[r][j];
-            atomicAdd(G.colsum + j0 + j, sum);
+            G.colsum[(size_t)blockIdx.y * G.N + j0 + j] = sum;
         }
     }
 }
 
 // 128 x 128 tiles once they give every SM one (n x 256 outputs: n >= 64 per
 // SM), else 64 x 64 ones, four times as many blocks
+// returns the number of tile rows
 template <bool A_K, bool B_K, int EPI>
-void gemm(cudaStream_t s, int sms, const GemmArgs& G) {
-    if (EPI != EPI_WEIGHTS && (int64_t)((G.M + 127) / 128) * ((G.N + 127) / 128) < sms)
-        gemm_f32<4, 4, A_K, B_K, EPI><<<dim3((G.N + 63) / 64, (G.M + 63) / 64), 256, 0, s>>>(G);
-    else if (EPI != EPI_WEIGHTS)
-        gemm_f32<8, 8, A_K, B_K, EPI><<<dim3((G.N + 127) / 128, (G.M + 127) / 128), 256, 0, s>>>(G);
-    else {
+uint32_t gemm(cudaStream_t s, int sms, const GemmArgs& G) {
+    if (EPI == EPI_WEIGHTS) {
         // K = the points: slices of at least 64, two blocks per SM
         const int tiles = ((G.N + 127) / 128) * ((G.M + 127) / 128);
         const int slices = std::max(1, std::min(2 * sms / tiles, (G.K + 63) / 64));
         gemm_f32<8, 8, A_K, B_K, EPI><<<dim3((G.N + 127) / 128, (G.M + 127) / 128, slices), 256, 0, s>>>(G);
+        return (uint32_t)((G.M + 127) / 128);
     }
+    if ((int64_t)((G.M + 127) / 128) * ((G.N + 127) / 128) < sms) {
+        gemm_f32<4, 4, A_K, B_K, EPI><<<dim3((G.N + 63) / 64, (G.M + 63) / 64), 256, 0, s>>>(G);
+        return (uint32_t)((G.M + 63) / 64);
+    }
+    gemm_f32<8, 8, A_K, B_K, EPI><<<dim3((G.N + 127) / 128, (G.M + 127) / 128), 256, 0, s>>>(G);
+    return (uint32_t)((G.M + 127) / 128);
 }
 
 // ------------------------------------------------------- elementwise kernels ---
@@ -304,8 +308,8 @@ __global__ void loss_l1(const float* y, const float* t, uint32_t n, float clampd
 
 // The backward pass of the output layer in one read of the last layer's z
 // and a (thread = column, a range of points per block):
-//   dz[p][k] = dy[p] w[k] sigmoid(z[p][k]), its column sums into gb, and
-//   gw[k] += sum_p dy[p] a[p][k]
+//   dz[p][k] = dy[p] w[k] sigmoid(z[p][k]), each block's column sums of it in
+//   gb[block][k], and of dy[p] a[p][k] in gw[block][k]
 __global__ void __launch_bounds__(HID) out_backward(const float* __restrict__ dy, const float* __restrict__ w,
                                                     const float* __restrict__ z, const float* __restrict__ a,
                                                     uint32_t n, float* __restrict__ dz, float* gw, float* gb) {
@@ -323,10 +327,31 @@ __global__ void __launch_bounds__(HID) out_backward(const float* __restrict__ dy
         sb += d;
         sw += g * a[at];
     }
-    if (p0 < p1) {
-        atomicAdd(gw + k, sw);
-        atomicAdd(gb + k, sb);
-    }
+    gw[(size_t)blockIdx.x * HID + k] = sw;
+    gb[(size_t)blockIdx.x * HID + k] = sb;
+}
+
+// The gradients that are sums over the points (the biases', the output
+// weights'), from the tiles' or blocks' partial sums: added in fp64, where
+// hundreds of fp32 atomics on one word would each round the running sum.
+struct ColumnSums {
+    const float* part[NLAYERS + 1];  // rows x HID
+    uint32_t rows[NLAYERS + 1];
+    float* out[NLAYERS + 1];
+};
+
+__global__ void __launch_bounds__(256) add_partials(ColumnSums S) {
+    __shared__ double s_sum[8][32];
+    const uint32_t c = threadIdx.x % 32, r0 = threadIdx.x / 32, k = 32 * blockIdx.x + c;
+    const float* p = S.part[blockIdx.y] + k;
+    double sum = 0.0;
+#pragma unroll 8
+    for (uint32_t r = r0; r < S.rows[blockIdx.y]; r += 8) sum += (double)__ldg(p + (size_t)r * HID);
+    s_sum[r0][c] = sum;
+    __syncthreads();
+    if (r0) return;
+    for (int w = 1; w < 8; ++w) sum += s_sum[w][c];
+    S.out[blockIdx.y][k] = (float)sum;
 }
 
 __global__ void adam(float* p, const float* g, float* m, float* v, uint64_t n, float lr, float b1, float b2,
@@ -394,8 +419,12 @@ using namespace iso::mlp;
 namespace {
 
 struct Views {
-    float *pts, *ff, *z[NLAYERS], *a[NLAYERS], *y, *t, *dy, *d[2], *loss;
+    float *pts, *ff, *z[NLAYERS], *a[NLAYERS], *y, *t, *dy, *d[2], *part, *loss;
+    uint32_t part_rows;  // rows of each of part's NLAYERS + 1 arrays
 };
+
+// partial sums per column: a row per 64 points (the smaller GEMM tile) or per block of out_backward
+inline uint32_t partial_rows(const iso_mlp* net, uint32_t n) { return std::max<uint32_t>((n + 63) / 64, 4 * (uint32_t)net->ctx->sms); }
 
 // each piece starts on a 256-byte boundary (the GEMMs load 16 bytes at once)
 inline size_t piece(size_t floats) { return (floats + 63) & ~(size_t)63; }
@@ -405,7 +434,7 @@ iso_status ensure_work(iso_mlp* net, uint32_t n) {
     if (net->work) cudaFree(net->work);
     net->work = nullptr;
     const size_t floats = piece(3 * (size_t)n) + piece(FF * (size_t)n) + (2 * NLAYERS + 2) * piece(HID * (size_t)n) +
-                          3 * piece(n) + 1024;
+                          3 * piece(n) + (NLAYERS + 1) * piece(HID * (size_t)partial_rows(net, n)) + 1024;
     cudaError_t e = cudaMalloc(&net->work, floats * 4);
     if (e != cudaSuccess) return cuda_fail(net->ctx, e, "mlp work");
     net->work_bytes = floats * 4;
@@ -431,6 +460,8 @@ Views views(iso_mlp* net) {
     w.dy = take(n);
     w.d[0] = take(HID * n);
     w.d[1] = take(HID * n);
+    w.part_rows = partial_rows(net, net->cap);
+    w.part = take((NLAYERS + 1) * (size_t)HID * w.part_rows);
     w.loss = p;
     return w;
 }
@@ -465,8 +496,15 @@ void backward(iso_mlp* net, const Views& w, uint32_t n, float clampd) {
     // dz of the last layer and the output layer's gradients
     const int last = NLAYERS - 1;
     float *dz = w.d[0], *below = w.d[1];
-    out_backward<<<std::min<unsigned>(blocks(n, 16), 4 * (unsigned)net->ctx->sms), HID, 0, s>>>(
-        w.dy, P + OUT_W, w.z[last], w.a[last], n, dz, G + OUT_W, G + bias_offset(last));
+    ColumnSums sums{};  // entry l: layer l's biases; the last: the output weights
+    for (int l = 0; l <= NLAYERS; ++l) {
+        sums.part[l] = w.part + (size_t)l * HID * w.part_rows;
+        sums.out[l] = G + (l < NLAYERS ? bias_offset(l) : OUT_W);
+    }
+    const unsigned out_blocks = std::min<unsigned>(blocks(n, 16), 4 * (unsigned)net->ctx->sms);
+    sums.rows[last] = sums.rows[NLAYERS] = out_blocks;
+    out_backward<<<out_blocks, HID, 0, s>>>(w.dy, P + OUT_W, w.z[last], w.a[last], n, dz,
+                                            const_cast<float*>(sums.part[NLAYERS]), const_cast<float*>(sums.part[last]));
     for (int l = last; l >= 0; --l) {
         const int in_dim = l ? HID : FF;
         // dW = dz^T [HID x n] * in [n x in_dim]
@@ -477,12 +515,13 @@ void backward(iso_mlp* net, const Views& w, uint32_t n, float clampd) {
             // dz of the layer below = (dz [n x HID] * W [HID x HID]) sigmoid(z), and its bias' gradient
             GemmArgs g{(int)n, HID, HID, dz, P + weight_offset(l), HID, HID, below, HID};
             g.Z = w.z[l - 1];
-            g.colsum = G + bias_offset(l - 1);
-            gemm<true, false, EPI_BACKWARD>(s, net->ctx->sms, g);
+            g.colsum = const_cast<float*>(sums.part[l - 1]);
+            sums.rows[l - 1] = gemm<true, false, EPI_BACKWARD>(s, net->ctx->sms, g);
             std::swap(dz, below);
         }
     }
-    net->ctx->launches += 2 + 2 * NLAYERS - 1;
+    add_partials<<<dim3(HID / 32, NLAYERS + 1), 256, 0, s>>>(sums);
+    net->ctx->launches += 2 + 2 * NLAYERS;
 }
 
 }  // namespace
