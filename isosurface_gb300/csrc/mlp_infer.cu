@@ -1,27 +1,36 @@
 // BF16 tensor-core inference of the surrogate MLP on sm_103a (tcgen05).
 //
-// One CTA of 256 threads per SM runs tiles of M = 128 points through the whole
-// network:
-//   * features / activations: the A operand, 128 rows x K bf16 in shared
-//     memory, K-major with the 128-byte swizzle, as K-blocks of 64 columns
-//     (16 KB each; layer 0's 96 features are padded to 128);
+// One CTA per SM runs two tiles of M = 128 points at a time through the whole
+// network, so that one tile's matrix products run on the tensor cores while
+// the other's activations run on the SM's own pipes:
+//   * features / activations: the A operand of each tile, 128 rows x K bf16 in
+//     shared memory, K-major with the 128-byte swizzle, as K-blocks of 64
+//     columns (16 KB each; layer 0's 96 features are padded to 128);
 //   * weights: the B operand, 256 rows (N) x 64 K bf16 per K-block (32 KB),
 //     the same layout, copied by TMA bulk copies from a pre-swizzled bf16
-//     image made once per parameter update (prepare_images) into four slots;
-//     the next layer's copies run during the current layer's epilogue;
+//     image made once per parameter update (prepare_images) through a ring of
+//     three slots by a producer thread that runs ahead;
 //   * one thread issues tcgen05.mma.cta_group::1.kind::f16 (M=128, N=256,
-//     K=16, fp32 accumulate) into a 256-column TMEM accumulator and commits to
-//     an mbarrier; every wait is bounded (error flag, copies drained, TMEM
-//     freed);
-//   * epilogue: eight warps read the accumulator with tcgen05.ld (warp w: 32
-//     lanes = rows, 128 columns), add the bias, apply softplus_beta and write
-//     the bf16 operand of the next layer; after the last layer they dot with
-//     w_out (fp32) instead.
+//     K=16, fp32 accumulate) for the two tiles' layers in turn, each into its
+//     own 256 TMEM columns, and commits to an mbarrier; every wait is bounded
+//     (error flag, copies drained, TMEM freed);
+//   * epilogue: eight warps per tile read the accumulator with tcgen05.ld (warp
+//     w: 32 lanes = rows, 128 columns), add the bias, apply softplus_beta and
+//     write the bf16 operand of the next layer; after the last layer they dot
+//     with w_out (fp32) instead, and make the next tile's features.
+// What bounds it is the SM's shared-memory / L1 bandwidth: a tile's layer
+// moves 192 KB of MMA operands, 128 KB of weights in and 64 KB of activations
+// out (3072 cycles at 128 bytes, against 2048 of MMA).  250001 points: 0.293
+// ms with one tile at a time (products and activations in turn), 0.219 with
+// two, 0.197 with the biases by value (read from memory they took another
+// 128 KB per tile and layer).  Pairs of CTAs sharing the weights by multicast
+// copies changed nothing.
 // Descriptor formats (tcgen05 shared-memory matrix descriptor and the
 // kind::f16 instruction descriptor) follow the PTX ISA for sm_100-class MMA.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "internal.h"
@@ -34,6 +43,7 @@ struct MlpImages {
     __nv_bfloat16* w = nullptr;  // per layer: NK/64 K-blocks of 256 rows x 128 B, swizzled
     float* bias = nullptr;       // NLAYERS x 256
     float* wout = nullptr;       // 256 + 1
+    std::vector<float> host;     // bias, then wout: the kernel takes them by value
     bool valid = false;
 };
 
@@ -102,9 +112,10 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
-// parity wait on an mbarrier, bounded in polls and in time (about a second)
-__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase) {
-    const uint64_t t0 = global_ns();
+// parity wait on an mbarrier, bounded in polls and in time (about a second);
+// also given up once another role of the CTA gave up (*abort)
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase, const volatile uint32_t* abort) {
+    uint64_t t0 = 0;
     for (uint32_t it = 0; it < WAIT_LIMIT; ++it) {
         uint32_t done;
         asm volatile(
@@ -113,7 +124,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase) {
             : "r"(addr), "r"(phase)
             : "memory");
         if (done) return true;
-        if ((it & 255u) == 255u && global_ns() - t0 > WAIT_NS) return false;
+        if ((it & 63u) == 63u) {
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > WAIT_NS || (abort && *abort)) return false;
+        }
     }
     return false;
 }
@@ -204,8 +219,11 @@ __device__ __forceinline__ void sincos_reduced(float a, float* s, float* c) {
 
 struct InferArgs {
     const unsigned char* w;  // swizzled bf16 weight image (K-blocks of 32 KB)
-    const float* bias;
-    const float* wout;
+    // by value, so that the epilogue reads them through the constant cache:
+    // loaded from memory, each lane's copy of 128 biases per layer took a
+    // quarter of the shared-memory / L1 bandwidth, which bounds this kernel
+    float bias[NLAYERS * HID];
+    float wout[HID + 4];
     // points: either explicit (pts != null, n points, out[i]) or a grid of
     // nx x ny x nz lattice points (i, j, k) at p = (i*step*inv, j*step*inv,
     // k*step*inv) mapped by q = p * scale + offset, out[(k*ny + j)*nx + i]
@@ -214,6 +232,7 @@ struct InferArgs {
     uint32_t nx, ny, nz, step;
     float inv;
     float scale[3], offset[3];
+    uint32_t groups;  // tiles a CTA works on at a time: 1 or 2
     float* out;
     uint32_t* err;
 };
@@ -235,10 +254,12 @@ __device__ __forceinline__ void point_of(const InferArgs& A, uint64_t i, float* 
     q[2] = __fadd_rn(__fmul_rn(__fmul_rn((float)(z * A.step), A.inv), A.scale[2]), A.offset[2]);
 }
 
-constexpr int THREADS = 256;
-constexpr size_t SMEM_A = 4 * KBLOCK_BYTES_A;          // 64 KB: activations, 4 K-blocks
-constexpr size_t SMEM_B = 4 * KBLOCK_BYTES_B;          // 128 KB: weight slots, one K-block each
-constexpr size_t SMEM_TOTAL = SMEM_A + SMEM_B + 1024;  // + alignment slack
+constexpr int GROUP = 256;                 // threads of a tile's epilogue
+constexpr int THREADS = 2 * GROUP + 64;    // two tiles, the MMA warp, the copying warp
+constexpr int SLOTS = 3;                   // weight K-blocks in flight
+constexpr size_t SMEM_A = 4 * KBLOCK_BYTES_A;                   // 64 KB: one tile's activations, 4 K-blocks
+constexpr size_t SMEM_B = SLOTS * KBLOCK_BYTES_B;               // 96 KB: weight slots
+constexpr size_t SMEM_TOTAL = 2 * SMEM_A + SMEM_B + 1024;       // + alignment slack
 
 __host__ __device__ constexpr int kblocks_of(int l) { return l == 0 ? KB0 : KB; }
 
@@ -246,192 +267,245 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
 }
 
-// weights of layer l into the slots: one bulk copy per K-block, completing
-// on that slot's barrier
-__device__ __forceinline__ void load_layer(const InferArgs& A, int l, uint32_t sB, uint32_t full0) {
-    const unsigned char* src = A.w + 2 * image_offset(l);
-    for (int kb = 0; kb < kblocks_of(l); ++kb) {
-        const uint32_t bar = full0 + 8 * kb;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
-                     "r"((uint32_t)KBLOCK_BYTES_B)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                sB + kb * (uint32_t)KBLOCK_BYTES_B),
-            "l"(src + kb * KBLOCK_BYTES_B), "r"((uint32_t)KBLOCK_BYTES_B), "r"(bar)
-            : "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void commit_to(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
+// a barrier of the 256 threads of group g; whether `ok` held for all of them
+__device__ __forceinline__ bool group_all(int g, bool ok) {
+    uint32_t all;
+    asm volatile(
+        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(all)
+        : "r"((uint32_t)ok), "r"(1 + g), "r"(GROUP)
+        : "memory");
+    return all != 0;
+}
+
+// Fourier features of point q as row `row` of a tile's operand: k in
+// [64*half, 64*half + 64) (96..127 zero)
+__device__ __forceinline__ void write_features(unsigned char* sA, int row, int half, const float* q) {
+    for (int k0 = 64 * half; k0 < 64 * half + 64; k0 += 8) {
+        uint32_t packed[4] = {0u, 0u, 0u, 0u};
+        if (k0 < FF) {
+            const int a = k0 / 32;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int j = (k0 % 32) / 2 + i;
+                float s, c;
+                sincos_reduced(ffreq(j) * q[a], &s, &c);
+                __nv_bfloat162 h = __floats2bfloat162_rn(s, c);
+                packed[i] = *reinterpret_cast<uint32_t*>(&h);
+            }
+        }
+        *reinterpret_cast<uint4*>(sA + swz(row, k0, 128)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
 }
 
-// One CTA per SM, 8 warps.  Warp w reads TMEM lanes 32*(w%4).. (rows) and
-// accumulator columns 128*(w/4).. in the epilogue; thread 0 also issues the
-// weight copies and the MMAs.  Per layer:
-//   thread 0: wait for each weight K-block, 4 MMAs (K = 16) per K-block,
-//             commit to `done`;
-//   all:      wait `done`; thread 0 starts copying the next layer's weights
-//             (the slots are free once the MMAs completed), which overlaps
-//             the epilogue; epilogue from TMEM into the next A operand.
-// Every wait is bounded; a timeout anywhere ends the CTA's loop uniformly
-// (the decision is a block-wide OR), drains what it started and frees TMEM.
-__global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferArgs A) {
+// Barriers (per tile g: ready = its operand is written, one arrival per warp; acc =
+// its layer's MMAs are done; per slot: full = the K-block has landed, empty =
+// the MMAs that read it are done).  Tile g's chain is ready -> MMA -> acc ->
+// epilogue -> ready ...; the MMA thread takes the chains' steps in turn, so
+// while it works on one tile the other's epilogue runs.  The operand and the
+// accumulator need no second copy: the epilogue writes and reads them after
+// acc (the MMAs are done with both), the MMAs after ready.
+// Every wait is bounded; a role that gives up raises s_abort, which ends the
+// others' waits; the MMAs and copies in flight are then waited for (again
+// with a limit) before TMEM is freed.
+__global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(const __grid_constant__ InferArgs A) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t s_full[4];
-    __shared__ uint64_t s_done;
+    __shared__ uint64_t s_full[SLOTS], s_empty[SLOTS], s_ready[2], s_acc[2], s_drain;
     __shared__ uint32_t s_tmem;
-    __shared__ float s_part[128];
+    __shared__ volatile uint32_t s_abort;
+    __shared__ float s_part[2][128];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* sA = smem;
-    const uint32_t sB = smem_u32(smem + SMEM_A);
+    const uint32_t sB = smem_u32(smem + 2 * SMEM_A);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t full0 = smem_u32(&s_full[0]), done = smem_u32(&s_done);
+    const uint32_t full0 = smem_u32(&s_full[0]), empty0 = smem_u32(&s_empty[0]);
+    const uint32_t ready0 = smem_u32(&s_ready[0]), acc0 = smem_u32(&s_acc[0]), drain = smem_u32(&s_drain);
     const uint64_t ntiles = (A.n + 127) / 128;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;\n" ::"r"(smem_u32(&s_tmem)));
+    const uint64_t steps = (ntiles + A.groups - 1) / A.groups;  // tiles in groups of one or two
+    if (warp == 16) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (tid == 0) {
-        for (int i = 0; i < 4; ++i) mbar_init(full0 + 8 * i, 1);
-        mbar_init(done, 1);
+        for (int i = 0; i < SLOTS; ++i) {
+            mbar_init(full0 + 8 * i, 1);
+            mbar_init(empty0 + 8 * i, 1);
+        }
+        for (int g = 0; g < 2; ++g) {
+            mbar_init(ready0 + 8 * g, GROUP / 32);
+            mbar_init(acc0 + 8 * g, 1);
+        }
+        mbar_init(drain, 1);
+        s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        if ((uint64_t)blockIdx.x < ntiles) load_layer(A, 0, sB, full0);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = s_tmem;
-    uint32_t full_phase = 0;   // thread 0: parity per slot
-    uint32_t pending = 0;      // thread 0: slots with a copy not yet waited on
-    if (tid == 0 && (uint64_t)blockIdx.x < ntiles) pending = (1u << KB0) - 1u;
-    uint32_t done_phase = 0;
-    bool aborted = false;
-    const int row = tid & 127, half = tid >> 7;  // features: point row, 64-feature half
-    const int erow = 32 * (warp & 3) + lane, ecol0 = 128 * (warp >> 2);  // epilogue
-    for (uint64_t tile = blockIdx.x; tile < ntiles && !aborted; tile += gridDim.x) {
-        const uint64_t pidx = tile * 128 + row;
-        float q[3] = {0.0f, 0.0f, 0.0f};
-        if (pidx < A.n) point_of(A, pidx, q);
-        // Fourier features k in [64*half, 64*half + 64) of row `row` (96..127 zero)
-        for (int k0 = 64 * half; k0 < 64 * half + 64; k0 += 8) {
-            uint32_t packed[4] = {0u, 0u, 0u, 0u};
-            if (k0 < FF) {
-                const int a = k0 / 32;
+    if (warp < 16) {
+        // ---- a tile's features and epilogues
+        const int g = warp >> 3, gt = tid & (GROUP - 1), gw = warp & 7;
+        unsigned char* sA = smem + g * SMEM_A;
+        const int row = gt & 127, half = gt >> 7;                                  // features: point row, 64-feature half
+        const int erow = 32 * (gw & 3) + lane, ecol0 = 128 * (gw >> 2);            // epilogue
+        const uint32_t taddr = tmem + (uint32_t)(256 * g) + ((uint32_t)(32 * (gw & 3)) << 16);
+        uint32_t phase = 0;
+        bool ok = g < (int)A.groups;
+        for (uint64_t step = blockIdx.x; step < steps && ok; step += gridDim.x) {
+            const uint64_t tile = step * A.groups + g, pidx = tile * 128 + row;
+            float q[3] = {0.0f, 0.0f, 0.0f};
+            if (pidx < A.n) point_of(A, pidx, q);
+            write_features(sA, row, half, q);
+            float y = 0.0f;
+            for (int l = 0; l < NLAYERS; ++l) {
+                // the operand is written and the accumulator read
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready0 + 8 * g);
+                const float* bias = A.bias + l * HID;
+                // one decision for the group: its barriers need every thread
+                ok = group_all(g, mbar_wait(acc0 + 8 * g, phase, &s_abort));
+                phase ^= 1;
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                // row erow, columns [ecol0, ecol0 + 128), 16 at a time; the
+                // TMEM load of the next 16 overlaps the arithmetic on these
+                uint32_t ra[16], rb[16];
+                uint64_t sum = f2(0.0f, 0.0f);
+                tmem_ld16(taddr + ecol0, ra);
+                tmem_wait(ra);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int j = (k0 % 32) / 2 + i;
-                    float s, c;
-                    sincos_reduced(ffreq(j) * q[a], &s, &c);
-                    __nv_bfloat162 h = __floats2bfloat162_rn(s, c);
-                    packed[i] = *reinterpret_cast<uint32_t*>(&h);
+                for (int c = 0; c < 8; ++c) {
+                    uint32_t(&cur)[16] = (c & 1) ? rb : ra;
+                    uint32_t(&nxt)[16] = (c & 1) ? ra : rb;
+                    const int c0 = ecol0 + 16 * c;
+                    if (c + 1 < 8) tmem_ld16(taddr + c0 + 16, nxt);
+                    uint64_t r[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        r[i] = softplus2(f2(__uint_as_float(cur[2 * i]), __uint_as_float(cur[2 * i + 1])),
+                                         f2(bias[c0 + 2 * i], bias[c0 + 2 * i + 1]));
+                    if (l + 1 < NLAYERS) {
+                        uint32_t p[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float a0, a1;
+                            uf2(r[i], a0, a1);
+                            __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
+                            p[i] = *reinterpret_cast<uint32_t*>(&h);
+                        }
+                        *reinterpret_cast<uint4*>(sA + swz(erow, c0, 128)) = make_uint4(p[0], p[1], p[2], p[3]);
+                        *reinterpret_cast<uint4*>(sA + swz(erow, c0 + 8, 128)) = make_uint4(p[4], p[5], p[6], p[7]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            sum = fma2(r[i], f2(A.wout[c0 + 2 * i], A.wout[c0 + 2 * i + 1]), sum);
+                        }
+                    }
+                    if (c + 1 < 8) tmem_wait(nxt);
+                }
+                if (l + 1 == NLAYERS) {
+                    float a0, a1;
+                    uf2(sum, a0, a1);
+                    y = a0 + a1;
                 }
             }
-            *reinterpret_cast<uint4*>(sA + swz(row, k0, 128)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            if (!ok) break;
+            // output: the two column halves of each row
+            if (ecol0) s_part[g][erow] = y;
+            group_all(g, true);
+            if (!ecol0) {
+                const uint64_t o = tile * 128 + erow;
+                if (o < A.n) A.out[o] = y + s_part[g][erow] + A.wout[HID];
+            }
         }
-        float y = 0.0f;
-        for (int l = 0; l < NLAYERS; ++l) {
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncthreads();
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            bool ok = true;
-            if (tid == 0) {
-                for (int kb = 0; kb < kblocks_of(l) && ok; ++kb) {
-                    ok = mbar_wait(full0 + 8 * kb, (full_phase >> kb) & 1u);
+        if (!ok && g < (int)A.groups) {
+            s_abort = 1;
+            if (gt == 0) atomicOr(A.err, DERR_QUEUE_TIMEOUT);
+        }
+    } else if (warp == 16 && lane == 0) {
+        // ---- the tiles' layers in turn
+        uint32_t phase = 0;   // both tiles' ready barriers move together
+        uint32_t kbi = 0;     // K-blocks taken so far
+        const uint64_t bdesc = sdesc(sB);
+        bool ok = true;
+        for (uint64_t step = blockIdx.x; step < steps && ok; step += gridDim.x) {
+            for (int l = 0; l < NLAYERS && ok; ++l, phase ^= 1) {
+                for (int g = 0; g < (int)A.groups && ok; ++g) {
+                    ok = mbar_wait(ready0 + 8 * g, phase, &s_abort);
                     if (!ok) break;
-                    full_phase ^= 1u << kb;
-                    pending &= ~(1u << kb);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    for (int s = 0; s < 4; ++s) {
-                        const uint64_t ad = sdesc(smem_u32(sA + kb * KBLOCK_BYTES_A + s * 32));
-                        const uint64_t bd = sdesc(sB + kb * (uint32_t)KBLOCK_BYTES_B + s * 32);
-                        mma(tmem, ad, bd, (kb | s) ? 1u : 0u);
+                    // (descriptor addresses count 16 bytes: a K = 16 step is 2 on)
+                    uint64_t ad = sdesc(smem_u32(smem + g * SMEM_A));
+                    for (int kb = 0; kb < kblocks_of(l); ++kb, ++kbi) {
+                        const uint32_t slot = kbi % SLOTS;
+                        ok = mbar_wait(full0 + 8 * slot, (kbi / SLOTS) & 1u, &s_abort);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        const uint64_t bd = bdesc + slot * (uint32_t)(KBLOCK_BYTES_B >> 4);
+#pragma unroll
+                        for (int s = 0; s < 4; ++s)
+                            mma(tmem + (uint32_t)(256 * g), ad + 2 * s, bd + 2 * s, (kb | s) ? 1u : 0u);
+                        ad += KBLOCK_BYTES_A >> 4;
+                        commit_to(empty0 + 8 * slot);
                     }
+                    if (ok) commit_to(acc0 + 8 * g);
                 }
-                // commit even after a failed wait: `done` then tracks the MMAs issued so far
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 done)
-                             : "memory");
-            }
-            const bool ok_done = mbar_wait(done, done_phase);
-            done_phase ^= 1;
-            if (__syncthreads_or(!(ok && ok_done))) {
-                if (tid == 0) atomicOr(A.err, DERR_QUEUE_TIMEOUT);
-                if (!ok_done) mbar_wait(done, done_phase ^ 1);  // bounded: let issued MMAs drain
-                aborted = true;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            // the slots are free: copy the next layer's weights during the epilogue
-            if (tid == 0) {
-                const bool more = l + 1 < NLAYERS || tile + gridDim.x < ntiles;
-                if (more) {
-                    const int nl = (l + 1) % NLAYERS;
-                    load_layer(A, nl, sB, full0);
-                    pending |= (1u << kblocks_of(nl)) - 1u;
-                }
-            }
-            // epilogue: row erow, columns [ecol0, ecol0 + 128), 16 at a time;
-            // the TMEM load of the next 16 overlaps the arithmetic on these
-            const float* bias = A.bias + l * HID;
-            const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-            uint32_t ra[16], rb[16];
-            uint64_t acc = f2(0.0f, 0.0f);
-            tmem_ld16(taddr + ecol0, ra);
-            tmem_wait(ra);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint32_t(&cur)[16] = (c & 1) ? rb : ra;
-                uint32_t(&nxt)[16] = (c & 1) ? ra : rb;
-                const int c0 = ecol0 + 16 * c;
-                if (c + 1 < 8) tmem_ld16(taddr + c0 + 16, nxt);
-                uint64_t r[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 bb = __ldg(reinterpret_cast<const float2*>(bias + c0) + i);
-                    r[i] = softplus2(f2(__uint_as_float(cur[2 * i]), __uint_as_float(cur[2 * i + 1])), f2(bb.x, bb.y));
-                }
-                if (l + 1 < NLAYERS) {
-                    uint32_t p[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float a0, a1;
-                        uf2(r[i], a0, a1);
-                        __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
-                        p[i] = *reinterpret_cast<uint32_t*>(&h);
-                    }
-                    *reinterpret_cast<uint4*>(sA + swz(erow, c0, 128)) = make_uint4(p[0], p[1], p[2], p[3]);
-                    *reinterpret_cast<uint4*>(sA + swz(erow, c0 + 8, 128)) = make_uint4(p[4], p[5], p[6], p[7]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float2 ww = __ldg(reinterpret_cast<const float2*>(A.wout + c0) + i);
-                        acc = fma2(r[i], f2(ww.x, ww.y), acc);
-                    }
-                }
-                if (c + 1 < 8) tmem_wait(nxt);
-            }
-            if (l + 1 == NLAYERS) {
-                float a0, a1;
-                uf2(acc, a0, a1);
-                y = a0 + a1;
             }
         }
-        if (aborted) break;
-        // output: the two column halves of each row
-        if (ecol0) s_part[erow] = y;
-        __syncthreads();
-        if (!ecol0) {
-            const uint64_t o = tile * 128 + erow;
-            if (o < A.n) A.out[o] = y + s_part[erow] + __ldg(A.wout + HID);
+        if (!ok) {
+            s_abort = 1;
+            atomicOr(A.err, DERR_QUEUE_TIMEOUT);
         }
+        // nothing issued here is still running when TMEM is freed
+        commit_to(drain);
+        mbar_wait(drain, 0, nullptr);
+    } else if (warp == 17 && lane == 0) {
+        // ---- weights: the K-blocks of the layers in the order the MMAs take them
+        uint32_t kbi = 0;
+        bool ok = true;
+        for (uint64_t step = blockIdx.x; step < steps && ok; step += gridDim.x) {
+            for (int l = 0; l < NLAYERS && ok; ++l) {
+                const unsigned char* src = A.w + 2 * image_offset(l);
+                for (int g = 0; g < (int)A.groups && ok; ++g) {
+                    for (int kb = 0; kb < kblocks_of(l); ++kb, ++kbi) {
+                        const uint32_t slot = kbi % SLOTS, bar = full0 + 8 * slot;
+                        ok = mbar_wait(empty0 + 8 * slot, ((kbi / SLOTS) & 1u) ^ 1u, &s_abort);
+                        if (!ok) break;
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
+                                     "r"((uint32_t)KBLOCK_BYTES_B)
+                                     : "memory");
+                        asm volatile(
+                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
+                                "r"(sB + slot * (uint32_t)KBLOCK_BYTES_B),
+                            "l"(src + kb * KBLOCK_BYTES_B), "r"((uint32_t)KBLOCK_BYTES_B), "r"(bar)
+                            : "memory");
+                    }
+                }
+            }
+        }
+        if (!ok) {
+            s_abort = 1;
+            atomicOr(A.err, DERR_QUEUE_TIMEOUT);
+        }
+        // the last copy into each slot has landed before the CTA ends
+        for (uint32_t i = kbi > SLOTS ? kbi - SLOTS : 0; i < kbi; ++i)
+            mbar_wait(full0 + 8 * (i % SLOTS), (i / SLOTS) & 1u, nullptr);
     }
-    if (tid == 0) {  // bounded drain of copies started and not consumed (after an abort)
-        for (int kb = 0; kb < 4; ++kb)
-            if ((pending >> kb) & 1u) mbar_wait(full0 + 8 * kb, (full_phase >> kb) & 1u);
-    }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem));
+    if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
 }
 
 }  // namespace
@@ -472,6 +546,10 @@ static iso_status ready(iso_mlp* net, MlpImages** out) {
         ctx->launches++;
         iso_status s = check_launch(ctx, "prepare images");
         if (s != ISO_OK) return s;
+        m->host.resize(NLAYERS * HID + HID + 1);
+        cudaError_t e = cudaMemcpyAsync(m->host.data(), m->bias, 4 * m->host.size(), cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp biases");
         m->valid = true;
     }
     *out = m;
@@ -485,8 +563,8 @@ iso_status mlp_infer_launch(iso_mlp* net, const float* d_pts, uint64_t n, const 
     if (s != ISO_OK) return s;
     InferArgs a{};
     a.w = reinterpret_cast<const unsigned char*>(m->w);
-    a.bias = m->bias;
-    a.wout = m->wout;
+    std::copy(m->host.begin(), m->host.begin() + NLAYERS * HID, a.bias);
+    std::copy(m->host.begin() + NLAYERS * HID, m->host.end(), a.wout);
     a.pts = d_pts;
     a.n = n;
     if (grid) {
@@ -509,8 +587,10 @@ iso_status mlp_infer_launch(iso_mlp* net, const float* d_pts, uint64_t n, const 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (a.n == 0) return ISO_OK;
+    // two tiles per CTA once every SM has one
     const uint64_t tiles = (a.n + 127) / 128;
-    const unsigned blocks = (unsigned)std::min<uint64_t>(tiles, (uint64_t)sms);
+    a.groups = tiles > (uint64_t)sms ? 2 : 1;
+    const unsigned blocks = (unsigned)std::min<uint64_t>((tiles + a.groups - 1) / a.groups, (uint64_t)sms);
     {
         StageTimer timer(ctx, ISO_STAGE_MLP);
         mlp_infer_kernel<<<blocks, THREADS, SMEM_TOTAL, ctx->stream>>>(a);
