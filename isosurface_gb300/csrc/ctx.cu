@@ -41,11 +41,13 @@ iso_status fork_side(iso_ctx* ctx, cudaStream_t* side) {
     e = cudaEventRecord(ctx->side_fork, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fork side stream");
+    ctx->side_open = true;
     *side = ctx->side;
     return ISO_OK;
 }
 
 iso_status join_side(iso_ctx* ctx) {
+    ctx->side_open = false;
     cudaError_t e = cudaEventRecord(ctx->side_join, ctx->side);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->side_join, 0);
     return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "join side stream");
@@ -597,6 +599,7 @@ iso_status parse_program(const uint8_t* bytes, size_t len, iso_program* p, std::
     if (!validate(p, err)) return ISO_ERR_BAD_PROGRAM;
     classify(p);
     cull_bounds(p);
+    for (float c : p->consts) p->tiny = p->tiny || (c != 0.0f && std::fabs(c) < 1e-18f);
     uint64_t hash = 0xCBF29CE484222325ull;  // FNV-1a 64
     for (size_t i = 0; i < len; ++i) hash = (hash ^ bytes[i]) * 0x100000001B3ull;
     p->content_hash = hash;

@@ -11,15 +11,20 @@
 // the last two passes are mc_extract_lattice.
 //
 // Passes: (1) grid sampler (sign bits everywhere; for a program with a
-// Lipschitz bound, values only near the surface, NaN elsewhere), (2) dc_dual:
-// sign bits of every dual vertex, value and centre of those marching cubes
-// can read, active primal cells appended to a list, (3) dc_place:
-// one thread per active cell -- eight normals from the program
-// (sample_normals_at_corners, marching_cubes_impl.rs:58-69), tangent planes,
-// the planar cells' centre of mass or particle placement, the non-planar
-// cells listed for (3b) dc_feature: their MinimiseQEF (f64 SVD) in full
-// warps, (4)+(5) the lattice marching-cubes passes.
+// Lipschitz bound, values only near the surface), (2) dc_signs: dual sign
+// words and the active primal cells, from the primal sign bits, (3) dc_edges:
+// the active cells at an end of a crossing dual edge, and the values and
+// centres that marching cubes reads there, (4) dc_place: one thread per
+// such cell -- eight normals from the program (sample_normals_at_corners,
+// marching_cubes_impl.rs:58-69), tangent planes, the planar cells' centre of
+// mass or particle placement, the non-planar cells listed for (5) dc_feature:
+// their MinimiseQEF (f64 SVD) in full warps; (4) and (5) on a side stream
+// beside (6) the lattice marching-cubes passes, whose emission waits for them.
+// A program without a bound takes its full field through dc_dual in place of
+// (2) and (3).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "internal.h"
 #include "qef.cuh"
@@ -29,12 +34,15 @@
 namespace iso {
 // jit.cu: dc_place with the program's compiled normals; false (nothing
 // launched) when the program has none
-bool jit_dc_place(iso_ctx* ctx, const iso_program* prog, const DcCells& cells, uint64_t blocks, cudaError_t* err);
+bool jit_dc_place(cudaStream_t stream, const iso_program* prog, const DcCells& cells, uint64_t blocks,
+                  cudaError_t* err);
 
 namespace {
 
+constexpr uint32_t FULL = 0xFFFFFFFFu;
+
 struct DualArgs {
-    const float* field;   // primal values; NaN where the sampler left them unwritten
+    const float* field;   // primal values
     const uint32_t* bits; // primal sign bits (bit set iff !(v > 0)), W words per row
     uint32_t W;
     uint64_t pitch;       // primal row pitch
@@ -46,22 +54,182 @@ struct DualArgs {
     uint64_t dpitch;
     float4* dpos;         // dual positions, dense (n-1) x (n-1) x nzd
     uint32_t* dbits;      // dual sign bits (bit set iff !(value > 0)), dW words per row
+    uint32_t* abits;      // active primal cells, laid out as dbits
     uint32_t dW;
     uint32_t* list;       // active primal cells (linear dual index)
     uint32_t* count;
+    uint32_t* ends;       // dc_edges: those at an end of a crossing dual edge
+    uint32_t* nends;
     uint32_t cap;
     uint32_t* err;
-    bool near;            // the sampler wrote values only near the surface (NaN elsewhere)
+    uint32_t run;         // dc_signs: layers per warp
 };
 
-// One warp per 32 dual vertices of a dual row (x = 32 w + lane): value,
-// centre, sign word (by ballot) and the active primal cells.  A dual vertex
-// whose primal corners 0 or 6 the near-surface sampler skipped gets its sign
-// only: those corners lie more than 2.5 lattice steps' worth of value change
-// from zero, so (by the Lipschitz bound) v0 and v6 share the sign of corner 0
-// and the dual value lies more than 1.6 steps' worth from zero, while both
-// ends of a crossing dual edge lie within one step's worth; marching cubes
-// reads values and positions only at those ends.
+// Vec3::lerp / Signed::lerp with f = 0.5: (1 - f) * a + f * b
+__device__ __forceinline__ float half_lerp(float a, float b) {
+    const float of = 1.0f - 0.5f;
+    return of * a + 0.5f * b;
+}
+
+__device__ __forceinline__ float4 dual_centre(const DualArgs& A, uint32_t x, uint32_t y, uint32_t z) {
+    const float c0x = (float)x * A.inv, c0y = (float)y * A.inv, c0z = (float)(z + A.zoff) * A.inv;
+    const float c6x = (float)(x + 1) * A.inv, c6y = (float)(y + 1) * A.inv, c6z = (float)(z + 1 + A.zoff) * A.inv;
+    return make_float4(half_lerp(c0x, c6x), half_lerp(c0y, c6y), half_lerp(c0z, c6z), 0.0f);
+}
+
+// corners 0 and 6 of dual vertex (x, y, z)'s primal cell
+__device__ __forceinline__ void dual_corners(const DualArgs& A, uint32_t x, uint32_t y, uint32_t z, float* v0,
+                                             float* v6) {
+    const float* f0 = A.field + ((size_t)z * A.n + y) * A.pitch + x;
+    *v0 = __ldg(f0);
+    *v6 = __ldg(f0 + (size_t)A.n * A.pitch + A.pitch + 1);
+}
+
+// Dual sign words and active cells, from sign bits alone wherever the cell's
+// corners 0 and 6 agree: the dual value, their mean, then has their sign
+// (no program here produces values within an ulp of zero's neighbours, see
+// iso_program::tiny).  Where they differ the surface passes between two points
+// sqrt(3) lattice steps apart, so both lie within that of zero and the
+// sampler (which keeps 2.5 steps) wrote them.  Lane = 32 dual vertices of a
+// row; a warp marches its 32 words up `run` layers, the sign words of a layer
+// serving the cells below and above it.  The active cells of a step are
+// handed out one per lane.
+__global__ void __launch_bounds__(256) dc_signs(DualArgs A) {
+    __shared__ uint32_t s_word[8][32];
+    const uint32_t m = A.n - 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t S = A.dW * m, SL = (S + 31) / 32;
+    const uint32_t task = blockIdx.x * 8 + warp, seg = task % SL, z0 = task / SL * A.run;
+    if (z0 >= A.nzd) return;  // warp-uniform
+    const uint32_t l = 32 * seg + lane, y = l / A.dW, c = l - y * A.dW;
+    const bool in = l < S, nxt = in && c + 1 < A.W;
+    const uint32_t left = in ? m - 32 * c : 0u;
+    const uint32_t valid = left >= 32 ? FULL : (1u << left) - 1u;
+    const uint64_t layer = (uint64_t)A.n * A.W;
+    const uint32_t* p = A.bits + z0 * layer + (uint64_t)y * A.W + c;
+    auto quad = [&](const uint32_t* q) {  // corners (x,y) (x+1,y) (x+1,y+1) (x,y+1)
+        const uint32_t a0 = in ? __ldg(q) : 0u, an = nxt ? __ldg(q + 1) : 0u;
+        const uint32_t b0 = in ? __ldg(q + A.W) : 0u, bn = nxt ? __ldg(q + A.W + 1) : 0u;
+        return make_uint4(a0, __funnelshift_r(a0, an, 1), __funnelshift_r(b0, bn, 1), b0);
+    };
+    uint4 lo = quad(p);
+    const uint32_t z1 = min(z0 + A.run, A.nzd);
+    for (uint32_t z = z0; z < z1; ++z) {
+        p += layer;
+        const uint4 hi = quad(p);
+        const uint32_t any = lo.x | lo.y | lo.z | lo.w | hi.x | hi.y | hi.z | hi.w;
+        const uint32_t all = lo.x & lo.y & lo.z & lo.w & hi.x & hi.y & hi.z & hi.w;
+        const uint32_t act = any & ~all & valid, diff = (lo.x ^ hi.z) & valid;
+        uint32_t word = lo.x & hi.z & valid;
+        if (__any_sync(FULL, act != 0)) {
+            const uint32_t n = __popc(act);
+            uint32_t incl = n;
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const uint32_t excl = incl - n, total = __shfl_sync(FULL, incl, 31);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(A.count, total);
+            base = __shfl_sync(FULL, base, 0);
+            s_word[warp][lane] = word;
+            __syncwarp();
+            for (uint32_t b0 = 0; b0 < total; b0 += 32) {
+                const uint32_t kk = b0 + lane;
+                uint32_t src = 0;  // the last lane whose prefix is <= kk
+#pragma unroll
+                for (uint32_t step = 16; step > 0; step >>= 1) {
+                    const uint32_t e = __shfl_sync(FULL, excl, (src + step) & 31);
+                    if (src + step < 32 && e <= kk) src += step;
+                }
+                uint32_t bits = __shfl_sync(FULL, act, src), r = kk - __shfl_sync(FULL, excl, src), i = 0;
+                const uint32_t dsrc = __shfl_sync(FULL, diff, src), lsrc = __shfl_sync(FULL, lo.x, src);
+                const uint32_t ysrc = __shfl_sync(FULL, y, src), csrc = __shfl_sync(FULL, c, src);
+                if (kk >= total) continue;
+#pragma unroll
+                for (uint32_t w = 16; w > 0; w >>= 1) {  // set bit number r
+                    const uint32_t below = __popc(bits & ((1u << w) - 1u));
+                    if (r >= below) {
+                        r -= below;
+                        bits >>= w;
+                        i += w;
+                    }
+                }
+                const uint32_t x = 32 * csrc + i;
+                if (base + kk < A.cap) A.list[base + kk] = (uint32_t)(((uint64_t)z * m + ysrc) * m + x);
+                else atomicOr(A.err, DERR_CAPACITY);
+                if ((dsrc >> i) & 1u) {
+                    float v0, v6;
+                    dual_corners(A, x, ysrc, z, &v0, &v6);
+                    const bool inside = v0 == v0 && v6 == v6 ? !(half_lerp(v0, v6) > 0.0f) : (lsrc >> i) & 1u;
+                    if (inside) atomicOr(&s_word[warp][src], 1u << i);
+                }
+            }
+            __syncwarp();
+            word = s_word[warp][lane];
+            __syncwarp();
+        }
+        if (in) {
+            const uint64_t at = ((uint64_t)z * m + y) * A.dW + c;
+            A.dbits[at] = word;
+            A.abits[at] = act;
+        }
+        lo = hi;
+    }
+}
+
+// One thread per active cell: marching cubes reads the value and position of
+// a dual vertex only at the ends of crossing dual edges, and of the two ends
+// at least one belongs to an active cell (cells that share four corners and
+// have no sign change have the same sign).  An active cell with such an edge
+// gets its value here and its position from the placement; its inactive
+// neighbours across such edges get their value and cell centre here.
+__global__ void __launch_bounds__(256) dc_edges(DualArgs A) {
+    const uint32_t m = A.n - 1, lane = threadIdx.x & 31, n = *A.count;
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        bool end = false;
+        uint32_t id = 0;
+        if (i < n) {
+            id = A.list[i];
+            const uint32_t x = id % m, r = id / m, y = r % m, z = r / m;
+            auto bit = [&](const uint32_t* words, uint32_t xx, uint32_t yy, uint32_t zz) {
+                return (__ldg(words + ((uint64_t)zz * m + yy) * A.dW + (xx >> 5)) >> (xx & 31)) & 1u;
+            };
+            const uint32_t own = bit(A.dbits, x, y, z);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const uint32_t axis = k >> 1, up = k & 1;
+                const uint32_t at = axis == 0 ? x : axis == 1 ? y : z, lim = axis == 2 ? A.nzd : m;
+                if (up ? at + 1 >= lim : at == 0) continue;
+                const uint32_t d = up ? 1u : 0xFFFFFFFFu;
+                const uint32_t xx = x + (axis == 0 ? d : 0u), yy = y + (axis == 1 ? d : 0u), zz = z + (axis == 2 ? d : 0u);
+                if (bit(A.dbits, xx, yy, zz) == own) continue;
+                end = true;
+                if (bit(A.abits, xx, yy, zz)) continue;  // it looks after itself
+                float v0, v6;
+                dual_corners(A, xx, yy, zz, &v0, &v6);
+                A.dval[((size_t)zz * m + yy) * A.dpitch + xx] = half_lerp(v0, v6);
+                A.dpos[((uint64_t)zz * m + yy) * m + xx] = dual_centre(A, xx, yy, zz);
+            }
+            if (end) {
+                float v0, v6;
+                dual_corners(A, x, y, z, &v0, &v6);
+                A.dval[((size_t)z * m + y) * A.dpitch + x] = half_lerp(v0, v6);
+            }
+        }
+        const uint32_t mask = __ballot_sync(FULL, end);
+        if (mask) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(A.nends, (uint32_t)__popc(mask));
+            base = __shfl_sync(FULL, base, 0);
+            if (end) A.ends[base + __popc(mask & ((1u << lane) - 1u))] = id;
+        }
+    }
+}
+
+// A full field (every value sampled): one warp per 32 dual vertices of a dual
+// row (x = 32 w + lane): value, centre, sign word (by ballot) and the active
+// primal cells.
 __global__ void __launch_bounds__(256) dc_dual(DualArgs A) {
     const uint32_t m = A.n - 1, lane = threadIdx.x & 31;
     const uint64_t gw = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -80,34 +248,23 @@ __global__ void __launch_bounds__(256) dc_dual(DualArgs A) {
                             sign_bit(x, y + 1, z) << 3 | sign_bit(x, y, z + 1) << 4 |
                             sign_bit(x + 1, y, z + 1) << 5 | sign_bit(x + 1, y + 1, z + 1) << 6 |
                             sign_bit(x, y + 1, z + 1) << 7;
-        const float* f0 = A.field + ((size_t)z * A.n + y) * A.pitch + x;
-        const float v0 = __ldg(f0), v6 = __ldg(f0 + (size_t)A.n * A.pitch + A.pitch + 1);
-        const uint64_t id = ((uint64_t)z * m + y) * m + x;
-        const bool sampled = v0 == v0 && v6 == v6;
-        if (sampled || !A.near) {
-            // Vec3::lerp / Signed::lerp with f = 0.5: (1 - f) * a + f * b (a
-            // full field's own NaN gets a signed sentinel in its place)
-            const float of = 1.0f - 0.5f;
-            const float c0x = (float)x * A.inv, c0y = (float)y * A.inv, c0z = (float)(z + A.zoff) * A.inv;
-            const float c6x = (float)(x + 1) * A.inv, c6y = (float)(y + 1) * A.inv,
-                        c6z = (float)(z + 1 + A.zoff) * A.inv;
-            const float dv = sampled ? of * v0 + 0.5f * v6 : ((cs & 1u) ? -3.0e38f : 3.0e38f);
-            A.dpos[id] = make_float4(of * c0x + 0.5f * c6x, of * c0y + 0.5f * c6y, of * c0z + 0.5f * c6z, 0.0f);
-            A.dval[((size_t)z * m + y) * A.dpitch + x] = dv;
-            inside = !(dv > 0.0f);
-        } else {
-            inside = (cs & 1u) != 0;
-        }
+        float v0, v6;
+        dual_corners(A, x, y, z, &v0, &v6);
+        // the field's own NaN gets a signed sentinel in its place
+        const float dv = v0 == v0 && v6 == v6 ? half_lerp(v0, v6) : ((cs & 1u) ? -3.0e38f : 3.0e38f);
+        A.dpos[((uint64_t)z * m + y) * m + x] = dual_centre(A, x, y, z);
+        A.dval[((size_t)z * m + y) * A.dpitch + x] = dv;
+        inside = !(dv > 0.0f);
         active = cs != 0 && cs != 255;
     }
-    const uint32_t word = __ballot_sync(0xFFFFFFFFu, inside);
+    const uint32_t word = __ballot_sync(FULL, inside);
     if (lane == 0) A.dbits[row * A.dW + w] = word;
     // warp-aggregated append of the active cells (their order does not matter)
-    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, active);
+    const uint32_t mask = __ballot_sync(FULL, active);
     if (mask) {
         uint32_t base = 0;
         if (lane == (uint32_t)__ffs(mask) - 1) base = atomicAdd(A.count, (uint32_t)__popc(mask));
-        base = __shfl_sync(0xFFFFFFFFu, base, __ffs(mask) - 1);
+        base = __shfl_sync(FULL, base, __ffs(mask) - 1);
         if (active) {
             const uint32_t at = base + __popc(mask & ((1u << lane) - 1u));
             if (at < A.cap) A.list[at] = (uint32_t)(((uint64_t)z * m + y) * m + x);
@@ -192,63 +349,91 @@ static iso_status dc_lattice(iso_ctx* ctx, const iso_program* prog, uint32_t n, 
     const uint64_t ndual = (uint64_t)m * m * nzd;
     const uint64_t dpitch = default_pitch(m), dW = words_per_row(m);
     iso_status s;
-    // primal field + bits | dual values | dual positions | dual bits | active list
+    // primal field + bits | dual values | dual positions | dual bits, active
+    // bits, counts, active list, end list, features' normals
     if ((s = ensure(ctx, ctx->field, 4ull * pitch * n * nzp)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->bits, 4ull * W * n * nzp)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->aux, 4ull * dpitch * m * nzd)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->aux2, 16ull * ndual)) != ISO_OK) return s;
-    const uint64_t list_words = (ndual + 63) & ~(uint64_t)63;
+    const uint64_t list_words = (ndual + 63) & ~(uint64_t)63, dwords = (dW * m * nzd + 63) & ~(uint64_t)63;
     // normals kept for the first feature cells (96 bytes each, at most 96 MB)
     const uint32_t fcap = (uint32_t)std::min<uint64_t>(list_words, 1u << 20);
-    if ((s = ensure(ctx, ctx->aux3, 4ull * dW * m * nzd + 8ull * list_words + 256 + 96ull * fcap)) != ISO_OK)
-        return s;
+    if ((s = ensure(ctx, ctx->aux3, 8ull * dwords + 8ull * list_words + 256 + 96ull * fcap)) != ISO_OK) return s;
     float* field = (float*)ctx->field.p;
     uint32_t* bits = (uint32_t*)ctx->bits.p;
     float* dval = (float*)ctx->aux.p;
     float4* dpos = (float4*)ctx->aux2.p;
     uint32_t* dbits = (uint32_t*)ctx->aux3.p;
-    uint32_t* count = dbits + dW * m * nzd;  // active cells, then (count + 1) non-planar ones
+    uint32_t* abits = dbits + dwords;
+    uint32_t* count = abits + dwords;  // active cells, then those at crossing edges, then the non-planar ones
     uint32_t* list = count + 64;
-    uint32_t* features = list + list_words;
-    qef::F3* fnormals = reinterpret_cast<qef::F3*>(features + list_words);
+    uint32_t* ends = list + list_words;
+    qef::F3* fnormals = reinterpret_cast<qef::F3*>(ends + list_words);
     const float inv = 1.0f / (float)(n - 1);
     // values only near the surface (programs with a Lipschitz bound): the
     // dual values read the primal ones up to 1 + sqrt(3)/2 lattice steps'
     // worth of change from zero (a dual crossing end within one step's
     // worth, and half the cell diagonal between its two corners); the
-    // sampler keeps 2.5, and the others stay NaN for dc_dual to recognise
-    const bool near = prog->lip > 0.0f;
-    cudaError_t e = cudaSuccess;
-    if (near) e = cudaMemsetAsync(field, 0xFF, 4ull * pitch * n * nzp, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "clear field");
+    // sampler keeps 2.5
+    const bool near = prog->lip > 0.0f && !prog->tiny;
     if ((s = launch_sample_grid(ctx, prog, n, n, nzp, inv, field, pitch, bits, near, zlo, 2.5f)) != ISO_OK) return s;
-    e = cudaMemsetAsync(count, 0, 8, ctx->stream);
+    cudaError_t e = cudaMemsetAsync(count, 0, 12, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "memset");
-    {
-        StageTimer timer(ctx, ISO_STAGE_PLACE);
-        DualArgs da{field, bits, (uint32_t)W, pitch, n, nzd, zlo, inv, dval, dpitch, dpos, dbits, (uint32_t)dW,
-                    list, count, (uint32_t)ndual, ctx->d_err, near};
+    const uint64_t sms = (uint64_t)std::max(ctx->sms, 1);
+    DualArgs da{field, bits, (uint32_t)W, pitch, n, nzd, zlo, inv, dval, dpitch, dpos, dbits, abits, (uint32_t)dW,
+                list, count, ends, count + 1, (uint32_t)ndual, ctx->d_err, 1};
+    // the cells to place; the features' list takes the place of the one the placement does not read
+    DcCells cells{n, zlo, inv, ends, count + 1, reinterpret_cast<DcPos*>(dpos), (int)placer, list, count + 2, fnormals,
+                  fcap};
+    StageTimer timer(ctx, ISO_STAGE_PLACE);
+    if (near) {
+        const uint64_t SL = (dW * m + 31) / 32;
+        // as mc_cell_count: long runs share sign words, short ones keep the warps many
+        da.run = (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, SL * nzd / (160 * sms)));
+        const uint64_t warps = SL * ((nzd + da.run - 1) / da.run);
+        dc_signs<<<(unsigned)((warps + 7) / 8), 256, 0, ctx->stream>>>(da);
+        dc_edges<<<(unsigned)std::min<uint64_t>((ndual + 255) / 256, 8 * sms), 256, 0, ctx->stream>>>(da);
+        ctx->launches++;
+    } else {
         const uint64_t dual_warps = dW * m * nzd;
         dc_dual<<<(unsigned)((dual_warps + 7) / 8), 256, 0, ctx->stream>>>(da);
-        const DcCells cells{n, zlo, inv, list, count, reinterpret_cast<DcPos*>(dpos), (int)placer, features,
-                            count + 1, fnormals, fcap};
-        const VmHermite ev{prog->view()};
-        const uint64_t place_blocks = std::min<uint64_t>((ndual + 127) / 128, 152 * 64);
-        cudaError_t je = cudaSuccess;
-        if (!jit_dc_place(ctx, prog, cells, place_blocks, &je))  // the program's compiled normals (jit.cu)
-            dc_place<<<(unsigned)place_blocks, 128, 0, ctx->stream>>>(ev, cells);
-        else if (je != cudaSuccess)
-            return cuda_fail(ctx, je, "compiled dc_place launch");
-        if (placer == 0) {
-            // one warp for each of the SMs' four sub-partitions
-            dc_feature<<<(unsigned)(4 * std::max(ctx->sms, 1)), 32, 0, ctx->stream>>>(ev, cells, ctx->d_err);
-            ctx->launches++;
-        }
+        cells.list = list;
+        cells.count = count;
+        cells.features = ends;
+    }
+    // placement on the side stream: only the mesh's vertices wait for it
+    // (count and scan of a 256^3 lattice, 17 us, run beside it)
+    cudaStream_t side;
+    if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
+    const VmHermite ev{prog->view()};
+    const uint64_t place_blocks = std::min<uint64_t>((ndual + 127) / 128, 152 * 64);
+    cudaError_t je = cudaSuccess;
+    if (!jit_dc_place(side, prog, cells, place_blocks, &je))  // the program's compiled normals (jit.cu)
+        dc_place<<<(unsigned)place_blocks, 128, 0, side>>>(ev, cells);
+    if (placer == 0 && je == cudaSuccess) {
+        // one warp for each of the SMs' four sub-partitions
+        dc_feature<<<(unsigned)(4 * sms), 32, 0, side>>>(ev, cells, ctx->d_err);
+        ctx->launches++;
     }
     ctx->launches += 2;
-    if ((s = check_launch(ctx, "dc passes")) != ISO_OK) return s;
+    if (je != cudaSuccess || (s = check_launch(ctx, "dc passes")) != ISO_OK) {
+        join_side(ctx);
+        return je != cudaSuccess ? cuda_fail(ctx, je, "compiled dc_place launch") : s;
+    }
     *L = Lattice{m, m, nzd, dpitch, dval, dbits, (uint32_t)dW, 0.0f, dpos, zlo};
+    L->join = true;
     return ISO_OK;
+}
+
+// marching cubes over the dual lattice; the side stream's placement is always
+// joined, also when the passes end early
+static iso_status dc_mesh(iso_ctx* ctx, const Lattice& L, uint32_t flags, iso_mesh_info* info) {
+    const iso_status s = mc_extract_lattice(ctx, L, flags, info);
+    if (ctx->side_open) {
+        const iso_status j = join_side(ctx);
+        if (s == ISO_OK) return j;
+    }
+    return s;
 }
 
 static iso_status dc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32_t size, uint32_t placer,
@@ -261,7 +446,7 @@ static iso_status dc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32_
     }
     Lattice L;
     if ((s = dc_lattice(ctx, prog, size, placer, 0, size, &L)) != ISO_OK) return s;
-    return mc_extract_lattice(ctx, L, flags, info);
+    return dc_mesh(ctx, L, flags, info);
 }
 
 // One slab of a z-partition of DualContouring::new(size): dual cube layers
@@ -279,8 +464,11 @@ extern "C" iso_status iso_dc_extract_slab(iso_ctx* ctx, const iso_program* prog,
     Lattice L;
     if ((s = dc_lattice(ctx, prog, size, placer, zlo, z_end - zlo + 1, &L)) != ISO_OK) return s;
     uint64_t hv = 0, ht = 0;
-    if (halo && (s = mc_first_layer_counts(ctx, L, &hv, &ht)) != ISO_OK) return s;
-    if ((s = mc_extract_lattice(ctx, L, flags, info)) != ISO_OK) return s;
+    if (halo && (s = mc_first_layer_counts(ctx, L, &hv, &ht)) != ISO_OK) {
+        join_side(ctx);
+        return s;
+    }
+    if ((s = dc_mesh(ctx, L, flags, info)) != ISO_OK) return s;
     if (halo_vertices) *halo_vertices = hv;
     if (halo_triangles) *halo_triangles = ht;
     return ISO_OK;

@@ -314,9 +314,9 @@ __host__ __device__ inline qef::F3 minimise_qef_n(const PlanesN& t, bool* ok) {
         u[i][2] = (double)t.normal[i].z;
     }
     double tau_v[2] = {0.0, 0.0};
-    bidiagonalise<12>(u, d, tau_v, t.n);
+    bidiagonalise(u, d, tau_v, t.n);
     unpack(u, v, d, tau_v, t.n);
-    *ok = diagonalise<12>(u, v, d, tau_v, t.n);
+    *ok = diagonalise(u, v, d, tau_v, t.n);
     singularise(u, v, d, t.n);
     if (t.feature == EDGE) {
         double s_min = 1.7976931348623157e308;

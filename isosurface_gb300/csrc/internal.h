@@ -100,6 +100,7 @@ struct iso_ctx {
     // first use) and the events that fork it from and join it to that stream
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    bool side_open = false;  // forked and not joined yet
     // page-locked host buffers (device-side pointers) that the MarchingCubes
     // kernels fill alongside the device mesh (iso_mc_extract_host); `armed`
     // reports whether the last lattice pass could deliver there
@@ -182,6 +183,10 @@ struct iso_program {
     float4* d_prims = nullptr;
     int32_t prim_dom_at = -1;
     float lip = 0.0f, slack = 0.0f;  // see ProgView
+    // some constant is nonzero and below 1e-18: only then can a value come
+    // out next to zero by a few units of f32's smallest step (differences of
+    // ordinary numbers are multiples of their own last places)
+    bool tiny = false;
     size_t block_bytes = 0;          // capacity of d_block
     uint64_t content_hash = 0;       // FNV-1a of the program bytes
     uint64_t uid = 0;  // unique per program created in this process
@@ -236,6 +241,7 @@ struct Lattice {
     float inv;               // point position = (x*inv, y*inv, z*inv)
     const float4* positions; // DC: explicit xyz per point (w unused); null = regular grid
     uint32_t zoff = 0;       // regular grid: lattice z of layer 0 (a slab of a larger grid)
+    bool join = false;       // the side stream still writes positions: the emission waits for it
 };
 iso_status mc_extract_lattice(iso_ctx* ctx, const Lattice& L, uint32_t flags, iso_mesh_info* info);
 iso_status mc_extract_slab(iso_ctx* ctx, const iso_program* prog, uint32_t size, uint32_t z_begin, uint32_t z_end,

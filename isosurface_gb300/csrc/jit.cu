@@ -437,12 +437,13 @@ bool jit_sample_bricks(iso_ctx* ctx, const iso_program* prog, const GridTiles& t
     return true;
 }
 
-bool jit_dc_place(iso_ctx* ctx, const iso_program* prog, const DcCells& cells, uint64_t blocks, cudaError_t* err) {
+bool jit_dc_place(cudaStream_t stream, const iso_program* prog, const DcCells& cells, uint64_t blocks,
+                  cudaError_t* err) {
     Module* m = module_for(prog);
     if (!m || !m->dc_place) return false;
     DcCells a = cells;
     void* args[] = {&a};
-    *err = cudaLaunchKernel((const void*)m->dc_place, dim3((unsigned)blocks), dim3(128), args, 0, ctx->stream);
+    *err = cudaLaunchKernel((const void*)m->dc_place, dim3((unsigned)blocks), dim3(128), args, 0, stream);
     return true;
 }
 

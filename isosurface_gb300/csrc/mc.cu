@@ -721,6 +721,10 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
         if (keys) cap_v = std::min<uint64_t>(cap_v, ctx->mesh_k.bytes / 16);
         const iso_ctx::HostOut& H = ctx->host_out;
         uint64_t* out_k = keys ? (uint64_t*)ctx->mesh_k.p : nullptr;
+        if (L.join && ctx->side_open) {
+            const iso_status js = join_side(ctx);
+            if (js != ISO_OK) return js;
+        }
         {
             StageTimer timer(ctx, ISO_STAGE_EMIT);
             if (cells) {

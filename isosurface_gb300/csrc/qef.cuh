@@ -42,12 +42,11 @@ __host__ __device__ inline double householder(double** x, int n) {
             for (int i = 1; i < n; ++i) {
                 const double v = fabs(*x[i]);
                 if (v != 0.0) {
-                    if (scl < v) {
-                        ssq = 1.0 + ssq * (scl / v) * (scl / v);
-                        scl = v;
-                    } else {
-                        ssq += v / scl * (v / scl);
-                    }
+                    // one division for either branch: a warp's lanes take both
+                    const bool grow = scl < v;
+                    const double r = (grow ? scl : v) / (grow ? v : scl);
+                    ssq = grow ? 1.0 + ssq * r * r : ssq + r * r;
+                    scl = grow ? v : scl;
                 }
             }
             xnorm = scl * sqrt(ssq);
@@ -161,16 +160,15 @@ __host__ __device__ inline void givens(double a, double b, double* c, double* s)
     if (b == 0.0) {
         *c = 1.0;
         *s = 0.0;
-    } else if (fabs(b) > fabs(a)) {
-        const double t = -a / b;
-        const double s1 = 1.0 / sqrt(1.0 + t * t);
-        *s = s1;
-        *c = s1 * t;
     } else {
-        const double t = -b / a;
-        const double c1 = 1.0 / sqrt(1.0 + t * t);
-        *c = c1;
-        *s = c1 * t;
+        // the larger of the two divides; the divisions and the root are
+        // shared by both orders, as a warp's lanes take both
+        const bool big_b = fabs(b) > fabs(a);
+        const double t = (big_b ? -a : -b) / (big_b ? b : a);
+        const double r = 1.0 / sqrt(1.0 + t * t);
+        const double rt = r * t;
+        *c = big_b ? rt : r;
+        *s = big_b ? r : rt;
     }
 }
 
@@ -180,10 +178,10 @@ __host__ __device__ inline void schur(double a1, double a2, double a3, double* c
         *c = 1.0;
         *s = 0.0;
     } else {
-        double t;
         const double tau = (a2 * a2 + (a3 + a1) * (a3 - a1)) / apq;
-        if (tau >= 0.0) t = 1.0 / (tau + sqrt(1.0 + tau * tau));
-        else t = -1.0 / (sqrt(1.0 + tau * tau) - tau);
+        const double root = sqrt(1.0 + tau * tau);
+        const bool up = tau >= 0.0;
+        const double t = (up ? 1.0 : -1.0) / (up ? tau + root : root - tau);
         *c = 1.0 / sqrt(1.0 + t * t);
         *s = t * *c;
     }
@@ -242,8 +240,10 @@ __host__ __device__ inline double shift(const double* tau_u, const double* tau_v
     const double tb = tau_u[2] * tau_u[2] + tau_v[1] * tau_v[1];
     const double tab = tau_u[1] * tau_v[1];
     const double dt = (ta - tb) / 2.0;
-    if (dt >= 0.0) return tb - tab * tab / (dt + sqrt(dt * dt + tab * tab));
-    return tb + tab * tab / (sqrt(dt * dt + tab * tab) - dt);
+    const double root = sqrt(dt * dt + tab * tab);
+    const bool up = dt >= 0.0;
+    const double q = tab * tab / (up ? dt + root : root - dt);
+    return up ? tb - q : tb + q;
 }
 
 __host__ __device__ inline void qr_cols2(double (*u)[3], double (*v)[3], double* tau_u, double* tau_v, int rows) {
@@ -353,7 +353,6 @@ __host__ __device__ inline void qr_step(double (*u)[3], double (*v)[3], double* 
 }
 
 // returns false when the sweep bound was reached
-template <int R = 8>
 __host__ __device__ inline bool diagonalise(double (*u)[3], double (*v)[3], double* tau_u, double* tau_v, int rows) {
     chop(tau_u, tau_v, 3);
     int b = 2;
@@ -366,18 +365,10 @@ __host__ __device__ inline bool diagonalise(double (*u)[3], double (*v)[3], doub
             int a = b - 1;
             while (a > 0 && tau_v[a - 1] != 0.0) a -= 1;
             const int n = b - a + 1;
-            double u1[R][3], v1[3][3];
-            for (int i = 0; i < rows; ++i) u1[i][0] = u1[i][1] = u1[i][2] = 0.0;
-            for (int i = 0; i < 3; ++i) v1[i][0] = v1[i][1] = v1[i][2] = 0.0;
-            for (int j = a; j <= b; ++j) {
-                for (int i = 0; i < rows; ++i) u1[i][j - a] = u[i][j];
-                for (int i = 0; i < 3; ++i) v1[i][j - a] = v[i][j];
-            }
-            qr_step(u1, v1, tau_u + a, tau_v + a, rows, n);
-            for (int j = a; j <= b; ++j) {
-                for (int i = 0; i < rows; ++i) u[i][j] = u1[i][j - a];
-                for (int i = 0; i < 3; ++i) v[i][j] = v1[i][j - a];
-            }
+            // columns a..b in place: rows are three apart, so the sub-matrix
+            // that starts at column a is addressed from there
+            qr_step(reinterpret_cast<double (*)[3]>(&u[0][a]), reinterpret_cast<double (*)[3]>(&v[0][a]), tau_u + a,
+                    tau_v + a, rows, n);
             chop(tau_u + a, tau_v + a, n);
         }
     }
