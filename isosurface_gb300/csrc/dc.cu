@@ -290,7 +290,11 @@ __global__ void __launch_bounds__(128) dc_place(VmHermite ev, DcCells A) { dc_pl
 // (the SVD, in the reference's order), and a warp's f64 instruction holds
 // its sub-partition's f64 unit for many cycles however few of its lanes are
 // active, so packing the chains into full warps cuts the f64 instructions
-// the scattered cells of dc_place would have issued.
+// the scattered cells of dc_place would have issued.  (Spread evenly over the
+// sub-partitions below 32 cells for each it was no faster alone, 129 us
+// against 121 for the 257 lattice, and slower beside the counting passes.)
+// The chain of one warp is the whole time: its matrices in registers took it
+// from 138 us to 121 (qef.cuh).
 __global__ void __launch_bounds__(32) dc_feature(VmHermite ev, DcCells A, uint32_t* err) {
     const uint32_t n = *A.nfeatures;
     for (uint32_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += gridDim.x * 32) {

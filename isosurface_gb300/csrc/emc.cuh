@@ -307,45 +307,10 @@ __host__ __device__ inline qef::F3 minimise_qef_n(const PlanesN& t, bool* ok) {
     using namespace qef;
     *ok = true;
     if (t.feature == PLANAR) return t.com;
-    double u[12][3], v[3][3], d[3] = {0.0, 0.0, 0.0};
-    for (int i = 0; i < t.n; ++i) {
-        u[i][0] = (double)t.normal[i].x;
-        u[i][1] = (double)t.normal[i].y;
-        u[i][2] = (double)t.normal[i].z;
-    }
-    double tau_v[2] = {0.0, 0.0};
-    bidiagonalise(u, d, tau_v, t.n);
-    unpack(u, v, d, tau_v, t.n);
-    *ok = diagonalise(u, v, d, tau_v, t.n);
-    singularise(u, v, d, t.n);
-    if (t.feature == EDGE) {
-        double s_min = 1.7976931348623157e308;
-        int id = 0;
-        for (int i = 0; i < 3; ++i)
-            if (d[i] < s_min) {
-                s_min = d[i];
-                id = i;
-            }
-        d[id] = 0.0;
-    }
-    if (d[2] < 0.1) d[2] = 0.0;
-    if (d[1] < 0.1) d[1] = 0.0;
-    if (d[0] < 0.1) d[0] = 0.0;
-    double w[3] = {0.0, 0.0, 0.0};
-    for (int i = 0; i < t.n; ++i) {
-        const double b = (double)t.d[i];
-        if (b != 0.0)
-            for (int j = 0; j < 3; ++j) w[j] += b * u[i][j];
-    }
-    for (int i = 0; i < 3; ++i)
-        if (d[i] != 0.0) w[i] /= d[i];
-    double x[3];
-    for (int i = 0; i < 3; ++i) {
-        double s = 0.0;
-        for (int j = 0; j < 3; ++j) s += w[j] * v[i][j];
-        x[i] = s;
-    }
-    return add(t.com, f3((float)x[0], (float)x[1], (float)x[2]));
+    // a surface that is nearly flat in a cell crosses at most six edges
+    const F3 x = t.n <= 6 ? solve_planes<6>(t.normal, t.d, t.n, t.feature == EDGE, ok)
+                          : solve_planes<12>(t.normal, t.d, t.n, t.feature == EDGE, ok);
+    return add(t.com, x);
 }
 
 // The tangent planes of an active cell: the normal (sample_normal,
