@@ -5,15 +5,21 @@
 // to size the mesh.
 //
 //   emc_sample     Directed value of every lattice point (float4 per point)
-//   emc_active     case of every cell; the cells with corners on both sides
-//                  go to a list, which the later passes walk instead of the grid
-//   emc_count      feature decision, vertex and triangle counts per active
-//                  cell; the feature cells go to a second list
-//   scan_u32 x 2   first vertex and first triangle of every cell
+//                  and one sign bit per point
+//   emc_active     case of every cell, from the sign bits; the cells with
+//                  corners on both sides go to a list, which the later passes
+//                  walk instead of the grid
+//   emc_count      feature decision per active cell; vertices and triangles
+//                  of every block of 1024 cells; the feature cells go to a
+//                  second list with their tangent planes
+//   emc_features   the feature points (MinimiseQEF), a few cells per warp, on
+//                  a side stream beside everything below but the last pass
+//   emc_scan       first vertex and first triangle of every block
+//   emc_offsets    those of every active cell
 //   emc_vertices   owned edge vertices; the edge map
-//   emc_features   the feature points (MinimiseQEF), a few cells per warp
 //   emc_triangles  marching-cubes triangles and fans, in traversal order
 //   emc_flips      feature-edge rotations
+//   emc_points     the feature points to their places among the vertices
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,88 +40,269 @@
 namespace iso {
 namespace {
 
-__global__ void __launch_bounds__(256) emc_sample(emc::Args A, uint64_t points) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < points; i += (uint64_t)gridDim.x * blockDim.x)
-        emc::sample_item(A, i);
+constexpr uint32_t BLOCK_CELLS = 1024;  // cells with one entry in the scan
+// feature cells whose tangent planes and points are kept, per lattice line:
+// sharp edges are curves, so their cells grow with the size, not its square
+constexpr uint32_t FEATURES_PER_LINE = 48;
+
+// emc_count's result for a feature cell, and emc_features'
+struct Feature {
+    emc::PlanesN planes;
+    qef::F3 point;
+};
+
+// device counters of one extraction
+struct Ctrl {
+    uint32_t active, features;
+    uint32_t vertices, triangles;
+    unsigned long long flips;
+};
+
+// sign bit i & 31 of word i >> 5: lattice point i is inside
+__global__ void __launch_bounds__(256) emc_sample(emc::Args A, uint32_t points, uint32_t* bits) {
+    for (uint32_t i0 = blockIdx.x * 256; i0 < points; i0 += gridDim.x * 256) {
+        const uint32_t i = i0 + threadIdx.x;
+        const uint32_t word = __ballot_sync(0xFFFFFFFFu, i < points && emc::sample_item(A, i));
+        if ((threadIdx.x & 31) == 0) bits[i >> 5] = word;
+    }
 }
 
-// Every cell's case; the cells with corners on both sides (the only ones
-// with work in the later passes) are appended to `list` in any order, the
-// others get their case and zero counts here.
-__global__ void __launch_bounds__(256) emc_active(emc::Args A, uint64_t cells, uint32_t* list, uint32_t* count) {
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint64_t c0 = (uint64_t)blockIdx.x * blockDim.x; c0 < cells; c0 += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = c0 + threadIdx.x;
+// Every cell's case, from two neighbouring sign bits in each of its four rows
+// (reading the eight values themselves was 16 times the bytes); the cells
+// with corners on both sides (the only ones with work in the later passes)
+// are appended to `list` in any order.
+__global__ void __launch_bounds__(256) emc_active(emc::Args A, uint32_t cells, const uint32_t* bits, uint32_t* list,
+                                                  Ctrl* ctrl) {
+    const uint32_t lane = threadIdx.x & 31, n = A.g.n;
+    for (uint32_t c0 = blockIdx.x * 256; c0 < cells; c0 += gridDim.x * 256) {
+        const uint32_t c = c0 + threadIdx.x;
         bool active = false;
         if (c < cells) {
             uint32_t x, y, z;
-            emc::cell_xyz(A.g.n, c, &x, &y, &z);
-            V3 corners[8], values[8];
-            emc::load_cell(A.field, A.g, x, y, z, corners, values);
-            const int cube = emc::classify_directed(values);
+            emc::cell_xyz(n, c, &x, &y, &z);
+            // points i and i + 1; the word after the last one is allocated
+            auto pair = [&](uint32_t i) {
+                const uint32_t* w = bits + (i >> 5);
+                return __funnelshift_r(__ldg(w), __ldg(w + 1), i & 31) & 3u;
+            };
+            const uint32_t p = (z * n + y) * n + x;
+            const uint32_t a = pair(p), b = pair(p + n), d = pair(p + n * n), e = pair(p + n * n + n);
+            // corners 0-1-2-3 go round a face (marching_cubes_tables.rs:16-25)
+            const uint32_t cube = a | (b & 2u) << 1 | (b & 1u) << 3 | d << 4 | (e & 2u) << 5 | (e & 1u) << 7;
             active = cube != 0 && cube != 255;
-            if (!active) {
-                A.cell[c] = (uint16_t)cube;
-                A.voff[c] = 0;
-                A.toff[c] = 0;
-            }
+            A.cell[c] = (uint16_t)cube;
         }
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, active);
         if (m) {
             const uint32_t leader = (uint32_t)__ffs(m) - 1;
             uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(m));
+            if (lane == leader) base = atomicAdd(&ctrl->active, (uint32_t)__popc(m));
             base = __shfl_sync(0xFFFFFFFFu, base, leader);
-            if (active) list[base + __popc(m & ((1u << lane) - 1u))] = (uint32_t)c;
+            if (active) list[base + __popc(m & ((1u << lane) - 1u))] = c;
         }
     }
 }
 
-// The per-cell passes over the active cells only (one thread per cell,
-// grid-stride).  The counting pass also lists the feature cells.
-__global__ void __launch_bounds__(128) emc_count(emc::Args A, const uint32_t* list, const uint32_t* count,
-                                                 uint32_t* features, uint32_t* nfeatures) {
-    const uint32_t n = *count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = list[i];
-        emc::count_item(A, c);
-        if ((A.cell[c] >> 8) & 1) features[atomicAdd(nfeatures, 1u)] = c;
+// The feature decision of every active cell, four lanes to a cell: the
+// program's normal at a crossing is the long chain here, a cell has three to
+// twelve of them and there are too few active cells to hide it, so each lane
+// takes every fourth crossing (one thread per cell, with its crossings in
+// local memory, took 58 us for a solid at 128).
+__global__ void __launch_bounds__(128) emc_count(emc::Args A, const uint32_t* list, Ctrl* ctrl, uint32_t* features,
+                                                 Feature* kept, uint32_t cap, unsigned long long* sums) {
+    __shared__ qef::F3 vtx[32][12], nrm[32][12];
+    const uint32_t n = ctrl->active, sub = threadIdx.x & 3, g = threadIdx.x >> 2;
+    for (uint32_t i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {
+        const uint32_t i = i0 + g;
+        const bool live = i < n;
+        uint32_t c = 0, x = 0, y = 0, z = 0;
+        int cube = 0, count = 0;
+        if (live) {
+            c = list[i];
+            cube = A.cell[c];
+            emc::cell_xyz(A.g.n, c, &x, &y, &z);
+            const uint32_t mask = iso_edge_mask[cube];
+            count = __popc(mask);
+            uint32_t rest = mask;
+            for (int k = 0; k < count; ++k, rest &= rest - 1) {
+                if ((k & 3) != (int)sub) continue;
+                const V3 p = emc::edge_crossing(A, x, y, z, __ffs(rest) - 1);
+                V3 nn;
+                eval_hermite(A.prog, p, &nn);
+                vtx[g][k] = qef::f3(p.x, p.y, p.z);
+                nrm[g][k] = qef::normalised_or_zero(qef::f3(nn.x, nn.y, nn.z));
+            }
+        }
+        __syncwarp();
+        // TangentPlanes (tangent_planes_n): the pair of normals with the
+        // smallest product, the first in (i, j) order of equals, each lane
+        // over a quarter of the rows i
+        float least = emc::F32_MAX;
+        uint32_t pair = ~0u;
+        for (int r = (int)sub; r < count; r += 4)
+            for (int k = 0; k < count; ++k) {
+                const float angle = qef::dot(nrm[g][r], nrm[g][k]);
+                if (angle < least) {
+                    least = angle;
+                    pair = (uint32_t)(16 * r + k);
+                }
+            }
+        for (uint32_t o = 1; o < 4; o <<= 1) {
+            const float a2 = __shfl_xor_sync(0xFFFFFFFFu, least, o);
+            const uint32_t p2 = __shfl_xor_sync(0xFFFFFFFFu, pair, o);
+            if (a2 < least || (a2 == least && p2 < pair)) {
+                least = a2;
+                pair = p2;
+            }
+        }
+        if (live && sub == 0) {
+            const uint32_t feature = !(least > qef::FEATURE_ANGLE);
+            uint32_t nv, nt;
+            emc::cell_counts(x, y, z, cube, feature, &nv, &nt);
+            atomicAdd(sums + c / BLOCK_CELLS, (unsigned long long)nt << 32 | nv);
+            if (feature) {
+                A.cell[c] = (uint16_t)(cube | 256);
+                const uint32_t at = atomicAdd(&ctrl->features, 1u);
+                features[at] = c;
+                if (at < cap) {
+                    const qef::F3 axis = pair == ~0u ? qef::f3(0.0f, 0.0f, 0.0f)
+                                                     : qef::cross(nrm[g][pair >> 4], nrm[g][pair & 15]);
+                    emc::planes_about(vtx[g], nrm[g], count, least, axis, &kept[at].planes);
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Exclusive scan of the blocks' sums in place (triangles in the high half),
+// by one thread block, four entries per thread and turn.
+__global__ void __launch_bounds__(1024) emc_scan(unsigned long long* sums, uint32_t nblocks, Ctrl* ctrl) {
+    __shared__ unsigned long long part[32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (uint32_t b0 = 0; b0 < nblocks; b0 += 4096) {
+        const uint32_t at = b0 + 4 * threadIdx.x;
+        unsigned long long v[4], mine = 0;
+        for (uint32_t k = 0; k < 4; ++k) {
+            v[k] = at + k < nblocks ? sums[at + k] : 0;
+            mine += v[k];
+        }
+        unsigned long long incl = mine;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) part[w] = incl;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
+        for (uint32_t k = 0; k < 32; ++k) {
+            if (k < w) before += part[k];
+            all += part[k];
+        }
+        unsigned long long run = carry + before + incl - mine;
+        for (uint32_t k = 0; k < 4; ++k) {
+            // a block without active cells keeps its mark: emc_offsets skips it
+            if (at + k < nblocks) sums[at + k] = v[k] ? run : ~0ull;
+            run += v[k];
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        ctrl->vertices = (uint32_t)carry;
+        ctrl->triangles = (uint32_t)(carry >> 32);
+    }
+}
+
+// First vertex and first triangle of every active cell (nothing reads those
+// of the others): a thread block per block of cells, four cells per thread.
+__global__ void __launch_bounds__(256) emc_offsets(emc::Args A, uint32_t cells, const unsigned long long* sums) {
+    __shared__ unsigned long long part[8];
+    const unsigned long long base = sums[blockIdx.x];
+    if (base == ~0ull) return;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t c0 = blockIdx.x * BLOCK_CELLS + 4 * threadIdx.x;
+    unsigned long long v[4], mine = 0;
+    for (uint32_t k = 0; k < 4; ++k) {
+        v[k] = 0;
+        if (c0 + k >= cells) continue;
+        const uint32_t info = A.cell[c0 + k];
+        const int cube = (int)(info & 255);
+        if (cube == 0 || cube == 255) continue;
+        uint32_t x, y, z, nv, nt;
+        emc::cell_xyz(A.g.n, c0 + k, &x, &y, &z);
+        emc::cell_counts(x, y, z, cube, info >> 8, &nv, &nt);
+        v[k] = (unsigned long long)nt << 32 | nv;
+        mine += v[k];
+    }
+    unsigned long long incl = mine;
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) part[w] = incl;
+    __syncthreads();
+    unsigned long long run = base + incl - mine;
+    for (uint32_t k = 0; k < w; ++k) run += part[k];
+    for (uint32_t k = 0; k < 4; ++k) {
+        if (v[k]) {
+            A.voff[c0 + k] = (uint32_t)run;
+            A.toff[c0 + k] = (uint32_t)(run >> 32);
+        }
+        run += v[k];
     }
 }
 
 // every vertex but the feature points
-__global__ void __launch_bounds__(128) emc_vertices(emc::Args A, const uint32_t* list, const uint32_t* count) {
-    const uint32_t n = *count;
+__global__ void __launch_bounds__(128) emc_vertices(emc::Args A, const uint32_t* list, const Ctrl* ctrl) {
+    const uint32_t n = ctrl->active;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         emc::vertex_item(A, list[i], false);
 }
 
-// The feature points: `per` listed feature cells to a one-warp block.  Each
-// is one serial chain of f64 operations (the SVD, in the reference's order),
-// and a warp's f64 instruction holds its sub-partition's f64 unit for many
-// cycles whatever its active lanes, so the chains go to as many warps as the
-// SMs' sub-partitions can take, each warp with a few, rather than scattered
-// over every warp of the vertex pass.
-__global__ void __launch_bounds__(32) emc_features(emc::Args A, const uint32_t* features, const uint32_t* nfeatures,
-                                                   uint32_t per) {
-    const uint32_t lane = threadIdx.x;
-    const uint64_t i = (uint64_t)blockIdx.x * per + lane;
-    if (lane < per && i < *nfeatures) emc::feature_item(A, features[i]);
+// The feature points of the kept feature cells.  Each is one serial chain of
+// f64 operations (the SVD, in the reference's order), and a warp's f64
+// instruction holds its sub-partition's f64 unit for many cycles whatever its
+// active lanes, so the chains go to as many warps as the SMs' sub-partitions
+// can take (the grid), each warp with a few, rather than scattered over every
+// warp of a pass over cells.  They start as soon as the cells are known.
+__global__ void __launch_bounds__(32) emc_features(emc::Args A, Feature* kept, uint32_t cap, const Ctrl* ctrl) {
+    const uint32_t n = min(ctrl->features, cap);
+    const uint32_t per = min(32u, (n + gridDim.x - 1) / gridDim.x);
+    if (threadIdx.x >= per) return;
+    for (uint32_t i = blockIdx.x * per + threadIdx.x; i < n; i += gridDim.x * per) {
+        bool ok;
+        const qef::F3 p = emc::minimise_qef_n(kept[i].planes, &ok);
+        if (!ok) atomicOr(A.err, DERR_SVD_ITER);
+        kept[i].point = p;
+    }
 }
 
-__global__ void __launch_bounds__(256) emc_triangles(emc::Args A, const uint32_t* list, const uint32_t* count) {
-    const uint32_t n = *count;
+// the feature points to the first vertex of their cells; those of the cells
+// that were not kept are found here
+__global__ void __launch_bounds__(32) emc_points(emc::Args A, const uint32_t* features, const Feature* kept, uint32_t cap,
+                                                 uint32_t n) {
+    for (uint32_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += gridDim.x * 32) {
+        const uint32_t c = features[i];
+        if (i < cap) emc::put_vertex(A, A.voff[c], kept[i].point);
+        else emc::feature_item(A, c);
+    }
+}
+
+__global__ void __launch_bounds__(256) emc_triangles(emc::Args A, const uint32_t* list, const Ctrl* ctrl) {
+    const uint32_t n = ctrl->active;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         emc::triangle_item(A, list[i]);
 }
 
-__global__ void __launch_bounds__(256) emc_flips(emc::Args A, const uint32_t* list, const uint32_t* count,
-                                                 unsigned long long* flips) {
-    const uint32_t n = *count;
+// a flip's first face is a feature cell's
+__global__ void __launch_bounds__(64) emc_flips(emc::Args A, const uint32_t* features, uint32_t n, Ctrl* ctrl) {
     uint32_t mine = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        mine += emc::flip_item(A, list[i]);
-    if (mine) atomicAdd(flips, (unsigned long long)mine);
+        mine += emc::flip_item(A, features[i]);
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&ctrl->flips, (unsigned long long)mine);
 }
 
 enum : uint32_t {
@@ -152,6 +339,42 @@ unsigned grid_for(const iso_ctx* ctx, uint64_t items, unsigned threads, unsigned
 
 using namespace iso;
 
+// everything after the scan; leaves the counters in h_pinned[0 .. 2]
+static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t nblocks, uint32_t cap,
+                           const uint32_t* active, const uint32_t* features, const Feature* kept, Ctrl* ctrl,
+                           const unsigned long long* sums) {
+    iso_status s;
+    cudaError_t e = cudaMemcpyAsync(ctx->h_pinned, ctrl, 16, cudaMemcpyDeviceToHost, ctx->stream);
+    emc_offsets<<<nblocks, 256, 0, ctx->stream>>>(A, (uint32_t)cells, sums);
+    ctx->launches++;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counts");
+    const Ctrl* h = (const Ctrl*)ctx->h_pinned;
+    const uint32_t nactive = h->active, nfeat = h->features;
+    if ((s = ensure(ctx, ctx->mesh_v, 12ull * h->vertices + 16)) != ISO_OK) return s;
+    if ((s = ensure(ctx, ctx->mesh_i, 12ull * h->triangles + 16)) != ISO_OK) return s;
+    A.vertices = (float*)ctx->mesh_v.p;
+    A.indices = (uint32_t*)ctx->mesh_i.p;
+    A.cap_v = h->vertices;
+    A.cap_t = h->triangles;
+    if (nactive) {
+        StageTimer timer(ctx, ISO_STAGE_EMIT);
+        emc_vertices<<<grid_for(ctx, nactive, 128, 32), 128, 0, ctx->stream>>>(A, active, ctrl);
+        emc_triangles<<<grid_for(ctx, nactive, 256, 16), 256, 0, ctx->stream>>>(A, active, ctrl);
+        ctx->launches += 2;
+        if (nfeat) {
+            emc_flips<<<grid_for(ctx, nfeat, 64, 32), 64, 0, ctx->stream>>>(A, features, nfeat, ctrl);
+            if ((s = join_side(ctx)) != ISO_OK) return s;
+            emc_points<<<grid_for(ctx, nfeat, 32, 32), 32, 0, ctx->stream>>>(A, features, kept, cap, nfeat);
+            ctx->launches += 2;
+        }
+    }
+    if ((s = check_launch(ctx, "emc emit")) != ISO_OK) return s;
+    e = cudaMemcpyAsync(ctx->h_pinned + 2, &ctrl->flips, 8, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "emc emit");
+}
+
 static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32_t size, iso_mesh_info* info,
                                    uint64_t* flips_out) {
     if (prog->ctx != ctx) return fail(ctx, ISO_ERR_INVALID_ARG, "program belongs to another context");
@@ -171,87 +394,62 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
     }
     const uint32_t n = size;
     const uint64_t points = emc::num_points(n), cells = emc::num_cells(n);
-    const uint32_t nsums = (uint32_t)((cells + 1023) / 1024);
-    // Directed field | case + feature per cell | vertex and triangle offsets,
-    // scan sums, totals, flip counter | edge map
+    const uint32_t nblocks = (uint32_t)((cells + BLOCK_CELLS - 1) / BLOCK_CELLS);
+    const uint32_t cap = (uint32_t)std::min<uint64_t>(cells, (uint64_t)FEATURES_PER_LINE * n);
+    const uint64_t bit_words = (((points + 31) / 32 + 1) + 63) & ~(uint64_t)63;
+    // Directed field | case + feature per cell | counters and the blocks'
+    // sums, vertex and triangle offsets | edge map
     if ((s = ensure(ctx, ctx->field, 16 * points)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->aux, 2 * cells)) != ISO_OK) return s;
-    const uint64_t off_words = 2 * cells, sum_words = 2ull * nsums;
-    if ((s = ensure(ctx, ctx->scan, 4 * (off_words + sum_words) + 64)) != ISO_OK) return s;
+    const size_t ctrl_bytes = sizeof(Ctrl) + 8ull * nblocks;
+    if ((s = ensure(ctx, ctx->scan, ctrl_bytes + 8 * cells)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->edges, 12 * points)) != ISO_OK) return s;
-    // the active cells, their count, the feature cells' count, the feature cells
+    // the active cells, the feature cells, sign bits, the kept features
     const uint64_t list_words = (cells + 63) & ~(uint64_t)63;
-    if ((s = ensure(ctx, ctx->aux2, 4 * (2 * list_words + 64))) != ISO_OK) return s;
+    if ((s = ensure(ctx, ctx->aux2, 4 * (2 * list_words + bit_words) + sizeof(Feature) * (uint64_t)cap)) != ISO_OK) return s;
     uint32_t* active = (uint32_t*)ctx->aux2.p;
-    uint32_t* nactive = active + list_words;
-    uint32_t* nfeatures = nactive + 1;
-    uint32_t* features = nactive + 64;
-    uint32_t* scan_base = (uint32_t*)ctx->scan.p;
-    uint32_t* sums = scan_base + off_words;
-    uint32_t* totals = sums + sum_words;  // vertices, triangles, then the flip counter (8-byte aligned)
-    unsigned long long* flips = (unsigned long long*)(totals + 2);
+    uint32_t* features = active + list_words;
+    uint32_t* bits = features + list_words;
+    Feature* kept = (Feature*)(bits + bit_words);
+    Ctrl* ctrl = (Ctrl*)ctx->scan.p;
+    unsigned long long* sums = (unsigned long long*)(ctrl + 1);
 
     emc::Args A{};
     A.prog = prog->view();
     A.g = emc::Grid{n, 1.0f / (float)(n - 1)};
     A.field = (float4*)ctx->field.p;
     A.cell = (uint16_t*)ctx->aux.p;
-    A.voff = scan_base;
-    A.toff = scan_base + cells;
+    A.voff = (uint32_t*)(sums + nblocks);
+    A.toff = A.voff + cells;
     A.edge_map = (uint32_t*)ctx->edges.p;
     A.err = ctx->d_err;
+    cudaError_t e = cudaMemsetAsync(ctrl, 0, ctrl_bytes, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counters");
     {
         StageTimer timer(ctx, ISO_STAGE_SAMPLE);
-        emc_sample<<<grid_for(ctx, points, 256, 16), 256, 0, ctx->stream>>>(A, points);
+        emc_sample<<<grid_for(ctx, points, 256, 16), 256, 0, ctx->stream>>>(A, (uint32_t)points, bits);
     }
+    cudaStream_t side;
     {
         StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
-        cudaError_t me = cudaMemsetAsync(nactive, 0, 8, ctx->stream);  // and nfeatures
-        if (me != cudaSuccess) return cuda_fail(ctx, me, "emc active count");
-        emc_active<<<grid_for(ctx, cells, 256, 16), 256, 0, ctx->stream>>>(A, cells, active, nactive);
-        emc_count<<<grid_for(ctx, cells, 128, 32), 128, 0, ctx->stream>>>(A, active, nactive, features, nfeatures);
+        emc_active<<<grid_for(ctx, cells, 256, 16), 256, 0, ctx->stream>>>(A, (uint32_t)cells, bits, active, ctrl);
+        emc_count<<<grid_for(ctx, cells, 32, 16), 128, 0, ctx->stream>>>(A, active, ctrl, features, kept, cap, sums);
         ctx->launches += 3;
         if ((s = check_launch(ctx, "emc count")) != ISO_OK) return s;
-        if ((s = scan_u32(ctx, A.voff, A.voff, (uint32_t)cells, sums, totals)) != ISO_OK) return s;
-        if ((s = scan_u32(ctx, A.toff, A.toff, (uint32_t)cells, sums + nsums, totals + 1)) != ISO_OK) return s;
+        // the feature points on a side stream: the passes below neither read
+        // nor wait for them
+        if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
+        emc_features<<<(unsigned)(4 * std::max(ctx->sms, 1)), 32, 0, side>>>(A, kept, cap, ctrl);
+        emc_scan<<<1, 1024, 0, ctx->stream>>>(sums, nblocks, ctrl);
+        ctx->launches += 2;
     }
-    cudaError_t e = cudaMemsetAsync(flips, 0, 8, ctx->stream);
-    uint32_t tot[2] = {0, 0}, nfeat = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tot, totals, 8, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nfeat, nfeatures, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counts");
-    const uint64_t nv = tot[0], nt = tot[1];
-    if ((s = ensure(ctx, ctx->mesh_v, 12 * nv + 16)) != ISO_OK) return s;
-    if ((s = ensure(ctx, ctx->mesh_i, 12 * nt + 16)) != ISO_OK) return s;
-    A.vertices = (float*)ctx->mesh_v.p;
-    A.indices = (uint32_t*)ctx->mesh_i.p;
-    A.cap_v = nv;
-    A.cap_t = nt;
-    {
-        StageTimer timer(ctx, ISO_STAGE_EMIT);
-        if (nfeat) {
-            // the feature points on a side stream, beside the other passes
-            // (none reads them): a few feature cells per warp, one warp for
-            // each of the SMs' four sub-partitions while there are enough
-            cudaStream_t side;
-            if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
-            const uint64_t slots = 4ull * (uint64_t)std::max(ctx->sms, 1);
-            const uint32_t per = (uint32_t)std::min<uint64_t>(32, (nfeat + slots - 1) / slots);
-            emc_features<<<(unsigned)((nfeat + per - 1) / per), 32, 0, side>>>(A, features, nfeatures, per);
-            ctx->launches++;
-        }
-        emc_vertices<<<grid_for(ctx, cells, 128, 32), 128, 0, ctx->stream>>>(A, active, nactive);
-        emc_triangles<<<grid_for(ctx, cells, 256, 16), 256, 0, ctx->stream>>>(A, active, nactive);
-        emc_flips<<<grid_for(ctx, cells, 256, 16), 256, 0, ctx->stream>>>(A, active, nactive, flips);
-        if (nfeat && (s = join_side(ctx)) != ISO_OK) return s;
+    s = emc_emit(ctx, A, cells, nblocks, cap, active, features, kept, ctrl, sums);
+    if (ctx->side_open) {  // the passes ended early
+        const iso_status j = join_side(ctx);
+        if (s == ISO_OK) s = j;
     }
-    ctx->launches += 3;
-    if ((s = check_launch(ctx, "emc emit")) != ISO_OK) return s;
-    unsigned long long nflips = 0;
-    e = cudaMemcpyAsync(&nflips, flips, 8, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "emc emit");
+    if (s != ISO_OK) return s;
+    const uint64_t nv = ctx->h_pinned[1] & 0xFFFFFFFFu, nt = ctx->h_pinned[1] >> 32, nflips = ctx->h_pinned[2];
     if ((s = read_device_errors(ctx)) != ISO_OK) return s;
     ctx->last.num_vertices = nv;
     ctx->last.num_triangles = nt;

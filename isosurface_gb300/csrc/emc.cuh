@@ -131,11 +131,19 @@ __host__ __device__ __forceinline__ V3 dir_torus(V3 p, float R, float t) {
 // component-wise min, max and max(b, -a) (csg.rs:41-45, 74-78, 102-106), and
 // CentralDifference passes the inner source's vector through (source.rs:76-80).
 // The host accepts only programs made of these ops (directed_ops_only).
+// The top of the value stack is `top`; vs[1 .. vsp - 1] holds the rest (a
+// run-time index keeps vs in local memory, which a chain of two-operand ops
+// would otherwise read and write three times per op).
 static __host__ __device__ __noinline__ V3 eval_vector(const ProgView& pv, V3 p) {
     V3 vs[VSTACK];
     V3 ps[PSTACK];
     int vsp = 0, psp = 0;
-    V3 q = p;
+    V3 q = p, top = p;
+    auto push = [&](V3 v) {
+        if (vsp) vs[vsp] = top;
+        ++vsp;
+        top = v;
+    };
     for (uint32_t pc = 0; pc < pv.n_ops; ++pc) {
         const uint32_t w = ld_ro(pv.ops + pc);
         const uint32_t op = w & 0xFFu;
@@ -146,22 +154,22 @@ static __host__ __device__ __noinline__ V3 eval_vector(const ProgView& pv, V3 p)
             q = pt_apply(op, k, q);
             break;
         case OP_PT_POP: q = ps[--psp]; break;
-        case OP_SPHERE: vs[vsp++] = dir_sphere(q, k[0]); break;
-        case OP_BOX: vs[vsp++] = dir_box(q, k[0], k[1], k[2]); break;
-        case OP_CYLINDER: vs[vsp++] = dir_cylinder(q, k[0], k[1]); break;
-        case OP_TORUS: vs[vsp++] = dir_torus(q, k[0], k[1]); break;
-        case OP_UNION: --vsp; vs[vsp - 1] = vmin(vs[vsp - 1], vs[vsp]); break;
-        case OP_INTERSECTION: --vsp; vs[vsp - 1] = vmax3(vs[vsp - 1], vs[vsp]); break;
+        case OP_SPHERE: push(dir_sphere(q, k[0])); break;
+        case OP_BOX: push(dir_box(q, k[0], k[1], k[2])); break;
+        case OP_CYLINDER: push(dir_cylinder(q, k[0], k[1])); break;
+        case OP_TORUS: push(dir_torus(q, k[0], k[1])); break;
+        case OP_UNION: --vsp; top = vmin(vs[vsp], top); break;
+        case OP_INTERSECTION: --vsp; top = vmax3(vs[vsp], top); break;
         case OP_DIFFERENCE: {
             --vsp;
-            const V3 a = vs[vsp - 1], b = vs[vsp];
-            vs[vsp - 1] = vmax3(b, v3(-a.x, -a.y, -a.z));
+            const V3 a = vs[vsp];
+            top = vmax3(top, v3(-a.x, -a.y, -a.z));
             break;
         }
         default: break;  // CD_BEGIN / CD_END: the vector is the inner source's
         }
     }
-    return vs[0];
+    return top;
 }
 
 // ---------------------------------------------------------------------------
@@ -179,11 +187,11 @@ __host__ __device__ __forceinline__ uint64_t point_index(uint32_t n, uint32_t x,
     return ((uint64_t)z * n + y) * n + x;
 }
 __host__ __device__ __forceinline__ void cell_xyz(uint32_t n, uint64_t c, uint32_t* x, uint32_t* y, uint32_t* z) {
-    const uint32_t m = n - 1;
-    *x = (uint32_t)(c % m);
-    const uint64_t r = c / m;
-    *y = (uint32_t)(r % m);
-    *z = (uint32_t)(r / m);
+    // sizes up to 513: below 2^28 cells, and a 64-bit division costs several
+    const uint32_t m = n - 1, i = (uint32_t)c, r = i / m;
+    *x = i - r * m;
+    *z = r / m;
+    *y = r - *z * m;
 }
 
 // lattice point position, `x as f32 * one_over_size` (primal_grid.rs:50-70)
@@ -208,10 +216,12 @@ __host__ __device__ __forceinline__ bool owns_edge(uint32_t x, uint32_t y, uint3
 
 // Directed::is_positive (distance.rs:87-90): outside when any component is
 // positive; classify_corners sets bit i when corner i is not outside
+__host__ __device__ __forceinline__ bool directed_inside(V3 v) { return !(v.x > 0.0f || v.y > 0.0f || v.z > 0.0f); }
+
 __host__ __device__ __forceinline__ int classify_directed(const V3* v) {
     int cube = 0;
     for (int i = 0; i < 8; ++i)
-        if (!(v[i].x > 0.0f || v[i].y > 0.0f || v[i].z > 0.0f)) cube |= 1 << i;
+        if (directed_inside(v[i])) cube |= 1 << i;
     return cube;
 }
 
@@ -261,19 +271,14 @@ struct PlanesN {
     int feature;
 };
 
-__host__ __device__ inline void tangent_planes_n(const qef::F3* vtx, const qef::F3* nrm, int n, PlanesN* t) {
+// the planes, once the smallest product of two normals and the cross product
+// of the two are known
+__host__ __device__ inline void planes_about(const qef::F3* vtx, const qef::F3* nrm, int n, float min_angle,
+                                             qef::F3 axis, PlanesN* t) {
     using namespace qef;
-    F3 com = f3(0.0f, 0.0f, 0.0f), axis = f3(0.0f, 0.0f, 0.0f);
-    float min_angle = 3.40282347e+38f;
+    F3 com = f3(0.0f, 0.0f, 0.0f);
     float count = 0.0f;
     for (int i = 0; i < n; ++i) {
-        for (int j = 0; j < n; ++j) {
-            const float angle = dot(nrm[i], nrm[j]);
-            if (angle < min_angle) {
-                axis = cross(nrm[i], nrm[j]);
-                min_angle = angle;
-            }
-        }
         com = add(com, vtx[i]);
         count += 1.0f;
     }
@@ -300,6 +305,21 @@ __host__ __device__ inline void tangent_planes_n(const qef::F3* vtx, const qef::
     t->n = n;
     t->com = com;
     t->feature = feature;
+}
+
+__host__ __device__ inline void tangent_planes_n(const qef::F3* vtx, const qef::F3* nrm, int n, PlanesN* t) {
+    using namespace qef;
+    F3 axis = f3(0.0f, 0.0f, 0.0f);
+    float min_angle = 3.40282347e+38f;
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) {
+            const float angle = dot(nrm[i], nrm[j]);
+            if (angle < min_angle) {
+                axis = cross(nrm[i], nrm[j]);
+                min_angle = angle;
+            }
+        }
+    planes_about(vtx, nrm, n, min_angle, axis, t);
 }
 
 // *ok = false if the QR sweep bound was reached
@@ -348,14 +368,24 @@ struct Args {
     uint32_t* err;       // DERR_* bits
 };
 
-// the Directed value of lattice point `i`
-__host__ __device__ inline void sample_item(const Args& A, uint64_t i) {
+// the Directed value of lattice point `i`; whether it is inside
+__host__ __device__ inline bool sample_item(const Args& A, uint64_t i) {
     const uint32_t n = A.g.n;
-    const uint32_t x = (uint32_t)(i % n);
-    const uint64_t r = i / n;
-    const uint32_t y = (uint32_t)(r % n), z = (uint32_t)(r / n);
+    const uint32_t p = (uint32_t)i, r = p / n, x = p - r * n, z = r / n, y = r - z * n;
     const V3 v = eval_vector(A.prog, point_pos(A.g, x, y, z));
     A.field[i] = make_float4(v.x, v.y, v.z, 0.0f);
+    return directed_inside(v);
+}
+
+// vertices and triangles cell (x, y, z) of case `cube` adds
+__host__ __device__ inline void cell_counts(uint32_t x, uint32_t y, uint32_t z, int cube, uint32_t feature, uint32_t* nv,
+                                            uint32_t* nt) {
+    const uint32_t mask = iso_edge_mask[cube];
+    uint32_t v = feature;
+    for (int e = 0; e < 12; ++e)
+        if ((mask & (1u << e)) && owns_edge(x, y, z, e)) ++v;
+    *nv = v;
+    *nt = feature ? iso_emc_fan_count[cube] : iso_tri_count[cube];
 }
 
 // case, feature decision and counts of cell `c`
@@ -371,15 +401,27 @@ __host__ __device__ inline void count_item(const Args& A, uint64_t c) {
         PlanesN t;
         cell_planes(A.prog, cube, vtx, &t);
         feature = t.feature != qef::PLANAR;
-        const uint32_t mask = iso_edge_mask[cube];
-        for (int e = 0; e < 12; ++e)
-            if ((mask & (1u << e)) && owns_edge(x, y, z, e)) ++nv;
-        nv += feature;
-        nt = feature ? iso_emc_fan_count[cube] : iso_tri_count[cube];
+        cell_counts(x, y, z, cube, feature, &nv, &nt);
     }
     A.cell[c] = (uint16_t)(cube | (feature << 8));
     A.voff[c] = nv;
     A.toff[c] = nt;
+}
+
+// crossing `e` of cell (x, y, z) alone: as edge_crossings gives it
+__host__ __device__ __forceinline__ V3 edge_crossing(const Args& A, uint32_t x, uint32_t y, uint32_t z, int e) {
+    const int u = iso_edge_connection[e][0], v = iso_edge_connection[e][1];
+    const uint32_t ux = x + iso_corners[u][0], uy = y + iso_corners[u][1], uz = z + iso_corners[u][2];
+    const uint32_t vx = x + iso_corners[v][0], vy = y + iso_corners[v][1], vz = z + iso_corners[v][2];
+    const float4 a = ld_ro(A.field + point_index(A.g.n, ux, uy, uz)), b = ld_ro(A.field + point_index(A.g.n, vx, vy, vz));
+    return crossing_directed(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), point_pos(A.g, ux, uy, uz), point_pos(A.g, vx, vy, vz));
+}
+
+__host__ __device__ __forceinline__ void put_vertex(const Args& A, uint32_t id, qef::F3 p) {
+    if (id >= A.cap_v) return;
+    A.vertices[3 * (uint64_t)id] = p.x;
+    A.vertices[3 * (uint64_t)id + 1] = p.y;
+    A.vertices[3 * (uint64_t)id + 2] = p.z;
 }
 
 // the feature point of a feature cell (case `cube`, edge crossings `vtx`)
@@ -390,11 +432,7 @@ __host__ __device__ inline void put_feature(const Args& A, int cube, const V3* v
     bool ok;
     const qef::F3 p = minimise_qef_n(t, &ok);
     if (!ok) set_err(A.err, DERR_SVD_ITER);
-    if (id < A.cap_v) {
-        A.vertices[3 * (uint64_t)id] = p.x;
-        A.vertices[3 * (uint64_t)id + 1] = p.y;
-        A.vertices[3 * (uint64_t)id + 2] = p.z;
-    }
+    put_vertex(A, id, p);
 }
 
 // the vertices cell `c` adds (offsets already scanned); with
