@@ -1,11 +1,13 @@
 // Batched MarchingCubes: thousands of independent chunks, each a
 // MarchingCubes::new(size_i).extract over its own source, in one pass.
 //
-// * Sampling: one persistent kernel drains a work queue of (chunk, z-slab,
-//   y-range) tiles (largest cost first); each block samples its tile with the
-//   culled sampler of bricks.cuh (sign bits everywhere, values where marching
-//   cubes can read them, primitives pruned per sub-brick).  The slab depth
-//   per chunk-size class comes from iso_batch_autotune.
+// * Sampling: the culled sampler of bricks.cuh (sign bits everywhere, values
+//   where marching cubes can read them, primitives pruned per sub-brick) in
+//   two launches: a warp classifies up to 32 sub-bricks of one chunk and
+//   lists the mixed ones, and a persistent grid evaluates the list, four
+//   sub-bricks of one chunk to a warp.  Warps do not cross a chunk's z-slabs;
+//   the slab depth per chunk-size class is the whole chunk unless
+//   iso_batch_set_slab or iso_batch_autotune chooses another.
 // * Classification, scan and emission: the chunked marching-cubes passes of
 //   mc.cu over a table of grids whose 32-cell chunks are laid out
 //   range-aligned in one global index space (mc_chunk.cuh).
@@ -58,45 +60,103 @@ struct SampleGrid {
     uint32_t W;
 };
 
-struct Tile {
-    uint32_t grid, z0, z1, y0, y1;  // layers [z0, z1), rows [y0, y1), all x
+// Up to eight groups of four sub-bricks along x (32 x 4 x 4 samples) of one
+// grid, from group `first` in (z, y, x) order: a classifying warp's work.
+struct Task {
+    uint32_t grid, first, groups;
 };
 
-// A persistent grid: each block takes tiles from the work queue (largest
-// first) and samples them whole with the culled sampler (bricks.cuh).
-__global__ void __launch_bounds__(256) batch_sample(const Tile* tiles, const SampleGrid* grids, uint32_t ntiles,
-                                                    uint32_t* next) {
-    __shared__ uint32_t s_tile, s_n;
-    __shared__ uint8_t s_cls[BRICK_MAX];
-    __shared__ uint64_t s_keep[BRICK_MAX];
-    __shared__ uint32_t s_list[BRICK_MAX];
-    while (true) {
-        __syncthreads();  // the previous tile is done with the shared arrays
-        if (threadIdx.x == 0) s_tile = atomicAdd(next, 1u);
-        __syncthreads();
-        const uint32_t t = s_tile;
-        if (t >= ntiles) return;
-        const Tile tl = tiles[t];
-        const SampleGrid sg = grids[tl.grid];
-        const BrickTile T{BrickLattice{sg.pv.lip, sg.pv.slack, sg.n, sg.n, sg.n + 1, sg.inv, sg.field, sg.pitch,
-                                       sg.bits, sg.W, 0, 1.0f},
-                          tl.y0, tl.y1, tl.z0, tl.z1};
-        brick_tile(VmEval{sg.pv}, T, s_cls, s_keep, s_list, &s_n);
+// A mixed sub-brick: its grid, its place sx | sy << 8 | sz << 17 (NO_BRICK:
+// none, filling up a warp's four) and the primitives it keeps.
+struct Mixed {
+    uint32_t grid, at;
+    uint64_t keep;
+};
+constexpr uint32_t NO_BRICK = 0xFFFFFFFFu;
+
+__device__ __forceinline__ BrickLattice lattice_of(const SampleGrid& sg) {
+    return BrickLattice{sg.pv.lip, sg.pv.slack, sg.n,     sg.n,  sg.n + 1, sg.inv,
+                        sg.field,  sg.pitch,    sg.bits, sg.W, 0,        1.0f};
+}
+
+// A warp per task, a lane per sub-brick: no barrier, and no lane waits for
+// another grid's primitives.  (Blocks that classified a tile, listed its
+// mixed sub-bricks in shared memory and sampled them between barriers spent
+// 44 % of their warps' time at those, on tiles of 20 sub-bricks for a 16^3
+// chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells.)
+__global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const SampleGrid* grids, uint32_t ntasks,
+                                                      Mixed* list, uint32_t* count) {
+    const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (t >= ntasks) return;
+    const Task k = tasks[t];
+    const SampleGrid sg = grids[k.grid];
+    const BrickLattice g = lattice_of(sg);
+    const VmEval ev{sg.pv};
+    const uint32_t SY = (g.ny + 3) / 4, gi = k.first + (lane >> 2), j = lane & 3;
+    const bool have = (lane >> 2) < k.groups;
+    const uint32_t w = gi % g.W, sy = gi / g.W % SY, sz = gi / (g.W * SY), sx = 4 * w + j;
+    const uint32_t xa = 8 * sx, ya = 4 * sy, za = 4 * sz;
+    uint32_t cls = BRICK_MIXED;
+    uint64_t keep = ~0ull;
+    if (!have || (g.lip > 0.0f && xa >= g.nx)) cls = BRICK_OUT;  // no samples: sign bits stay clear
+    else if (g.lip > 0.0f)
+        cls = brick_class(ev, g, xa, min(xa + 7, g.nx - 1), ya, min(ya + 3, g.ny - 1), za, min(za + 3, g.nz - 1), &keep);
+    const uint32_t mixed = __ballot_sync(0xFFFFFFFFu, cls == BRICK_MIXED);
+    // the group's sign words: its four lanes take four rows each
+    uint32_t cls4 = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) cls4 |= __shfl_sync(0xFFFFFFFFu, cls, (lane & ~3u) + i) << (8 * i);
+    const uint32_t mine = mixed >> (lane & ~3u) & 15u;
+    if (have) {
+        const uint32_t word = decided_word(cls4, g.nx, w), z = za + j;
+        for (uint32_t r = 0; r < 4 && z < g.nz; ++r) {
+            const uint32_t y = ya + r;
+            if (y >= g.ny) break;
+            uint32_t* at = g.bits + ((uint64_t)z * g.ny + y) * g.W + w;
+            if (!mine) {
+                *at = word;
+            } else {
+                for (uint32_t i = 0; i < 4; ++i)
+                    if (!(mine >> i & 1u))
+                        reinterpret_cast<uint8_t*>(at)[i] = decided_byte(cls4 >> (8 * i) & 0xFFu, g.nx, 4 * w + i);
+            }
+        }
+    }
+    if (!mixed) return;
+    // the task's part of the list, filled up to whole fours
+    const uint32_t n = __popc(mixed), padded = (n + 3) & ~3u;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, padded);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (cls == BRICK_MIXED)
+        list[base + __popc(mixed & ((1u << lane) - 1u))] = Mixed{k.grid, sx | sy << 8 | sz << 17, keep};
+    if (lane < padded - n) list[base + n + lane] = Mixed{k.grid, NO_BRICK, 0};
+}
+
+// The listed sub-bricks, four of one grid to a warp, over a persistent grid.
+__global__ void __launch_bounds__(256) batch_rows(const SampleGrid* grids, const Mixed* list, const uint32_t* count) {
+    const uint32_t n = *count, lane = threadIdx.x & 31;
+    for (uint32_t q = 4 * (blockIdx.x * 8 + (threadIdx.x >> 5)); q < n; q += 32 * gridDim.x) {
+        const Mixed m = list[q + (lane >> 3)];
+        const SampleGrid& sg = grids[__shfl_sync(0xFFFFFFFFu, m.grid, 0)];
+        const BrickLattice g = lattice_of(sg);
+        const bool have = m.at != NO_BRICK;
+        const uint32_t sx = have ? m.at & 255u : 0u, ya = have ? 4 * (m.at >> 8 & 511u) : 0u,
+                       za = have ? 4 * (m.at >> 17) : 0u;
+        brick_fill(VmEval{sg.pv}, g, have, sx, ya, za, g.ny, g.nz, warp_or64(m.keep));
     }
 }
 
-// The tiles of one chunk of `n` (n x n x (n + 1) samples) for slab depth
-// `depth` (0: the whole chunk), rounded up to whole sub-bricks (4 layers)
-// and cut in y so that a tile holds at most BRICK_MAX sub-bricks.
+// The tasks of one chunk of `n` (n x n x (n + 1) samples) for slab depth
+// `depth` (0: the whole chunk), rounded up to whole sub-bricks (4 layers).
 template <class F>
-void chunk_tiles(uint32_t grid, uint32_t n, uint32_t depth, F&& add) {
-    const uint32_t nz = n + 1, SX = 4 * words_per_row(n);
-    uint32_t zg = ((depth ? depth : nz) + 3) / 4;
-    zg = std::max(1u, std::min(zg, BRICK_MAX / SX));
-    const uint32_t ty = std::max(1u, std::min((n + 3) / 4, BRICK_MAX / (SX * zg)));
-    for (uint32_t z0 = 0; z0 < nz; z0 += 4 * zg)
-        for (uint32_t y0 = 0; y0 < n; y0 += 4 * ty)
-            add(Tile{grid, z0, std::min(nz, z0 + 4 * zg), y0, std::min(n, y0 + 4 * ty)});
+void chunk_tasks(uint32_t grid, uint32_t n, uint32_t depth, F&& add) {
+    const uint32_t layer = words_per_row(n) * ((n + 3) / 4), nsz = (n + 1 + 3) / 4;  // groups per four layers
+    const uint32_t zg = depth ? std::min((depth + 3) / 4, nsz) : nsz;
+    for (uint32_t z = 0; z < nsz; z += zg) {
+        const uint32_t end = layer * std::min(z + zg, nsz);
+        for (uint32_t first = layer * z; first < end; first += 8) add(Task{grid, first, std::min(8u, end - first)});
+    }
 }
 
 struct Chunk {
@@ -116,9 +176,9 @@ struct iso_batch {
     SampleGrid* d_sgrids = nullptr;
     void* d_grids = nullptr;
     uint32_t* d_range_grid = nullptr;
-    Tile* d_tiles = nullptr;
-    uint32_t ntiles = 0;
-    uint32_t* d_next = nullptr;  // the sampler's work-queue counter
+    Task* d_tasks = nullptr;  // the sampler's tasks, then room for their mixed sub-bricks
+    uint32_t ntasks = 0;
+    uint32_t* d_next = nullptr;  // how many mixed sub-bricks are listed
     uint32_t* d_extents = nullptr;   // 4 per chunk
     uint64_t* d_totals = nullptr;    // [0] triangles [1] vertices
     void* d_scratch = nullptr;       // chunk-pass scratch
@@ -141,30 +201,25 @@ struct iso_batch {
 
 namespace {
 
-// Device copy of `tiles`.
-cudaError_t upload_tiles(const std::vector<Tile>& tiles, Tile** d_tiles) {
-    cudaError_t e = cudaMalloc((void**)d_tiles, sizeof(Tile) * std::max<size_t>(tiles.size(), 1));
-    if (e == cudaSuccess && !tiles.empty())
-        e = cudaMemcpy(*d_tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice);
+// where the list of mixed sub-bricks starts behind `n` tasks
+size_t list_at(size_t n) { return (sizeof(Task) * n + 255) & ~(size_t)255; }
+
+// Device copy of `tasks`, with room for every sub-brick of theirs behind it.
+cudaError_t upload_tasks(const std::vector<Task>& tasks, Task** d_tasks) {
+    const size_t n = tasks.size();
+    cudaError_t e = cudaMalloc((void**)d_tasks, list_at(n) + 32 * sizeof(Mixed) * std::max<size_t>(n, 1));
+    if (e == cudaSuccess && n) e = cudaMemcpy(*d_tasks, tasks.data(), sizeof(Task) * n, cudaMemcpyHostToDevice);
     return e;
 }
 
-iso_status build_tiles(iso_batch* b) {
-    std::vector<std::pair<double, Tile>> t;
-    for (uint32_t i = 0; i < b->chunks.size(); ++i) {
-        const uint32_t n = b->chunks[i].size;
-        const double cost_per_point = (double)b->programs[b->chunks[i].prog]->ops.size();
-        chunk_tiles(i, n, b->slab[i], [&](const Tile& tl) {
-            t.push_back({cost_per_point * ((n + 31) / 32 * 32) * (tl.y1 - tl.y0) * (tl.z1 - tl.z0), tl});
-        });
-    }
-    std::stable_sort(t.begin(), t.end(), [](const auto& a, const auto& c) { return a.first > c.first; });
-    std::vector<Tile> tiles(t.size());
-    for (size_t i = 0; i < t.size(); ++i) tiles[i] = t[i].second;
-    if (b->d_tiles) cudaFree(b->d_tiles);
-    b->d_tiles = nullptr;
-    b->ntiles = (uint32_t)tiles.size();
-    cudaError_t e = upload_tiles(tiles, &b->d_tiles);
+iso_status build_tasks(iso_batch* b) {
+    std::vector<Task> tasks;
+    for (uint32_t i = 0; i < b->chunks.size(); ++i)
+        chunk_tasks(i, b->chunks[i].size, b->slab[i], [&](const Task& t) { tasks.push_back(t); });
+    if (b->d_tasks) cudaFree(b->d_tasks);
+    b->d_tasks = nullptr;
+    b->ntasks = (uint32_t)tasks.size();
+    cudaError_t e = upload_tasks(tasks, &b->d_tasks);
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
@@ -173,21 +228,23 @@ iso_status build_tiles(iso_batch* b) {
         cudaGraphDestroy(b->graph);
         b->graph = nullptr;
     }
-    return e == cudaSuccess ? ISO_OK : cuda_fail(b->ctx, e, "tiles");
+    return e == cudaSuccess ? ISO_OK : cuda_fail(b->ctx, e, "tasks");
 }
 
-// blocks of batch_sample that fill every SM (looked up once per process)
-unsigned sample_blocks(int sms) {
+// blocks of batch_rows that fill every SM (looked up once per process)
+unsigned rows_blocks(int sms) {
     static std::atomic<int> per_sm{0};
-    return persistent_blocks((const void*)batch_sample, per_sm, sms);
+    return persistent_blocks((const void*)batch_rows, per_sm, sms);
 }
 
-// the culled sampler over `ntiles` tiles (the queue counter zeroed first)
-cudaError_t launch_sampler(iso_ctx* ctx, const Tile* d_tiles, uint32_t ntiles, const SampleGrid* d_sgrids,
-                           uint32_t* next) {
-    cudaError_t e = cudaMemsetAsync(next, 0, 4, ctx->stream);
+// the culled sampler over `ntasks` tasks
+cudaError_t launch_sampler(iso_ctx* ctx, const Task* d_tasks, uint32_t ntasks, const SampleGrid* d_sgrids,
+                           uint32_t* count) {
+    cudaError_t e = cudaMemsetAsync(count, 0, 4, ctx->stream);
     if (e != cudaSuccess) return e;
-    batch_sample<<<sample_blocks(ctx->sms), 256, 0, ctx->stream>>>(d_tiles, d_sgrids, ntiles, next);
+    Mixed* list = (Mixed*)((char*)d_tasks + list_at(ntasks));
+    batch_classify<<<(ntasks + 7) / 8, 256, 0, ctx->stream>>>(d_tasks, d_sgrids, ntasks, list, count);
+    batch_rows<<<rows_blocks(ctx->sms), 256, 0, ctx->stream>>>(d_sgrids, list, count);
     return cudaGetLastError();
 }
 
@@ -196,10 +253,10 @@ iso_status enqueue(iso_batch* b, bool sync_sizes) {
     iso_ctx* ctx = b->ctx;
     {
         StageTimer timer(ctx, ISO_STAGE_SAMPLE);
-        cudaError_t e = launch_sampler(ctx, b->d_tiles, b->ntiles, b->d_sgrids, b->d_next);
+        cudaError_t e = launch_sampler(ctx, b->d_tasks, b->ntasks, b->d_sgrids, b->d_next);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch sampler");
     }
-    ctx->launches++;
+    ctx->launches += 2;
     return mc_extract_grids(ctx, b->d_grids, (uint32_t)b->chunks.size(), b->d_range_grid, b->total_chunks, b->max_cw,
                             b->d_scratch, b->cap_v, b->cap_t, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p,
                             b->d_extents, b->d_totals, sync_sizes);
@@ -249,7 +306,7 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
         }
         b->chunks.push_back(Chunk{chunks[i].program, chunks[i].size});
     }
-    b->slab.assign(nchunks, 4);
+    b->slab.assign(nchunks, 0);
     // layout: per chunk field + bits; grid tables; chunk-pass scratch
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -316,7 +373,7 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
         iso_batch_destroy(b);
         return cuda_fail(ctx, e, "batch tables");
     }
-    if ((s = build_tiles(b)) != ISO_OK) {
+    if ((s = build_tasks(b)) != ISO_OK) {
         iso_batch_destroy(b);
         return s;
     }
@@ -329,7 +386,7 @@ iso_status iso_batch_destroy(iso_batch* b) {
     cudaSetDevice(b->ctx->device);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
-    if (b->d_tiles) cudaFree(b->d_tiles);
+    if (b->d_tasks) cudaFree(b->d_tasks);
     if (b->arena) cudaFree(b->arena);
     if (b->d_solo_grids) cudaFree(b->d_solo_grids);
     delete b;
@@ -340,7 +397,7 @@ iso_status iso_batch_set_slab(iso_batch* b, uint32_t size, uint32_t depth) {
     if (!b) return ISO_ERR_INVALID_ARG;
     for (size_t i = 0; i < b->chunks.size(); ++i)
         if (size == 0 || b->chunks[i].size == size) b->slab[i] = depth;
-    return build_tiles(b);
+    return build_tasks(b);
 }
 
 iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
@@ -403,7 +460,7 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
         cudaError_t e = cudaGraphLaunch(b->exec, ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "graph launch");
     }
-    ctx->launches += 6;
+    ctx->launches += 7;
     s = finish(b, info);
     if (s == ISO_ERR_CAPACITY || ctx->last.num_vertices > b->cap_v || ctx->last.num_triangles > b->cap_t) {
         b->sized = false;  // grow and run eagerly
@@ -540,7 +597,7 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, ctx->device);
     // cached depths are for this sampler design on this GPU model
-    const std::string gpu = std::string(prop.name) + " bricks";
+    const std::string gpu = std::string(prop.name) + " brick list";
     std::map<uint32_t, uint32_t> classes;  // size -> chunk count
     for (auto& c : b->chunks) classes[c.size]++;
     std::map<uint32_t, uint32_t> best;
@@ -567,26 +624,24 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
     for (auto& cl : classes) {
         if (best.count(cl.first)) continue;
         float best_ms = 1e30f;
-        uint32_t best_depth = 4;
+        uint32_t best_depth = 0;
         for (uint32_t d : candidates) {
             // time the sampler on this class's chunks only, slab depth d
-            std::vector<std::pair<double, Tile>> t;
+            std::vector<Task> tasks;
             for (uint32_t i = 0; i < b->chunks.size(); ++i) {
                 if (b->chunks[i].size != cl.first) continue;
-                chunk_tiles(i, cl.first, d, [&](const Tile& tl) { t.push_back({0.0, tl}); });
+                chunk_tasks(i, cl.first, d, [&](const Task& t) { tasks.push_back(t); });
             }
-            std::vector<Tile> tiles(t.size());
-            for (size_t i = 0; i < t.size(); ++i) tiles[i] = t[i].second;
-            Tile* d_t = nullptr;
-            if (upload_tiles(tiles, &d_t) != cudaSuccess) {
+            Task* d_t = nullptr;
+            if (upload_tasks(tasks, &d_t) != cudaSuccess) {
                 if (d_t) cudaFree(d_t);
                 cudaGetLastError();
-                return fail(ctx, ISO_ERR_OUT_OF_MEMORY, "autotune tiles");
+                return fail(ctx, ISO_ERR_OUT_OF_MEMORY, "autotune tasks");
             }
             float ms = 1e30f;
             for (int rep = 0; rep < 4; ++rep) {
                 cudaEventRecord(e0, ctx->stream);
-                launch_sampler(ctx, d_t, (uint32_t)tiles.size(), b->d_sgrids, b->d_next);
+                launch_sampler(ctx, d_t, (uint32_t)tasks.size(), b->d_sgrids, b->d_next);
                 cudaEventRecord(e1, ctx->stream);
                 cudaEventSynchronize(e1);
                 float t_ms = 0.0f;
@@ -622,7 +677,7 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
         }
     }
     (void)saved;
-    return build_tiles(b);
+    return build_tasks(b);
 }
 
 }  // extern "C"

@@ -23,7 +23,28 @@ struct VmEval {
     __device__ __forceinline__ uint32_t nprims() const { return pv.nprims; }
     __device__ __forceinline__ V3 point(V3 p) const { return prims_point(pv, p); }
     __device__ __forceinline__ float prim(uint32_t i, V3 q) const { return prim_at(pv, i, q); }
-    __device__ __forceinline__ float value_kept(uint64_t keep, V3 p) const { return eval_prims_kept(pv, keep, p); }
+    __device__ __forceinline__ void values_kept(uint64_t keep, const V3 (&p)[4], float (&v)[16]) const {
+        V3 q[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[j] = point(p[j]);
+        // fminf returns its other operand for a NaN, so the first primitive's value replaces it
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = __int_as_float(0x7FFFFFFF);
+        for (; keep; keep &= keep - 1) {
+            const uint32_t i = lowest_bit(keep);
+            const float4 c = ld_ro(pv.prims + 2 * i), a = ld_ro(pv.prims + 2 * i + 1);
+            auto each = [&](auto&& sd) {
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                    v[r] = fminf(v[r], sd(v3(q[0].x - c.x, q[r & 3].y - c.y, q[r >> 2].z - c.z)));
+            };
+            const uint32_t type = float_bits(c.w);
+            if (type == OP_SPHERE) each([&](V3 t) { return sd_sphere(t, a.x); });
+            else if (type == OP_BOX) each([&](V3 t) { return sd_box(t, a.x, a.y, a.z); });
+            else if (type == OP_CYLINDER) each([&](V3 t) { return sd_cylinder(t, a.x, a.y); });
+            else each([&](V3 t) { return sd_torus(t, a.x, a.y); });
+        }
+    }
 };
 
 // The culling bounds of a program for a lattice.

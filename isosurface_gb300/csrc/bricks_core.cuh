@@ -28,18 +28,15 @@
 // at once; in a mixed group the decided sub-bricks get their sign bytes and
 // every sample of the mixed ones is evaluated, four mixed sub-bricks to a
 // warp (eight lanes each, one sign byte per row), so that no lane idles on a
-// decided sub-brick.  Two schedules:
-//  * one lattice (brick_classify + brick_rows): one block per tile
-//    classifies and appends its mixed sub-bricks to a list; a persistent
-//    grid then samples the list, so the evaluation is spread evenly however
-//    the surface falls;
-//  * many small lattices (brick_tile, the chunk batch): a block takes whole
-//    tiles from a work queue and samples its own mixed sub-bricks from a list
-//    in shared memory.
+// decided sub-brick.  Classification appends the mixed sub-bricks to a list (a block
+// per tile here; a warp per 32 sub-bricks for many small lattices, batch.cu);
+// a persistent grid then samples the list, so the evaluation is spread evenly
+// however the surface falls.
 //
 // The evaluator `Ev` provides value(p) and, for pruned unions, prunable(),
-// nprims(), point(p) (the point after a leading domain map), prim(i, q) and
-// value_kept(keep, p).
+// nprims(), point(p) (the point after a leading domain map, which keeps the
+// axes apart), prim(i, q) and values_kept(keep, p, v): v[4 k + j] is the
+// union's value at (p[0].x, p[j].y, p[k].z).
 #pragma once
 
 namespace iso {
@@ -96,6 +93,41 @@ __host__ __device__ __forceinline__ uint32_t brick_count(uint32_t W, uint32_t ro
     return 4 * W * ((rows + 3) / 4) * ((layers + 3) / 4);
 }
 
+// Class of the sub-brick of samples [xa, xb] x [ya, yb] x [za, zb] and the
+// primitives it keeps (a program with a bound).
+template <class Ev>
+__device__ __forceinline__ uint32_t brick_class(const Ev& ev, const BrickLattice& g, uint32_t xa, uint32_t xb,
+                                                uint32_t ya, uint32_t yb, uint32_t za, uint32_t zb, uint64_t* keep) {
+    // both ends of a crossing edge lie within lip * inv of zero (rounded up);
+    // a caller may need values further out (reach_steps > 1)
+    const float reach = g.lip * g.inv * g.reach_steps * (1.0f + 1.0f / 1024.0f) + g.slack;
+    const float hx = 0.5f * (float)(xb - xa), hy = 0.5f * (float)(yb - ya), hz = 0.5f * (float)(zb - za);
+    const V3 c = v3(((float)xa + hx) * g.inv, ((float)ya + hy) * g.inv, ((float)(za + g.zoff) + hz) * g.inv);
+    // the largest change of any value over the sub-brick, rounded up
+    const float spread = g.lip * sqrtf((hx * hx + hy * hy) + hz * hz) * g.inv * (1.0f + 1.0f / 1024.0f) + g.slack;
+    float v;
+    if (ev.prunable()) {
+        const V3 q = ev.point(c);
+        const uint32_t n = ev.nprims();
+        float upper = __int_as_float(0x7F800000);  // +infinity
+        v = 0.0f;
+        for (uint32_t i = 0; i < n; ++i) {
+            const float d = ev.prim(i, q);
+            v = (i == 0) ? d : fminf(v, d);
+            upper = fminf(upper, d + spread);
+        }
+        uint64_t k = 0;
+        for (uint32_t i = 0; i < n; ++i)
+            if (!(ev.prim(i, q) - spread > upper)) k |= 1ull << i;
+        *keep = k;
+    } else {
+        v = ev.value(c);
+    }
+    if (v - spread > reach) return BRICK_OUT;
+    if (v + spread < -reach) return BRICK_IN;
+    return BRICK_MIXED;
+}
+
 // Class and kept primitives of every sub-brick of a tile, into shared memory
 // (every thread of the block calls it; no barrier at the end).
 template <class Ev>
@@ -103,46 +135,16 @@ __device__ __forceinline__ void brick_classes(const Ev& ev, const BrickTile& T, 
     const BrickLattice& g = T.g;
     const uint32_t SX = 4 * g.W, SY = (T.y1 - T.y0 + 3) / 4, SZ = (T.z1 - T.z0 + 3) / 4;
     const uint32_t nsb = SX * SY * SZ;
-    const bool cull = g.lip > 0.0f;
-    const bool prune = cull && ev.prunable();
-    // both ends of a crossing edge lie within lip * inv of zero (rounded up);
-    // a caller may need values further out (reach_steps > 1)
-    const float reach = g.lip * g.inv * g.reach_steps * (1.0f + 1.0f / 1024.0f) + g.slack;
     for (uint32_t s = threadIdx.x; s < nsb; s += blockDim.x) {
         uint32_t cls = BRICK_MIXED;
         uint64_t keep = ~0ull;
-        if (cull) {
+        if (g.lip > 0.0f) {
             const uint32_t sx = s % SX, sy = (s / SX) % SY, sz = s / (SX * SY);
             const uint32_t xa = 8 * sx, ya = T.y0 + 4 * sy, za = T.z0 + 4 * sz;
-            if (xa >= g.nx) {
-                cls = BRICK_OUT;  // no samples: sign bits stay clear
-            } else {
-                const uint32_t xb = min(xa + 7, g.nx - 1), yb = min(ya + 3, T.y1 - 1), zb = min(za + 3, T.z1 - 1);
-                const float hx = 0.5f * (float)(xb - xa), hy = 0.5f * (float)(yb - ya), hz = 0.5f * (float)(zb - za);
-                const V3 c = v3(((float)xa + hx) * g.inv, ((float)ya + hy) * g.inv, ((float)(za + g.zoff) + hz) * g.inv);
-                // the largest change of any value over the sub-brick, rounded up
-                const float spread = g.lip * sqrtf((hx * hx + hy * hy) + hz * hz) * g.inv * (1.0f + 1.0f / 1024.0f) +
-                                     g.slack;
-                float v;
-                if (prune) {
-                    const V3 q = ev.point(c);
-                    const uint32_t n = ev.nprims();
-                    float upper = __int_as_float(0x7F800000);  // +infinity
-                    v = 0.0f;
-                    for (uint32_t i = 0; i < n; ++i) {
-                        const float d = ev.prim(i, q);
-                        v = (i == 0) ? d : fminf(v, d);
-                        upper = fminf(upper, d + spread);
-                    }
-                    keep = 0;
-                    for (uint32_t i = 0; i < n; ++i)
-                        if (!(ev.prim(i, q) - spread > upper)) keep |= 1ull << i;
-                } else {
-                    v = ev.value(c);
-                }
-                if (v - spread > reach) cls = BRICK_OUT;
-                else if (v + spread < -reach) cls = BRICK_IN;
-            }
+            if (xa >= g.nx) cls = BRICK_OUT;  // no samples: sign bits stay clear
+            else
+                cls = brick_class(ev, g, xa, min(xa + 7, g.nx - 1), ya, min(ya + 3, T.y1 - 1), za,
+                                  min(za + 3, T.z1 - 1), &keep);
         }
         s_cls[s] = (uint8_t)cls;
         s_keep[s] = keep;
@@ -197,11 +199,52 @@ __device__ __forceinline__ uint32_t brick_group_bits(const BrickTile& T, uint32_
     return mixed;
 }
 
-// The 16 rows of up to four mixed sub-bricks, one per eight lanes: lane l
-// samples x = 8 sx + l % 8 of sub-brick `sb` of tile `T` (both its own; sb
-// = ~0u: none) and the eight lanes' signs go out as one byte of the row's
-// sign word.  `keep` (the same in every lane) holds every primitive any of
-// the sub-bricks keeps.  Every lane of the warp calls it.
+// The 16 rows of up to four mixed sub-bricks, one per eight lanes (sx, ya,
+// za and have: the lane's own sub-brick; y1, z1: the ends of its rows): lane
+// l samples x = 8 sx + l % 8, and the eight lanes' signs go out as one byte
+// of the row's sign word.  `keep` (the same in every lane) holds every
+// primitive any of the sub-bricks keeps.  Every lane of the warp calls it.
+//
+// A pruned union is evaluated a primitive at a time over the lane's 4 x 4
+// points (values_kept): the primitive is read and told apart once for 16
+// points, and what depends on one or two of the coordinates is computed
+// once per coordinate.  The chunk batch's 1024 chunks, a point at a time:
+// 348 M warp instructions.
+template <class Ev>
+__device__ __forceinline__ void brick_fill(const Ev& ev, const BrickLattice& g, bool have, uint32_t sx, uint32_t ya,
+                                           uint32_t za, uint32_t y1, uint32_t z1, uint64_t keep) {
+    const uint32_t lane = threadIdx.x & 31, x = 8 * sx + (lane & 7);
+    auto put = [&](uint32_t r, float v) {
+        const uint32_t y = ya + (r & 3), z = za + (r >> 2);
+        const bool row_ok = have && y < y1 && z < z1;
+        const uint64_t row = (uint64_t)z * g.ny + y;
+        const bool in = row_ok && x < g.nx;
+        if (in) g.field[row * g.pitch + x] = v;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, in && !(v > 0.0f));
+        if (row_ok && (lane & 7) == 0)
+            reinterpret_cast<uint8_t*>(g.bits + row * g.W + sx / 4)[sx % 4] = (uint8_t)(b >> (lane & ~7u));
+    };
+    if (g.lip > 0.0f && ev.prunable()) {
+        V3 p[4];  // (x, y_j, z_j)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            p[j] = v3((float)x * g.inv, (float)(ya + j) * g.inv, (float)(za + j + g.zoff) * g.inv);
+        float v[16];
+        ev.values_kept(keep, p, v);
+#pragma unroll
+        for (uint32_t r = 0; r < 16; ++r) put(r, v[r]);
+        return;
+    }
+    for (uint32_t r = 0; r < 16; ++r) {
+        const uint32_t y = ya + (r & 3), z = za + (r >> 2);
+        float v = 0.0f;
+        if (have && y < y1 && z < z1 && x < g.nx)
+            v = ev.value(v3((float)x * g.inv, (float)y * g.inv, (float)(z + g.zoff) * g.inv));
+        put(r, v);
+    }
+}
+
+// brick_fill of sub-brick `sb` of tile `T` (the lane's own; sb = ~0u: none)
 template <class Ev>
 __device__ __forceinline__ void brick_quad(const Ev& ev, const BrickTile& T, uint32_t sb, uint64_t keep) {
     const BrickLattice& g = T.g;
@@ -214,23 +257,7 @@ __device__ __forceinline__ void brick_quad(const Ev& ev, const BrickTile& T, uin
         ya = T.y0 + 4 * ((sb / SX) % SY);
         za = T.z0 + 4 * (sb / (SX * SY));
     }
-    const uint32_t x = 8 * sx + (lane & 7);
-    const bool prune = g.lip > 0.0f && ev.prunable();
-    for (uint32_t r = 0; r < 16; ++r) {
-        const uint32_t y = ya + (r & 3), z = za + (r >> 2);
-        const bool row_ok = have && y < T.y1 && z < T.z1;
-        const uint64_t row = (uint64_t)z * g.ny + y;
-        bool inside = false;
-        if (row_ok && x < g.nx) {
-            const V3 p = v3((float)x * g.inv, (float)y * g.inv, (float)(z + g.zoff) * g.inv);
-            const float v = prune ? ev.value_kept(keep, p) : ev.value(p);
-            g.field[row * g.pitch + x] = v;
-            inside = !(v > 0.0f);
-        }
-        const uint32_t b = __ballot_sync(0xFFFFFFFFu, inside);
-        if (row_ok && (lane & 7) == 0)
-            reinterpret_cast<uint8_t*>(g.bits + row * g.W + sx / 4)[sx % 4] = (uint8_t)(b >> (lane & ~7u));
-    }
+    brick_fill(ev, g, have, sx, ya, za, T.y1, T.z1, keep);
 }
 
 // Classify one tile, write its decided sign bits and list its mixed
@@ -263,33 +290,6 @@ __device__ __forceinline__ void brick_classify_tile(const Ev& ev, const BrickTil
                 else atomicOr(err, BRICK_ERR_CAPACITY);
             }
         }
-    }
-}
-
-// Sample a whole tile in the block: classes, decided sign bits, then the
-// mixed sub-bricks four to a warp from a list in shared memory (every thread
-// of the block calls it).
-template <class Ev>
-__device__ __forceinline__ void brick_tile(const Ev& ev, const BrickTile& T, uint8_t* s_cls, uint64_t* s_keep,
-                                           uint32_t* s_list, uint32_t* s_n) {
-    if (threadIdx.x == 0) *s_n = 0;
-    brick_classes(ev, T, s_cls, s_keep);
-    __syncthreads();
-    const uint32_t groups = brick_count(T.g.W, T.y1 - T.y0, T.z1 - T.z0) / 4;
-    for (uint32_t gi = threadIdx.x; gi < groups; gi += blockDim.x) {
-        uint32_t mixed = brick_group_bits(T, gi, s_cls);
-        if (mixed) {
-            uint32_t at = atomicAdd(s_n, (uint32_t)__popc(mixed));
-            for (; mixed; mixed &= mixed - 1) s_list[at++] = 4 * gi + (uint32_t)(__ffs(mixed) - 1);
-        }
-    }
-    __syncthreads();
-    const uint32_t n = *s_n, lane = threadIdx.x & 31;
-    for (uint32_t q = 4 * (threadIdx.x >> 5); q < n; q += 4 * (blockDim.x >> 5)) {
-        const uint32_t e = q + (lane >> 3);
-        const uint32_t sb = e < n ? s_list[e] : 0xFFFFFFFFu;
-        const uint64_t keep = warp_or64(e < n ? s_keep[sb] : 0ull);
-        brick_quad(ev, T, sb, keep);
     }
 }
 

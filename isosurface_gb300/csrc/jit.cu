@@ -290,7 +290,7 @@ std::string module_source(const std::string& value_body, const std::string& herm
          "    __device__ __forceinline__ uint32_t nprims() const { return 0; }\n"
          "    __device__ __forceinline__ V3 point(V3 p) const { return p; }\n"
          "    __device__ __forceinline__ float prim(uint32_t, V3) const { return 0.0f; }\n"
-         "    __device__ __forceinline__ float value_kept(uint64_t, V3 p) const { return value(p); }\n"
+         "    __device__ __forceinline__ void values_kept(uint64_t, const V3 (&)[4], float (&)[16]) const {}\n"
          "};\n}  // namespace iso\n"
          "extern \"C\" __global__ void __launch_bounds__(256) iso_jit_classify(iso::GridTiles tiles, "
          "iso::BrickTask* list, uint32_t* count, uint32_t cap, uint32_t* err) {\n"
