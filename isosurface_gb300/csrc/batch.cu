@@ -8,9 +8,11 @@
 //   sub-bricks of one chunk to a warp.  Warps do not cross a chunk's z-slabs;
 //   the slab depth per chunk-size class is the whole chunk unless
 //   iso_batch_set_slab or iso_batch_autotune chooses another.
-// * Classification, scan and emission: the chunked marching-cubes passes of
-//   mc.cu over a table of grids whose 32-cell chunks are laid out
-//   range-aligned in one global index space (mc_chunk.cuh).
+// * Counting, scan and emission: the cell passes of mc_cells.cuh over a table
+//   of grids that share one edge map; when the grids' edges do not fit its
+//   32-bit keys, or there is no memory for it (4 B per lattice edge), the
+//   block emit over grids whose 32-cell chunks are laid out range-aligned in
+//   one global index space (mc_chunk.cuh).
 // * iso_batch_run with ISO_BATCH_GRAPH captures all of it in one CUDA graph
 //   and replays it; output capacities come from the previous run (the first
 //   run is eager and sizes them), and an overflow is detected on the device
@@ -44,6 +46,12 @@ iso_status mc_extract_grids(iso_ctx* ctx, const void* d_grids, uint32_t ngrids, 
 size_t mc_grid_bytes();
 void mc_fill_grid(void* dst, const Lattice& L, uint32_t chunk0, uint32_t* nchunks, uint32_t* cw);
 size_t mc_grids_scratch_bytes(uint32_t chunks, uint32_t ngrids);
+struct CellTable;
+CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n);
+void mc_table_destroy(CellTable* t);
+uint64_t mc_table_edges(const CellTable* t);
+iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, uint64_t cap_t, float* out_v,
+                            uint32_t* out_i, uint32_t* extents, uint64_t* totals, bool sync_sizes);
 }  // namespace iso
 
 using namespace iso;
@@ -73,6 +81,7 @@ struct Mixed {
     uint64_t keep;
 };
 constexpr uint32_t NO_BRICK = 0xFFFFFFFFu;
+constexpr uint32_t HELD = 16;  // primitives whose values a classifying lane keeps in shared memory
 
 __device__ __forceinline__ BrickLattice lattice_of(const SampleGrid& sg) {
     return BrickLattice{sg.pv.lip, sg.pv.slack, sg.n,     sg.n,  sg.n + 1, sg.inv,
@@ -83,9 +92,11 @@ __device__ __forceinline__ BrickLattice lattice_of(const SampleGrid& sg) {
 // another grid's primitives.  (Blocks that classified a tile, listed its
 // mixed sub-bricks in shared memory and sampled them between barriers spent
 // 44 % of their warps' time at those, on tiles of 20 sub-bricks for a 16^3
-// chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells.)
+// chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells; now 47 and 143 for
+// batch_rows, which issues in 73 % of its slots.)
 __global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const SampleGrid* grids, uint32_t ntasks,
                                                       Mixed* list, uint32_t* count) {
+    __shared__ float s_held[HELD][256];
     const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (t >= ntasks) return;
     const Task k = tasks[t];
@@ -100,7 +111,8 @@ __global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const S
     uint64_t keep = ~0ull;
     if (!have || (g.lip > 0.0f && xa >= g.nx)) cls = BRICK_OUT;  // no samples: sign bits stay clear
     else if (g.lip > 0.0f)
-        cls = brick_class(ev, g, xa, min(xa + 7, g.nx - 1), ya, min(ya + 3, g.ny - 1), za, min(za + 3, g.nz - 1), &keep);
+        cls = brick_class(ev, g, xa, min(xa + 7, g.nx - 1), ya, min(ya + 3, g.ny - 1), za, min(za + 3, g.nz - 1), &keep,
+                          &s_held[0][threadIdx.x], HELD, 256);
     const uint32_t mixed = __ballot_sync(0xFFFFFFFFu, cls == BRICK_MIXED);
     // the group's sign words: its four lanes take four rows each
     uint32_t cls4 = 0;
@@ -193,6 +205,8 @@ struct iso_batch {
     // extraction on the context may regrow (free and reallocate) them
     void* graph_v = nullptr;
     void* graph_i = nullptr;
+    void* graph_e = nullptr;  // its edge map (null: captured with the block emit)
+    CellTable* table = nullptr;
     bool sized = false;
     // iso_batch_run_per_chunk_async: each chunk as a grid of its own
     void* d_solo_grids = nullptr;
@@ -248,8 +262,18 @@ cudaError_t launch_sampler(iso_ctx* ctx, const Task* d_tasks, uint32_t ntasks, c
     return cudaGetLastError();
 }
 
-// enqueue the whole batch on the context's stream (no host sync)
-iso_status enqueue(iso_batch* b, bool sync_sizes) {
+// whether the cell passes can run: the table exists and the edge map is there
+bool edge_map_ready(iso_batch* b) {
+    if (!b->table) return false;
+    if (ensure(b->ctx, b->ctx->edges, 4 * mc_table_edges(b->table)) == ISO_OK) return true;
+    cudaGetLastError();
+    b->ctx->last_error.clear();
+    return false;
+}
+
+// enqueue the whole batch on the context's stream (sync_sizes: the counts are
+// read back before the emit)
+iso_status enqueue(iso_batch* b, bool cells, bool sync_sizes) {
     iso_ctx* ctx = b->ctx;
     {
         StageTimer timer(ctx, ISO_STAGE_SAMPLE);
@@ -257,6 +281,9 @@ iso_status enqueue(iso_batch* b, bool sync_sizes) {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch sampler");
     }
     ctx->launches += 2;
+    if (cells)
+        return mc_extract_table(ctx, b->table, b->cap_v, b->cap_t, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p,
+                                b->d_extents, b->d_totals, sync_sizes);
     return mc_extract_grids(ctx, b->d_grids, (uint32_t)b->chunks.size(), b->d_range_grid, b->total_chunks, b->max_cw,
                             b->d_scratch, b->cap_v, b->cap_t, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p,
                             b->d_extents, b->d_totals, sync_sizes);
@@ -353,6 +380,7 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
     b->d_scratch = base + scr_off;
     std::vector<char> grids(mc_grid_bytes() * nchunks);
     std::vector<uint32_t> range_grid(nranges);
+    std::vector<Lattice> lattices;
     b->sgrids.resize(nchunks);
     for (uint32_t i = 0; i < nchunks; ++i) {
         const uint32_t n = b->chunks[i].size;
@@ -361,6 +389,7 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
                       (uint32_t*)(base + bits_off[i]), words_per_row(n)};
         b->sgrids[i] = sg;
         Lattice L{n, n, n + 1, default_pitch(n), sg.field, sg.bits, sg.W, sg.inv, nullptr};
+        lattices.push_back(L);
         uint32_t nch = 0, cw = 0;
         mc_fill_grid(grids.data() + mc_grid_bytes() * i, L, b->grid_chunk0[i], &nch, &cw);
         for (uint32_t r = b->grid_chunk0[i] / 256; r < (b->grid_chunk0[i] + nch + 255) / 256; ++r) range_grid[r] = i;
@@ -377,6 +406,7 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
         iso_batch_destroy(b);
         return s;
     }
+    b->table = mc_table_create(ctx, lattices.data(), nchunks);
     *out = b;
     return ISO_OK;
 }
@@ -387,6 +417,7 @@ iso_status iso_batch_destroy(iso_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     if (b->d_tasks) cudaFree(b->d_tasks);
+    mc_table_destroy(b->table);
     if (b->arena) cudaFree(b->arena);
     if (b->d_solo_grids) cudaFree(b->d_solo_grids);
     delete b;
@@ -407,9 +438,10 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
     iso_status s = set_device(ctx);
     if (s != ISO_OK) return s;
     const bool graph = (flags & ISO_BATCH_GRAPH) != 0;
+    const bool cells = edge_map_ready(b);
     if (!graph || !b->sized) {
         // eager: sizes are read back between the count and the emit passes
-        s = enqueue(b, true);
+        s = enqueue(b, cells, true);
         if (s != ISO_OK) return s;
         if ((s = finish(b, info)) != ISO_OK) return s;
         if (!b->sized || ctx->last.num_vertices > b->cap_v || ctx->last.num_triangles > b->cap_t) {
@@ -429,7 +461,8 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
     }
     if ((s = ensure(ctx, ctx->mesh_v, 12 * b->cap_v)) != ISO_OK) return s;
     if ((s = ensure(ctx, ctx->mesh_i, 12 * b->cap_t)) != ISO_OK) return s;
-    if (b->exec && (b->graph_v != ctx->mesh_v.p || b->graph_i != ctx->mesh_i.p)) {
+    void* const edges = cells ? ctx->edges.p : nullptr;
+    if (b->exec && (b->graph_v != ctx->mesh_v.p || b->graph_i != ctx->mesh_i.p || b->graph_e != edges)) {
         cudaGraphExecDestroy(b->exec);
         cudaGraphDestroy(b->graph);
         b->exec = nullptr;
@@ -440,7 +473,7 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "begin capture");
         const bool timing = ctx->timing;
         ctx->timing = false;  // no events inside the graph
-        s = enqueue(b, false);
+        s = enqueue(b, cells, false);
         ctx->timing = timing;
         cudaGraph_t g = nullptr;
         e = cudaStreamEndCapture(ctx->stream, &g);
@@ -454,6 +487,7 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "instantiate graph");
         b->graph_v = ctx->mesh_v.p;
         b->graph_i = ctx->mesh_i.p;
+        b->graph_e = edges;
     }
     {
         StageTimer timer(ctx, ISO_STAGE_OTHER);

@@ -94,10 +94,13 @@ __host__ __device__ __forceinline__ uint32_t brick_count(uint32_t W, uint32_t ro
 }
 
 // Class of the sub-brick of samples [xa, xb] x [ya, yb] x [za, zb] and the
-// primitives it keeps (a program with a bound).
+// primitives it keeps (a program with a bound).  The values of the first
+// `nheld` primitives are held at held[0], held[stride], ... for the second
+// look at them (null: all are evaluated twice).
 template <class Ev>
 __device__ __forceinline__ uint32_t brick_class(const Ev& ev, const BrickLattice& g, uint32_t xa, uint32_t xb,
-                                                uint32_t ya, uint32_t yb, uint32_t za, uint32_t zb, uint64_t* keep) {
+                                                uint32_t ya, uint32_t yb, uint32_t za, uint32_t zb, uint64_t* keep,
+                                                float* held = nullptr, uint32_t nheld = 0, uint32_t stride = 0) {
     // both ends of a crossing edge lie within lip * inv of zero (rounded up);
     // a caller may need values further out (reach_steps > 1)
     const float reach = g.lip * g.inv * g.reach_steps * (1.0f + 1.0f / 1024.0f) + g.slack;
@@ -115,10 +118,13 @@ __device__ __forceinline__ uint32_t brick_class(const Ev& ev, const BrickLattice
             const float d = ev.prim(i, q);
             v = (i == 0) ? d : fminf(v, d);
             upper = fminf(upper, d + spread);
+            if (i < nheld) held[i * stride] = d;
         }
         uint64_t k = 0;
-        for (uint32_t i = 0; i < n; ++i)
-            if (!(ev.prim(i, q) - spread > upper)) k |= 1ull << i;
+        for (uint32_t i = 0; i < n; ++i) {
+            const float d = i < nheld ? held[i * stride] : ev.prim(i, q);
+            if (!(d - spread > upper)) k |= 1ull << i;
+        }
         *keep = k;
     } else {
         v = ev.value(c);
@@ -208,8 +214,9 @@ __device__ __forceinline__ uint32_t brick_group_bits(const BrickTile& T, uint32_
 // A pruned union is evaluated a primitive at a time over the lane's 4 x 4
 // points (values_kept): the primitive is read and told apart once for 16
 // points, and what depends on one or two of the coordinates is computed
-// once per coordinate.  The chunk batch's 1024 chunks, a point at a time:
-// 348 M warp instructions.
+// once per coordinate.  The chunk batch's 1024 chunks: 109 M warp
+// instructions for the mixed sub-bricks, 348 M with a point at a time
+// (classification included).
 template <class Ev>
 __device__ __forceinline__ void brick_fill(const Ev& ev, const BrickLattice& g, bool have, uint32_t sx, uint32_t ya,
                                            uint32_t za, uint32_t y1, uint32_t z1, uint64_t keep) {

@@ -619,6 +619,26 @@ cudaError_t emit_smem_attribute(size_t smem) {
 }
 }  // namespace
 
+// list entries per emitting warp: several pool their cells into full rounds
+// of 32, while that leaves about four waves of warps (a warp's chain of loads
+// takes a few us whatever its cells)
+static uint32_t emit_group(const iso_ctx* ctx, uint64_t nsegs) {
+    return (uint32_t)std::min<uint64_t>(4, std::max<uint64_t>(1, nsegs / (128 * (uint64_t)std::max(ctx->sms, 1))));
+}
+
+// layers per counting warp: long runs share the sign words between layers;
+// short ones keep the warps many (a step is one round trip to memory) and
+// their ends even
+static uint32_t count_run(const iso_ctx* ctx, uint64_t nsegs) {
+    return (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, nsegs / (160 * (uint64_t)std::max(ctx->sms, 1))));
+}
+
+// persistent: five blocks of 256 threads per SM, or a warp for every group the list could hold
+static unsigned cell_emit_blocks(const iso_ctx* ctx, const CellArgs& ca) {
+    const uint64_t groups = ca.nsegs / ca.group + ca.nblocks;
+    return (unsigned)std::min<uint64_t>((groups + 7) / 8, 5ull * (uint64_t)std::max(ctx->sms, 1));
+}
+
 // One synchronisation per extraction: count, scan and emit are queued back to
 // back, the emit writing into the context's mesh buffers as sized by earlier
 // extractions (its writes are capacity-checked); the totals come back with
@@ -653,11 +673,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     const size_t smem = block_emit_smem(CW);
     if (smem > 220 * 1024) return fail(ctx, ISO_ERR_INVALID_ARG, "rows too long for the emit pass");
     iso_status s;
-    // list entries per emitting warp: several pool their cells into full
-    // rounds of 32, while that leaves about four waves of warps (a warp's
-    // chain of loads takes a few us whatever its cells)
-    const uint32_t group = (uint32_t)std::min<uint64_t>(
-        4, std::max<uint64_t>(1, nsegs / (128 * (uint64_t)std::max(ctx->sms, 1))));
+    const uint32_t group = emit_group(ctx, nsegs);
     // cell passes: per segment its counts, active chunks and list entry (and
     // the padding of each scan block's part); block emit: per-chunk prefixes
     const size_t masks_at = (8 * (size_t)nsegs + 255) & ~(size_t)255;
@@ -683,10 +699,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     if (cells) {
         ca.grid = grid;
         ca.nsegs = (uint32_t)nsegs;
-        // layers per counting warp: long runs share the sign words between
-        // layers; short ones keep the warps many (a step is one round trip to
-        // memory) and their ends even
-        ca.run = (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, nsegs / (160 * (uint64_t)std::max(ctx->sms, 1))));
+        ca.run = count_run(ctx, nsegs);
         ca.ntasks = grid.SL * ((L.nz - 1 + ca.run - 1) / ca.run);
         ca.segs = (uint2*)ctx->rowtri.p;
         ca.masks = (uint32_t*)((char*)ctx->rowtri.p + masks_at);
@@ -730,10 +743,8 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
             if (cells) {
                 const CellEmitArgs ea{ca, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p, out_k, cap_v, cap_t,
                                       (uint32_t*)ctx->edges.p, H.v, H.cap_v, H.cap_t};
-                // persistent: five blocks of 256 threads per SM, or a warp for every group the list could hold
-                const uint64_t groups = nsegs / group + nblocks;
-                const uint64_t blocks = std::min<uint64_t>((groups + 7) / 8, 5ull * (uint64_t)std::max(ctx->sms, 1));
-                cudaError_t le = launch_pdl(mc_cell_emit<false>, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, ea);
+                cudaError_t le = launch_pdl(mc_cell_emit<false>, dim3(cell_emit_blocks(ctx, ca)), dim3(256), 0,
+                                            ctx->stream, ea);
                 if (le == cudaSuccess)
                     le = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream,
                                     (uint32_t*)ctx->mesh_i.p, (const uint64_t*)totals, cap_t,
@@ -981,6 +992,133 @@ void mc_fill_grid(void* dst, const Lattice& L, uint32_t chunk0, uint32_t* nchunk
     std::memcpy(dst, &g, sizeof(Grid));
     *nchunks = g.nchunks;
     *cw = g.CW;
+}
+
+// The cell passes over a table of lattices: the device table (lattices,
+// counting tasks, the lattice of every segment) and the passes' arrays, in
+// one allocation.
+struct CellTable {
+    CellArgs a{};
+    void* arena = nullptr;
+    uint32_t ngrids = 0, nedges = 0;
+};
+
+void mc_table_destroy(CellTable* t) {
+    if (!t) return;
+    if (t->arena) cudaFree(t->arena);
+    delete t;
+}
+
+// entries of the edge map the table's passes need (ctx->edges, 4 bytes each)
+uint64_t mc_table_edges(const CellTable* t) { return t->nedges; }
+
+// null: the lattices' edge keys or segments do not fit 32 bits (or the
+// allocation failed), and the block emit has to do
+CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n) {
+    uint64_t nsegs = 0, nedges = 0;
+    std::vector<Grid> grids(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        if (nsegs >= (1ull << 31) || nedges >= (1ull << 32)) return nullptr;
+        grids[i] = make_grid(L[i], 0, (uint32_t)nsegs, (uint32_t)nedges);
+        nsegs += (uint64_t)grids[i].SL * (L[i].nz - 1);
+        nedges += 3ull * L[i].nx * L[i].ny * L[i].nz;
+    }
+    if (nsegs >= (1ull << 31) || nedges >= (1ull << 32)) return nullptr;
+    const uint32_t run = count_run(ctx, nsegs);
+    std::vector<uint4> tasks;
+    std::vector<uint32_t> seg_grid(nsegs);
+    for (uint32_t i = 0; i < n; ++i) {
+        const Grid& g = grids[i];
+        std::fill_n(seg_grid.begin() + g.seg0, (size_t)g.SL * (g.nz - 1), i);
+        for (uint32_t z = 0; z < g.nz - 1; z += run)
+            for (uint32_t j = 0; j < g.SL; ++j) tasks.push_back(make_uint4(i, j, z, std::min(run, g.nz - 1 - z)));
+    }
+    CellTable* t = new CellTable();
+    t->ngrids = n;
+    t->nedges = (uint32_t)nedges;
+    CellArgs& a = t->a;
+    a.nsegs = (uint32_t)nsegs;
+    a.nblocks = (uint32_t)((nsegs + SCAN_BLOCK_SEGS - 1) / SCAN_BLOCK_SEGS);
+    a.group = emit_group(ctx, nsegs);
+    a.run = run;
+    a.ntasks = (uint32_t)tasks.size();
+    a.err = ctx->d_err;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = off;
+        off = (off + bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t g_at = take(sizeof(Grid) * n), t_at = take(16 * tasks.size()), sg_at = take(4 * nsegs),
+                 s_at = take(8 * nsegs), m_at = take(4 * nsegs), b_at = take(8ull * a.nblocks),
+                 l_at = take(16 * (nsegs + (uint64_t)a.group * a.nblocks)), c_at = take(64);
+    cudaError_t e = cudaMalloc(&t->arena, off);
+    char* base = (char*)t->arena;
+    if (e == cudaSuccess) e = cudaMemcpy(base + g_at, grids.data(), sizeof(Grid) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + t_at, tasks.data(), 16 * tasks.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + sg_at, seg_grid.data(), 4 * nsegs, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        mc_table_destroy(t);
+        return nullptr;
+    }
+    a.grids = (const Grid*)(base + g_at);
+    a.tasks = (const uint4*)(base + t_at);
+    a.seg_grid = (const uint32_t*)(base + sg_at);
+    a.segs = (uint2*)(base + s_at);
+    a.masks = (uint32_t*)(base + m_at);
+    a.blocks = (uint2*)(base + b_at);
+    a.list = (uint4*)(base + l_at);
+    a.ctrl = (uint32_t*)(base + c_at);
+    return t;
+}
+
+// Count, scan and emit of a table's lattices into one mesh (each lattice's
+// indices from its own first vertex) and their extents.  sync_sizes: the
+// counts are read back and size the context's mesh buffers before the emit;
+// otherwise it writes into out_v and out_i with the given capacities (no
+// host synchronisation: a graph capture).  ctx->edges holds the edge map.
+iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, uint64_t cap_t, float* out_v,
+                            uint32_t* out_i, uint32_t* extents, uint64_t* totals, bool sync_sizes) {
+    CellArgs a = t->a;
+    a.totals = totals;
+    cudaError_t e;
+    iso_status s;
+    {
+        StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
+        e = launch_pdl(mc_cell_count<true>, dim3((a.ntasks + 7) / 8), dim3(256), 0, ctx->stream, a);
+        if (e == cudaSuccess) e = launch_pdl(mc_cell_scan, dim3(a.nblocks), dim3(512), 0, ctx->stream, a);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "batch count");
+    }
+    if (sync_sizes) {
+        std::vector<uint2> blocks(a.nblocks);
+        e = cudaMemcpyAsync(blocks.data(), a.blocks, 8ull * a.nblocks, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "batch totals");
+        cap_v = cap_t = 0;
+        for (const uint2& b : blocks) {
+            cap_v += b.x;
+            cap_t += b.y;
+        }
+        if (cap_v >= (1ull << 31) || cap_t >= (1ull << 31)) return fail(ctx, ISO_ERR_TOO_LARGE, "batch mesh too large");
+        if ((s = ensure(ctx, ctx->mesh_v, 12 * std::max<uint64_t>(cap_v, 1))) != ISO_OK) return s;
+        if ((s = ensure(ctx, ctx->mesh_i, 12 * std::max<uint64_t>(cap_t, 1))) != ISO_OK) return s;
+        out_v = (float*)ctx->mesh_v.p;
+        out_i = (uint32_t*)ctx->mesh_i.p;
+    }
+    const CellEmitArgs ea{a, out_v, out_i, nullptr, cap_v, cap_t, (uint32_t*)ctx->edges.p, nullptr, 0, 0};
+    {
+        StageTimer timer(ctx, ISO_STAGE_EMIT);
+        e = launch_pdl(mc_cell_emit<true>, dim3(cell_emit_blocks(ctx, a)), dim3(256), 0, ctx->stream, ea);
+        if (e == cudaSuccess)
+            e = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream, out_i,
+                           (const uint64_t*)totals, cap_t, (const uint32_t*)ctx->edges.p, t->nedges,
+                           (uint32_t*)nullptr, (uint64_t)0, (uint64_t)0, cap_v);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "batch emit");
+        mc_cell_extents<<<(t->ngrids + 7) / 8, 256, 0, ctx->stream>>>(a, t->ngrids, (uint4*)extents);
+    }
+    ctx->launches += 5;
+    return check_launch(ctx, "batch emit");
 }
 
 size_t mc_grids_scratch_bytes(uint32_t chunks, uint32_t ngrids) {

@@ -22,7 +22,9 @@
 // chunk's eight words in each of two kernels and looked every active cell's
 // triangle count up: count and scan 55, emit 79.  401 x 401 x 301 samples of
 // a dense field: 18 + 8 + 114 against 48 + 126.  A dual lattice of 256^3: 9 +
-// 8 + 28 against 19 + 4 + 50 with the block emit.
+// 8 + 28 against 19 + 4 + 50 with the block emit.  A table of 1024 lattices
+// of 16^3 to 64^3 cells: 23 + 8 + 150 and 44 for the ids against 55 + 9 + 305
+// with the block emit.
 constexpr uint32_t SCAN_BLOCK_SEGS = 4096;  // segments per block of mc_cell_scan (512 threads x 8)
 
 struct CellArgs {
@@ -251,6 +253,21 @@ __device__ __forceinline__ void write_totals(const CellArgs& A, uint32_t lane) {
         A.totals[1] = v;
         if (v > 0xFFFFFFFFull || t > 0xFFFFFFFFull) atomicOr(A.err, DERR_CAPACITY);
     }
+}
+
+// Mesh extents of every lattice of a table (first vertex, vertices, first
+// triangle, triangles), a warp each, from the prefixes of its first segment
+// and of the one after its last.
+__global__ void __launch_bounds__(256) mc_cell_extents(CellArgs A, uint32_t ngrids, uint4* out) {
+    const uint32_t lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= ngrids) return;
+    auto prefix = [&](uint32_t seg) {
+        const uint2 b = blocks_before(A, seg < A.nsegs ? seg / SCAN_BLOCK_SEGS : A.nblocks, lane);
+        const uint2 p = seg < A.nsegs ? A.segs[seg] : make_uint2(0, 0);
+        return make_uint2(b.x + p.x, b.y + p.y);
+    };
+    const uint2 a = prefix(A.grids[i].seg0), b = prefix(i + 1 < ngrids ? A.grids[i + 1].seg0 : A.nsegs);
+    if (lane == 0) out[i] = make_uint4(a.x, b.x - a.x, a.y, b.y - a.y);
 }
 
 // ---------------------------------------------------------------- emission ---
