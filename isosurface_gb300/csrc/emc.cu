@@ -14,7 +14,7 @@
 //                  second list with their tangent planes
 //   emc_features   the feature points (MinimiseQEF), a few cells per warp, on
 //                  a side stream beside everything below but the last pass
-//   emc_scan       first vertex and first triangle of every block
+//   scan_block_sums  first vertex and first triangle of every block
 //   emc_offsets    those of every active cell
 //   emc_vertices   owned edge vertices; the edge map
 //   emc_triangles  marching-cubes triangles and fans, in traversal order
@@ -24,6 +24,7 @@
 
 #include <algorithm>
 
+#include "block_sums.cuh"
 #include "internal.h"
 
 #define ISO_TABLE static __device__ const
@@ -54,7 +55,7 @@ struct Feature {
 // device counters of one extraction
 struct Ctrl {
     uint32_t active, features;
-    uint32_t vertices, triangles;
+    uint2 totals;  // vertices, triangles
     unsigned long long flips;
 };
 
@@ -175,53 +176,11 @@ __global__ void __launch_bounds__(128) emc_count(emc::Args A, const uint32_t* li
     }
 }
 
-// Exclusive scan of the blocks' sums in place (triangles in the high half),
-// by one thread block, four entries per thread and turn.
-__global__ void __launch_bounds__(1024) emc_scan(unsigned long long* sums, uint32_t nblocks, Ctrl* ctrl) {
-    __shared__ unsigned long long part[32];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned long long carry = 0;
-    for (uint32_t b0 = 0; b0 < nblocks; b0 += 4096) {
-        const uint32_t at = b0 + 4 * threadIdx.x;
-        unsigned long long v[4], mine = 0;
-        for (uint32_t k = 0; k < 4; ++k) {
-            v[k] = at + k < nblocks ? sums[at + k] : 0;
-            mine += v[k];
-        }
-        unsigned long long incl = mine;
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += up;
-        }
-        if (lane == 31) part[w] = incl;
-        __syncthreads();
-        unsigned long long before = 0, all = 0;
-        for (uint32_t k = 0; k < 32; ++k) {
-            if (k < w) before += part[k];
-            all += part[k];
-        }
-        unsigned long long run = carry + before + incl - mine;
-        for (uint32_t k = 0; k < 4; ++k) {
-            // a block without active cells keeps its mark: emc_offsets skips it
-            if (at + k < nblocks) sums[at + k] = v[k] ? run : ~0ull;
-            run += v[k];
-        }
-        carry += all;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        ctrl->vertices = (uint32_t)carry;
-        ctrl->triangles = (uint32_t)(carry >> 32);
-    }
-}
-
 // First vertex and first triangle of every active cell (nothing reads those
 // of the others): a thread block per block of cells, four cells per thread.
 __global__ void __launch_bounds__(256) emc_offsets(emc::Args A, uint32_t cells, const unsigned long long* sums) {
-    __shared__ unsigned long long part[8];
     const unsigned long long base = sums[blockIdx.x];
-    if (base == ~0ull) return;
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (base == NO_ITEMS) return;
     const uint32_t c0 = blockIdx.x * BLOCK_CELLS + 4 * threadIdx.x;
     unsigned long long v[4], mine = 0;
     for (uint32_t k = 0; k < 4; ++k) {
@@ -236,15 +195,7 @@ __global__ void __launch_bounds__(256) emc_offsets(emc::Args A, uint32_t cells, 
         v[k] = (unsigned long long)nt << 32 | nv;
         mine += v[k];
     }
-    unsigned long long incl = mine;
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-        const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += up;
-    }
-    if (lane == 31) part[w] = incl;
-    __syncthreads();
-    unsigned long long run = base + incl - mine;
-    for (uint32_t k = 0; k < w; ++k) run += part[k];
+    unsigned long long run = offset_in_block(base, mine);
     for (uint32_t k = 0; k < 4; ++k) {
         if (v[k]) {
             A.voff[c0 + k] = (uint32_t)run;
@@ -351,12 +302,12 @@ static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t n
     if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counts");
     const Ctrl* h = (const Ctrl*)ctx->h_pinned;
     const uint32_t nactive = h->active, nfeat = h->features;
-    if ((s = ensure(ctx, ctx->mesh_v, 12ull * h->vertices + 16)) != ISO_OK) return s;
-    if ((s = ensure(ctx, ctx->mesh_i, 12ull * h->triangles + 16)) != ISO_OK) return s;
+    if ((s = ensure(ctx, ctx->mesh_v, 12ull * h->totals.x + 16)) != ISO_OK) return s;
+    if ((s = ensure(ctx, ctx->mesh_i, 12ull * h->totals.y + 16)) != ISO_OK) return s;
     A.vertices = (float*)ctx->mesh_v.p;
     A.indices = (uint32_t*)ctx->mesh_i.p;
-    A.cap_v = h->vertices;
-    A.cap_t = h->triangles;
+    A.cap_v = h->totals.x;
+    A.cap_t = h->totals.y;
     if (nactive) {
         StageTimer timer(ctx, ISO_STAGE_EMIT);
         emc_vertices<<<grid_for(ctx, nactive, 128, 32), 128, 0, ctx->stream>>>(A, active, ctrl);
@@ -440,7 +391,7 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
         // nor wait for them
         if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
         emc_features<<<(unsigned)(4 * std::max(ctx->sms, 1)), 32, 0, side>>>(A, kept, cap, ctrl);
-        emc_scan<<<1, 1024, 0, ctx->stream>>>(sums, nblocks, ctrl);
+        scan_block_sums<<<1, 1024, 0, ctx->stream>>>(sums, nblocks, &ctrl->totals);
         ctx->launches += 2;
     }
     s = emc_emit(ctx, A, cells, nblocks, cap, active, features, kept, ctrl, sums);

@@ -140,11 +140,11 @@ struct iso_ctx {
         uint64_t prog_uid = 0;
         uint32_t depth = 0, flags = 0;
         void* bufs[6] = {};
-        std::vector<uint32_t> nref;
-        uint32_t ncubes = 0, nt = 0, nv = 0;
+        uint32_t nodes = 0, ncubes = 0, nt = 0, nv = 0;
         uint64_t launches = 0;
     } lhmc_plan;
     uint64_t lhmc_last_key[3] = {};
+    uint64_t lhmc_room = 0;  // nodes the largest octree so far was given room for
 };
 
 namespace iso {

@@ -4,27 +4,48 @@
 // (src/linear_hashed_octree.rs:30-51), with Morton keys (src/morton.rs).
 //
 // GPU form:
-// 1. Octree build, one generation at a time: evaluate the source at every
-//    frontier node's centre, apply should_refine (level < 2 || (level <
-//    max_depth && |d| < size * sqrt 3)), and write the children of refined
-//    nodes, in order, as the next frontier.  Generation g holds keys with
-//    3g+1 bits in ascending order, so the concatenated node array is sorted
-//    and a binary search replaces the HashMap<Morton, Node>.
-// 2. Primal vertices: every leaf emits primal_vertex(level, i) for i < 8; a
-//    GPU hash table keeps, per vertex, the deepest level (the reference's
-//    max-level map) and, among leaves of that level, the smallest key.  That
-//    leaf owns the vertex, which gives a deterministic order (leaf order, then
-//    i) for the walk the reference does in HashMap order.
+// 1. Octree build in one cooperative launch (oct_build), generation by
+//    generation: evaluate the source
+//    at the centres of the children of every refined node, apply
+//    should_refine (level < 2 || (level < max_depth && |d| < size * sqrt 3)),
+//    and append them in order.  Where a refined node's children go follows
+//    from how many nodes before it are refined, which the previous generation
+//    left as sums over tiles of nodes; the generations' sizes stay on the
+//    device.  Generation g holds keys with 3g+1 bits in ascending order.
+// 2. Primal vertices: every leaf emits primal_vertex(level, i) for i < 8; the
+//    reference keeps, per vertex, the deepest level (its max-level map).  Of
+//    the leaves of that level the one with the smallest key owns the vertex
+//    here, which gives a deterministic order (leaf order, then i) for the walk
+//    the reference does in HashMap order.  A leaf finds out alone: the cells
+//    of its level around the vertex are nodes that are refined (deeper leaves
+//    have it), leaves (the smaller key has it) or part of a coarser leaf.
+//    That takes the families around: a warp per family of eight children
+//    looks up the 27 families around it and tests the family's 27 vertices.
 // 3. Dual cubes: for each primal vertex and corner i, dual_vertex(level,
 //    REMAP_CUBE[i]) walks parent() until a node exists; the corner is that
 //    node's centre and value.  A corner with no ancestor keeps the previous
 //    corner's data in the reference (an order-dependent case); it is counted
 //    and reported through iso_lhmc_stale_corners.  No input reaches it: all
 //    64 level-2 nodes always exist and primal vertices lie strictly inside,
-//    so every walk meets a node at level 2 or deeper.
-// 4. Marching cubes on the dual cubes with MortonKey dedup: each vertex is
+//    so every walk meets a node at level 2 or deeper.  The same warps find
+//    them once the vertices before theirs are counted: a corner is a child of
+//    one of the 27 families, or the node one of those walks ends at.  The
+//    cubes with corners on both sides go to a list, which the later passes
+//    walk.
+// 4. Marching cubes on the listed cubes with MortonKey dedup: each vertex is
 //    owned by the first (cube, first-use rank) that references its key, found
 //    with a 64-bit atomicMin in a second hash table.
+//
+// The host waits twice: for the number of nodes (it sizes the arrays) and for
+// the mesh, which is written into the buffers as earlier extractions sized
+// them and again where it did not fit.  Every later size is bounded by the
+// nodes: splitting a cell adds at most 19 vertices to the octree's 8 nodes,
+// so vertices and cubes are below 3 per node.
+//
+// csg at depth 8 (313 k nodes, 502 k cubes): 690 us with a host round trip
+// and three to five launches per generation, hash tables of vertices (128 MB)
+// and edges (64 MB) with three lookups per visit, and every pass over all
+// cubes.
 //
 // The reference's output order is that of a RandomState HashMap, so only the
 // triangle set (keyed by MortonKey pairs) is defined; this order is
@@ -34,8 +55,10 @@
 #include <cstring>
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
+#include "block_sums.cuh"
 #include "internal.h"
 #include "vm.cuh"
 #define ISO_TABLE static __device__ const
@@ -105,9 +128,11 @@ __device__ inline V3 center(uint64_t k) {  // morton.rs:78-116
     bz &= length_mask;
     by &= length_mask;
     bx &= length_mask;
-    const float s = 1.0f / (float)((uint64_t)2 << lv);
+    // coordinates are below 2^21: as 32-bit numbers they convert on the FP32
+    // side, where 64-bit ones go through the (slow) f64 unit
+    const float s = 1.0f / (float)(2u << lv);
     const float s2 = s * 2.0f;
-    return v3((float)bx * s2 + s, (float)by * s2 + s, (float)bz * s2 + s);
+    return v3((float)(uint32_t)bx * s2 + s, (float)(uint32_t)by * s2 + s, (float)(uint32_t)bz * s2 + s);
 }
 __device__ inline uint64_t primal_vertex(uint64_t self, int lv, uint64_t which) {  // morton.rs:120-136
     const uint64_t k = 1ull << (3 * lv);
@@ -128,25 +153,29 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-// open-addressing table: key 0 = empty; returns the slot or UINT32_MAX when full
-__device__ __forceinline__ uint32_t ht_insert(unsigned long long* keys, uint32_t mask, uint64_t key) {
+// open-addressing table of (key, value) slots: key 0 = empty; the slot, or
+// NO_SLOT when full
+struct alignas(16) Slot {
+    unsigned long long key, val;
+};
+constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
+
+// The slot of `key`, taken if it has none; *val: a value the slot has held (a
+// slot's value only moves one way, so one that `key`'s code cannot improve on
+// needs no atomic; neither does a key that is already there).
+__device__ __forceinline__ uint32_t ht_insert(Slot* table, uint32_t mask, uint64_t key, unsigned long long* val) {
     uint32_t slot = (uint32_t)mix64(key) & mask;
     for (uint32_t probe = 0; probe <= mask; ++probe) {
-        const unsigned long long prev = atomicCAS(keys + slot, 0ull, (unsigned long long)key);
-        if (prev == 0ull || prev == key) return slot;
+        const ulonglong2 q = __ldcg(reinterpret_cast<const ulonglong2*>(table + slot));
+        *val = q.y;
+        if (q.x == key) return slot;
+        if (q.x == 0ull) {
+            const unsigned long long prev = atomicCAS(&table[slot].key, 0ull, (unsigned long long)key);
+            if (prev == 0ull || prev == key) return slot;
+        }
         slot = (slot + 1) & mask;
     }
-    return 0xFFFFFFFFu;
-}
-__device__ __forceinline__ uint32_t ht_find(const unsigned long long* keys, uint32_t mask, uint64_t key) {
-    uint32_t slot = (uint32_t)mix64(key) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-        const unsigned long long k = keys[slot];
-        if (k == key) return slot;
-        if (k == 0ull) return 0xFFFFFFFFu;
-        slot = (slot + 1) & mask;
-    }
-    return 0xFFFFFFFFu;
+    return NO_SLOT;
 }
 
 // ----------------------------------------------------------- exclusive scan ---
@@ -235,174 +264,415 @@ __global__ void __launch_bounds__(1024) scan_small(const uint32_t* in, uint32_t*
 }
 
 // ------------------------------------------------------------ octree build ---
-struct GenArgs {
+constexpr uint32_t TILE = 32;     // nodes with one count of refined ones
+constexpr uint32_t SUPER = 64;    // tiles with one
+constexpr uint32_t MAX_GENS = 16; // of any octree (keys fit 31 bits)
+constexpr uint32_t BLOCK_FAMILIES = 32;  // families with one sum of primal vertices (block_sums.cuh)
+constexpr uint32_t BLOCK_CUBES = 256;    // cubes with one sum of vertices and triangles
+
+// what the passes find out, read back by the host in one copy
+struct Ctl {
+    uint32_t nodes;
+    uint32_t arrived;                       // blocks at the barriers of oct_build
+    uint32_t pad[30];
+    uint32_t released, pad2;                // turns of the barrier that are over (a cache line of its own)
+    unsigned long long need;                // nodes the arena had no room for (0: all fit)
+    unsigned long long work;                // crossing edges of the listed cubes << 32 | listed cubes
+    unsigned long long stale;
+    uint2 cubes;                            // dual cubes, 0
+    uint2 mesh;                             // vertices, triangles
+};
+
+struct OctArgs {
     ProgView pv;
     unsigned long long* keys;  // all nodes, BFS (= ascending) order
     float* vals;
-    uint32_t* refine;         // 1 = refined
-    uint32_t off, cnt;        // this generation
+    uint8_t* refine;           // per family (nodes 8 f + 1 .. 8 f + 8): its refined children
+    unsigned long long* families;  // refined node's key << 32 | its first child (family_insert)
+    uint32_t fmask;
+    uint32_t cap;
     uint32_t max_depth;
-};
-
-__global__ void oct_eval(GenArgs A) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.cnt) return;
-    const uint64_t key = A.keys[A.off + i];
-    const float d = eval_scalar(A.pv, morton::center(key));  // construct_node, implicit_octree.rs:56-59
-    const int lv = morton::level(key);
-    const float sz = 1.0f / (float)((uint64_t)2 << lv);
-    // should_refine (implicit_octree.rs:47-55) with Signed::within_extent (distance.rs:60-62)
-    const bool r = lv < 2 || (lv < (int)A.max_depth && fabsf(d) < sz * 1.73205080757f);
-    A.vals[A.off + i] = d;
-    A.refine[A.off + i] = r ? 1u : 0u;
-}
-
-__global__ void set_root(unsigned long long* keys) { keys[0] = 1ull; }
-
-__global__ void oct_expand(unsigned long long* keys, const uint32_t* refine, const uint32_t* rank, uint32_t off,
-                           uint32_t cnt, uint32_t next_off) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cnt || !refine[off + i]) return;
-    const uint64_t key = keys[off + i];
-    const uint32_t at = next_off + 8 * rank[i];
-    for (uint32_t c = 0; c < 8; ++c) keys[at + c] = (key << 3) | c;  // Morton::child
-}
-
-// ----------------------------------------------------------- primal vertices ---
-constexpr uint64_t MASK58 = (1ull << 58) - 1;
-
-__device__ __forceinline__ uint64_t owner_code(int lv, uint64_t key) { return ((uint64_t)lv << 58) | (MASK58 - key); }
-
-struct LeafArgs {
-    const unsigned long long* keys;
-    const uint32_t* refine;
-    uint32_t nodes;
-    unsigned long long* hkeys;
-    unsigned long long* hvals;
-    uint32_t hmask;
-    uint32_t* counts;   // per node: owned primal vertices
+    uint32_t* tiles;           // refined nodes of every tile, of every super tile: generation g's from
+    uint32_t* supers;          // off / TILE + g and off / (TILE * SUPER) + g
+    Ctl* c;
     uint32_t* err;
 };
 
-__global__ void leaf_insert(LeafArgs A) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t node = t >> 3, i = t & 7;
-    if (node >= A.nodes || A.refine[node]) return;
-    const uint64_t key = A.keys[node];
+__device__ __forceinline__ bool oct_node(const OctArgs& A, uint32_t at, uint64_t key) {
+    const float d = eval_scalar(A.pv, morton::center(key));  // construct_node, implicit_octree.rs:56-59
     const int lv = morton::level(key);
-    const uint64_t v = morton::primal_vertex(key, lv, i);
-    if (v == 0) return;
-    const uint32_t slot = ht_insert(A.hkeys, A.hmask, v);
-    if (slot == 0xFFFFFFFFu) {
-        atomicOr(A.err, DERR_CAPACITY);
-        return;
-    }
-    atomicMax(A.hvals + slot, (unsigned long long)owner_code(lv, key));
+    const float sz = 1.0f / (float)(2u << lv);
+    // should_refine (implicit_octree.rs:47-55) with Signed::within_extent (distance.rs:60-62)
+    const bool r = lv < 2 || (lv < (int)A.max_depth && fabsf(d) < sz * 1.73205080757f);
+    A.keys[at] = key;
+    A.vals[at] = d;
+    return r;
 }
 
-__global__ void leaf_count(LeafArgs A) {
-    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= A.nodes) return;
-    uint32_t n = 0;
-    if (!A.refine[node]) {
-        const uint64_t key = A.keys[node];
-        const int lv = morton::level(key);
-        for (uint32_t i = 0; i < 8; ++i) {
-            const uint64_t v = morton::primal_vertex(key, lv, i);
-            if (v == 0) continue;
-            const uint32_t slot = ht_find(A.hkeys, A.hmask, v);
-            if (slot != 0xFFFFFFFFu && A.hvals[slot] == owner_code(lv, key)) ++n;
-        }
+// The nodes by key: a refined node's eight children follow one another in the
+// node array, so a table of the refined nodes (0 empty, at most half full)
+// finds any node with an eighth of the entries.  A refined node's key fits 32
+// bits at the depths allowed.
+__device__ __forceinline__ uint32_t family_slot(uint64_t parent, uint32_t mask) {
+    const uint32_t h = (uint32_t)parent * 0x9E3779B1u;
+    return (h ^ h >> 15) & mask;
+}
+__device__ __forceinline__ void family_insert(const OctArgs& A, uint64_t parent, uint32_t first) {
+    uint32_t slot = family_slot(parent, A.fmask);
+    for (uint32_t probe = 0; probe <= A.fmask; ++probe) {
+        if (atomicCAS(A.families + slot, 0ull, parent << 32 | first) == 0ull) return;
+        slot = (slot + 1) & A.fmask;
     }
-    A.counts[node] = n;
+}
+// the first child of the node with key `parent`, 0 if that is no refined node
+__device__ __forceinline__ uint32_t find_family(const unsigned long long* families, uint32_t mask, uint64_t parent) {
+    uint32_t slot = family_slot(parent, mask);
+    for (uint32_t probe = 0; probe <= mask; ++probe) {
+        const unsigned long long w = __ldg(families + slot);
+        if (w == 0ull) return 0;
+        if (w >> 32 == parent) return (uint32_t)w;
+        slot = (slot + 1) & mask;
+    }
+    return 0;
 }
 
-__global__ void leaf_write(LeafArgs A, const uint32_t* offsets, unsigned long long* pv_key, uint8_t* pv_level) {
-    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= A.nodes || A.refine[node]) return;
-    const uint64_t key = A.keys[node];
-    const int lv = morton::level(key);
-    uint32_t at = offsets[node];
-    for (uint32_t i = 0; i < 8; ++i) {
-        const uint64_t v = morton::primal_vertex(key, lv, i);
-        if (v == 0) continue;
-        const uint32_t slot = ht_find(A.hkeys, A.hmask, v);
-        if (slot != 0xFFFFFFFFu && A.hvals[slot] == owner_code(lv, key)) {
-            pv_key[at] = v;
-            pv_level[at] = (uint8_t)lv;
-            ++at;
+// All blocks of the (cooperative) launch have come here `turn` times; the
+// last one to come releases the others, which wait on a word of its own.
+// Bounded, and reported when the bound is reached.
+constexpr uint32_t BARRIER_SPINS = 1u << 22;
+__device__ __forceinline__ void grid_barrier(Ctl* c, uint32_t turn, uint32_t* err) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&c->arrived, 1u) + 1 == turn * gridDim.x) {
+            __threadfence();
+            *(volatile uint32_t*)&c->released = turn;
+        } else {
+            uint32_t spins = 0;
+            while (*(volatile uint32_t*)&c->released < turn && ++spins < BARRIER_SPINS) __nanosleep(20);
+            if (spins == BARRIER_SPINS) atomicOr(err, DERR_QUEUE_TIMEOUT);
+        }
+        __threadfence();
+    }
+    __syncthreads();
+}
+
+// The whole octree in one cooperative launch, a grid barrier between
+// generations.  Bound by one evaluation's chain per generation: launched
+// generation by generation the interpreter's code and the program came from
+// L2 again each time (10-18 us each; 95 us for csg at depth 8).
+// Generations 0 to 2 (nodes 0, 1-8 and 9-72) every octree has; after that a
+// block takes the refined nodes of a tile and evaluates their children.
+// What other blocks wrote is read past L1.
+__global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
+    __shared__ unsigned long long s_key[TILE];
+    __shared__ uint32_t s_sum[8], s_n;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    auto block_sum = [&](uint32_t v) {
+        v = __reduce_add_sync(FULL, v);
+        __syncthreads();  // the previous sum and the previous tile are used
+        if (lane == 0) s_sum[tid >> 5] = v;
+        __syncthreads();
+        uint32_t all = 0;
+        for (int k = 0; k < 8; ++k) all += s_sum[k];
+        return all;
+    };
+    if (blockIdx.x == 0 && tid < 96) {
+        // nodes 1-72 to threads 0-71, so that families are eights of lanes
+        const uint32_t at = tid == 72 ? 0 : tid + 1;
+        bool r = false;
+        if (tid <= 72) r = oct_node(A, at, at == 0 ? 1 : at < 9 ? 7 + at : 55 + at);
+        const uint32_t m = __ballot_sync(FULL, r) >> (lane & ~7u) & 0xFFu;
+        if (tid < 72 && (tid & 7) == 0) {
+            A.refine[at >> 3] = (uint8_t)m;
+            family_insert(A, at == 1 ? 1 : 7 + (at >> 3), at);
+            if (at >= 9) {
+                atomicAdd(A.tiles + 9 / TILE + 2 + (at - 9) / TILE, (uint32_t)__popc(m));
+                atomicAdd(A.supers + 9 / (TILE * SUPER) + 2, (uint32_t)__popc(m));
+            }
         }
     }
+    uint32_t off = 9, cnt = 64;
+    for (uint32_t g = 2; g < last; ++g) {
+        grid_barrier(A.c, g - 1, A.err);
+        const uint32_t next = off + cnt;
+        const uint32_t ntiles = (cnt + TILE - 1) / TILE, nsupers = (ntiles + SUPER - 1) / SUPER;
+        const uint32_t* tiles = A.tiles + off / TILE + g;
+        const uint32_t* supers = A.supers + off / (TILE * SUPER) + g;
+        uint32_t* ntile = A.tiles + next / TILE + g + 1;
+        uint32_t* nsuper = A.supers + next / (TILE * SUPER) + g + 1;
+        for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const uint32_t s = t / SUPER;
+            uint32_t sum = 0;
+            for (uint32_t k = tid; k < s; k += 256) sum += __ldcg(supers + k);
+            for (uint32_t k = s * SUPER + tid; k < t; k += 256) sum += __ldcg(tiles + k);
+            const uint32_t before = block_sum(sum);
+            // the tile's refined nodes, in order
+            const uint32_t i = t * TILE + tid;
+            if (tid < TILE) {
+                const uint32_t at = off + i;  // node 8 f + 1 + bit
+                const bool r = i < cnt && (__ldcg(A.refine + ((at - 1) >> 3)) >> ((at - 1) & 7) & 1);
+                const uint32_t m = __ballot_sync(FULL, r);
+                if (r) s_key[__popc(m & ((1u << lane) - 1u))] = __ldcg(A.keys + at);
+                if (lane == 0) s_n = __popc(m);
+            }
+            __syncthreads();
+            const uint32_t n = 8 * s_n;
+            for (uint32_t c0 = 0; c0 < n; c0 += 256) {
+                const uint32_t c = c0 + tid, rel = 8 * before + c;
+                bool cr = false;
+                if (c < n && next + rel < A.cap)
+                    cr = oct_node(A, next + rel, s_key[c >> 3] << 3 | (c & 7));  // Morton::child
+                const uint32_t cm = __ballot_sync(FULL, cr) >> (lane & ~7u) & 0xFFu;
+                if ((lane & 7) == 0 && c < n && next + rel < A.cap) {  // a family lies in one tile
+                    A.refine[(next + rel) >> 3] = (uint8_t)cm;
+                    family_insert(A, s_key[c >> 3], next + rel);
+                    if (cm) {
+                        atomicAdd(ntile + rel / TILE, (uint32_t)__popc(cm));
+                        atomicAdd(nsuper + rel / (TILE * SUPER), (uint32_t)__popc(cm));
+                    }
+                }
+            }
+        }
+        // the next generation's size, in every block
+        uint32_t sum = 0;
+        for (uint32_t k = tid; k < nsupers; k += 256) sum += __ldcg(supers + k);
+        const uint64_t children = 8ull * block_sum(sum);
+        const bool fits = next + children <= A.cap;
+        off = next;
+        cnt = fits ? (uint32_t)children : 0u;
+        if (cnt == 0) {
+            if (blockIdx.x == 0 && tid == 0 && !fits) A.c->need = next + children;
+            break;
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) A.c->nodes = off + cnt;
 }
 
 // ---------------------------------------------------------------- dual cubes ---
 struct CubeArgs {
-    const unsigned long long* ntable;  // node key -> index (node_insert)
-    uint32_t nmask;
+    const unsigned long long* nkeys;
     const float* nvals;
-    const unsigned long long* pv_key;
-    const uint8_t* pv_level;
-    uint32_t ncubes;
-    uint32_t* corner;      // 8 node indices per cube (UINT32_MAX: no ancestor)
-    uint8_t* cases;
-    uint32_t* tri_counts;
-    unsigned long long* stale;
+    const uint8_t* refine;
+    const unsigned long long* families;
+    uint32_t fmask;
+    uint32_t nfamilies;
+    uint8_t* fcount;         // per family: primal vertices its children own
+    unsigned long long* fsums;  // per BLOCK_FAMILIES families
+    uint32_t cap;            // room for cubes
+    Ctl* c;
+    uint8_t* cases;          // per cube
+    uint2* list;             // listed cubes (both kinds of corners): cube, case
+    uint32_t* corner;        // 8 node indices per listed cube (UINT32_MAX: no ancestor)
+    uint32_t* slots;         // 12 per listed cube: the slots of its edges' keys, by first-use rank
+    Slot* table;             // edge key -> first visitor: cube << 4 | first-use rank
+    uint32_t table_cap;
+    uint16_t* owned;         // per cube: owned first-use ranks
+    unsigned long long* sums;  // per BLOCK_CUBES cubes: triangles << 32 | vertices
+    uint32_t *vbase, *tbase;   // per cube, of the listed ones
+    float* out_v;
+    uint32_t* out_i;
+    uint64_t* out_k;
+    uint32_t cap_v, cap_t;
+    uint32_t* err;
 };
 
-// Node key -> index for the parent walks: open addressing over
-// (key << 32 | index) words, 0 empty (keys lie in [1, 2^31)), at most half
-// full, so a lookup takes one or two probes where a binary search over the
-// sorted keys took twenty dependent loads.
-__global__ void node_insert(const unsigned long long* keys, uint32_t n, unsigned long long* table, uint32_t mask) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t key = keys[i];
-    const unsigned long long word = (key << 32) | i;
-    uint32_t slot = (uint32_t)mix64(key) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-        if (atomicCAS(table + slot, 0ull, word) == 0ull) return;
-        slot = (slot + 1) & mask;
+// What a warp knows of family f (first child 8 f + 1) and its surroundings:
+// lane n < 27 looks after the family at offset (n % 3, n / 3 % 3, n / 9) - 1
+// and the vertex at that offset (0..2 per axis, in children's sizes).
+struct Around {
+    uint32_t first;  // that family's first child, 0: none
+    uint32_t refine; // its refined children
+    uint64_t key;    // its parent's key
+    bool own;        // a child of this family owns the lane's vertex
+    uint32_t code;   // child * 8 + vertex of it
+    uint32_t lo, hi; // the set of all such codes (in every lane)
+};
+
+// the cells around vertex offset v on one axis: cell a = 0 (below), 1 (above)
+// is child bit `bit` of the family at offset `fam`
+__device__ __forceinline__ uint32_t axis_fam(uint32_t v, uint32_t a) { return (v + 1 + a) >> 1; }
+__device__ __forceinline__ uint32_t axis_bit(uint32_t v, uint32_t a) { return (v + 1 + a) & 1; }
+
+__device__ __forceinline__ Around look_around(const CubeArgs& A, uint32_t f) {
+    const uint32_t lane = threadIdx.x & 31, n = min(lane, 26u);
+    const uint32_t vx = n % 3, vy = n / 3 % 3, vz = n / 9;
+    const uint64_t P = __ldg(A.nkeys + 8 * f + 1) >> 3;
+    const int L = (63 - __clzll((long long)P)) / 3;
+    Around q;
+    // (P - (1, 1, 1)) + offset, per axis; past the domain's faces this is some
+    // other key, which only a vertex on the face would look at
+    q.key = morton::add(morton::sub(P, 7), (uint64_t)((vx & 1) | (vx >> 1) << 3 | (vy & 1) << 1 | (vy >> 1) << 4 |
+                                                       (vz & 1) << 2 | (vz >> 1) << 5));
+    q.first = n == 13 ? 8 * f + 1 : find_family(A.families, A.fmask, q.key);
+    q.refine = q.first ? __ldg(A.refine + (q.first >> 3)) : 0u;
+    // strictly inside the domain (primal_vertex, morton.rs:120-136)
+    const uint64_t lead = 1ull << (3 * L), low = P ^ lead;
+    auto inside = [&](uint32_t v, uint64_t axis) {
+        const uint64_t all = axis & (lead - 1), at = low & axis;
+        return !(v == 0 && at == 0) && !(v == 2 && at == all);
+    };
+    bool own = lane < 27 && inside(vx, morton::DILATE_TX) && inside(vy, morton::DILATE_TY) && inside(vz, morton::DILATE_TZ);
+    uint64_t least = ~0ull;
+    uint32_t mine = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t a = k & 1, b = k >> 1 & 1, c = k >> 2;
+        const uint32_t from = axis_fam(vx, a) + 3 * axis_fam(vy, b) + 9 * axis_fam(vz, c);
+        const uint32_t ci = axis_bit(vx, a) | axis_bit(vy, b) << 1 | axis_bit(vz, c) << 2;
+        const uint32_t word = __shfl_sync(FULL, q.refine | (q.first ? 256u : 0u), from);
+        const uint64_t key = (uint64_t)__shfl_sync(FULL, (uint32_t)q.key, from) << 3 | ci;
+        if (!(word & 256u)) continue;  // a coarser leaf's
+        if (word >> ci & 1u) own = false;
+        // key 8^lv has one level less by morton::level, and no vertices
+        if (key < least && key != lead << 3) {
+            least = key;
+            mine = from == 13 ? ci + 1 : 0;
+        }
+    }
+    q.own = own && mine;
+    const uint32_t child = mine - 1;
+    q.code = 8 * child + ((vx - (child & 1)) | (vy - (child >> 1 & 1)) << 1 | (vz - (child >> 2)) << 2);
+    q.lo = __reduce_or_sync(FULL, q.own && q.code < 32 ? 1u << q.code : 0u);
+    q.hi = __reduce_or_sync(FULL, q.own && q.code >= 32 ? 1u << (q.code - 32) : 0u);
+    return q;
+}
+
+// Primal vertices of every family: a warp each, a block's 8 warps over
+// BLOCK_FAMILIES.  (A hash table of vertices with an insertion per leaf and
+// corner and two lookups took 41 + 31 + 33 us for 313 k nodes, a lane per
+// leaf and corner with its seven lookups 72.)
+__global__ void __launch_bounds__(256) family_count(CubeArgs A) {
+    __shared__ uint32_t s_n[8];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t n = 0;
+    for (uint32_t k = warp; k < BLOCK_FAMILIES; k += 8) {
+        const uint32_t f = blockIdx.x * BLOCK_FAMILIES + k;
+        if (f >= A.nfamilies) break;
+        const Around q = look_around(A, f);
+        const uint32_t own = __popc(q.lo) + __popc(q.hi);
+        if (lane == 0) A.fcount[f] = (uint8_t)own;
+        n += own;
+    }
+    if (lane == 0) s_n[warp] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+        for (int w = 0; w < 8; ++w) all += s_n[w];
+        A.fsums[blockIdx.x] = all;
     }
 }
 
-__device__ __forceinline__ uint32_t find_node(const unsigned long long* table, uint32_t mask, uint64_t key) {
-    uint32_t slot = (uint32_t)mix64(key) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-        const unsigned long long w = __ldg(table + slot);
-        if (w == 0ull) return 0xFFFFFFFFu;
-        if ((w >> 32) == key) return (uint32_t)w;
-        slot = (slot + 1) & mask;
+// The dual cubes of the families' vertices (in order of leaf, then vertex):
+// corners, case, and the list of those with corners on both sides, with one
+// place in it for a block's eight families (one for every warp's cubes, all
+// at one address, cost more than the walks).
+__global__ void __launch_bounds__(256) cube_gather(CubeArgs A) {
+    __shared__ uint32_t s_listed[8], s_edges[8], s_base;
+    const unsigned long long base = A.fsums[blockIdx.x];
+    if (base == NO_ITEMS) return;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, f0 = blockIdx.x * BLOCK_FAMILIES;
+    // vertices before each of the block's families (lane = family)
+    const uint32_t count = f0 + lane < A.nfamilies ? A.fcount[f0 + lane] : 0u;
+    uint32_t before = count;
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(FULL, before, o);
+        if (lane >= o) before += up;
     }
-    return 0xFFFFFFFFu;
+    before += (uint32_t)base - count;
+    for (uint32_t k = warp; k < BLOCK_FAMILIES; k += 8) {
+        const uint32_t f = f0 + k, n = __shfl_sync(FULL, count, k), j0 = __shfl_sync(FULL, before, k);
+        bool listed = false;
+        uint32_t corner[8], cs = 0, j = 0;
+        if (n) {  // warp-uniform
+            Around q = look_around(A, f);
+            // where there is no family, or its children's keys are past 32
+            // bits, the walk goes on at its parent
+            uint32_t ref = q.first;
+            if (lane < 27 && (!q.first || q.key >> 29)) {
+                uint64_t m = q.key;
+                uint32_t found = 0xFFFFFFFFu;
+                while (m > 1) {
+                    const uint32_t g = m >> 32 ? 0u : find_family(A.families, A.fmask, m >> 3);
+                    if (g) {
+                        found = g + (uint32_t)(m & 7);
+                        break;
+                    }
+                    m = morton::parent(m);
+                }
+                ref = found;
+                q.first = 0;
+            }
+            const uint32_t vx = min(lane, 26u) % 3, vy = min(lane, 26u) / 3 % 3, vz = min(lane, 26u) / 9;
+            uint32_t prev = 0xFFFFFFFFu;
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                constexpr uint8_t REMAP[8] = {2, 3, 1, 0, 6, 7, 5, 4};  // iso_remap_cube: vertex - REMAP = cell
+                const uint32_t a = ~REMAP[i] & 1, b = ~REMAP[i] >> 1 & 1, c = ~REMAP[i] >> 2 & 1;
+                const uint32_t from = axis_fam(vx, a) + 3 * axis_fam(vy, b) + 9 * axis_fam(vz, c);
+                const uint32_t ci = axis_bit(vx, a) | axis_bit(vy, b) << 1 | axis_bit(vz, c) << 2;
+                uint32_t found = __shfl_sync(FULL, ref, from);
+                if (__shfl_sync(FULL, q.first, from)) found += ci;
+                if (q.own && found == 0xFFFFFFFFu) {
+                    // the reference keeps the previous corner's data here (implicit_octree.rs:84-95)
+                    atomicAdd(&A.c->stale, 1ull);
+                    found = prev;
+                }
+                corner[i] = found;
+                prev = found;
+            }
+            if (q.own) {
+                const unsigned long long set = (unsigned long long)q.hi << 32 | q.lo;
+                j = j0 + __popcll(set & ((1ull << q.code) - 1));
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const float d = corner[i] != 0xFFFFFFFFu ? __ldg(A.nvals + corner[i]) : 0.0f;
+                    if (!(d > 0.0f)) cs |= 1u << i;
+                }
+                if (j < A.cap) A.cases[j] = (uint8_t)cs;
+                else atomicOr(A.err, DERR_CAPACITY);
+                listed = j < A.cap && cs != 0 && cs != 255;
+            }
+        }
+        const uint32_t lm = __ballot_sync(FULL, listed);
+        const uint32_t edges = __reduce_add_sync(FULL, listed ? (uint32_t)iso_edge_count[cs] : 0u);
+        if (lane == 0) {
+            s_listed[warp] = __popc(lm);
+            s_edges[warp] = edges;
+        }
+        __syncthreads();
+        uint32_t at = 0, all = 0, ne = 0;
+        for (uint32_t w = 0; w < 8; ++w) {
+            if (w < warp) at += s_listed[w];
+            all += s_listed[w];
+            ne += s_edges[w];
+        }
+        if (threadIdx.x == 0 && all)
+            s_base = (uint32_t)atomicAdd(&A.c->work, (unsigned long long)ne << 32 | (unsigned long long)all);
+        __syncthreads();
+        if (listed) {
+            at += s_base + __popc(lm & ((1u << lane) - 1u));
+            A.list[at] = make_uint2(j, cs);
+            uint4* c = reinterpret_cast<uint4*>(A.corner + 8 * (size_t)at);
+            c[0] = make_uint4(corner[0], corner[1], corner[2], corner[3]);
+            c[1] = make_uint4(corner[4], corner[5], corner[6], corner[7]);
+        }
+        __syncthreads();  // s_base and s_listed are used
+    }
 }
 
-__global__ void cube_gather(CubeArgs A) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= A.ncubes) return;
-    const uint64_t v = A.pv_key[j];
-    const int lv = A.pv_level[j];
-    uint32_t cs = 0;
-    uint32_t prev = 0xFFFFFFFFu;
-    for (int i = 0; i < 8; ++i) {
-        uint64_t m = morton::dual_vertex(v, lv, iso_remap_cube[i]);
-        uint32_t found = 0xFFFFFFFFu;
-        while (m > 1) {
-            found = find_node(A.ntable, A.nmask, m);
-            if (found != 0xFFFFFFFFu) break;
-            m = morton::parent(m);
-        }
-        if (found == 0xFFFFFFFFu) {
-            // the reference keeps the previous corner's data here (implicit_octree.rs:84-95)
-            atomicAdd(A.stale, 1ull);
-            found = prev;
-        }
-        A.corner[8 * (size_t)j + i] = found;
-        const float d = found != 0xFFFFFFFFu ? A.nvals[found] : 0.0f;
-        if (!(d > 0.0f)) cs |= 1u << i;
-        prev = found;
-    }
-    A.cases[j] = (uint8_t)cs;
-    A.tri_counts[j] = iso_tri_count[cs];
+// the edge table's mask: three slots for every two crossing edges of listed
+// cubes (an edge has about four cubes), as far as there is room
+__device__ __forceinline__ uint32_t edge_mask(const CubeArgs& A) {
+    const uint32_t visits = (uint32_t)(A.c->work >> 32), want = max(visits + visits / 2, 1024u);
+    const uint32_t bits = 32 - __clz(want - 1);
+    return min(bits >= 31 ? 1u << 31 : 1u << bits, A.table_cap) - 1;
+}
+
+__global__ void __launch_bounds__(256) edge_clear(CubeArgs A) {
+    const uint32_t mask = edge_mask(A);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i <= mask; i += gridDim.x * 256)
+        reinterpret_cast<ulonglong2*>(A.table)[i] = make_ulonglong2(0ull, ~0ull);
 }
 
 __device__ __forceinline__ uint64_t edge_key(const unsigned long long* nkeys, const uint32_t* corner, uint32_t e) {
@@ -411,119 +681,116 @@ __device__ __forceinline__ uint64_t edge_key(const unsigned long long* nkeys, co
     return a > b ? ((b << 32) | a) : ((a << 32) | b);  // MortonKey::new, index_cache.rs:63-73
 }
 
-struct EdgeArgs {
-    const unsigned long long* nkeys;
-    const uint32_t* corner;
-    const uint8_t* cases;
-    uint32_t ncubes;
-    unsigned long long* hkeys;
-    unsigned long long* hvals;  // first visitor: cube << 4 | first-use rank
-    uint32_t hmask;
-    uint32_t* vcounts;
-    uint16_t* owned;            // per cube: owned first-use ranks
-    uint32_t* err;
-};
+// in the table an edge goes by its two nodes, as its keys do one by one
+// (+ 1: never 0)
+__device__ __forceinline__ uint64_t edge_nodes(const uint32_t* corner, uint32_t e) {
+    const uint32_t u = corner[iso_edge_connection[e][0]], w = corner[iso_edge_connection[e][1]];
+    const uint32_t a = u != 0xFFFFFFFFu ? u : 0u, b = w != 0xFFFFFFFFu ? w : 0u;  // node 0 has key 1
+    return (a > b ? (uint64_t)b << 32 | a : (uint64_t)a << 32 | b) + 1;
+}
 
-__global__ void edge_visit(EdgeArgs A) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= A.ncubes) return;
-    const uint32_t cs = A.cases[j];
-    const uint64_t ord = iso_edge_order[cs];
-    const uint32_t ne = iso_edge_count[cs];
-    for (uint32_t r = 0; r < ne; ++r) {
-        const uint32_t e = (uint32_t)(ord >> (4 * r)) & 15u;
-        const uint64_t k = edge_key(A.nkeys, A.corner + 8 * (size_t)j, e);
-        const uint32_t slot = ht_insert(A.hkeys, A.hmask, k);
-        if (slot == 0xFFFFFFFFu) {
-            atomicOr(A.err, DERR_CAPACITY);
-            continue;
+// Four lanes per cube: a visit is a chain of dependent accesses to L2.
+__global__ void __launch_bounds__(256) edge_visit(CubeArgs A) {
+    const uint32_t n = (uint32_t)A.c->work, mask = edge_mask(A), sub = threadIdx.x & 3;
+    for (uint32_t p = blockIdx.x * 64 + (threadIdx.x >> 2); p < n; p += gridDim.x * 64) {
+        const uint2 q = A.list[p];
+        const uint64_t ord = iso_edge_order[q.y];
+        const uint32_t ne = iso_edge_count[q.y];
+        for (uint32_t r = sub; r < ne; r += 4) {
+            const uint32_t e = (uint32_t)(ord >> (4 * r)) & 15u;
+            const unsigned long long code = (unsigned long long)q.x << 4 | r;
+            unsigned long long held;
+            const uint32_t slot = ht_insert(A.table, mask, edge_nodes(A.corner + 8 * (size_t)p, e), &held);
+            A.slots[12 * (size_t)p + r] = slot;
+            if (slot == NO_SLOT) atomicOr(A.err, DERR_CAPACITY);
+            else if (held > code) atomicMin(&A.table[slot].val, code);
         }
-        atomicMin(A.hvals + slot, (unsigned long long)(((uint64_t)j << 4) | r));
     }
 }
 
-__global__ void edge_own(EdgeArgs A) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= A.ncubes) return;
-    const uint32_t cs = A.cases[j];
-    const uint64_t ord = iso_edge_order[cs];
-    const uint32_t ne = iso_edge_count[cs];
-    uint32_t mask = 0;
-    for (uint32_t r = 0; r < ne; ++r) {
-        const uint32_t e = (uint32_t)(ord >> (4 * r)) & 15u;
-        const uint32_t slot = ht_find(A.hkeys, A.hmask, edge_key(A.nkeys, A.corner + 8 * (size_t)j, e));
-        if (slot != 0xFFFFFFFFu && A.hvals[slot] == (((uint64_t)j << 4) | r)) mask |= 1u << r;
+__global__ void __launch_bounds__(128) edge_own(CubeArgs A) {
+    const uint32_t n = (uint32_t)A.c->work, lane = threadIdx.x & 31;
+    for (uint32_t p0 = blockIdx.x * 128 + (threadIdx.x & ~31u); p0 < n; p0 += gridDim.x * 128) {
+        const uint32_t p = p0 + lane;
+        const uint2 q = p < n ? A.list[p] : make_uint2(0, 0);
+        const uint32_t ne = iso_edge_count[q.y];
+        uint32_t own = 0;
+        for (uint32_t r = 0; r < ne; ++r) {
+            const uint32_t slot = A.slots[12 * (size_t)p + r];
+            if (slot != NO_SLOT && A.table[slot].val == (((uint64_t)q.x << 4) | r)) own |= 1u << r;
+        }
+        if (p < n) A.owned[q.x] = (uint16_t)own;
+        // the list keeps a block's cubes together, so a warp mostly adds to one sum
+        const uint32_t b = q.x / BLOCK_CUBES, b0 = __shfl_sync(FULL, b, 0);
+        const bool same = p < n && b == b0;
+        const uint32_t nv = __popc(own), nt = iso_tri_count[q.y];
+        const uint32_t sv = __reduce_add_sync(FULL, same ? nv : 0u), st = __reduce_add_sync(FULL, same ? nt : 0u);
+        if (lane == 0) atomicAdd(A.sums + b0, (unsigned long long)st << 32 | (unsigned long long)sv);
+        else if (p < n && !same) atomicAdd(A.sums + b, (unsigned long long)nt << 32 | (unsigned long long)nv);
     }
-    A.owned[j] = (uint16_t)mask;
-    A.vcounts[j] = __popc(mask);
 }
 
-struct EmitArgs {
-    const unsigned long long* nkeys;
-    const float* nvals;
-    const uint32_t* corner;
-    const uint8_t* cases;
-    const uint16_t* owned;
-    const uint32_t* vbase;
-    const uint32_t* tbase;
-    uint32_t ncubes;
-    const unsigned long long* hkeys;
-    const unsigned long long* hvals;
-    uint32_t hmask;
-    float* out_v;
-    uint32_t* out_i;
-    uint64_t* out_k;
-    uint32_t* err;
-};
+// a thread block per BLOCK_CUBES cubes, a thread per cube
+__global__ void __launch_bounds__(256) cube_offsets(CubeArgs A) {
+    const unsigned long long base = A.sums[blockIdx.x];
+    if (base == NO_ITEMS) return;
+    const uint32_t n = min(A.c->cubes.x, A.cap), j = blockIdx.x * BLOCK_CUBES + threadIdx.x;
+    const uint32_t cs = j < n ? A.cases[j] : 0u;
+    const bool listed = cs != 0 && cs != 255;
+    const unsigned long long mine =
+        listed ? (unsigned long long)iso_tri_count[cs] << 32 | (unsigned long long)__popc(A.owned[j]) : 0ull;
+    const unsigned long long run = offset_in_block(base, mine);
+    if (listed) {
+        A.vbase[j] = (uint32_t)run;
+        A.tbase[j] = (uint32_t)(run >> 32);
+    }
+}
 
-__global__ void cube_emit(EmitArgs A) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= A.ncubes) return;
-    const uint32_t cs = A.cases[j];
-    const uint32_t nt = iso_tri_count[cs];
-    if (nt == 0) return;
-    const uint32_t* corner = A.corner + 8 * (size_t)j;
-    const uint64_t ord = iso_edge_order[cs];
-    const uint32_t ne = iso_edge_count[cs];
-    const uint32_t own = A.owned[j];
-    const uint32_t vb = A.vbase[j];
-    uint32_t ids[12];
-    for (uint32_t r = 0; r < ne; ++r) {
-        const uint32_t e = (uint32_t)(ord >> (4 * r)) & 15u;
-        const uint64_t k = edge_key(A.nkeys, corner, e);
-        if ((own >> r) & 1u) {
-            // find_crossing_point over the two corner nodes (distance.rs:64-69)
-            const uint32_t u = corner[iso_edge_connection[e][0]], w = corner[iso_edge_connection[e][1]];
-            const uint64_t ku = u != 0xFFFFFFFFu ? A.nkeys[u] : 1ull, kw = w != 0xFFFFFFFFu ? A.nkeys[w] : 1ull;
-            const float fa = u != 0xFFFFFFFFu ? A.nvals[u] : 0.0f, fb = w != 0xFFFFFFFFu ? A.nvals[w] : 0.0f;
-            const V3 pa = morton::center(ku), pb = morton::center(kw);
-            const float delta = fb - fa;
-            const float t = (delta == 0.0f) ? 0.5f : -fa / delta;
-            const float omt = 1.0f - t;
-            const uint32_t vid = vb + __popc(own & ((1u << r) - 1u));
-            A.out_v[3 * (size_t)vid + 0] = pa.x * omt + pb.x * t;
-            A.out_v[3 * (size_t)vid + 1] = pa.y * omt + pb.y * t;
-            A.out_v[3 * (size_t)vid + 2] = pa.z * omt + pb.z * t;
-            if (A.out_k) {
-                A.out_k[2 * (size_t)vid] = k >> 32;
-                A.out_k[2 * (size_t)vid + 1] = k & 0xFFFFFFFFull;
-            }
-            ids[r] = vid;
-        } else {
-            const uint32_t slot = ht_find(A.hkeys, A.hmask, k);
-            if (slot == 0xFFFFFFFFu) {
-                atomicOr(A.err, DERR_CAPACITY);
+__global__ void __launch_bounds__(128) cube_emit(CubeArgs A) {
+    const uint32_t n = (uint32_t)A.c->work;
+    for (uint32_t p = blockIdx.x * 128 + threadIdx.x; p < n; p += gridDim.x * 128) {
+        const uint2 q = A.list[p];
+        const uint32_t j = q.x, cs = q.y, nt = iso_tri_count[cs], ne = iso_edge_count[cs];
+        const uint32_t* corner = A.corner + 8 * (size_t)p;
+        const uint64_t ord = iso_edge_order[cs];
+        const uint32_t own = A.owned[j], vb = A.vbase[j];
+        uint32_t ids[12];
+        for (uint32_t r = 0; r < ne; ++r) {
+            if ((own >> r) & 1u) {
+                const uint32_t e = (uint32_t)(ord >> (4 * r)) & 15u;
+                const uint32_t vid = vb + __popc(own & ((1u << r) - 1u));
+                ids[r] = vid;
+                if (vid >= A.cap_v) continue;
+                // find_crossing_point over the two corner nodes (distance.rs:64-69)
+                const uint32_t u = corner[iso_edge_connection[e][0]], w = corner[iso_edge_connection[e][1]];
+                const uint64_t ku = u != 0xFFFFFFFFu ? A.nkeys[u] : 1ull, kw = w != 0xFFFFFFFFu ? A.nkeys[w] : 1ull;
+                const float fa = u != 0xFFFFFFFFu ? A.nvals[u] : 0.0f, fb = w != 0xFFFFFFFFu ? A.nvals[w] : 0.0f;
+                const V3 pa = morton::center(ku), pb = morton::center(kw);
+                const float delta = fb - fa;
+                const float t = (delta == 0.0f) ? 0.5f : -fa / delta;
+                const float omt = 1.0f - t;
+                A.out_v[3 * (size_t)vid + 0] = pa.x * omt + pb.x * t;
+                A.out_v[3 * (size_t)vid + 1] = pa.y * omt + pb.y * t;
+                A.out_v[3 * (size_t)vid + 2] = pa.z * omt + pb.z * t;
+                if (A.out_k) {
+                    const uint64_t k = edge_key(A.nkeys, corner, e);
+                    A.out_k[2 * (size_t)vid] = k >> 32;
+                    A.out_k[2 * (size_t)vid + 1] = k & 0xFFFFFFFFull;
+                }
+            } else {
+                const uint32_t slot = A.slots[12 * (size_t)p + r];
                 ids[r] = 0;
-                continue;
+                if (slot == NO_SLOT) continue;  // reported when it found no room
+                const uint64_t code = A.table[slot].val;
+                const uint32_t oj = (uint32_t)(code >> 4), orank = (uint32_t)(code & 15u);
+                ids[r] = A.vbase[oj] + __popc((uint32_t)A.owned[oj] & ((1u << orank) - 1u));
             }
-            const uint64_t code = A.hvals[slot];
-            const uint32_t oj = (uint32_t)(code >> 4), orank = (uint32_t)(code & 15u);
-            ids[r] = A.vbase[oj] + __popc((uint32_t)A.owned[oj] & ((1u << orank) - 1u));
         }
+        const uint64_t slotw = iso_tri_slot[cs];
+        const uint32_t t0 = A.tbase[j];
+        for (uint32_t k = 0; k < 3 * nt; ++k)
+            if (t0 + k / 3 < A.cap_t) A.out_i[3 * (size_t)t0 + k] = ids[(slotw >> (4 * k)) & 15u];
     }
-    const uint64_t slotw = iso_tri_slot[cs];
-    const size_t t0 = A.tbase[j];
-    for (uint32_t k = 0; k < 3 * nt; ++k) A.out_i[3 * t0 + k] = ids[(slotw >> (4 * k)) & 15u];
 }
 
 }  // namespace
@@ -570,28 +837,44 @@ uint32_t pow2_at_least(uint64_t v) {
     return (uint32_t)std::min<uint64_t>(p, 1ull << 31);
 }
 
-iso_status read_u32(iso_ctx* ctx, const uint32_t* d, uint32_t* h) {
-    cudaError_t e = cudaMemcpyAsync(ctx->h_pinned, d, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "read count");
-    *h = *(uint32_t*)ctx->h_pinned;
-    return ISO_OK;
+unsigned blocks_for(const iso_ctx* ctx, uint64_t items, unsigned per_block, unsigned per_sm) {
+    const uint64_t want = (items + per_block - 1) / per_block;
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)std::max(ctx->sms, 1) * per_sm));
 }
-
-inline size_t scan_sums_for(uint64_t n) { return (size_t)((n + 1023) / 1024) + 64; }
 
 }  // namespace
 
-// The counts an extraction discovered: the refined nodes of each generation,
-// the dual cubes, the triangles and vertices.  An eager run fills one; a run
-// recorded into a CUDA graph replays one (queueing everything, synchronising
-// nowhere) and copies each count it computes to pinned memory, so that the
-// replay can be checked against the trace.
+// The counts an extraction discovered: its nodes, dual cubes, triangles and
+// vertices.  An eager run fills one; a run recorded into a CUDA graph replays
+// one (queueing everything, synchronising nowhere) and copies each count it
+// computes to pinned memory, so that the replay can be checked against the
+// trace.
 struct LhmcTrace {
-    std::vector<uint32_t> nref;
-    uint32_t ncubes = 0, nt = 0, nv = 0;
+    uint32_t nodes = 0, ncubes = 0, nt = 0, nv = 0;
 };
-constexpr int LHMC_PIN_GEN = 8;  // h_pinned slots: [0] nt|nv, [2] stale, [3] error flags, [7] ncubes, [8+g] nref
+// h_pinned slots: [3] error flags, [8 ..] the device counters
+constexpr int LHMC_PIN_CTL = 8;
+static_assert(8 * LHMC_PIN_CTL + sizeof(Ctl) <= 4096, "pinned scratch");
+
+static LhmcTrace counts_of(const iso_ctx* ctx) {
+    const Ctl* c = (const Ctl*)(ctx->h_pinned + LHMC_PIN_CTL);
+    return LhmcTrace{c->nodes, c->cubes.x, c->mesh.y, c->mesh.x};
+}
+
+// blocks of oct_build, all of which are resident at once (looked up once per process)
+static unsigned oct_blocks(const iso_ctx* ctx) {
+    static std::atomic<int> per_sm{0};
+    int b = per_sm.load(std::memory_order_relaxed);
+    if (b == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, oct_build, 256, 0) != cudaSuccess || b < 1) {
+            cudaGetLastError();
+            b = 1;
+        }
+        b = std::min(b, 4);
+        per_sm.store(b, std::memory_order_relaxed);
+    }
+    return (unsigned)(b * std::max(ctx->sms, 1));
+}
 
 static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32_t max_depth, uint32_t flags,
                                        iso_mesh_info* info, LhmcTrace* trace, const LhmcTrace* replay) {
@@ -618,211 +901,142 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
             if (max_nodes > (1ull << 28)) break;
         }
     }
-    // node arrays grow as generations are built
-    auto node_bytes = [](size_t cap) { return cap * (8 + 4 + 4 + 4) + 4 * scan_sums_for(cap) + 4 * 1024 + 4096; };
-    size_t node_cap = (size_t)std::min<uint64_t>(max_nodes, 1ull << 20);
-    // reuse an arena that earlier extractions grew
-    while (node_cap < max_nodes && node_bytes(2 * node_cap) <= ctx->aux.bytes) node_cap *= 2;
-    if ((s = ensure(ctx, ctx->aux, node_bytes(node_cap))) != ISO_OK) return s;
-    auto carve = [&](size_t cap, unsigned long long** keys, float** vals, uint32_t** refine, uint32_t** rank,
-                     uint32_t** sums, uint32_t** total) {
+    // counters, tile counts and the table of families | keys | values | refine flags
+    auto tile_words = [](size_t cap) { return cap / TILE + cap / (TILE * SUPER) + 3 * MAX_GENS; };
+    auto table_at = [&](size_t cap) { return (sizeof(Ctl) + 4 * tile_words(cap) + 255) & ~(size_t)255; };
+    auto head_bytes = [&](size_t cap) { return table_at(cap) + 8 * (size_t)pow2_at_least(cap / 4); };
+    auto node_bytes = [&](size_t cap) { return head_bytes(cap) + 12 * cap + cap / 8 + 4096; };
+    // a first guess, or the room an earlier octree needed
+    size_t node_cap = (size_t)std::min<uint64_t>(max_nodes, std::max<uint64_t>(1ull << 20, ctx->lhmc_room));
+    const uint32_t last = std::max(2u, max_depth) + 1;  // the last generation there can be: see morton::level
+    Ctl* const h = (Ctl*)(ctx->h_pinned + LHMC_PIN_CTL);
+    cudaError_t e;
+    OctArgs oa{};
+    uint32_t nodes = 0;
+    while (true) {
+        if ((s = ensure(ctx, ctx->aux, node_bytes(node_cap))) != ISO_OK) return s;
         Arena a{(char*)ctx->aux.p, 0, ctx->aux.bytes};
-        *keys = a.take<unsigned long long>(cap);
-        *vals = a.take<float>(cap);
-        *refine = a.take<uint32_t>(cap);
-        *rank = a.take<uint32_t>(cap);
-        *sums = a.take<uint32_t>(scan_sums_for(cap));
-        *total = a.take<uint32_t>(64);
-    };
-    unsigned long long* nkeys;
-    float* nvals;
-    uint32_t *refine, *rank, *sums, *total;
-    carve(node_cap, &nkeys, &nvals, &refine, &rank, &sums, &total);
-    set_root<<<1, 1, 0, ctx->stream>>>(nkeys);
-    ctx->launches++;
-    cudaError_t e = cudaSuccess;
-    uint32_t off = 0, cnt = 1, gen_i = 0;
-    if (trace) *trace = LhmcTrace{};
-    while (cnt > 0) {
-        GenArgs ga{prog->view(), nkeys, nvals, refine, off, cnt, max_depth};
-        oct_eval<<<(cnt + 127) / 128, 128, 0, ctx->stream>>>(ga);
+        char* head = a.take<char>(head_bytes(node_cap));
+        oa.pv = prog->view();
+        oa.keys = a.take<unsigned long long>(node_cap);
+        oa.vals = a.take<float>(node_cap);
+        oa.refine = a.take<uint8_t>(node_cap / 8 + 1);
+        oa.families = (unsigned long long*)(head + table_at(node_cap));
+        oa.fmask = pow2_at_least(node_cap / 4) - 1;
+        oa.cap = (uint32_t)node_cap;
+        oa.max_depth = max_depth;
+        oa.c = (Ctl*)head;
+        oa.err = ctx->d_err;
+        oa.tiles = (uint32_t*)(oa.c + 1);
+        oa.supers = oa.tiles + node_cap / TILE + MAX_GENS;
+        e = cudaMemsetAsync(head, 0, head_bytes(node_cap), ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "octree counters");
+        // blocks beyond the widest generation's tiles would only come to the barriers
+        const uint64_t most = std::min<uint64_t>(1ull << std::min(3 * (last - 1), 32u), node_cap);
+        const unsigned blocks = (unsigned)std::min<uint64_t>(oct_blocks(ctx), (most + TILE - 1) / TILE);
+        uint32_t last_arg = last;
+        void* args[] = {&oa, &last_arg};
+        e = cudaLaunchCooperativeKernel(oct_build, dim3(blocks), dim3(256), args, 0, ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "octree launch");
         ctx->launches++;
-        if ((s = scan_u32(ctx, refine + off, rank, cnt, sums, total)) != ISO_OK) return s;
-        uint32_t nref = 0;
+        if ((s = check_launch(ctx, "octree")) != ISO_OK) return s;
         if (rec) {
-            if (gen_i >= replay->nref.size() || LHMC_PIN_GEN + gen_i >= 512)
-                return fail(ctx, ISO_ERR_INVALID_ARG, "trace shorter than the octree");
-            nref = replay->nref[gen_i];
-            e = cudaMemcpyAsync(ctx->h_pinned + LHMC_PIN_GEN + gen_i, total, 4, cudaMemcpyDeviceToHost, ctx->stream);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "copy count");
-        } else {
-            if ((s = read_u32(ctx, total, &nref)) != ISO_OK) return s;
-            if (trace) trace->nref.push_back(nref);
+            nodes = replay->nodes;
+            break;
         }
-        ++gen_i;
-        const uint64_t next = 8ull * nref;
-        const uint64_t need = (uint64_t)off + cnt + next;
-        if (need >= 0xFFFFFFF0ull) return fail(ctx, ISO_ERR_TOO_LARGE, "octree too large");
-        if (need > node_cap && rec) return fail(ctx, ISO_ERR_INVALID_ARG, "octree arena would grow while recording");
-        if (need > node_cap) {
-            // grow: copy the built prefix into a larger arena
-            const size_t new_cap = (size_t)std::max<uint64_t>(need, 2 * node_cap);
-            void* fresh = nullptr;
-            e = cudaMalloc(&fresh, node_bytes(new_cap));
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "grow octree");
-            Arena a{(char*)fresh, 0, node_bytes(new_cap)};
-            unsigned long long* k2 = a.take<unsigned long long>(new_cap);
-            float* v2 = a.take<float>(new_cap);
-            uint32_t* r2 = a.take<uint32_t>(new_cap);
-            uint32_t* q2 = a.take<uint32_t>(new_cap);
-            cudaMemcpyAsync(k2, nkeys, 8ull * (off + cnt), cudaMemcpyDeviceToDevice, ctx->stream);
-            cudaMemcpyAsync(v2, nvals, 4ull * (off + cnt), cudaMemcpyDeviceToDevice, ctx->stream);
-            cudaMemcpyAsync(r2, refine, 4ull * (off + cnt), cudaMemcpyDeviceToDevice, ctx->stream);
-            cudaMemcpyAsync(q2, rank, 4ull * cnt, cudaMemcpyDeviceToDevice, ctx->stream);
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(ctx->aux.p);
-            ctx->aux.p = fresh;
-            ctx->aux.bytes = node_bytes(new_cap);
-            node_cap = new_cap;
-            nkeys = k2;
-            nvals = v2;
-            refine = r2;
-            rank = q2;
-            Arena rest{(char*)fresh, 0, ctx->aux.bytes};
-            rest.take<unsigned long long>(new_cap);
-            rest.take<float>(new_cap);
-            rest.take<uint32_t>(new_cap);
-            rest.take<uint32_t>(new_cap);
-            sums = rest.take<uint32_t>(scan_sums_for(new_cap));
-            total = rest.take<uint32_t>(64);
-        }
-        if (nref) {
-            oct_expand<<<(cnt + 127) / 128, 128, 0, ctx->stream>>>(nkeys, refine, rank, off, cnt, off + cnt);
-            ctx->launches++;
-        }
-        off += cnt;
-        cnt = (uint32_t)next;
-    }
-    const uint32_t nodes = off;
-    if ((s = check_launch(ctx, "octree")) != ISO_OK) return s;
-
-    // ---- 2. primal vertices (hash: vertex -> deepest level, smallest key)
-    const uint32_t hcap1 = pow2_at_least(16ull * nodes);
-    const size_t pv_cap = 8ull * nodes;
-    {
-        const size_t bytes = 16ull * hcap1 + 4ull * nodes * 2 + 9ull * pv_cap + 4 * scan_sums_for(nodes) + 4096;
-        if ((s = ensure(ctx, ctx->aux2, bytes)) != ISO_OK) return s;
-    }
-    Arena a2{(char*)ctx->aux2.p, 0, ctx->aux2.bytes};
-    unsigned long long* hk1 = a2.take<unsigned long long>(hcap1);
-    unsigned long long* hv1 = a2.take<unsigned long long>(hcap1);
-    uint32_t* counts = a2.take<uint32_t>(nodes);
-    uint32_t* offsets = a2.take<uint32_t>(nodes);
-    unsigned long long* pv_key = a2.take<unsigned long long>(pv_cap);
-    uint8_t* pv_level = a2.take<uint8_t>(pv_cap);
-    uint32_t* sums2 = a2.take<uint32_t>(scan_sums_for(nodes));
-    uint32_t* total2 = a2.take<uint32_t>(64);
-    e = cudaMemsetAsync(hk1, 0, 16ull * hcap1, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "memset table");
-    LeafArgs la{nkeys, refine, nodes, hk1, hv1, hcap1 - 1, counts, ctx->d_err};
-    leaf_insert<<<(unsigned)((8ull * nodes + 255) / 256), 256, 0, ctx->stream>>>(la);
-    leaf_count<<<(nodes + 255) / 256, 256, 0, ctx->stream>>>(la);
-    ctx->launches += 2;
-    if ((s = scan_u32(ctx, counts, offsets, nodes, sums2, total2)) != ISO_OK) return s;
-    leaf_write<<<(nodes + 255) / 256, 256, 0, ctx->stream>>>(la, offsets, pv_key, pv_level);
-    // the node table for the parent walks, in the primal-vertex table's
-    // memory (2 slots per node against its 16, and done with it now)
-    const uint32_t ncap = pow2_at_least(2ull * nodes);
-    unsigned long long* ntable = hk1;
-    e = cudaMemsetAsync(ntable, 0, 8ull * ncap, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "memset node table");
-    node_insert<<<(nodes + 255) / 256, 256, 0, ctx->stream>>>(nkeys, nodes, ntable, ncap - 1);
-    ctx->launches += 2;
-    uint32_t ncubes = 0;
-    if (rec) {
-        ncubes = replay->ncubes;
-        e = cudaMemcpyAsync(ctx->h_pinned + 7, total2, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "copy count");
-    } else {
-        if ((s = read_u32(ctx, total2, &ncubes)) != ISO_OK) return s;
-        if (trace) trace->ncubes = ncubes;
-    }
-
-    // ---- 3./4. dual cubes and their marching cubes
-    const uint32_t hcap2 = pow2_at_least(8ull * ncubes + 1024);
-    {
-        const size_t bytes = 32ull * ncubes + ncubes + 4ull * ncubes * 4 + 2ull * ncubes + 16ull * hcap2 +
-                             8 * scan_sums_for(ncubes) + 8192;
-        if ((s = ensure(ctx, ctx->aux3, bytes)) != ISO_OK) return s;
-    }
-    Arena a3{(char*)ctx->aux3.p, 0, ctx->aux3.bytes};
-    uint32_t* corner = a3.take<uint32_t>(8ull * ncubes);
-    uint8_t* cases = a3.take<uint8_t>(ncubes);
-    uint32_t* tcount = a3.take<uint32_t>(ncubes);
-    uint32_t* tbase = a3.take<uint32_t>(ncubes);
-    uint32_t* vcount = a3.take<uint32_t>(ncubes);
-    uint32_t* vbase = a3.take<uint32_t>(ncubes);
-    uint16_t* owned = a3.take<uint16_t>(ncubes);
-    unsigned long long* hk2 = a3.take<unsigned long long>(hcap2);
-    unsigned long long* hv2 = a3.take<unsigned long long>(hcap2);
-    uint32_t* sums3 = a3.take<uint32_t>(2 * scan_sums_for(ncubes));
-    uint32_t* tot3 = a3.take<uint32_t>(16);
-    unsigned long long* stale = (unsigned long long*)(tot3 + 8);
-    e = cudaMemsetAsync(hk2, 0, 8ull * hcap2, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(hv2, 0xFF, 8ull * hcap2, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(stale, 0, 8, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "memset");
-    if (ncubes) {
-        CubeArgs ca{ntable, ncap - 1, nvals, pv_key, pv_level, ncubes, corner, cases, tcount, stale};
-        cube_gather<<<(ncubes + 127) / 128, 128, 0, ctx->stream>>>(ca);
-        EdgeArgs ea{nkeys, corner, cases, ncubes, hk2, hv2, hcap2 - 1, vcount, owned, ctx->d_err};
-        edge_visit<<<(ncubes + 127) / 128, 128, 0, ctx->stream>>>(ea);
-        edge_own<<<(ncubes + 127) / 128, 128, 0, ctx->stream>>>(ea);
-        ctx->launches += 3;
-    }
-    if ((s = scan_u32(ctx, tcount, tbase, ncubes, sums3, tot3)) != ISO_OK) return s;
-    if ((s = scan_u32(ctx, vcount, vbase, ncubes, sums3 + scan_sums_for(ncubes), tot3 + 1)) != ISO_OK) return s;
-    e = cudaMemcpyAsync(ctx->h_pinned, tot3, 8, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 2, stale, 8, cudaMemcpyDeviceToHost, ctx->stream);
-    uint32_t nt, nv;
-    if (rec) {
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "copy totals");
-        nt = replay->nt;
-        nv = replay->nv;
-    } else {
+        e = cudaMemcpyAsync(h, oa.c, sizeof(Ctl), cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "read totals");
-        if ((s = read_device_errors(ctx)) != ISO_OK) return s;
-        nt = ((uint32_t*)ctx->h_pinned)[0];
-        nv = ((uint32_t*)ctx->h_pinned)[1];
-        ctx->lhmc_stale = ctx->h_pinned[2];
-        if (trace) {
-            trace->nt = nt;
-            trace->nv = nv;
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "read octree size");
+        if (h->need == 0) {
+            nodes = h->nodes;
+            ctx->lhmc_room = std::max<uint64_t>(ctx->lhmc_room, node_cap);
+            break;
         }
+        // a generation did not fit: again in a larger arena
+        if (h->need >= 0xFFFFFFF0ull) return fail(ctx, ISO_ERR_TOO_LARGE, "octree too large");
+        node_cap = (size_t)std::max<uint64_t>(h->need, std::min<uint64_t>(2 * (uint64_t)node_cap, 0xFFFFFFF0ull));
     }
+    if (trace) trace->nodes = nodes;
+
+    // ---- 2. to 4. primal vertices, dual cubes and their marching cubes
+    const uint64_t bound = 3ull * nodes + 1024;  // vertices, and the dual cubes around them
+    const uint32_t nfam = (nodes - 1) / 8;
+    const uint32_t fblocks = (nfam + BLOCK_FAMILIES - 1) / BLOCK_FAMILIES;
+    const uint32_t cblocks = (uint32_t)((bound + BLOCK_CUBES - 1) / BLOCK_CUBES);
+    if ((s = ensure(ctx, ctx->aux2, 8ull * (fblocks + cblocks) + nfam + 4096)) != ISO_OK) return s;
+    const uint32_t ecap = pow2_at_least(4 * bound);
+    if ((s = ensure(ctx, ctx->aux3, (32ull + 8 + 48 + 1 + 2 + 8) * bound + 16ull * ecap + 8192)) != ISO_OK) return s;
+    // a first extraction starts from a modest guess; later ones reuse what grew
     const bool keys = (flags & ISO_FLAG_KEYS) != 0;
-    if ((s = ensure(ctx, ctx->mesh_v, 12ull * std::max<uint32_t>(nv, 1))) != ISO_OK) return s;
-    if ((s = ensure(ctx, ctx->mesh_i, 12ull * std::max<uint32_t>(nt, 1))) != ISO_OK) return s;
-    if (keys && (s = ensure(ctx, ctx->mesh_k, 16ull * std::max<uint32_t>(nv, 1))) != ISO_OK) return s;
-    if (nt) {
-        EmitArgs ma{nkeys, nvals, corner, cases, owned, vbase, tbase, ncubes, hk2, hv2, hcap2 - 1,
-                    (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p, keys ? (uint64_t*)ctx->mesh_k.p : nullptr,
-                    ctx->d_err};
-        cube_emit<<<(ncubes + 127) / 128, 128, 0, ctx->stream>>>(ma);
+    if ((s = ensure(ctx, ctx->mesh_v, 12 * (size_t)65536)) != ISO_OK) return s;
+    if ((s = ensure(ctx, ctx->mesh_i, 12 * (size_t)131072)) != ISO_OK) return s;
+    if (keys && (s = ensure(ctx, ctx->mesh_k, 16 * (size_t)65536)) != ISO_OK) return s;
+    Arena a3{(char*)ctx->aux3.p, 0, ctx->aux3.bytes};
+    Arena a2{(char*)ctx->aux2.p, 0, ctx->aux2.bytes};
+    CubeArgs ca{};
+    ca.nkeys = oa.keys;
+    ca.nvals = oa.vals;
+    ca.refine = oa.refine;
+    ca.families = oa.families;
+    ca.fmask = oa.fmask;
+    ca.nfamilies = nfam;
+    ca.fsums = a2.take<unsigned long long>(fblocks);
+    ca.sums = a2.take<unsigned long long>(cblocks);
+    ca.fcount = a2.take<uint8_t>(nfam);
+    ca.cap = (uint32_t)bound;
+    ca.c = oa.c;
+    ca.table = a3.take<Slot>(ecap);
+    ca.table_cap = ecap;
+    ca.corner = a3.take<uint32_t>(8 * bound);
+    ca.list = a3.take<uint2>(bound);
+    ca.slots = a3.take<uint32_t>(12 * bound);
+    ca.cases = a3.take<uint8_t>(bound);
+    ca.owned = a3.take<uint16_t>(bound);
+    ca.vbase = a3.take<uint32_t>(bound);
+    ca.tbase = a3.take<uint32_t>(bound);
+    ca.err = ctx->d_err;
+    e = cudaMemsetAsync(ca.sums, 0, 8ull * cblocks, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "clear sums");
+    family_count<<<fblocks, 256, 0, ctx->stream>>>(ca);
+    scan_block_sums<<<1, 1024, 0, ctx->stream>>>(ca.fsums, fblocks, &oa.c->cubes);
+    cube_gather<<<fblocks, 256, 0, ctx->stream>>>(ca);
+    edge_clear<<<blocks_for(ctx, ecap, 256, 8), 256, 0, ctx->stream>>>(ca);
+    const unsigned pblocks = blocks_for(ctx, bound, 128, 16);
+    edge_visit<<<blocks_for(ctx, bound, 64, 8), 256, 0, ctx->stream>>>(ca);
+    edge_own<<<pblocks, 128, 0, ctx->stream>>>(ca);
+    scan_block_sums<<<1, 1024, 0, ctx->stream>>>(ca.sums, cblocks, &oa.c->mesh);
+    cube_offsets<<<cblocks, 256, 0, ctx->stream>>>(ca);
+    ctx->launches += 8;
+    if ((s = check_launch(ctx, "dual cubes")) != ISO_OK) return s;
+    LhmcTrace t{};
+    while (true) {
+        ca.out_v = (float*)ctx->mesh_v.p;
+        ca.out_i = (uint32_t*)ctx->mesh_i.p;
+        ca.out_k = keys ? (uint64_t*)ctx->mesh_k.p : nullptr;
+        auto room = [](size_t n) { return (uint32_t)std::min<size_t>(n, 0xFFFFFFFFu); };
+        ca.cap_v = room(keys ? std::min(ctx->mesh_v.bytes / 12, ctx->mesh_k.bytes / 16) : ctx->mesh_v.bytes / 12);
+        ca.cap_t = room(ctx->mesh_i.bytes / 12);
+        cube_emit<<<pblocks, 128, 0, ctx->stream>>>(ca);
         ctx->launches++;
         if ((s = check_launch(ctx, "cube_emit")) != ISO_OK) return s;
+        e = cudaMemcpyAsync(h, oa.c, sizeof(Ctl), cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 3, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (rec) return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "copy counts");
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "read counts");
+        if ((uint32_t)ctx->h_pinned[3] && (s = read_device_errors(ctx)) != ISO_OK) return s;
+        t = counts_of(ctx);
+        ctx->lhmc_stale = h->stale;
+        if (t.nv <= ca.cap_v && t.nt <= ca.cap_t) break;
+        // it did not all fit (the counts are exact): again into buffers of that size
+        if ((s = ensure(ctx, ctx->mesh_v, 12ull * t.nv)) != ISO_OK) return s;
+        if ((s = ensure(ctx, ctx->mesh_i, 12ull * t.nt)) != ISO_OK) return s;
+        if (keys && (s = ensure(ctx, ctx->mesh_k, 16ull * t.nv)) != ISO_OK) return s;
     }
-    if (rec) {
-        e = cudaMemcpyAsync(ctx->h_pinned + 3, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "copy error flags");
-    }
-    e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "sync");
-    if ((s = read_device_errors(ctx)) != ISO_OK) return s;
-    ctx->last.num_vertices = nv;
-    ctx->last.num_triangles = nt;
-    ctx->last.num_cells = ncubes;
+    if (trace) *trace = t;
+    ctx->last.num_vertices = t.nv;
+    ctx->last.num_triangles = t.nt;
+    ctx->last.num_cells = t.ncubes;
     if (info) *info = ctx->last;
     return ISO_OK;
 }
@@ -855,20 +1069,19 @@ static iso_status lhmc_planned(iso_ctx* ctx, const iso_program* prog, uint32_t d
         cudaError_t e = cudaGraphLaunch(P.exec, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "octree graph");
-        const uint64_t* h = ctx->h_pinned;
-        bool same = (uint32_t)h[0] == P.nt && (uint32_t)(h[0] >> 32) == P.nv && (uint32_t)h[7] == P.ncubes &&
-                    (uint32_t)h[3] == 0;
-        for (size_t g = 0; same && g < P.nref.size(); ++g) same = (uint32_t)h[LHMC_PIN_GEN + g] == P.nref[g];
+        const LhmcTrace t = counts_of(ctx);
+        const bool same = t.nodes == P.nodes && t.ncubes == P.ncubes && t.nt == P.nt && t.nv == P.nv &&
+                          (uint32_t)ctx->h_pinned[3] == 0;
         if (same) {
             ctx->launches += P.launches;
             ctx->last = iso_mesh_info{P.nv, P.nt, P.ncubes};
             ctx->last_flags = flags;
             ctx->last_vertex_floats = 3;
-            ctx->lhmc_stale = h[2];
+            ctx->lhmc_stale = ((const Ctl*)(ctx->h_pinned + LHMC_PIN_CTL))->stale;
             if (info) *info = ctx->last;
             return ISO_OK;
         }
-        if ((uint32_t)h[3]) cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
+        if ((uint32_t)ctx->h_pinned[3]) cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
         lhmc_plan_release(ctx);
     }
     LhmcTrace tr;
@@ -877,7 +1090,7 @@ static iso_status lhmc_planned(iso_ctx* ctx, const iso_program* prog, uint32_t d
     const uint64_t key[3] = {prog->uid, depth, flags};
     const bool repeat = std::memcmp(key, ctx->lhmc_last_key, sizeof(key)) == 0;
     std::memcpy(ctx->lhmc_last_key, key, sizeof(key));
-    if (ctx->timing || !repeat || tr.nref.size() + LHMC_PIN_GEN >= 512) return ISO_OK;
+    if (ctx->timing || !repeat) return ISO_OK;
     // record the same extraction with the counts just found
     lhmc_plan_release(ctx);
     const uint64_t launches0 = ctx->launches;
@@ -905,7 +1118,7 @@ static iso_status lhmc_planned(iso_ctx* ctx, const iso_program* prog, uint32_t d
             P.depth = depth;
             P.flags = flags;
             lhmc_buffers(ctx, P.bufs);
-            P.nref = tr.nref;
+            P.nodes = tr.nodes;
             P.ncubes = tr.ncubes;
             P.nt = tr.nt;
             P.nv = tr.nv;
