@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(1024) scan_small(const uint32_t* in, uint32_t*
 
 // ------------------------------------------------------------ octree build ---
 constexpr uint32_t TILE = 32;     // nodes with one count of refined ones
+constexpr uint32_t OCT_THREADS = 256;
 constexpr uint32_t SUPER = 64;    // tiles with one
 constexpr uint32_t MAX_GENS = 16; // of any octree (keys fit 31 bits)
 constexpr uint32_t BLOCK_FAMILIES = 32;  // families with one sum of primal vertices (block_sums.cuh)
@@ -317,12 +318,9 @@ __device__ __forceinline__ uint32_t family_slot(uint64_t parent, uint32_t mask) 
     const uint32_t h = (uint32_t)parent * 0x9E3779B1u;
     return (h ^ h >> 15) & mask;
 }
-__device__ __forceinline__ void family_insert(const OctArgs& A, uint64_t parent, uint32_t first) {
-    uint32_t slot = family_slot(parent, A.fmask);
-    for (uint32_t probe = 0; probe <= A.fmask; ++probe) {
-        if (atomicCAS(A.families + slot, 0ull, parent << 32 | first) == 0ull) return;
-        slot = (slot + 1) & A.fmask;
-    }
+__device__ __forceinline__ void family_insert(const OctArgs& A, uint64_t parent, uint32_t first, uint32_t slot) {
+    for (uint32_t probe = 0; probe <= A.fmask; ++probe, ++slot)
+        if (atomicCAS(A.families + (slot & A.fmask), 0ull, parent << 32 | first) == 0ull) return;
 }
 // the first child of the node with key `parent`, 0 if that is no refined node
 __device__ __forceinline__ uint32_t find_family(const unsigned long long* families, uint32_t mask, uint64_t parent) {
@@ -364,9 +362,9 @@ __device__ __forceinline__ void grid_barrier(Ctl* c, uint32_t turn, uint32_t* er
 // Generations 0 to 2 (nodes 0, 1-8 and 9-72) every octree has; after that a
 // block takes the refined nodes of a tile and evaluates their children.
 // What other blocks wrote is read past L1.
-__global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
-    __shared__ unsigned long long s_key[TILE];
-    __shared__ uint32_t s_sum[8], s_n;
+__global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t last) {
+    __shared__ unsigned long long s_key[OCT_THREADS];
+    __shared__ uint32_t s_sum[OCT_THREADS / 32], s_n[OCT_THREADS / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     auto block_sum = [&](uint32_t v) {
         v = __reduce_add_sync(FULL, v);
@@ -374,7 +372,7 @@ __global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
         if (lane == 0) s_sum[tid >> 5] = v;
         __syncthreads();
         uint32_t all = 0;
-        for (int k = 0; k < 8; ++k) all += s_sum[k];
+        for (int k = 0; k < OCT_THREADS / 32; ++k) all += s_sum[k];
         return all;
     };
     if (blockIdx.x == 0 && tid < 96) {
@@ -385,7 +383,7 @@ __global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
         const uint32_t m = __ballot_sync(FULL, r) >> (lane & ~7u) & 0xFFu;
         if (tid < 72 && (tid & 7) == 0) {
             A.refine[at >> 3] = (uint8_t)m;
-            family_insert(A, at == 1 ? 1 : 7 + (at >> 3), at);
+            family_insert(A, at == 1 ? 1 : 7 + (at >> 3), at, family_slot(at == 1 ? 1 : 7 + (at >> 3), A.fmask));
             if (at >= 9) {
                 atomicAdd(A.tiles + 9 / TILE + 2 + (at - 9) / TILE, (uint32_t)__popc(m));
                 atomicAdd(A.supers + 9 / (TILE * SUPER) + 2, (uint32_t)__popc(m));
@@ -401,32 +399,47 @@ __global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
         const uint32_t* supers = A.supers + off / (TILE * SUPER) + g;
         uint32_t* ntile = A.tiles + next / TILE + g + 1;
         uint32_t* nsuper = A.supers + next / (TILE * SUPER) + g + 1;
-        for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        // tiles a block takes together: one while there are blocks for all, up
+        // to a node per thread, so that a block's chain of loads and its lanes'
+        // last evaluation are paid for once
+        const uint32_t span = min((ntiles + gridDim.x - 1) / gridDim.x, OCT_THREADS / TILE);
+        for (uint32_t t = blockIdx.x * span; t < ntiles; t += gridDim.x * span) {
             const uint32_t s = t / SUPER;
             uint32_t sum = 0;
-            for (uint32_t k = tid; k < s; k += 256) sum += __ldcg(supers + k);
-            for (uint32_t k = s * SUPER + tid; k < t; k += 256) sum += __ldcg(tiles + k);
+            for (uint32_t k = tid; k < s; k += OCT_THREADS) sum += __ldcg(supers + k);
+            for (uint32_t k = s * SUPER + tid; k < t; k += OCT_THREADS) sum += __ldcg(tiles + k);
+            // its nodes and which of them are refined (on their way meanwhile)
+            const uint32_t i = t * TILE + tid, at = off + i;  // node 8 f + 1 + bit
+            const bool mine = tid < span * TILE && i < cnt;
+            const uint32_t flags = mine ? __ldcg(A.refine + ((at - 1) >> 3)) : 0u;
+            const unsigned long long node = mine ? __ldcg(A.keys + at) : 0ull;
             const uint32_t before = block_sum(sum);
-            // the tile's refined nodes, in order
-            const uint32_t i = t * TILE + tid;
-            if (tid < TILE) {
-                const uint32_t at = off + i;  // node 8 f + 1 + bit
-                const bool r = i < cnt && (__ldcg(A.refine + ((at - 1) >> 3)) >> ((at - 1) & 7) & 1);
-                const uint32_t m = __ballot_sync(FULL, r);
-                if (r) s_key[__popc(m & ((1u << lane) - 1u))] = __ldcg(A.keys + at);
-                if (lane == 0) s_n = __popc(m);
-            }
+            // the refined ones, in order
+            const bool r = flags >> ((at - 1) & 7) & 1;
+            const uint32_t m = __ballot_sync(FULL, r);
+            if (lane == 0) s_n[tid >> 5] = __popc(m);
             __syncthreads();
-            const uint32_t n = 8 * s_n;
-            for (uint32_t c0 = 0; c0 < n; c0 += 256) {
+            uint32_t n = 0;
+            for (uint32_t w = 0; w < OCT_THREADS / 32; ++w) {
+                if (r && w == tid >> 5) s_key[n + __popc(m & ((1u << lane) - 1u))] = node;
+                n += s_n[w];
+            }
+            n *= 8;
+            __syncthreads();
+            for (uint32_t c0 = 0; c0 < n; c0 += OCT_THREADS) {
                 const uint32_t c = c0 + tid, rel = 8 * before + c;
+                const bool live = c < n && next + rel < A.cap, leads = live && (lane & 7) == 0;
+                const unsigned long long parent = c < n ? s_key[c >> 3] : 0ull;
+                // the family's place in the table is asked for before the evaluation
+                uint32_t slot = family_slot(parent, A.fmask);
+                unsigned long long taken = 0;
+                if (leads) taken = atomicCAS(A.families + slot, 0ull, parent << 32 | (next + rel));
                 bool cr = false;
-                if (c < n && next + rel < A.cap)
-                    cr = oct_node(A, next + rel, s_key[c >> 3] << 3 | (c & 7));  // Morton::child
+                if (live) cr = oct_node(A, next + rel, parent << 3 | (c & 7));  // Morton::child
                 const uint32_t cm = __ballot_sync(FULL, cr) >> (lane & ~7u) & 0xFFu;
-                if ((lane & 7) == 0 && c < n && next + rel < A.cap) {  // a family lies in one tile
+                if (leads) {  // a family lies in one tile
+                    if (taken) family_insert(A, parent, next + rel, slot + 1);
                     A.refine[(next + rel) >> 3] = (uint8_t)cm;
-                    family_insert(A, s_key[c >> 3], next + rel);
                     if (cm) {
                         atomicAdd(ntile + rel / TILE, (uint32_t)__popc(cm));
                         atomicAdd(nsuper + rel / (TILE * SUPER), (uint32_t)__popc(cm));
@@ -436,7 +449,7 @@ __global__ void __launch_bounds__(256, 4) oct_build(OctArgs A, uint32_t last) {
         }
         // the next generation's size, in every block
         uint32_t sum = 0;
-        for (uint32_t k = tid; k < nsupers; k += 256) sum += __ldcg(supers + k);
+        for (uint32_t k = tid; k < nsupers; k += OCT_THREADS) sum += __ldcg(supers + k);
         const uint64_t children = 8ull * block_sum(sum);
         const bool fits = next + children <= A.cap;
         off = next;
@@ -866,7 +879,7 @@ static unsigned oct_blocks(const iso_ctx* ctx) {
     static std::atomic<int> per_sm{0};
     int b = per_sm.load(std::memory_order_relaxed);
     if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, oct_build, 256, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, oct_build, OCT_THREADS, 0) != cudaSuccess || b < 1) {
             cudaGetLastError();
             b = 1;
         }
@@ -936,7 +949,7 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         const unsigned blocks = (unsigned)std::min<uint64_t>(oct_blocks(ctx), (most + TILE - 1) / TILE);
         uint32_t last_arg = last;
         void* args[] = {&oa, &last_arg};
-        e = cudaLaunchCooperativeKernel(oct_build, dim3(blocks), dim3(256), args, 0, ctx->stream);
+        e = cudaLaunchCooperativeKernel(oct_build, dim3(blocks), dim3(OCT_THREADS), args, 0, ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "octree launch");
         ctx->launches++;
         if ((s = check_launch(ctx, "octree")) != ISO_OK) return s;
