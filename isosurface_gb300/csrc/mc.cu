@@ -619,6 +619,16 @@ cudaError_t emit_smem_attribute(size_t smem) {
 }
 }  // namespace
 
+// log2 of a segment's chunks: eight for a lattice with few segments of 32
+// (128^3 and below), where a segment's chain of rounds in one emitting warp
+// is the emission's time (128^3 torus: 23 us with 32 chunks, 11 with eight;
+// 65^3 sphere: 16 and 11), else 32, whose cells fill the rounds (257^3 csg:
+// 27 us with 32 chunks, 44 with eight)
+static uint32_t segment_shift(const iso_ctx* ctx, const Lattice& L) {
+    const uint64_t segs = ((uint64_t)((L.nx - 1 + 31) / 32) * (L.ny - 1) + 31) / 32 * (L.nz - 1);
+    return segs <= 16 * (uint64_t)std::max(ctx->sms, 1) ? 3 : 5;
+}
+
 // list entries per emitting warp: several pool their cells into full rounds
 // of 32, while that leaves about four waves of warps (a warp's chain of loads
 // takes a few us whatever its cells)
@@ -666,7 +676,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     // owners itself
     const uint64_t nedges = 3ull * L.nx * L.ny * L.nz;
     const bool cells = nedges < (1ull << 32);
-    const Grid grid = make_grid(L, 0);
+    const Grid grid = make_grid(L, 0, segment_shift(ctx, L));
     const uint32_t nranges = (uint32_t)((chunks + RANGE - 1) / RANGE);
     const uint64_t nsegs = (uint64_t)grid.SL * (L.nz - 1);
     const uint32_t nblocks = (uint32_t)((nsegs + SCAN_BLOCK_SEGS - 1) / SCAN_BLOCK_SEGS);
@@ -699,8 +709,8 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     if (cells) {
         ca.grid = grid;
         ca.nsegs = (uint32_t)nsegs;
-        ca.run = count_run(ctx, nsegs);
-        ca.ntasks = grid.SL * ((L.nz - 1 + ca.run - 1) / ca.run);
+        ca.run = count_run(ctx, (uint64_t)grid.WL * (L.nz - 1));
+        ca.ntasks = grid.WL * ((L.nz - 1 + ca.run - 1) / ca.run);
         ca.segs = (uint2*)ctx->rowtri.p;
         ca.masks = (uint32_t*)((char*)ctx->rowtri.p + masks_at);
         ca.list = (uint4*)((char*)ctx->rowtri.p + list_at);
@@ -713,7 +723,8 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
         // chained with programmatic dependent launch: each kernel's blocks
         // are resident when its predecessor finishes, and wait for it on the device
         StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
-        e = launch_pdl(mc_cell_count<false>, dim3((ca.ntasks + 7) / 8), dim3(256), 0, ctx->stream, ca);
+        e = launch_pdl(grid.shift == 5 ? mc_cell_count<false, 5> : mc_cell_count<false, 3>, dim3((ca.ntasks + 7) / 8),
+                       dim3(256), 0, ctx->stream, ca);
         if (e == cudaSuccess) e = launch_pdl(mc_cell_scan, dim3(nblocks), dim3(512), 0, ctx->stream, ca);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "count launch");
         ctx->launches += 2;
@@ -1015,23 +1026,24 @@ uint64_t mc_table_edges(const CellTable* t) { return t->nedges; }
 // null: the lattices' edge keys or segments do not fit 32 bits (or the
 // allocation failed), and the block emit has to do
 CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n) {
-    uint64_t nsegs = 0, nedges = 0;
+    uint64_t nsegs = 0, nwarps = 0, nedges = 0;
     std::vector<Grid> grids(n);
     for (uint32_t i = 0; i < n; ++i) {
         if (nsegs >= (1ull << 31) || nedges >= (1ull << 32)) return nullptr;
-        grids[i] = make_grid(L[i], 0, (uint32_t)nsegs, (uint32_t)nedges);
+        grids[i] = make_grid(L[i], 0, 3, (uint32_t)nsegs, (uint32_t)nedges);
         nsegs += (uint64_t)grids[i].SL * (L[i].nz - 1);
+        nwarps += (uint64_t)grids[i].WL * (L[i].nz - 1);
         nedges += 3ull * L[i].nx * L[i].ny * L[i].nz;
     }
     if (nsegs >= (1ull << 31) || nedges >= (1ull << 32)) return nullptr;
-    const uint32_t run = count_run(ctx, nsegs);
+    const uint32_t run = count_run(ctx, nwarps);
     std::vector<uint4> tasks;
     std::vector<uint32_t> seg_grid(nsegs);
     for (uint32_t i = 0; i < n; ++i) {
         const Grid& g = grids[i];
         std::fill_n(seg_grid.begin() + g.seg0, (size_t)g.SL * (g.nz - 1), i);
         for (uint32_t z = 0; z < g.nz - 1; z += run)
-            for (uint32_t j = 0; j < g.SL; ++j) tasks.push_back(make_uint4(i, j, z, std::min(run, g.nz - 1 - z)));
+            for (uint32_t j = 0; j < g.WL; ++j) tasks.push_back(make_uint4(i, j, z, std::min(run, g.nz - 1 - z)));
     }
     CellTable* t = new CellTable();
     t->ngrids = n;
@@ -1039,7 +1051,10 @@ CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n) {
     CellArgs& a = t->a;
     a.nsegs = (uint32_t)nsegs;
     a.nblocks = (uint32_t)((nsegs + SCAN_BLOCK_SEGS - 1) / SCAN_BLOCK_SEGS);
-    a.group = emit_group(ctx, nsegs);
+    // segments of eight chunks, four together: small lattices are dense (1024
+    // chunks of 16^3 to 64^3 cells: emit 120 us, 172 one at a time, 135 eight
+    // together, 152 with 32 chunks)
+    a.group = 4;
     a.run = run;
     a.ntasks = (uint32_t)tasks.size();
     a.err = ctx->d_err;
@@ -1086,7 +1101,7 @@ iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, ui
     iso_status s;
     {
         StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
-        e = launch_pdl(mc_cell_count<true>, dim3((a.ntasks + 7) / 8), dim3(256), 0, ctx->stream, a);
+        e = launch_pdl(mc_cell_count<true, 3>, dim3((a.ntasks + 7) / 8), dim3(256), 0, ctx->stream, a);
         if (e == cudaSuccess) e = launch_pdl(mc_cell_scan, dim3(a.nblocks), dim3(512), 0, ctx->stream, a);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch count");
     }

@@ -3,9 +3,10 @@
 // whose edge maps share one 32-bit key space.
 //
 // A segment is 32 consecutive chunks of one cell layer in (y, x) order (a
-// chunk is 32 cells of a row; a layer's last segment may be shorter), so
-// segments in order are the reference's (z, y, x) visit order and one warp
-// handles a segment with lane = chunk.
+// chunk is 32 cells of a row; a layer's last segment may be shorter), or
+// eight in small lattices and tables, so segments in order are the
+// reference's (z, y, x) visit order.  A counting warp handles 32 chunks with
+// lane = chunk.
 //
 //   mc_cell_count   owned vertices and triangles of every segment, from the
 //                   sign bits
@@ -70,7 +71,7 @@ __device__ __forceinline__ uint32_t maj(uint32_t a, uint32_t b, uint32_t c) { re
 // the tables when they are generated), only cases with six or more have a
 // second loop, and e summed over the chunk comes from bit-sliced adders; the
 // few cells with six or more look their case up.
-template <bool TABLE>
+template <bool TABLE, uint32_t SHIFT>
 __global__ void __launch_bounds__(256) mc_cell_count(CellArgs A) {
     __shared__ uint8_t s_extra[256];  // per case: loops after the first
     __shared__ uint16_t s_owned[8];
@@ -90,8 +91,8 @@ __global__ void __launch_bounds__(256) mc_cell_count(CellArgs A) {
     if (TABLE) {
         t = __ldg(A.tasks + task);
     } else {
-        const uint32_t r = fdiv(task, A.grid.div_sl);
-        t.y = task - r * A.grid.SL;
+        const uint32_t r = fdiv(task, A.grid.div_wl);
+        t.y = task - r * A.grid.WL;
         t.z = r * A.run;
         t.w = min(A.run, A.grid.nz - 1 - t.z);
     }
@@ -101,7 +102,11 @@ __global__ void __launch_bounds__(256) mc_cell_count(CellArgs A) {
     const uint32_t valid = in ? chunk_valid(c, g.nx - 1) : 0u;
     const uint64_t layer = (uint64_t)g.ny * g.W;
     const uint32_t* p = g.bits + t.z * layer + (uint64_t)y * g.W + c;
-    uint32_t seg = g.seg0 + t.z * g.SL + t.y;
+    // the lane's segment, and whether its first lane writes the counts
+    constexpr uint32_t per = 1u << SHIFT;
+    const uint32_t sl = l >> SHIFT, first = lane & ~(per - 1);
+    const bool writes = lane == first && sl < g.SL;
+    uint32_t seg = g.seg0 + t.z * g.SL + sl;
     Quad lo = load_quad(p, g.W, in, nxt);
     p += layer;
     Quad up = load_quad(p, g.W, in, nxt);
@@ -151,12 +156,20 @@ __global__ void __launch_bounds__(256) mc_cell_count(CellArgs A) {
                 tri = __popc(s0) + 2 * __popc(s1) + 4 * __popc(s2) + 8 * __popc(s3) - 2 * __popc(act);
                 for (uint32_t m = s3 | (s2 & s1); m; m &= m - 1) tri -= 2 * s_extra[case_at(q, __ffs(m) - 1)];
             }
-            v = __reduce_add_sync(FULL, v);
-            tri = __reduce_add_sync(FULL, tri);
+            // at most 32 x 32 x 12 of either in a segment
+            uint32_t both = v | tri << 16;
+            if (SHIFT == 5) {
+                both = __reduce_add_sync(FULL, both);
+            } else {
+#pragma unroll
+                for (uint32_t o = 1; o < per; o <<= 1) both += __shfl_xor_sync(FULL, both, o);
+            }
+            v = both & 0xFFFFu;
+            tri = both >> 16;
         }
-        if (lane == 0) {
+        if (writes) {
             A.segs[seg] = make_uint2(v, tri);
-            if (chunks) A.masks[seg] = chunks;
+            if (tri) A.masks[seg] = SHIFT == 5 ? chunks : chunks >> first & ((1u << (per & 31u)) - 1u);
         }
         lo = hi;
         any_lo = any_hi;
@@ -403,7 +416,7 @@ __global__ void __launch_bounds__(256, 5) mc_cell_emit(CellEmitArgs A) {
             uint32_t act = 0;
             {
                 const uint32_t ls = seg - g.seg0, zc = fdiv(ls, g.div_sl);
-                const uint32_t l = 32 * (ls - zc * g.SL) + bit, y = fdiv(l, g.div_cw), c = l - y * g.CW;
+                const uint32_t l = ((ls - zc * g.SL) << g.shift) + bit, y = fdiv(l, g.div_cw), c = l - y * g.CW;
                 if (live) {
                     const uint32_t* a = g.bits + ((uint64_t)zc * g.ny + y) * g.W + c;
                     const uint32_t* b = a + (uint64_t)g.ny * g.W;

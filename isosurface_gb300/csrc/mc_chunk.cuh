@@ -46,13 +46,14 @@ struct Grid {
     uint32_t zoff;     // lattice z of layer 0 (a slab of a larger grid): positions and keys use z + zoff
     uint32_t chunk0;   // first global chunk id (a multiple of RANGE)
     uint32_t nchunks;  // CW * (ny-1) * (nz-1)
-    // the cell passes: chunks per cell layer, segments of 32 chunks per layer,
-    // first global segment, first key of its edges in the edge map
-    uint32_t S, SL, seg0, edge0;
-    FastDiv div_sl;
+    // the cell passes: chunks per cell layer, segments of 2^shift chunks per
+    // layer, counting warps (32 chunks) per layer, first global segment, first
+    // key of its edges in the edge map
+    uint32_t S, SL, WL, shift, seg0, edge0;
+    FastDiv div_sl, div_wl;
 };
 
-inline Grid make_grid(const Lattice& L, uint32_t chunk0, uint32_t seg0 = 0, uint32_t edge0 = 0) {
+inline Grid make_grid(const Lattice& L, uint32_t chunk0, uint32_t shift = 5, uint32_t seg0 = 0, uint32_t edge0 = 0) {
     Grid g;
     g.bits = L.bits;
     g.values = L.values;
@@ -70,7 +71,10 @@ inline Grid make_grid(const Lattice& L, uint32_t chunk0, uint32_t seg0 = 0, uint
     g.chunk0 = chunk0;
     g.nchunks = g.CW * (L.ny - 1) * (L.nz - 1);
     g.S = g.CW * (L.ny - 1);
-    g.SL = (g.S + 31) / 32;
+    g.shift = shift;
+    g.SL = (g.S + (1u << shift) - 1) >> shift;
+    g.WL = (g.S + 31) / 32;
+    g.div_wl = make_fastdiv(g.WL);
     g.seg0 = seg0;
     g.edge0 = edge0;
     g.div_sl = make_fastdiv(g.SL);
@@ -531,8 +535,8 @@ __global__ void __launch_bounds__(256) mc_block_emit(ChunkEmitArgs A, uint32_t m
 
 // Triangle corners: edge-map key -> vertex id recorded by the owner, for the
 // 3 * min(triangles, capacity) corners written (the count is read on the
-// device, so no host round trip is needed).  Four corners per thread and
-// step, so four independent gathers are in flight; the resolved corners also
+// device, so no host round trip is needed).  Bound by the gathers' latency;
+// eight corners per thread and step, so eight independent ones are in flight; the resolved corners also
 // go to the page-locked host buffer when the mesh is delivered there.  Keys
 // outside the map (corners of triangles an emit without room skipped) are
 // left alone.
@@ -547,15 +551,22 @@ __global__ void __launch_bounds__(256) mc_resolve_ids(uint32_t* __restrict__ idx
     const uint64_t n4 = n / 4, stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint4* __restrict__ p = reinterpret_cast<uint4*>(idx);
-    for (uint64_t i = t0; i < n4; i += stride) {
-        uint4 v = p[i];
-        const uint32_t a = v.x < nedges ? __ldg(edge_id + v.x) : v.x;
-        const uint32_t b = v.y < nedges ? __ldg(edge_id + v.y) : v.y;
-        const uint32_t c = v.z < nedges ? __ldg(edge_id + v.z) : v.z;
-        const uint32_t d = v.w < nedges ? __ldg(edge_id + v.w) : v.w;
-        v = make_uint4(a, b, c, d);
+    auto id = [&](uint32_t key) { return key < nedges ? __ldg(edge_id + key) : key; };
+    auto put = [&](uint64_t i, uint4 v) {
         p[i] = v;
         if (to_host) reinterpret_cast<uint4*>(host_i)[i] = v;
+    };
+    uint64_t i = t0;
+    for (; i + stride < n4; i += 2 * stride) {
+        uint4 v = p[i], w = p[i + stride];
+        v = make_uint4(id(v.x), id(v.y), id(v.z), id(v.w));
+        w = make_uint4(id(w.x), id(w.y), id(w.z), id(w.w));
+        put(i, v);
+        put(i + stride, w);
+    }
+    if (i < n4) {
+        const uint4 v = p[i];
+        put(i, make_uint4(id(v.x), id(v.y), id(v.z), id(v.w)));
     }
     const uint64_t k = 4 * n4 + t0;  // the last n % 4 corners
     if (k < n) {
@@ -567,7 +578,7 @@ __global__ void __launch_bounds__(256) mc_resolve_ids(uint32_t* __restrict__ idx
 
 // grid of mc_resolve_ids for at most 3 * cap_t corners
 inline unsigned resolve_blocks(uint64_t cap_t) {
-    return (unsigned)std::min<uint64_t>(std::max<uint64_t>((3 * cap_t / 4 + 255) / 256, 1), 16384);
+    return (unsigned)std::min<uint64_t>(std::max<uint64_t>((3 * cap_t / 8 + 255) / 256, 1), 16384);
 }
 
 // Per-grid mesh extents: (first vertex, vertex count, first triangle, triangle count).
