@@ -211,6 +211,39 @@ __device__ __forceinline__ void sphere_column(const SetArgs& A, const float4* ke
 
 // The samples of column (x, y), layers z0..z1, from the nk kept spheres;
 // sign words go to word wx of each row.
+// The fold over nk spheres (sphere(i), in order) at 32 points of a row and
+// z0 .. z1: a sphere at a time over up to FOLD_Z layers, so that it is read
+// and its x and y terms computed once for them, and their chains overlap.
+// (A point at a time, 64 spheres and 16 layers took 72 us however few rows
+// there were.)
+constexpr uint32_t FOLD_Z = 8;
+template <class F>
+__device__ __forceinline__ void fold_column(const SetArgs& A, F&& sphere, uint32_t nk, float px, float py, uint32_t x,
+                                            uint32_t y, uint32_t z0, uint32_t z1, bool valid, int lane, uint32_t wx) {
+    for (uint32_t zb = z0; zb <= z1; zb += FOLD_Z) {
+        float v[FOLD_Z], pz[FOLD_Z];
+#pragma unroll
+        for (uint32_t j = 0; j < FOLD_Z; ++j) {
+            v[j] = nk ? __int_as_float(0x7FFFFFFF) : 0.0f;  // fminf takes the first sphere's value
+            pz[j] = world((float)(zb + j + A.zoff) * A.inv, A.sz, A.oz, A.domain);
+        }
+        for (uint32_t i = 0; i < nk; ++i) {
+            const float4 c = sphere(i);
+#pragma unroll
+            for (uint32_t j = 0; j < FOLD_Z; ++j) v[j] = fminf(v[j], vlen(v3(px - c.x, py - c.y, pz[j] - c.z)) - c.w);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < FOLD_Z; ++j) {
+            const uint32_t z = zb + j;
+            if (z > z1) break;
+            const uint64_t row = (uint64_t)z * A.ny + y;
+            if (valid) A.field[row * A.pitch + x] = v[j];  // near-only mode writes all values here: a superset
+            const uint32_t b = __ballot_sync(FULL, valid && !(v[j] > 0.0f));
+            if (lane == 0) A.bits[row * A.W + wx] = b;
+        }
+    }
+}
+
 __device__ __forceinline__ void sample_column(const SetArgs& A, const float4* keep, const float4* thr, uint32_t nk,
                                               float px, float py, uint32_t x, uint32_t y, uint32_t z0, uint32_t z1,
                                               bool valid, int lane, uint32_t wx) {
@@ -221,19 +254,7 @@ __device__ __forceinline__ void sample_column(const SetArgs& A, const float4* ke
     case 4: sphere_column<4>(A, keep, thr, px, py, x, y, z0, z1, valid, lane, wx); return;
     default: break;
     }
-    for (uint32_t z = z0; z <= z1; ++z) {
-        const float pz = world((float)(z + A.zoff) * A.inv, A.sz, A.oz, A.domain);
-        float v = 0.0f;
-        for (uint32_t i = 0; i < nk; ++i) {
-            float4 c = keep[i];
-            float d = vlen(v3(px - c.x, py - c.y, pz - c.z)) - c.w;
-            v = (i == 0) ? d : fminf(v, d);
-        }
-        const uint64_t row = (uint64_t)z * A.ny + y;
-        if (valid) A.field[row * A.pitch + x] = v;  // near-only mode writes all values here: a superset
-        uint32_t b = __ballot_sync(FULL, valid && !(v > 0.0f));
-        if (lane == 0) A.bits[row * A.W + wx] = b;
-    }
+    fold_column(A, [&](uint32_t i) { return keep[i]; }, nk, px, py, x, y, z0, z1, valid, lane, wx);
 }
 
 __global__ void __launch_bounds__(256) sample_sphere_set(SetArgs A) {
@@ -523,32 +544,94 @@ __global__ void __launch_bounds__(32 * TILE_WARPS) set_tiles(SetArgs A, uint32_t
     }
 }
 
-// persistent: warps stride over (mixed tile, row) items.  A row is first
-// bounded against the tile's kept spheres alone (they decide the minimum
-// everywhere in the tile): a row wholly beyond reach writes its sign words.
+// persistent: warps stride over (mixed tile, row) items, or over their halves
+// in z while there are warps for those.  A row is first bounded against the
+// tile's kept spheres alone (they decide the minimum everywhere in the tile):
+// a row wholly beyond reach writes its sign words.  Where the tile keeps more
+// spheres than its record holds (coarse lattices, whose tiles are large), the
+// row keeps its own of all of them.
 constexpr int SET_ROWS_BLOCKS = 3;  // resident blocks of set_rows per SM (4 measured slower)
 
 __global__ void __launch_bounds__(256, SET_ROWS_BLOCKS) set_rows(SetArgs A, uint32_t tiles_y, const TileRec* recs,
                                                    const uint32_t* mixed, const uint32_t* nmixed, const float4* thr_all) {
     __shared__ float4 s_keep[8][KEEP_MAX];
     __shared__ float4 s_thr[8][KEEP_MAX];
+    __shared__ uint8_t s_idx[8][WARP_SET_MAX];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float4* sp = reinterpret_cast<const float4*>(A.spheres);
-    const uint32_t items = 8 * *nmixed;
-    for (uint32_t it = blockIdx.x * 8 + warp; it < items; it += gridDim.x * 8) {
+    const uint32_t rows = 8 * *nmixed, half = 2 * rows <= gridDim.x * 8 ? 1 : 0, items = rows << half;
+    for (uint32_t ih = blockIdx.x * 8 + warp; ih < items; ih += gridDim.x * 8) {
+        const uint32_t it = ih >> half;
         const uint32_t t = mixed[it >> 3];
         const uint32_t wx = t % A.W, rt = t / A.W;
-        const TileBox tb = tile_box(A, wx, rt % tiles_y, rt / tiles_y);
+        TileBox tb = tile_box(A, wx, rt % tiles_y, rt / tiles_y);
         const uint32_t y = tb.y0 + (it & 7);
         if (y > tb.y1) continue;
+        if (half) {
+            const uint32_t mid = tb.z0 + TZ / 2;
+            if (ih & 1) tb.z0 = mid;
+            else tb.z1 = min(tb.z1, mid - 1);
+            if (tb.z0 > tb.z1) continue;
+        }
         const TileRec* rec = recs + t;
         const uint32_t nk = rec->nk;
         const uint32_t x = tb.x0 + lane;
         const bool valid = x < A.nx;
         const float px = world((float)x * A.inv, A.sx, A.ox, A.domain);
         const float py = world((float)y * A.inv, A.sy, A.oy, A.domain);
-        if (nk > KEEP_MAX) {  // the fold over every sphere: the same minimum
-            sample_column(A, sp, nullptr, A.n, px, py, x, y, tb.z0, tb.z1, valid, lane, wx);
+        // bounds of a sphere's value over the row box (margins as in sample_sphere_set)
+        const float ax = world((float)tb.x0 * A.inv, A.sx, A.ox, A.domain);
+        const float bx = world((float)tb.x1 * A.inv, A.sx, A.ox, A.domain);
+        const float az = world((float)(tb.z0 + A.zoff) * A.inv, A.sz, A.oz, A.domain);
+        const float bz = world((float)(tb.z1 + A.zoff) * A.inv, A.sz, A.oz, A.domain);
+        const float lox = fminf(ax, bx), hix = fmaxf(ax, bx), loz = fminf(az, bz), hiz = fmaxf(az, bz);
+        auto bounds = [&](float4 c, float* up, float* lo) {
+            const float fx = fmaxf(fabsf(c.x - lox), fabsf(c.x - hix)), fy = fabsf(c.y - py);
+            const float fz = fmaxf(fabsf(c.z - loz), fabsf(c.z - hiz));
+            const float far = sqrtf(fx * fx + fy * fy + fz * fz);
+            *up = far - c.w + (1e-4f + 1e-5f * (far + fabsf(c.w)));
+            const float dx = fmaxf(fmaxf(lox - c.x, c.x - hix), 0.0f);
+            const float dz = fmaxf(fmaxf(loz - c.z, c.z - hiz), 0.0f);
+            const float near = sqrtf(dx * dx + fy * fy + dz * dz);
+            *lo = near - c.w - (1e-4f + 1e-5f * (near + fabsf(c.w) + 4.0f));
+        };
+        // a row wholly beyond reach: its sign words
+        auto decided = [&](float up, float lo) {
+            if (!A.near_only || !(lo > A.reach || up < -A.reach)) return false;
+            const uint32_t word = __ballot_sync(FULL, up < -A.reach && valid);
+            if (lane <= (int)(tb.z1 - tb.z0)) A.bits[((size_t)(tb.z0 + lane) * A.ny + y) * A.W + wx] = word;
+            return true;
+        };
+        auto warp_min = [](float v) {
+            for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULL, v, o));
+            return v;
+        };
+        if (nk > KEEP_MAX) {
+            float U = 3.0e38f, LB = 3.0e38f, low[WARP_SET_MAX / 32];
+#pragma unroll
+            for (int k = 0; k < (int)(WARP_SET_MAX / 32); ++k) {
+                const uint32_t i = 32 * k + lane;
+                low[k] = 3.0e38f;
+                if (i >= A.n) continue;
+                float up;
+                bounds(__ldg(sp + i), &up, &low[k]);
+                U = fminf(U, up);
+                LB = fminf(LB, low[k]);
+            }
+            U = warp_min(U);
+            if (decided(U, warp_min(LB))) continue;
+            __syncwarp();  // the previous item's list is used
+            uint32_t n = 0;
+#pragma unroll
+            for (int k = 0; k < (int)(WARP_SET_MAX / 32); ++k) {
+                const bool keep = 32u * k + lane < A.n && low[k] <= U;
+                const uint32_t m = __ballot_sync(FULL, keep);
+                if (keep) s_idx[warp][n + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
+                n += __popc(m);
+            }
+            __syncwarp();
+            fold_column(A, [&](uint32_t i) { return __ldg(sp + s_idx[warp][i]); }, n, px, py, x, y, tb.z0, tb.z1, valid,
+                        lane, wx);
             continue;
         }
         __syncwarp();  // the previous item's reads of the staging slots are done
@@ -559,33 +642,10 @@ __global__ void __launch_bounds__(256, SET_ROWS_BLOCKS) set_rows(SetArgs A, uint
             s_keep[warp][lane] = c;
             if (A.near_only) {
                 s_thr[warp][lane] = __ldg(thr_all + i);
-                // bounds of this sphere's value over the row box
-                const float ax = world((float)tb.x0 * A.inv, A.sx, A.ox, A.domain);
-                const float bx = world((float)tb.x1 * A.inv, A.sx, A.ox, A.domain);
-                const float az = world((float)(tb.z0 + A.zoff) * A.inv, A.sz, A.oz, A.domain);
-                const float bz = world((float)(tb.z1 + A.zoff) * A.inv, A.sz, A.oz, A.domain);
-                const float lox = fminf(ax, bx), hix = fmaxf(ax, bx), loz = fminf(az, bz), hiz = fmaxf(az, bz);
-                const float fx = fmaxf(fabsf(c.x - lox), fabsf(c.x - hix)), fy = fabsf(c.y - py);
-                const float fz = fmaxf(fabsf(c.z - loz), fabsf(c.z - hiz));
-                const float far = sqrtf(fx * fx + fy * fy + fz * fz);
-                up = far - c.w + (1e-4f + 1e-5f * (far + fabsf(c.w)));
-                const float dx = fmaxf(fmaxf(lox - c.x, c.x - hix), 0.0f);
-                const float dz = fmaxf(fmaxf(loz - c.z, c.z - hiz), 0.0f);
-                const float near = sqrtf(dx * dx + fy * fy + dz * dz);
-                lo = near - c.w - (1e-4f + 1e-5f * (near + fabsf(c.w) + 4.0f));
+                bounds(c, &up, &lo);
             }
         }
-        if (A.near_only) {
-            for (int o = 16; o > 0; o >>= 1) {
-                up = fminf(up, __shfl_xor_sync(FULL, up, o));
-                lo = fminf(lo, __shfl_xor_sync(FULL, lo, o));
-            }
-            if (lo > A.reach || up < -A.reach) {
-                const uint32_t word = __ballot_sync(FULL, up < -A.reach && valid);
-                if (lane <= (int)(tb.z1 - tb.z0)) A.bits[((size_t)(tb.z0 + lane) * A.ny + y) * A.W + wx] = word;
-                continue;
-            }
-        }
+        if (decided(warp_min(up), warp_min(lo))) continue;
         __syncwarp();
         sample_column(A, s_keep[warp], s_thr[warp], nk, px, py, x, y, tb.z0, tb.z1, valid, lane, wx);
     }
