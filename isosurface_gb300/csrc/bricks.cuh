@@ -14,6 +14,41 @@ namespace iso {
 
 static_assert(BRICK_ERR_CAPACITY == DERR_CAPACITY, "the core's capacity bit is the library's");
 
+// A set bit of a mask of primitives.  The union over a subset (in the same
+// order) equals eval_prims wherever every dropped primitive's value exceeds
+// some kept one's: fminf returns one of its operands, so the minimum over a
+// subset that holds the minimiser is the minimum over all.
+__device__ __forceinline__ uint32_t lowest_bit(uint64_t m) { return (uint32_t)(__ffsll((long long)m) - 1); }
+
+// eval_scalar at N points
+template <int N>
+__device__ __forceinline__ void eval_scalars(const ProgView& pv, const V3 (&p)[N], float (&v)[N]) {
+    V3 q[N];
+    if (!pv.prims) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) q[j] = p[j];
+        eval_points<N>(pv, 0, pv.n_ops, q, v);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        q[j] = prims_point(pv, p[j]);
+        v[j] = pv.nprims ? __int_as_float(0x7FFFFFFF) : 0.0f;  // fminf takes the first primitive's value
+    }
+    for (uint32_t i = 0; i < pv.nprims; ++i) {
+        const float4 c = ld_ro(pv.prims + 2 * i), a = ld_ro(pv.prims + 2 * i + 1);
+        auto each = [&](auto&& sd) {
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = fminf(v[j], sd(v3(q[j].x - c.x, q[j].y - c.y, q[j].z - c.z)));
+        };
+        const uint32_t type = float_bits(c.w);
+        if (type == OP_SPHERE) each([&](V3 t) { return sd_sphere(t, a.x); });
+        else if (type == OP_BOX) each([&](V3 t) { return sd_box(t, a.x, a.y, a.z); });
+        else if (type == OP_CYLINDER) each([&](V3 t) { return sd_cylinder(t, a.x, a.y); });
+        else each([&](V3 t) { return sd_torus(t, a.x, a.y); });
+    }
+}
+
 // The interpreted evaluator: the program's ops, or its flat list of
 // translated primitives (pruned per sub-brick when there are at most 64).
 struct VmEval {

@@ -59,12 +59,25 @@ struct Ctrl {
     unsigned long long flips;
 };
 
-// sign bit i & 31 of word i >> 5: lattice point i is inside
+// Sign bit i & 31 of word i >> 5: lattice point i is inside.  A lane takes
+// four points, 32 apart (128 solid: 62 us a point at a time).
+constexpr uint32_t POINTS = 4;
 __global__ void __launch_bounds__(256) emc_sample(emc::Args A, uint32_t points, uint32_t* bits) {
-    for (uint32_t i0 = blockIdx.x * 256; i0 < points; i0 += gridDim.x * 256) {
-        const uint32_t i = i0 + threadIdx.x;
-        const uint32_t word = __ballot_sync(0xFFFFFFFFu, i < points && emc::sample_item(A, i));
-        if ((threadIdx.x & 31) == 0) bits[i >> 5] = word;
+    constexpr uint32_t span = 256 * POINTS;
+    for (uint32_t i0 = blockIdx.x * span; i0 < points; i0 += gridDim.x * span) {
+        const uint32_t i = i0 + (threadIdx.x >> 5) * 32 * POINTS + (threadIdx.x & 31);
+        V3 q[POINTS], v[POINTS];
+#pragma unroll
+        for (uint32_t j = 0; j < POINTS; ++j) q[j] = emc::item_pos(A.g, i + 32 * j);
+        emc::eval_vectors<POINTS>(A.prog, q, v);
+#pragma unroll
+        for (uint32_t j = 0; j < POINTS; ++j) {
+            const uint32_t at = i + 32 * j;
+            const bool in = at < points;
+            if (in) A.field[at] = make_float4(v[j].x, v[j].y, v[j].z, 0.0f);
+            const uint32_t word = __ballot_sync(0xFFFFFFFFu, in && emc::directed_inside(v[j]));
+            if ((threadIdx.x & 31) == 0 && in) bits[at >> 5] = word;
+        }
     }
 }
 
@@ -378,7 +391,7 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
     if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counters");
     {
         StageTimer timer(ctx, ISO_STAGE_SAMPLE);
-        emc_sample<<<grid_for(ctx, points, 256, 16), 256, 0, ctx->stream>>>(A, (uint32_t)points, bits);
+        emc_sample<<<grid_for(ctx, points, 256 * POINTS, 16), 256, 0, ctx->stream>>>(A, (uint32_t)points, bits);
     }
     cudaStream_t side;
     {

@@ -131,18 +131,30 @@ __host__ __device__ __forceinline__ V3 dir_torus(V3 p, float R, float t) {
 // component-wise min, max and max(b, -a) (csg.rs:41-45, 74-78, 102-106), and
 // CentralDifference passes the inner source's vector through (source.rs:76-80).
 // The host accepts only programs made of these ops (directed_ops_only).
-// The top of the value stack is `top`; vs[1 .. vsp - 1] holds the rest (a
-// run-time index keeps vs in local memory, which a chain of two-operand ops
-// would otherwise read and write three times per op).
-static __host__ __device__ __noinline__ V3 eval_vector(const ProgView& pv, V3 p) {
-    V3 vs[VSTACK];
-    V3 ps[PSTACK];
+// N points at a time (they share the decoding of an op and the loads of its
+// constants).  The tops of the value stacks are `top`; vs[1 .. vsp - 1] holds
+// the rest (a run-time index keeps vs in local memory, which a chain of
+// two-operand ops would otherwise read and write three times per op).
+template <int N>
+__host__ __device__ __forceinline__ void eval_vectors(const ProgView& pv, V3 (&q)[N], V3 (&top)[N]) {
+    V3 vs[VSTACK][N];
+    V3 ps[PSTACK][N];
     int vsp = 0, psp = 0;
-    V3 q = p, top = p;
-    auto push = [&](V3 v) {
-        if (vsp) vs[vsp] = top;
+    auto each = [&](auto&& f) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) f(j);
+    };
+    each([&](int j) { top[j] = q[j]; });
+    auto push = [&](auto&& value) {
+        each([&](int j) {
+            if (vsp) vs[vsp][j] = top[j];
+            top[j] = value(q[j]);
+        });
         ++vsp;
-        top = v;
+    };
+    auto join = [&](auto&& value) {
+        --vsp;
+        each([&](int j) { top[j] = value(vs[vsp][j], top[j]); });
     };
     for (uint32_t pc = 0; pc < pv.n_ops; ++pc) {
         const uint32_t w = ld_ro(pv.ops + pc);
@@ -150,26 +162,32 @@ static __host__ __device__ __noinline__ V3 eval_vector(const ProgView& pv, V3 p)
         const float* k = pv.k + (w >> 8);
         switch (op) {
         case OP_PT_DOMAIN: case OP_PT_TRANSLATE:
-            ps[psp++] = q;
-            q = pt_apply(op, k, q);
+            each([&](int j) {
+                ps[psp][j] = q[j];
+                q[j] = pt_apply(op, k, q[j]);
+            });
+            ++psp;
             break;
-        case OP_PT_POP: q = ps[--psp]; break;
-        case OP_SPHERE: push(dir_sphere(q, k[0])); break;
-        case OP_BOX: push(dir_box(q, k[0], k[1], k[2])); break;
-        case OP_CYLINDER: push(dir_cylinder(q, k[0], k[1])); break;
-        case OP_TORUS: push(dir_torus(q, k[0], k[1])); break;
-        case OP_UNION: --vsp; top = vmin(vs[vsp], top); break;
-        case OP_INTERSECTION: --vsp; top = vmax3(vs[vsp], top); break;
-        case OP_DIFFERENCE: {
-            --vsp;
-            const V3 a = vs[vsp];
-            top = vmax3(top, v3(-a.x, -a.y, -a.z));
+        case OP_PT_POP:
+            --psp;
+            each([&](int j) { q[j] = ps[psp][j]; });
             break;
-        }
+        case OP_SPHERE: push([&](V3 p) { return dir_sphere(p, k[0]); }); break;
+        case OP_BOX: push([&](V3 p) { return dir_box(p, k[0], k[1], k[2]); }); break;
+        case OP_CYLINDER: push([&](V3 p) { return dir_cylinder(p, k[0], k[1]); }); break;
+        case OP_TORUS: push([&](V3 p) { return dir_torus(p, k[0], k[1]); }); break;
+        case OP_UNION: join([](V3 a, V3 b) { return vmin(a, b); }); break;
+        case OP_INTERSECTION: join([](V3 a, V3 b) { return vmax3(a, b); }); break;
+        case OP_DIFFERENCE: join([](V3 a, V3 b) { return vmax3(b, v3(-a.x, -a.y, -a.z)); }); break;
         default: break;  // CD_BEGIN / CD_END: the vector is the inner source's
         }
     }
-    return top;
+}
+
+static __host__ __device__ __noinline__ V3 eval_vector(const ProgView& pv, V3 p) {
+    V3 q[1] = {p}, v[1];
+    eval_vectors<1>(pv, q, v);
+    return v[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -368,13 +386,16 @@ struct Args {
     uint32_t* err;       // DERR_* bits
 };
 
-// the Directed value of lattice point `i`; whether it is inside
-__host__ __device__ inline bool sample_item(const Args& A, uint64_t i) {
-    const uint32_t n = A.g.n;
-    const uint32_t p = (uint32_t)i, r = p / n, x = p - r * n, z = r / n, y = r - z * n;
-    const V3 v = eval_vector(A.prog, point_pos(A.g, x, y, z));
+// the position of lattice point `i`
+__host__ __device__ __forceinline__ V3 item_pos(const Grid& g, uint32_t i) {
+    const uint32_t r = i / g.n, z = r / g.n;
+    return point_pos(g, i - r * g.n, r - z * g.n, z);
+}
+
+// the Directed value of lattice point `i`
+__host__ __device__ inline void sample_item(const Args& A, uint64_t i) {
+    const V3 v = eval_vector(A.prog, item_pos(A.g, (uint32_t)i));
     A.field[i] = make_float4(v.x, v.y, v.z, 0.0f);
-    return directed_inside(v);
 }
 
 // vertices and triangles cell (x, y, z) of case `cube` adds

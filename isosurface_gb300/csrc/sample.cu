@@ -36,6 +36,32 @@ __global__ void __launch_bounds__(256) sample_generic(VmEval ev, BrickLattice g)
     field_warp(ev, g, (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5));
 }
 
+// The same with four rows to a warp: the interpreter decodes an op once for
+// four points of a lane, and their chains overlap (128^3 torus: 28 us a row
+// at a time).  For lattices that still give every scheduler several warps.
+constexpr uint32_t ROWS = 4;
+__global__ void __launch_bounds__(256) sample_generic_rows(VmEval ev, BrickLattice g) {
+    const uint32_t lane = threadIdx.x & 31, yq = (g.ny + ROWS - 1) / ROWS;
+    const uint64_t gw = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (gw >= (uint64_t)g.W * yq * g.nz) return;
+    const uint32_t w = (uint32_t)(gw % g.W), r = (uint32_t)(gw / g.W), y0 = ROWS * (r % yq), z = r / yq;
+    const uint32_t x = 32 * w + lane;
+    V3 p[ROWS];
+    float v[ROWS];
+#pragma unroll
+    for (uint32_t j = 0; j < ROWS; ++j)
+        p[j] = v3((float)x * g.inv, (float)(y0 + j) * g.inv, (float)(z + g.zoff) * g.inv);
+    eval_scalars<ROWS>(ev.pv, p, v);
+#pragma unroll
+    for (uint32_t j = 0; j < ROWS; ++j) {
+        if (y0 + j >= g.ny) break;
+        const uint64_t row = (uint64_t)z * g.ny + y0 + j;
+        if (x < g.nx) g.field[row * g.pitch + x] = v[j];
+        const uint32_t b = __ballot_sync(FULL, x < g.nx && !(v[j] > 0.0f));
+        if (lane == 0) g.bits[row * g.W + w] = b;
+    }
+}
+
 // Union of spheres, hard min, optionally behind a domain map.  Each block
 // samples a 32 x 8 x TZ tile of points; it first keeps only the spheres that
 // can attain the minimum somewhere in the tile:
@@ -807,7 +833,11 @@ iso_status launch_sample_grid(iso_ctx* ctx, const iso_program* prog, uint32_t nx
         if (!near_only && jit_sample_field(ctx, prog, g, (warps + 7) / 8, &je)) {
             if (je != cudaSuccess) return cuda_fail(ctx, je, "compiled field sampler launch");
         } else {
-            sample_generic<<<(unsigned)((warps + 7) / 8), 256, 0, ctx->stream>>>(VmEval{prog->view()}, g);
+            const uint64_t fours = (uint64_t)W * ((ny + ROWS - 1) / ROWS) * nz;
+            if (fours >= 16 * (uint64_t)ctx->sms && fours < (1ull << 31))
+                sample_generic_rows<<<(unsigned)((fours + 7) / 8), 256, 0, ctx->stream>>>(VmEval{prog->view()}, g);
+            else
+                sample_generic<<<(unsigned)((warps + 7) / 8), 256, 0, ctx->stream>>>(VmEval{prog->view()}, g);
         }
     }
     ctx->launches++;

@@ -50,20 +50,34 @@ __host__ __device__ __forceinline__ V3 pt_apply(uint32_t op, const float* k, V3 
               (m[6] * d.x + m[7] * d.y) + m[8] * d.z);
 }
 
-// Scalar evaluation of ops[begin, end) at p (one value left on the stack).
-// The top value and the current point live in registers; only the entries
-// below them are kept in (local-memory) stacks, so a primitive, a binary
-// operator and a point op each touch memory at most once.
-static __host__ __device__ __noinline__ float eval_range(const ProgView& pv, uint32_t begin, uint32_t end, V3 p) {
-    float vs[VSTACK];  // values below the top: vs[0 .. vsp-2]
-    V3 ps[PSTACK];     // points below the current one: ps[0 .. psp-1]
-    float tos = 0.0f;  // top value (vsp > 0)
-    V3 q = p;          // current point
+// Scalar evaluation of ops[begin, end) at the N points q (one value each left
+// on the stack, in tos).  The top values and the current points live in
+// registers; only the entries below them are kept in (local-memory) stacks,
+// so a primitive, a binary operator and a point op each touch memory at most
+// once.  Several points share the decoding of an op and the loads of its
+// constants, and their chains overlap.
+template <int N>
+__host__ __device__ __forceinline__ void eval_points(const ProgView& pv, uint32_t begin, uint32_t end, V3 (&q)[N],
+                                                     float (&tos)[N]) {
+    float vs[VSTACK][N];  // values below the top: vs[0 .. vsp-2]
+    V3 ps[PSTACK][N];     // points below the current ones: ps[0 .. psp-1]
     int vsp = 0, psp = 0;
-    auto push = [&](float x) {
-        if (vsp > 0) vs[vsp - 1] = tos;
-        tos = x;
+    auto each = [&](auto&& f) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) f(j);
+    };
+    each([&](int j) { tos[j] = 0.0f; });
+    auto push = [&](auto&& value) {
+        each([&](int j) {
+            if (vsp > 0) vs[vsp - 1][j] = tos[j];
+            tos[j] = value(q[j]);
+        });
         ++vsp;
+    };
+    // binary operators: a = the entry below the top, b = the top
+    auto join = [&](auto&& value) {
+        each([&](int j) { tos[j] = value(vs[vsp - 2][j], tos[j]); });
+        --vsp;
     };
     for (uint32_t pc = begin; pc < end; ++pc) {
         const uint32_t w = ld_ro(pv.ops + pc);
@@ -71,36 +85,55 @@ static __host__ __device__ __noinline__ float eval_range(const ProgView& pv, uin
         const float* k = pv.k + (w >> 8);
         switch (op) {
         case OP_PT_DOMAIN: case OP_PT_TRANSLATE: case OP_PT_RIGID:
-            ps[psp++] = q;
-            q = pt_apply(op, k, q);
+            each([&](int j) {
+                ps[psp][j] = q[j];
+                q[j] = pt_apply(op, k, q[j]);
+            });
+            ++psp;
             break;
-        case OP_PT_POP: q = ps[--psp]; break;
-        case OP_SPHERE: push(sd_sphere(q, k[0])); break;
-        case OP_BOX: push(sd_box(q, k[0], k[1], k[2])); break;
-        case OP_CYLINDER: push(sd_cylinder(q, k[0], k[1])); break;
-        case OP_TORUS: push(sd_torus(q, k[0], k[1])); break;
-        // binary operators: a = the entry below the top, b = the top
-        case OP_UNION: tos = fminf(vs[vsp - 2], tos); --vsp; break;
-        case OP_INTERSECTION: tos = fmaxf(vs[vsp - 2], tos); --vsp; break;
-        case OP_DIFFERENCE: tos = fmaxf(tos, -vs[vsp - 2]); --vsp; break;
-        case OP_SMOOTH_UNION: tos = smooth_min(vs[vsp - 2], tos, k[0]); --vsp; break;
+        case OP_PT_POP:
+            --psp;
+            each([&](int j) { q[j] = ps[psp][j]; });
+            break;
+        case OP_SPHERE: push([&](V3 p) { return sd_sphere(p, k[0]); }); break;
+        case OP_BOX: push([&](V3 p) { return sd_box(p, k[0], k[1], k[2]); }); break;
+        case OP_CYLINDER: push([&](V3 p) { return sd_cylinder(p, k[0], k[1]); }); break;
+        case OP_TORUS: push([&](V3 p) { return sd_torus(p, k[0], k[1]); }); break;
+        case OP_UNION: join([](float a, float b) { return fminf(a, b); }); break;
+        case OP_INTERSECTION: join([](float a, float b) { return fmaxf(a, b); }); break;
+        case OP_DIFFERENCE: join([](float a, float b) { return fmaxf(b, -a); }); break;
+        case OP_SMOOTH_UNION: join([&](float a, float b) { return smooth_min(a, b, k[0]); }); break;
         case OP_SPHERE_SET: {
-            uint32_t n = (uint32_t)k[0];
-            bool smooth = k[1] != 0.0f;
-            float kk = k[2];
-            float v = 0.0f;
+            const uint32_t n = (uint32_t)k[0];
+            const bool smooth = k[1] != 0.0f;
+            const float kk = k[2];
+            float v[N];
+            each([&](int j) { v[j] = 0.0f; });
             for (uint32_t i = 0; i < n; ++i) {
                 const float* c = k + 3 + 4 * i;
-                float d = vlen(v3(q.x - c[0], q.y - c[1], q.z - c[2])) - c[3];
-                v = (i == 0) ? d : (smooth ? smooth_min(v, d, kk) : fminf(v, d));
+                each([&](int j) {
+                    const float d = vlen(v3(q[j].x - c[0], q[j].y - c[1], q[j].z - c[2])) - c[3];
+                    v[j] = (i == 0) ? d : (smooth ? smooth_min(v[j], d, kk) : fminf(v[j], d));
+                });
             }
-            push(v);
+            each([&](int j) {
+                if (vsp > 0) vs[vsp - 1][j] = tos[j];
+                tos[j] = v[j];
+            });
+            ++vsp;
             break;
         }
         default: break;  // CD_BEGIN / CD_END are markers in scalar mode
         }
     }
-    return tos;
+}
+
+// the same at one point
+static __host__ __device__ __noinline__ float eval_range(const ProgView& pv, uint32_t begin, uint32_t end, V3 p) {
+    V3 q[1] = {p};
+    float v[1];
+    eval_points<1>(pv, begin, end, q, v);
+    return v[0];
 }
 
 // Primitive i of ProgView::prims at q (a point after the leading domain map):
@@ -130,12 +163,6 @@ static __host__ __device__ __noinline__ float eval_prims(const ProgView& pv, V3 
     }
     return v;
 }
-
-// A set bit of a mask of primitives.  The union over a subset (in the same
-// order) equals eval_prims wherever every dropped primitive's value exceeds
-// some kept one's: fminf returns one of its operands, so the minimum over a
-// subset that holds the minimiser is the minimum over all.
-__device__ __forceinline__ uint32_t lowest_bit(uint64_t m) { return (uint32_t)(__ffsll((long long)m) - 1); }
 
 __host__ __device__ __forceinline__ float eval_scalar(const ProgView& pv, V3 p) {
     return pv.prims ? eval_prims(pv, p) : eval_range(pv, 0, pv.n_ops, p);
