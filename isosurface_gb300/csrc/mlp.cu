@@ -238,7 +238,10 @@ __global__ void __launch_bounds__(256, 2) gemm_f32(GemmArgs G) {
 }
 
 // 128 x 128 tiles once they give every SM one (n x 256 outputs: n >= 64 per
-// SM), else 64 x 64 ones, four times as many blocks
+// SM), else 64 x 64 ones, four times as many blocks.  (65536 x 256 outputs are
+// 3.4 waves of two blocks to an SM; the last part of one as 64 x 128 tiles in
+// a launch of its own took 164 + 40 us against 189: a block whose SM has
+// fallen empty beside it already runs faster.)
 // returns the number of tile rows
 template <bool A_K, bool B_K, int EPI>
 uint32_t gemm(cudaStream_t s, int sms, const GemmArgs& G) {
@@ -269,15 +272,28 @@ __global__ void fourier(const float* pts, uint32_t n, float* out) {
     reinterpret_cast<float2*>(out)[i] = make_float2(sn, cs);
 }
 
-// y[p] = a[p] . w + b; warp per point
-__global__ void out_forward(const float* a, uint32_t n, const float* w, const float* b, float* y) {
-    const uint32_t p = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const int lane = threadIdx.x & 31;
-    if (p >= n) return;
-    float s = 0.0f;
-    for (int k = lane; k < HID; k += 32) s += a[(size_t)p * HID + k] * w[k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) y[p] = s + b[0];
+// y[p] = a[p] . w + b; a warp for every four points, bound by the read of a
+// (65536 points: 34 us with a point per warp and 4-byte loads)
+__global__ void __launch_bounds__(256) out_forward(const float* __restrict__ a, uint32_t n, const float* __restrict__ w,
+                                                   const float* b, float* __restrict__ y) {
+    static_assert(HID == 256, "two float4 per lane");
+    const uint32_t lane = threadIdx.x & 31, p0 = (blockIdx.x * 8 + threadIdx.x / 32) * 4;
+    if (p0 >= n) return;
+    const float4 w0 = __ldg(reinterpret_cast<const float4*>(w) + lane), w1 = __ldg(reinterpret_cast<const float4*>(w) + 32 + lane);
+    float4 q[4][2];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const float4* row = reinterpret_cast<const float4*>(a + (size_t)min(p0 + j, n - 1) * HID);
+        q[j][0] = __ldg(row + lane);
+        q[j][1] = __ldg(row + 32 + lane);
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const float4 u = q[j][0], v = q[j][1];
+        float s = ((u.x * w0.x + u.y * w0.y) + (u.z * w0.z + u.w * w0.w)) + ((v.x * w1.x + v.y * w1.y) + (v.z * w1.z + v.w * w1.w));
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        if (lane == 0 && p0 + j < n) y[p0 + j] = s + b[0];
+    }
 }
 
 // Truncated L1: e = y - t inside the band |t| < d; where the target is
@@ -307,28 +323,41 @@ __global__ void loss_l1(const float* y, const float* t, uint32_t n, float clampd
 }
 
 // The backward pass of the output layer in one read of the last layer's z
-// and a (thread = column, a range of points per block):
+// and a (a range of points per block; thread = four columns, every fourth
+// point):
 //   dz[p][k] = dy[p] w[k] sigmoid(z[p][k]), each block's column sums of it in
 //   gb[block][k], and of dy[p] a[p][k] in gw[block][k]
-__global__ void __launch_bounds__(HID) out_backward(const float* __restrict__ dy, const float* __restrict__ w,
+// Bound by memory (65536 points: 200 MB; 86 us with a column per thread, whose
+// 4-byte loads left too little in flight).
+__global__ void __launch_bounds__(256) out_backward(const float* __restrict__ dy, const float* __restrict__ w,
                                                     const float* __restrict__ z, const float* __restrict__ a,
                                                     uint32_t n, float* __restrict__ dz, float* gw, float* gb) {
-    const uint32_t k = threadIdx.x;
+    static_assert(HID == 256, "64 threads cover a row");
+    __shared__ float4 s_w[4][64], s_b[4][64];
+    const uint32_t c = threadIdx.x % 64, g = threadIdx.x / 64;
     const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
     const uint32_t p0 = blockIdx.x * per, p1 = min(n, p0 + per);
-    const float wk = w[k];
-    float sw = 0.0f, sb = 0.0f;
+    const float4 wk = __ldg(reinterpret_cast<const float4*>(w) + c);
+    float4 sw = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sb = sw;
 #pragma unroll 4
-    for (uint32_t p = p0; p < p1; ++p) {
-        const float g = __ldg(dy + p);
-        const size_t at = (size_t)p * HID + k;
-        const float d = g * wk * sigmoid(z[at]);
-        dz[at] = d;
-        sb += d;
-        sw += g * a[at];
+    for (uint32_t p = p0 + g; p < p1; p += 4) {
+        const float d = __ldg(dy + p);
+        const size_t at = (size_t)p * (HID / 4) + c;
+        const float4 zz = __ldg(reinterpret_cast<const float4*>(z) + at), aa = __ldg(reinterpret_cast<const float4*>(a) + at);
+        const float4 o = make_float4(d * wk.x * sigmoid(zz.x), d * wk.y * sigmoid(zz.y), d * wk.z * sigmoid(zz.z),
+                                     d * wk.w * sigmoid(zz.w));
+        reinterpret_cast<float4*>(dz)[at] = o;
+        sb = make_float4(sb.x + o.x, sb.y + o.y, sb.z + o.z, sb.w + o.w);
+        sw = make_float4(sw.x + d * aa.x, sw.y + d * aa.y, sw.z + d * aa.z, sw.w + d * aa.w);
     }
-    gw[(size_t)blockIdx.x * HID + k] = sw;
-    gb[(size_t)blockIdx.x * HID + k] = sb;
+    s_w[g][c] = sw;
+    s_b[g][c] = sb;
+    __syncthreads();
+    const float* fw = reinterpret_cast<const float*>(s_w);
+    const float* fb = reinterpret_cast<const float*>(s_b);
+    const uint32_t k = threadIdx.x;
+    gw[(size_t)blockIdx.x * HID + k] = (fw[k] + fw[HID + k]) + (fw[2 * HID + k] + fw[3 * HID + k]);
+    gb[(size_t)blockIdx.x * HID + k] = (fb[k] + fb[HID + k]) + (fb[2 * HID + k] + fb[3 * HID + k]);
 }
 
 // The gradients that are sums over the points (the biases', the output
@@ -340,17 +369,17 @@ struct ColumnSums {
     float* out[NLAYERS + 1];
 };
 
-__global__ void __launch_bounds__(256) add_partials(ColumnSums S) {
-    __shared__ double s_sum[8][32];
+__global__ void __launch_bounds__(1024) add_partials(ColumnSums S) {
+    __shared__ double s_sum[32][32];
     const uint32_t c = threadIdx.x % 32, r0 = threadIdx.x / 32, k = 32 * blockIdx.x + c;
     const float* p = S.part[blockIdx.y] + k;
     double sum = 0.0;
 #pragma unroll 8
-    for (uint32_t r = r0; r < S.rows[blockIdx.y]; r += 8) sum += (double)__ldg(p + (size_t)r * HID);
+    for (uint32_t r = r0; r < S.rows[blockIdx.y]; r += 32) sum += (double)__ldg(p + (size_t)r * HID);
     s_sum[r0][c] = sum;
     __syncthreads();
     if (r0) return;
-    for (int w = 1; w < 8; ++w) sum += s_sum[w][c];
+    for (int w = 1; w < 32; ++w) sum += s_sum[w][c];
     S.out[blockIdx.y][k] = (float)sum;
 }
 
@@ -481,7 +510,7 @@ void forward(iso_mlp* net, const Views& w, uint32_t n) {
         g.C2 = w.a[l];
         gemm<true, true, EPI_FORWARD>(s, net->ctx->sms, g);
     }
-    out_forward<<<blocks(n, 8), 256, 0, s>>>(w.a[NLAYERS - 1], n, P + OUT_W, P + OUT_B, w.y);
+    out_forward<<<blocks(n, 32), 256, 0, s>>>(w.a[NLAYERS - 1], n, P + OUT_W, P + OUT_B, w.y);
     net->ctx->launches += 2 + NLAYERS;
 }
 
@@ -503,7 +532,7 @@ void backward(iso_mlp* net, const Views& w, uint32_t n, float clampd) {
     }
     const unsigned out_blocks = std::min<unsigned>(blocks(n, 16), 4 * (unsigned)net->ctx->sms);
     sums.rows[last] = sums.rows[NLAYERS] = out_blocks;
-    out_backward<<<out_blocks, HID, 0, s>>>(w.dy, P + OUT_W, w.z[last], w.a[last], n, dz,
+    out_backward<<<out_blocks, 256, 0, s>>>(w.dy, P + OUT_W, w.z[last], w.a[last], n, dz,
                                             const_cast<float*>(sums.part[NLAYERS]), const_cast<float*>(sums.part[last]));
     for (int l = last; l >= 0; --l) {
         const int in_dim = l ? HID : FF;
@@ -520,7 +549,7 @@ void backward(iso_mlp* net, const Views& w, uint32_t n, float clampd) {
             std::swap(dz, below);
         }
     }
-    add_partials<<<dim3(HID / 32, NLAYERS + 1), 256, 0, s>>>(sums);
+    add_partials<<<dim3(HID / 32, NLAYERS + 1), 1024, 0, s>>>(sums);
     net->ctx->launches += 2 + 2 * NLAYERS;
 }
 
