@@ -40,7 +40,7 @@ UNITS = {
     "jit.cu": ["-fmad=false"],
 }
 HEADERS = ["internal.h", "vm.cuh", "vm_math.cuh", "bricks.cuh", "bricks_core.cuh", "smooth_set.cuh", "mc_tables.h", "mc_chunk.cuh", "mc_cells.cuh",
-           "qef.cuh", "qef_planes.cuh", "dc_core.cuh", "block_sums.cuh", "mlp.h", "emc.cuh", "emc_tables.h"]
+           "qef.cuh", "qef_rows.cuh", "qef_planes.cuh", "dc_core.cuh", "block_sums.cuh", "mlp.h", "emc.cuh", "emc_tables.h"]
 # sources the library compiles again at run time, for one program at a time
 # (jit.cu): embedded as string literals in _build/jit_sources.inc
 JIT_SOURCES = (("kJitVmMath", "vm_math.cuh"), ("kJitBricksCore", "bricks_core.cuh"),

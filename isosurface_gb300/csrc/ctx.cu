@@ -33,7 +33,10 @@ iso_status set_device(iso_ctx* ctx) {
 iso_status fork_side(iso_ctx* ctx, cudaStream_t* side) {
     cudaError_t e = cudaSuccess;
     if (!ctx->side) {
-        e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
+        // its kernels are what the passes beside them wait for in the end
+        int least = 0, greatest = 0;
+        cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        e = cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "side stream");

@@ -18,8 +18,8 @@
 // such cell -- eight normals from the program (sample_normals_at_corners,
 // marching_cubes_impl.rs:58-69), tangent planes, the planar cells' centre of
 // mass or particle placement, the non-planar cells listed for (5) dc_feature:
-// their MinimiseQEF (f64 SVD) in full warps; (4) and (5) on a side stream
-// beside (6) the lattice marching-cubes passes, whose emission waits for them.
+// their MinimiseQEF (f64 SVD); (4) and (5) on a side stream beside (6) the
+// lattice marching-cubes passes, whose vertices are placed last.
 // A program without a bound takes its full field through dc_dual in place of
 // (2) and (3).
 #include <cuda_runtime.h>
@@ -28,6 +28,7 @@
 
 #include "internal.h"
 #include "qef.cuh"
+#include "qef_rows.cuh"
 #include "vm.cuh"
 #include "dc_core.cuh"
 
@@ -285,18 +286,78 @@ struct VmHermite {
 
 __global__ void __launch_bounds__(128) dc_place(VmHermite ev, DcCells A) { dc_place_body(ev, A); }
 
-// MinimiseQEF of the non-planar cells dc_place listed, one per thread over
-// one-warp blocks (grid-stride): each is a serial chain of f64 operations
-// (the SVD, in the reference's order), and a warp's f64 instruction holds
-// its sub-partition's f64 unit for many cycles however few of its lanes are
-// active, so packing the chains into full warps cuts the f64 instructions
-// the scattered cells of dc_place would have issued.  (Spread evenly over the
-// sub-partitions below 32 cells for each it was no faster alone, 129 us
-// against 121 for the 257 lattice, and slower beside the counting passes.)
-// The chain of one warp is the whole time: its matrices in registers took it
-// from 138 us to 121 (qef.cuh).
+// MinimiseQEF of feature cell i (its normals kept) by the eight lanes of
+// `mask`, a corner each: tangent_planes, then the solve.
+__device__ __forceinline__ void feature_by_rows(const DcCells& A, uint32_t i, uint32_t mask, uint32_t* err) {
+    using namespace qef;
+    const uint32_t y = threadIdx.x & 7, id = A.features[i], m = A.n - 1;
+    const uint32_t cx = id % m, r = id / m, cy = r % m, cz = r / m + A.zoff;
+    const float px[2] = {(float)cx * A.inv, (float)(cx + 1) * A.inv};
+    const float py[2] = {(float)cy * A.inv, (float)(cy + 1) * A.inv};
+    const float pz[2] = {(float)cz * A.inv, (float)(cz + 1) * A.inv};
+    // corner k of CORNERS (marching_cubes_tables.rs:16-25)
+    auto corner = [&](uint32_t k) { return f3(px[(k + 1) >> 1 & 1], py[k >> 1 & 1], pz[k >> 2]); };
+    const F3 nrm = A.fnormals[8 * (uint64_t)i + y];
+    auto normal_of = [&](uint32_t k) {
+        return f3(__shfl_sync(mask, nrm.x, k, 8), __shfl_sync(mask, nrm.y, k, 8), __shfl_sync(mask, nrm.z, k, 8));
+    };
+    F3 com = f3(0.0f, 0.0f, 0.0f);
+    float least = 3.40282347e+38f;
+    uint32_t pair = ~0u;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        com = add(com, corner(k));
+        const float angle = dot(nrm, normal_of(k));
+        if (angle < least) {
+            least = angle;
+            pair = 8 * y + k;
+        }
+    }
+    com = f3(com.x / 8.0f, com.y / 8.0f, com.z / 8.0f);
+    for (uint32_t o = 1; o < 8; o <<= 1) {  // the first of equals in (i, j) order
+        const float a = __shfl_xor_sync(mask, least, o, 8);
+        const uint32_t q = __shfl_xor_sync(mask, pair, o, 8);
+        if (a < least || (a == least && q < pair)) {
+            least = a;
+            pair = q;
+        }
+    }
+    F3 p = com;
+    bool ok = true;
+    if (!(least > FEATURE_ANGLE)) {
+        const F3 na = normal_of(pair >> 3 & 7), nb = normal_of(pair & 7);
+        const F3 axis = normalised_or_zero(pair == ~0u ? f3(0.0f, 0.0f, 0.0f) : cross(na, nb));
+        const float along = dot(axis, nrm);
+        float lo = fminf(1.0f, along), hi = fmaxf(-1.0f, along);
+        for (uint32_t o = 1; o < 8; o <<= 1) {
+            lo = fminf(lo, __shfl_xor_sync(mask, lo, o, 8));
+            hi = fmaxf(hi, __shfl_xor_sync(mask, hi, o, 8));
+        }
+        float c = fmaxf(fabsf(lo), fabsf(hi));
+        c = sqrtf(1.0f - c * c);
+        p = add(com, solve_planes_rows(mask, nrm, dot(sub(corner(y), com), nrm), 8, c > FEATURE_ANGLE, &ok));
+    }
+    if (y != 0) return;
+    if (!ok) atomicOr(err, DERR_SVD_ITER);
+    A.dpos[id] = DcPos{p.x, p.y, p.z, 0.0f};
+}
+
+// MinimiseQEF of the non-planar cells dc_place listed, over one-warp blocks.
+// A solve is a serial chain of f64 operations (the SVD, in the reference's
+// order), and a warp's f64 instruction holds its sub-partition's unit for many
+// cycles however few of its lanes are active.  Few cells go to eight lanes
+// each (qef_rows.cuh), which shortens the chain; many, beyond what ten such
+// warps per SM take in a turn, to one lane each, in full warps, which issues
+// fewer instructions.  257 lattice: 121 us with a lane each (138 with its
+// matrices in local memory).
+constexpr uint32_t ROW_WARPS = 10;  // one-warp blocks per SM
 __global__ void __launch_bounds__(32) dc_feature(VmHermite ev, DcCells A, uint32_t* err) {
     const uint32_t n = *A.nfeatures;
+    if (n <= A.fcap && n <= 4 * gridDim.x) {
+        const uint32_t group = threadIdx.x >> 3, i = 4 * blockIdx.x + group;
+        if (i < n) feature_by_rows(A, i, 0xFFu << (8 * group), err);
+        return;
+    }
     for (uint32_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += gridDim.x * 32) {
         const uint32_t id = A.features[i];
         qef::F3 corners[8], normals[8];
@@ -416,7 +477,7 @@ static iso_status dc_lattice(iso_ctx* ctx, const iso_program* prog, uint32_t n, 
         dc_place<<<(unsigned)place_blocks, 128, 0, side>>>(ev, cells);
     if (placer == 0 && je == cudaSuccess) {
         // one warp for each of the SMs' four sub-partitions
-        dc_feature<<<(unsigned)(4 * sms), 32, 0, side>>>(ev, cells, ctx->d_err);
+        dc_feature<<<(unsigned)(ROW_WARPS * sms), 32, 0, side>>>(ev, cells, ctx->d_err);
         ctx->launches++;
     }
     ctx->launches += 2;

@@ -26,6 +26,7 @@
 
 #include "block_sums.cuh"
 #include "internal.h"
+#include "qef_rows.cuh"
 
 #define ISO_TABLE static __device__ const
 #include "emc_tables.h"
@@ -225,17 +226,35 @@ __global__ void __launch_bounds__(128) emc_vertices(emc::Args A, const uint32_t*
         emc::vertex_item(A, list[i], false);
 }
 
-// The feature points of the kept feature cells.  Each is one serial chain of
-// f64 operations (the SVD, in the reference's order), and a warp's f64
-// instruction holds its sub-partition's f64 unit for many cycles whatever its
-// active lanes, so the chains go to as many warps as the SMs' sub-partitions
-// can take (the grid), each warp with a few, rather than scattered over every
-// warp of a pass over cells.  They start as soon as the cells are known.
+// The feature points of the kept feature cells, over one-warp blocks, as soon
+// as the cells are known.  Each is one serial chain of f64 operations (the
+// SVD, in the reference's order), and a warp's f64 instruction holds its
+// sub-partition's f64 unit for many cycles whatever its active lanes.  Few
+// cells go to eight lanes each (qef_rows.cuh; a cell with more than eight
+// crossings to its first lane), which shortens the chain; many, beyond what
+// the grid takes in a turn, to one lane each, in full warps.  128 solid, 2200
+// cells: 92 us with a lane each, spread evenly.
+constexpr uint32_t ROW_WARPS = 10;  // one-warp blocks per SM
 __global__ void __launch_bounds__(32) emc_features(emc::Args A, Feature* kept, uint32_t cap, const Ctrl* ctrl) {
     const uint32_t n = min(ctrl->features, cap);
-    const uint32_t per = min(32u, (n + gridDim.x - 1) / gridDim.x);
-    if (threadIdx.x >= per) return;
-    for (uint32_t i = blockIdx.x * per + threadIdx.x; i < n; i += gridDim.x * per) {
+    if (n <= 4 * gridDim.x) {
+        const uint32_t group = threadIdx.x >> 3, y = threadIdx.x & 7, i = 4 * blockIdx.x + group;
+        if (i >= n) return;
+        const emc::PlanesN& t = kept[i].planes;
+        const int rows = t.n;
+        bool ok = true;
+        if (rows <= 8) {
+            const uint32_t at = min(y, (uint32_t)rows - 1);
+            const qef::F3 p = qef::add(t.com, qef::solve_planes_rows(0xFFu << (8 * group), t.normal[at], t.d[at], rows,
+                                                                     t.feature == qef::EDGE, &ok));
+            if (y == 0) kept[i].point = p;
+        } else if (y == 0) {
+            kept[i].point = emc::minimise_qef_n(t, &ok);
+        }
+        if (!ok && y == 0) atomicOr(A.err, DERR_SVD_ITER);
+        return;
+    }
+    for (uint32_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += gridDim.x * 32) {
         bool ok;
         const qef::F3 p = emc::minimise_qef_n(kept[i].planes, &ok);
         if (!ok) atomicOr(A.err, DERR_SVD_ITER);
@@ -403,7 +422,7 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
         // the feature points on a side stream: the passes below neither read
         // nor wait for them
         if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
-        emc_features<<<(unsigned)(4 * std::max(ctx->sms, 1)), 32, 0, side>>>(A, kept, cap, ctrl);
+        emc_features<<<ROW_WARPS * (unsigned)std::max(ctx->sms, 1), 32, 0, side>>>(A, kept, cap, ctrl);
         scan_block_sums<<<1, 1024, 0, ctx->stream>>>(sums, nblocks, &ctrl->totals);
         ctx->launches += 2;
     }
