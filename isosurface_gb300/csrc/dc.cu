@@ -18,8 +18,8 @@
 // such cell -- eight normals from the program (sample_normals_at_corners,
 // marching_cubes_impl.rs:58-69), tangent planes, the planar cells' centre of
 // mass or particle placement, the non-planar cells listed for (5) dc_feature:
-// their MinimiseQEF (f64 SVD); (4) and (5) on a side stream beside (6) the
-// lattice marching-cubes passes, whose vertices are placed last.
+// their MinimiseQEF (f64 SVD); (4) and (5) on a side stream
+// beside (6) the lattice marching-cubes passes, whose emission waits for them.
 // A program without a bound takes its full field through dc_dual in place of
 // (2) and (3).
 #include <cuda_runtime.h>
@@ -342,22 +342,29 @@ __device__ __forceinline__ void feature_by_rows(const DcCells& A, uint32_t i, ui
     A.dpos[id] = DcPos{p.x, p.y, p.z, 0.0f};
 }
 
-// MinimiseQEF of the non-planar cells dc_place listed, over one-warp blocks.
-// A solve is a serial chain of f64 operations (the SVD, in the reference's
-// order), and a warp's f64 instruction holds its sub-partition's unit for many
-// cycles however few of its lanes are active.  Few cells go to eight lanes
-// each (qef_rows.cuh), which shortens the chain; many, beyond what ten such
-// warps per SM take in a turn, to one lane each, in full warps, which issues
-// fewer instructions.  257 lattice: 121 us with a lane each (138 with its
-// matrices in local memory).
-constexpr uint32_t ROW_WARPS = 10;  // one-warp blocks per SM
+// MinimiseQEF of the non-planar cells dc_place listed, over one-warp blocks,
+// one warp for each of the SMs' four sub-partitions.  A solve is a serial
+// chain of f64 operations (the SVD, in the reference's order), and a warp's
+// f64 instruction holds its sub-partition's unit for many cycles however few
+// of its lanes are active.  Few cells go to eight lanes each (qef_rows.cuh),
+// which shortens the chain; more, beyond a warp of four cells for each
+// sub-partition, to one lane each, in full warps, which issues fewer
+// instructions.  257 lattice, about 10000 cells: 121 us with a lane each (138
+// with its matrices in local memory), 175 with four lanes each.  Two kernels,
+// of which one has nothing to do: in one, the one-lane solve took 131 us.
+constexpr uint32_t ROW_WARPS = 4;  // one-warp blocks per SM
+__device__ __forceinline__ bool by_rows(const DcCells& A, uint32_t n, uint32_t blocks) {
+    return n <= A.fcap && n <= 4 * blocks;
+}
+
+__global__ void __launch_bounds__(32) dc_feature_rows(DcCells A, uint32_t* err) {
+    const uint32_t n = *A.nfeatures, group = threadIdx.x >> 3, i = 4 * blockIdx.x + group;
+    if (by_rows(A, n, gridDim.x) && i < n) feature_by_rows(A, i, 0xFFu << (8 * group), err);
+}
+
 __global__ void __launch_bounds__(32) dc_feature(VmHermite ev, DcCells A, uint32_t* err) {
     const uint32_t n = *A.nfeatures;
-    if (n <= A.fcap && n <= 4 * gridDim.x) {
-        const uint32_t group = threadIdx.x >> 3, i = 4 * blockIdx.x + group;
-        if (i < n) feature_by_rows(A, i, 0xFFu << (8 * group), err);
-        return;
-    }
+    if (by_rows(A, n, gridDim.x)) return;
     for (uint32_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += gridDim.x * 32) {
         const uint32_t id = A.features[i];
         qef::F3 corners[8], normals[8];
@@ -477,8 +484,9 @@ static iso_status dc_lattice(iso_ctx* ctx, const iso_program* prog, uint32_t n, 
         dc_place<<<(unsigned)place_blocks, 128, 0, side>>>(ev, cells);
     if (placer == 0 && je == cudaSuccess) {
         // one warp for each of the SMs' four sub-partitions
+        dc_feature_rows<<<(unsigned)(ROW_WARPS * sms), 32, 0, side>>>(cells, ctx->d_err);
         dc_feature<<<(unsigned)(ROW_WARPS * sms), 32, 0, side>>>(ev, cells, ctx->d_err);
-        ctx->launches++;
+        ctx->launches += 2;
     }
     ctx->launches += 2;
     if (je != cudaSuccess || (s = check_launch(ctx, "dc passes")) != ISO_OK) {

@@ -231,10 +231,11 @@ __global__ void __launch_bounds__(128) emc_vertices(emc::Args A, const uint32_t*
 // SVD, in the reference's order), and a warp's f64 instruction holds its
 // sub-partition's f64 unit for many cycles whatever its active lanes.  Few
 // cells go to eight lanes each (qef_rows.cuh; a cell with more than eight
-// crossings to its first lane), which shortens the chain; many, beyond what
-// the grid takes in a turn, to one lane each, in full warps.  128 solid, 2200
-// cells: 92 us with a lane each, spread evenly.
-constexpr uint32_t ROW_WARPS = 10;  // one-warp blocks per SM
+// crossings to its first lane), which shortens the chain; more, beyond a warp
+// of four cells for each sub-partition, to one lane each, in full warps (dc.cu
+// has a case measured there).  128 solid, 2200 cells: 72 us, 92 with a lane
+// each, spread evenly.
+constexpr uint32_t ROW_WARPS = 4;  // one-warp blocks per SM
 __global__ void __launch_bounds__(32) emc_features(emc::Args A, Feature* kept, uint32_t cap, const Ctrl* ctrl) {
     const uint32_t n = min(ctrl->features, cap);
     if (n <= 4 * gridDim.x) {

@@ -643,13 +643,10 @@ static uint32_t count_run(const iso_ctx* ctx, uint64_t nsegs) {
     return (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, nsegs / (160 * (uint64_t)std::max(ctx->sms, 1))));
 }
 
-// persistent: five blocks of 256 threads per SM, or a warp for every group the
-// list could hold.  `beside` kernels of the side stream: two per SM, which
-// leaves registers for those (a dual lattice of 256^3: 323 us; with five the
-// placement waited for the emission, 425; one after the other 348)
-static unsigned cell_emit_blocks(const iso_ctx* ctx, const CellArgs& ca, bool beside = false) {
+// persistent: five blocks of 256 threads per SM, or a warp for every group the list could hold
+static unsigned cell_emit_blocks(const iso_ctx* ctx, const CellArgs& ca) {
     const uint64_t groups = ca.nsegs / ca.group + ca.nblocks;
-    return (unsigned)std::min<uint64_t>((groups + 7) / 8, (beside ? 2ull : 5ull) * (uint64_t)std::max(ctx->sms, 1));
+    return (unsigned)std::min<uint64_t>((groups + 7) / 8, 5ull * (uint64_t)std::max(ctx->sms, 1));
 }
 
 // One synchronisation per extraction: count, scan and emit are queued back to
@@ -704,7 +701,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     uint32_t* ctrl = (uint32_t*)(totals + 8);
     char* arrays = (char*)ctx->scan.p + 128;
     // only the cell emit delivers to host buffers
-    ctx->host_out.armed = cells && !L.join && ctx->host_out.v && ctx->host_out.i;
+    ctx->host_out.armed = cells && ctx->host_out.v && ctx->host_out.i;
     cudaError_t e = cudaSuccess;
     CellArgs ca{};
     uint2 *local = (uint2*)ctx->rowtri.p, *rangeagg = (uint2*)arrays, *rangepre = rangeagg + nranges;
@@ -748,7 +745,7 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
         if (keys) cap_v = std::min<uint64_t>(cap_v, ctx->mesh_k.bytes / 16);
         const iso_ctx::HostOut& H = ctx->host_out;
         uint64_t* out_k = keys ? (uint64_t*)ctx->mesh_k.p : nullptr;
-        if (!cells && L.join && ctx->side_open) {
+        if (L.join && ctx->side_open) {
             const iso_status js = join_side(ctx);
             if (js != ISO_OK) return js;
         }
@@ -756,26 +753,15 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
             StageTimer timer(ctx, ISO_STAGE_EMIT);
             if (cells) {
                 const CellEmitArgs ea{ca, (float*)ctx->mesh_v.p, (uint32_t*)ctx->mesh_i.p, out_k, cap_v, cap_t,
-                                      (uint32_t*)ctx->edges.p, L.join ? nullptr : H.v, H.cap_v, H.cap_t, L.join};
-                cudaError_t le = launch_pdl(mc_cell_emit<false>, dim3(cell_emit_blocks(ctx, ca, L.join)), dim3(256),
-                                            0, ctx->stream, ea);
+                                      (uint32_t*)ctx->edges.p, H.v, H.cap_v, H.cap_t};
+                cudaError_t le = launch_pdl(mc_cell_emit<false>, dim3(cell_emit_blocks(ctx, ca)), dim3(256), 0,
+                                            ctx->stream, ea);
                 if (le == cudaSuccess)
                     le = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream,
                                     (uint32_t*)ctx->mesh_i.p, (const uint64_t*)totals, cap_t,
-                                    (const uint32_t*)ctx->edges.p, (uint32_t)nedges, L.join ? nullptr : H.i, H.cap_v,
-                                    H.cap_t, cap_v);
+                                    (const uint32_t*)ctx->edges.p, (uint32_t)nedges, H.i, H.cap_v, H.cap_t, cap_v);
                 if (le != cudaSuccess) return cuda_fail(ctx, le, "emit launch");
                 ctx->launches++;
-                if (L.join) {
-                    // the side stream's positions come last
-                    if (ctx->side_open) {
-                        const iso_status js = join_side(ctx);
-                        if (js != ISO_OK) return js;
-                    }
-                    mc_place_vertices<<<(unsigned)std::min<uint64_t>((cap_v + 255) / 256, 8ull * (uint64_t)std::max(ctx->sms, 1)),
-                                        256, 0, ctx->stream>>>((float*)ctx->mesh_v.p, totals, cap_v, L.positions);
-                    ctx->launches++;
-                }
             } else {
                 const ChunkEmitArgs ea{d_grid, nullptr, (uint32_t)chunks, local, rangepre, (float*)ctx->mesh_v.p,
                                        (uint32_t*)ctx->mesh_i.p, out_k, cap_v, cap_t, ctx->d_err};
@@ -1135,7 +1121,7 @@ iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, ui
         out_v = (float*)ctx->mesh_v.p;
         out_i = (uint32_t*)ctx->mesh_i.p;
     }
-    const CellEmitArgs ea{a, out_v, out_i, nullptr, cap_v, cap_t, (uint32_t*)ctx->edges.p, nullptr, 0, 0, false};
+    const CellEmitArgs ea{a, out_v, out_i, nullptr, cap_v, cap_t, (uint32_t*)ctx->edges.p, nullptr, 0, 0};
     {
         StageTimer timer(ctx, ISO_STAGE_EMIT);
         e = launch_pdl(mc_cell_emit<true>, dim3(cell_emit_blocks(ctx, a)), dim3(256), 0, ctx->stream, ea);

@@ -295,9 +295,6 @@ struct CellEmitArgs {
     // receive the mesh when all of it fits both them and the device buffers
     float* host_v;
     uint64_t host_cap_v, host_cap_t;
-    // positions that are not there yet: a vertex is its two points' indices
-    // and where it lies between them, for mc_place_vertices
-    bool later;
 };
 
 // place of set bit number r (from 0, lowest first) of m
@@ -522,12 +519,12 @@ __global__ void __launch_bounds__(256, 5) mc_cell_emit(CellEmitArgs A) {
                     const float* val = g.values + (((uint64_t)cz * g.ny + cy) * g.pitch + cx);
                     const float fa = __ldg(val + S.uoff[k]), fb = __ldg(val + S.voff[k]);
                     const uint32_t cell = (cz * g.ny + cy) * g.nx + cx;
-                    const uint32_t lay = g.nx * g.ny;
-                    const uint32_t ia = cell + ((d & 1) + ((d & 2) ? g.nx : 0) + ((d & 4) ? lay : 0));
-                    const uint32_t ib = cell + ((d >> 3 & 1) + ((d & 16) ? g.nx : 0) + ((d & 32) ? lay : 0));
                     V3 pa, pb;
-                    if (g.positions && !A.later) {
-                        const float4 qa = __ldg(g.positions + ia), qb = __ldg(g.positions + ib);
+                    if (g.positions) {
+                        const float4* pos = g.positions + cell;
+                        const uint32_t lay = g.nx * g.ny;
+                        const float4 qa = __ldg(pos + ((d & 1) + ((d & 2) ? g.nx : 0) + ((d & 4) ? lay : 0)));
+                        const float4 qb = __ldg(pos + ((d >> 3 & 1) + ((d & 16) ? g.nx : 0) + ((d & 32) ? lay : 0)));
                         pa = v3(qa.x, qa.y, qa.z);
                         pb = v3(qb.x, qb.y, qb.z);
                     } else {
@@ -543,9 +540,9 @@ __global__ void __launch_bounds__(256, 5) mc_cell_emit(CellEmitArgs A) {
                     const uint32_t vid = vcarry + j;
                     if (vid < A.cap_v) {
                         float* o = A.out_v + 3 * (size_t)vid;
-                        o[0] = A.later ? __uint_as_float(ia) : pa.x * omt + pb.x * tt;
-                        o[1] = A.later ? __uint_as_float(ib) : pa.y * omt + pb.y * tt;
-                        o[2] = A.later ? tt : pa.z * omt + pb.z * tt;
+                        o[0] = pa.x * omt + pb.x * tt;
+                        o[1] = pa.y * omt + pb.y * tt;
+                        o[2] = pa.z * omt + pb.z * tt;
                         if (A.out_k) {
                             // the lattice edge's key: lower end point * 3 + axis
                             const uint32_t lo = d & d >> 3 & 7u;
@@ -594,21 +591,5 @@ __global__ void __launch_bounds__(256, 5) mc_cell_emit(CellEmitArgs A) {
             }
         }
         grp = gridDim.x * 8 + __shfl_sync(FULL, taken, 0);
-    }
-}
-
-// The vertices an emission left as two points and the place between them
-// (CellEmitArgs::later).  The emission of a dual lattice needs everything but
-// the placed positions, which take longer than it does.
-__global__ void __launch_bounds__(256) mc_place_vertices(float* __restrict__ v, const uint64_t* totals, uint64_t cap_v,
-                                                         const float4* __restrict__ positions) {
-    const uint64_t n = min(totals[1], cap_v);
-    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
-        float* o = v + 3 * i;
-        const float tt = o[2], omt = 1.0f - tt;
-        const float4 a = __ldg(positions + __float_as_uint(o[0])), b = __ldg(positions + __float_as_uint(o[1]));
-        o[0] = a.x * omt + b.x * tt;
-        o[1] = a.y * omt + b.y * tt;
-        o[2] = a.z * omt + b.z * tt;
     }
 }
