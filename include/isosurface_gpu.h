@@ -399,8 +399,8 @@ typedef struct iso_batch iso_batch;
 ISO_API iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, uint32_t nprograms,
                                     const iso_chunk_desc* chunks, uint32_t nchunks, iso_batch** out);
 ISO_API iso_status iso_batch_destroy(iso_batch* batch);
-/* Run every chunk: work-queue sampler + chunked classify/scan/emit over all
- * chunks at once.  The first run (and any run after a capacity overflow) is
+/* Run every chunk: sampling, counting, scan and emission over all chunks at
+ * once.  The first run (and any run after a capacity overflow) is
  * eager; with ISO_BATCH_GRAPH later runs replay one captured CUDA graph. */
 ISO_API iso_status iso_batch_run(iso_batch* batch, uint32_t flags, iso_mesh_info* info);
 /* The same chunks one extraction at a time (the per-chunk-launch baseline). */
@@ -411,8 +411,8 @@ ISO_API iso_status iso_batch_run_per_chunk(iso_batch* batch, iso_mesh_info* info
  * first), one synchronisation at the start and one at the end. */
 ISO_API iso_status iso_batch_run_per_chunk_async(iso_batch* batch, iso_mesh_info* info);
 ISO_API iso_status iso_batch_extents(iso_batch* batch, uint32_t* extents /* 4 per chunk */);
-/* Sampler slab depth (z layers per work-queue tile) for chunks of `size`
- * (0: all sizes); depth 0 = whole chunk. */
+/* Sampler slab depth for chunks of `size` (0: all sizes): a warp's sub-bricks
+ * stay within that many z layers; depth 0 = whole chunk (the default). */
 ISO_API iso_status iso_batch_set_slab(iso_batch* batch, uint32_t size, uint32_t depth);
 /* Times the sampler at each candidate slab depth for every chunk-size class
  * of the batch and keeps the fastest; results are cached per GPU model in
