@@ -343,16 +343,16 @@ __device__ __forceinline__ void feature_by_rows(const DcCells& A, uint32_t i, ui
 }
 
 // MinimiseQEF of the non-planar cells dc_place listed, over one-warp blocks,
-// one warp for each of the SMs' four sub-partitions.  A solve is a serial
+// six to an SM.  A solve is a serial
 // chain of f64 operations (the SVD, in the reference's order), and a warp's
 // f64 instruction holds its sub-partition's unit for many cycles however few
 // of its lanes are active.  Few cells go to eight lanes each (qef_rows.cuh),
-// which shortens the chain; more, beyond a warp of four cells for each
-// sub-partition, to one lane each, in full warps, which issues fewer
-// instructions.  257 lattice, about 10000 cells: 121 us with a lane each (138
+// which shortens the chain; more, beyond six warps of four cells per SM, to
+// one lane each, in full warps, which issues fewer instructions (csg at 65:
+// 163 us with six, 180 with four; more is no faster).  257 lattice, about 10000 cells: 121 us with a lane each (138
 // with its matrices in local memory), 175 with four lanes each.  Two kernels,
 // of which one has nothing to do: in one, the one-lane solve took 131 us.
-constexpr uint32_t ROW_WARPS = 4;  // one-warp blocks per SM
+constexpr uint32_t ROW_WARPS = 6;  // one-warp blocks per SM
 __device__ __forceinline__ bool by_rows(const DcCells& A, uint32_t n, uint32_t blocks) {
     return n <= A.fcap && n <= 4 * blocks;
 }
@@ -483,7 +483,6 @@ static iso_status dc_lattice(iso_ctx* ctx, const iso_program* prog, uint32_t n, 
     if (!jit_dc_place(side, prog, cells, place_blocks, &je))  // the program's compiled normals (jit.cu)
         dc_place<<<(unsigned)place_blocks, 128, 0, side>>>(ev, cells);
     if (placer == 0 && je == cudaSuccess) {
-        // one warp for each of the SMs' four sub-partitions
         dc_feature_rows<<<(unsigned)(ROW_WARPS * sms), 32, 0, side>>>(cells, ctx->d_err);
         dc_feature<<<(unsigned)(ROW_WARPS * sms), 32, 0, side>>>(ev, cells, ctx->d_err);
         ctx->launches += 2;

@@ -401,11 +401,9 @@ __host__ __device__ inline void sample_item(const Args& A, uint64_t i) {
 // vertices and triangles cell (x, y, z) of case `cube` adds
 __host__ __device__ inline void cell_counts(uint32_t x, uint32_t y, uint32_t z, int cube, uint32_t feature, uint32_t* nv,
                                             uint32_t* nt) {
-    const uint32_t mask = iso_edge_mask[cube];
-    uint32_t v = feature;
-    for (int e = 0; e < 12; ++e)
-        if ((mask & (1u << e)) && owns_edge(x, y, z, e)) ++v;
-    *nv = v;
+    // the edges that owns_edge gives a cell on these low faces
+    const uint32_t owned = iso_owned_mask[(x == 0 ? 1 : 0) | (y == 0 ? 2 : 0) | (z == 0 ? 4 : 0)];
+    *nv = feature + (uint32_t)popc(iso_edge_mask[cube] & owned);
     *nt = feature ? iso_emc_fan_count[cube] : iso_tri_count[cube];
 }
 
