@@ -92,7 +92,7 @@ __device__ __forceinline__ BrickLattice lattice_of(const SampleGrid& sg) {
 // another grid's primitives.  (Blocks that classified a tile, listed its
 // mixed sub-bricks in shared memory and sampled them between barriers spent
 // 44 % of their warps' time at those, on tiles of 20 sub-bricks for a 16^3
-// chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells; now 47 and 143 for
+// chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells; now 39 and 139 for
 // batch_rows, which issues in 73 % of its slots.)
 __global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const SampleGrid* grids, uint32_t ntasks,
                                                       Mixed* list, uint32_t* count) {
@@ -118,21 +118,10 @@ __global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const S
     uint32_t cls4 = 0;
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) cls4 |= __shfl_sync(0xFFFFFFFFu, cls, (lane & ~3u) + i) << (8 * i);
-    const uint32_t mine = mixed >> (lane & ~3u) & 15u;
     if (have) {
+        // (the mixed sub-bricks' bytes are batch_rows' to write, after this)
         const uint32_t word = decided_word(cls4, g.nx, w), z = za + j;
-        for (uint32_t r = 0; r < 4 && z < g.nz; ++r) {
-            const uint32_t y = ya + r;
-            if (y >= g.ny) break;
-            uint32_t* at = g.bits + ((uint64_t)z * g.ny + y) * g.W + w;
-            if (!mine) {
-                *at = word;
-            } else {
-                for (uint32_t i = 0; i < 4; ++i)
-                    if (!(mine >> i & 1u))
-                        reinterpret_cast<uint8_t*>(at)[i] = decided_byte(cls4 >> (8 * i) & 0xFFu, g.nx, 4 * w + i);
-            }
-        }
+        for (uint32_t y = ya; y < min(ya + 4, g.ny) && z < g.nz; ++y) g.bits[((uint64_t)z * g.ny + y) * g.W + w] = word;
     }
     if (!mixed) return;
     // the task's part of the list, filled up to whole fours

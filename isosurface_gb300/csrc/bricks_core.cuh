@@ -25,13 +25,13 @@
 // multiples of 4, at most BRICK_MAX sub-bricks.  One thread classifies one
 // sub-brick.  A group of four sub-bricks along x (32 x 4 x 4 points, one
 // sign word in each of 16 rows) that is wholly decided gets its sign words
-// at once; in a mixed group the decided sub-bricks get their sign bytes and
-// every sample of the mixed ones is evaluated, four mixed sub-bricks to a
-// warp (eight lanes each, one sign byte per row), so that no lane idles on a
-// decided sub-brick.  Classification appends the mixed sub-bricks to a list (a block
-// per tile here; a warp per 32 sub-bricks for many small lattices, batch.cu);
-// a persistent grid then samples the list, so the evaluation is spread evenly
-// however the surface falls.
+// at once; in a mixed group every sample of the mixed ones is evaluated
+// afterwards, four mixed sub-bricks to a warp (eight lanes each, one sign byte
+// per row), so that no lane idles on a decided sub-brick.  Classification
+// appends the mixed sub-bricks to a list (a block per tile here; a warp per 32
+// sub-bricks for many small lattices, batch.cu); a persistent grid then
+// samples the list, so the evaluation is spread evenly however the surface
+// falls.
 //
 // The evaluator `Ev` provides value(p) and, for pruned unions, prunable(),
 // nprims(), point(p) (the point after a leading domain map, which keeps the
@@ -157,8 +157,8 @@ __device__ __forceinline__ void brick_classes(const Ev& ev, const BrickTile& T, 
     }
 }
 
-// Sign word of a wholly decided group: its sub-bricks' classes, bits past
-// the row's last sample clear.
+// Sign word of a group from its sub-bricks' classes, bits of mixed ones and
+// past the row's last sample clear.
 __device__ __forceinline__ uint32_t decided_word(uint32_t cls4, uint32_t nx, uint32_t w) {
     uint32_t word = 0;
     for (uint32_t j = 0; j < 4; ++j)
@@ -167,18 +167,11 @@ __device__ __forceinline__ uint32_t decided_word(uint32_t cls4, uint32_t nx, uin
     return valid < 32 ? word & ((1u << valid) - 1u) : word;
 }
 
-// The sign byte (8 samples from x = 8 sx) of a decided sub-brick.
-__device__ __forceinline__ uint8_t decided_byte(uint32_t cls, uint32_t nx, uint32_t sx) {
-    if (cls != BRICK_IN || 8 * sx >= nx) return 0;
-    const uint32_t valid = nx - 8 * sx;
-    return valid < 8 ? (uint8_t)((1u << valid) - 1u) : (uint8_t)0xFFu;
-}
-
 // The sign bits of group gi of tile T (four sub-bricks along x, one sign
-// word in each of 16 rows), written by one thread: a wholly decided group
-// gets its words; in a mixed group the decided sub-bricks get their bytes
-// and the mixed ones are left to brick_quad.  Returns the mask of mixed
-// sub-bricks (bit j: sub-brick 4 gi + j).
+// word in each of 16 rows), written by one thread; brick_quad writes the
+// bytes of the mixed sub-bricks after that (writing only the decided ones'
+// here took up to 64 byte stores).  Returns the mask of mixed sub-bricks (bit
+// j: sub-brick 4 gi + j).
 __device__ __forceinline__ uint32_t brick_group_bits(const BrickTile& T, uint32_t gi, const uint8_t* s_cls) {
     const BrickLattice& g = T.g;
     const uint32_t SY = (T.y1 - T.y0 + 3) / 4;
@@ -193,14 +186,7 @@ __device__ __forceinline__ uint32_t brick_group_bits(const BrickTile& T, uint32_
     for (uint32_t r = 0; r < 16; ++r) {
         const uint32_t y = T.y0 + 4 * gy + (r & 3), z = T.z0 + 4 * gz + (r >> 2);
         if (y >= T.y1 || z >= T.z1) continue;
-        uint32_t* at = g.bits + ((uint64_t)z * g.ny + y) * g.W + w;
-        if (!mixed) {
-            *at = word;
-        } else {
-            for (uint32_t j = 0; j < 4; ++j)
-                if (!((mixed >> j) & 1u))
-                    reinterpret_cast<uint8_t*>(at)[j] = decided_byte((cls4 >> (8 * j)) & 0xFFu, g.nx, 4 * w + j);
-        }
+        g.bits[((uint64_t)z * g.ny + y) * g.W + w] = word;
     }
     return mixed;
 }

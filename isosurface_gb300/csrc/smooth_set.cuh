@@ -304,24 +304,13 @@ __global__ void __launch_bounds__(64) smooth_classify(SmoothArgs A) {
     }
     __syncthreads();
     // sign bits: thread = (row of the box, layer in steps), one word per row;
-    // the mixed sub-bricks' bytes are left to smooth_rows
+    // smooth_rows writes the mixed sub-bricks' bytes after this
     for (uint32_t r = t; r < A.rows * A.rows; r += 64) {
         const uint32_t yr = r % A.rows, zr = r / A.rows, y = b.y0 + yr, z = b.z0 + zr;
         if (y >= b.y1 || z >= b.z1) continue;
-        uint32_t cls4 = 0, any = 0;
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t cj = s_cls[((zr >> 2) * sy + (yr >> 2)) * 4 + j];
-            cls4 |= cj << (8 * j);
-            any |= (cj == BRICK_MIXED) << j;
-        }
-        uint32_t* at = g.bits + ((uint64_t)z * g.ny + y) * g.W + b.wx;
-        if (!any) {
-            *at = decided_word(cls4, g.nx, b.wx);
-        } else {
-            for (uint32_t j = 0; j < 4; ++j)
-                if (!((any >> j) & 1u))
-                    reinterpret_cast<uint8_t*>(at)[j] = decided_byte((cls4 >> (8 * j)) & 0xFFu, g.nx, 4 * b.wx + j);
-        }
+        uint32_t cls4 = 0;
+        for (uint32_t j = 0; j < 4; ++j) cls4 |= (uint32_t)s_cls[((zr >> 2) * sy + (yr >> 2)) * 4 + j] << (8 * j);
+        g.bits[((uint64_t)z * g.ny + y) * g.W + b.wx] = decided_word(cls4, g.nx, b.wx);
     }
 }
 
