@@ -587,6 +587,7 @@ iso_status iso_mlp_create(iso_ctx* ctx, uint64_t seed, iso_mlp** out) {
         iso_mlp_destroy(net);
         return cuda_fail(ctx, e, "mlp init");
     }
+    mlp_infer_invalidate(net, h.data());
     *out = net;
     return ISO_OK;
 }
@@ -613,7 +614,7 @@ iso_status iso_mlp_get_params(iso_mlp* net, float* host) {
 iso_status iso_mlp_set_params(iso_mlp* net, const float* host) {
     if (!net || !host) return ISO_ERR_INVALID_ARG;
     cudaError_t e = cudaMemcpy(net->params, host, 4ull * NPARAMS, cudaMemcpyHostToDevice);
-    mlp_infer_invalidate(net);
+    mlp_infer_invalidate(net, e == cudaSuccess ? host : nullptr);
     return e == cudaSuccess ? ISO_OK : cuda_fail(net->ctx, e, "set params");
 }
 
@@ -806,7 +807,7 @@ iso_status iso_mlp_load(iso_mlp* net, const char* path) {
     if (e == cudaSuccess) e = cudaMemcpy(net->m, host.data() + NPARAMS, 8ull * NPARAMS, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(net->ctx, e, "checkpoint load");
     net->step = h.step;
-    mlp_infer_invalidate(net);
+    mlp_infer_invalidate(net, host.data());
     return ISO_OK;
 }
 

@@ -52,7 +52,8 @@ constexpr size_t NPARAMS = OUT_B + 1;
 
 // mlp_infer.cu: the bf16 tensor-core copy of the parameters
 void mlp_infer_release(iso_mlp* net);
-void mlp_infer_invalidate(iso_mlp* net);
+// the parameters changed (params: their host copy, if there is one)
+void mlp_infer_invalidate(iso_mlp* net, const float* params = nullptr);
 // A lattice of nx x ny x nz points (i, j, k) at p = (i, j, k) * step * inv,
 // given to the network as q = p * scale + offset.
 struct MlpGrid {

@@ -44,6 +44,7 @@ struct MlpImages {
     float* bias = nullptr;       // NLAYERS x 256
     float* wout = nullptr;       // 256 + 1
     std::vector<float> host;     // bias, then wout: the kernel takes them by value
+    bool host_valid = false;
     bool valid = false;
 };
 
@@ -525,8 +526,16 @@ void mlp_infer_release(iso_mlp* net) {
     net->infer = nullptr;
 }
 
-void mlp_infer_invalidate(iso_mlp* net) {
-    if (net->infer) ((MlpImages*)net->infer)->valid = false;
+void mlp_infer_invalidate(iso_mlp* net, const float* params) {
+    if (!net->infer && !params) return;
+    MlpImages* m = images_of(net);
+    m->valid = m->host_valid = false;
+    if (!params) return;
+    // what the kernel takes by value need not come back from the device
+    m->host.resize(NLAYERS * HID + HID + 1);
+    for (int l = 0; l < NLAYERS; ++l) std::copy_n(params + bias_offset(l), HID, m->host.begin() + l * HID);
+    std::copy_n(params + OUT_W, HID + 1, m->host.begin() + NLAYERS * HID);
+    m->host_valid = true;
 }
 
 static iso_status ready(iso_mlp* net, MlpImages** out) {
@@ -546,10 +555,13 @@ static iso_status ready(iso_mlp* net, MlpImages** out) {
         ctx->launches++;
         iso_status s = check_launch(ctx, "prepare images");
         if (s != ISO_OK) return s;
-        m->host.resize(NLAYERS * HID + HID + 1);
-        cudaError_t e = cudaMemcpyAsync(m->host.data(), m->bias, 4 * m->host.size(), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp biases");
+        if (!m->host_valid) {  // trained on the device
+            m->host.resize(NLAYERS * HID + HID + 1);
+            cudaError_t e = cudaMemcpyAsync(m->host.data(), m->bias, 4 * m->host.size(), cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp biases");
+            m->host_valid = true;
+        }
         m->valid = true;
     }
     *out = m;
