@@ -759,7 +759,8 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
                 if (le == cudaSuccess)
                     le = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream,
                                     (uint32_t*)ctx->mesh_i.p, (const uint64_t*)totals, cap_t,
-                                    (const uint32_t*)ctx->edges.p, (uint32_t)nedges, H.i, H.cap_v, H.cap_t, cap_v);
+                                    (const uint32_t*)ctx->edges.p, (uint32_t)nedges, H.i, H.cap_v, H.cap_t, cap_v,
+                                    ctx->h_pinned, (const uint32_t*)ctx->d_err);
                 if (le != cudaSuccess) return cuda_fail(ctx, le, "emit launch");
                 ctx->launches++;
             } else {
@@ -771,8 +772,11 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
         ctx->launches++;
         iso_status st = check_launch(ctx, "mc emit");
         if (st != ISO_OK) return st;
-        cudaError_t ce = cudaMemcpyAsync(ctx->h_pinned, totals, 16, cudaMemcpyDeviceToHost, ctx->stream);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
+        cudaError_t ce = cudaSuccess;
+        if (!cells) {  // mc_resolve_ids has stored them otherwise
+            ce = cudaMemcpyAsync(ctx->h_pinned, totals, 16, cudaMemcpyDeviceToHost, ctx->stream);
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
+        }
         if (ce == cudaSuccess && !record) ce = cudaStreamSynchronize(ctx->stream);
         return ce == cudaSuccess ? ISO_OK : cuda_fail(ctx, ce, "sync after emit");
     };
@@ -1128,7 +1132,8 @@ iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, ui
         if (e == cudaSuccess)
             e = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream, out_i,
                            (const uint64_t*)totals, cap_t, (const uint32_t*)ctx->edges.p, t->nedges,
-                           (uint32_t*)nullptr, (uint64_t)0, (uint64_t)0, cap_v);
+                           (uint32_t*)nullptr, (uint64_t)0, (uint64_t)0, cap_v, (uint64_t*)nullptr,
+                           (const uint32_t*)nullptr);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch emit");
         mc_cell_extents<<<(t->ngrids + 7) / 8, 256, 0, ctx->stream>>>(a, t->ngrids, (uint4*)extents);
     }

@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(512) mc_cell_scan(CellArgs A) {
     pdl_trigger();
     const uint32_t i0 = blockIdx.x * SCAN_BLOCK_SEGS + threadIdx.x * 8;
     uint2 a[8];
+    uint32_t mask[8] = {};  // (of a segment without triangles: anything)
     uint64_t sum = 0;  // vertices << 38 | triangles << 13 | active segments
     auto packed = [](uint2 c) { return ((uint64_t)c.x << 38) | ((uint64_t)c.y << 13) | (c.y ? 1u : 0u); };
     if (i0 + 8 <= A.nsegs) {
@@ -201,9 +202,21 @@ __global__ void __launch_bounds__(512) mc_cell_scan(CellArgs A) {
             a[2 * k] = make_uint2(q.x, q.y);
             a[2 * k + 1] = make_uint2(q.z, q.w);
         }
+        const uint4* m = reinterpret_cast<const uint4*>(A.masks + i0);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint4 q = m[k];
+            mask[4 * k] = q.x;
+            mask[4 * k + 1] = q.y;
+            mask[4 * k + 2] = q.z;
+            mask[4 * k + 3] = q.w;
+        }
     } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) a[k] = i0 + k < A.nsegs ? A.segs[i0 + k] : make_uint2(0, 0);
+        for (int k = 0; k < 8; ++k) {
+            a[k] = i0 + k < A.nsegs ? A.segs[i0 + k] : make_uint2(0, 0);
+            if (a[k].y) mask[k] = A.masks[i0 + k];
+        }
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) sum += packed(a[k]);
@@ -232,7 +245,7 @@ __global__ void __launch_bounds__(512) mc_cell_scan(CellArgs A) {
     for (int k = 0; k < 8; ++k) {
         const uint2 pre = make_uint2((uint32_t)(run >> 38), (uint32_t)(run >> 13) & 0x1FFFFFFu);
         if (i0 + k < A.nsegs) A.segs[i0 + k] = pre;
-        if (a[k].y) A.list[base + ((uint32_t)run & 0x1FFFu)] = make_uint4(i0 + k, pre.x, pre.y, A.masks[i0 + k]);
+        if (a[k].y) A.list[base + ((uint32_t)run & 0x1FFFu)] = make_uint4(i0 + k, pre.x, pre.y, mask[k]);
         run += packed(a[k]);
     }
     if (active + threadIdx.x < padded) A.list[base + active + threadIdx.x] = make_uint4(0, 0, 0, 0);

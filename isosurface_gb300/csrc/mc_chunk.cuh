@@ -543,8 +543,17 @@ __global__ void __launch_bounds__(256) mc_block_emit(ChunkEmitArgs A, uint32_t m
 __global__ void __launch_bounds__(256) mc_resolve_ids(uint32_t* __restrict__ idx, const uint64_t* totals,
                                                       uint64_t cap_t, const uint32_t* __restrict__ edge_id,
                                                       uint32_t nedges, uint32_t* host_i, uint64_t host_cap_v,
-                                                      uint64_t host_cap_t, uint64_t cap_v) {
+                                                      uint64_t host_cap_t, uint64_t cap_v, uint64_t* host_totals,
+                                                      const uint32_t* err) {
     pdl_wait();  // the emitted keys and the edge map
+    // what the host looks at after its synchronisation (page-locked memory):
+    // stored from here, as two copies behind the kernel took longer than it
+    // on a small lattice
+    if (host_totals && blockIdx.x == 0 && threadIdx.x == 0) {
+        host_totals[0] = totals[0];
+        host_totals[1] = totals[1];
+        host_totals[2] = *err;
+    }
     const uint64_t n = 3 * min(totals[0], cap_t);
     const bool to_host = mesh_to_host(reinterpret_cast<const float*>(host_i), totals, host_cap_v, host_cap_t, cap_v,
                                       cap_t);
