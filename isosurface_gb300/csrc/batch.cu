@@ -278,10 +278,14 @@ iso_status enqueue(iso_batch* b, bool cells, bool sync_sizes) {
                             b->d_extents, b->d_totals, sync_sizes);
 }
 
-iso_status finish(iso_batch* b, iso_mesh_info* info) {
+// stored: the totals and the error flags are in h_pinned already (the cell passes)
+iso_status finish(iso_batch* b, bool stored, iso_mesh_info* info) {
     iso_ctx* ctx = b->ctx;
-    cudaError_t e = cudaMemcpyAsync(ctx->h_pinned, b->d_totals, 16, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaSuccess;
+    if (!stored) {
+        e = cudaMemcpyAsync(ctx->h_pinned, b->d_totals, 16, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 2, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "batch totals");
     const uint64_t nt = ctx->h_pinned[0], nv = ctx->h_pinned[1];
@@ -432,7 +436,7 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
         // eager: sizes are read back between the count and the emit passes
         s = enqueue(b, cells, true);
         if (s != ISO_OK) return s;
-        if ((s = finish(b, info)) != ISO_OK) return s;
+        if ((s = finish(b, cells, info)) != ISO_OK) return s;
         if (!b->sized || ctx->last.num_vertices > b->cap_v || ctx->last.num_triangles > b->cap_t) {
             b->cap_v = ctx->last.num_vertices + ctx->last.num_vertices / 4 + 1024;
             b->cap_t = ctx->last.num_triangles + ctx->last.num_triangles / 4 + 1024;
@@ -484,7 +488,7 @@ iso_status iso_batch_run(iso_batch* b, uint32_t flags, iso_mesh_info* info) {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "graph launch");
     }
     ctx->launches += 7;
-    s = finish(b, info);
+    s = finish(b, cells, info);
     if (s == ISO_ERR_CAPACITY || ctx->last.num_vertices > b->cap_v || ctx->last.num_triangles > b->cap_t) {
         b->sized = false;  // grow and run eagerly
         return iso_batch_run(b, 0, info);

@@ -323,7 +323,8 @@ unsigned grid_for(const iso_ctx* ctx, uint64_t items, unsigned threads, unsigned
 
 using namespace iso;
 
-// everything after the scan; leaves the counters in h_pinned[0 .. 2]
+// everything after the scan; leaves the counters in h_pinned[0 .. 2] and the
+// error flags in h_pinned[3]
 static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t nblocks, uint32_t cap,
                            const uint32_t* active, const uint32_t* features, const Feature* kept, Ctrl* ctrl,
                            const unsigned long long* sums) {
@@ -355,6 +356,7 @@ static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t n
     }
     if ((s = check_launch(ctx, "emc emit")) != ISO_OK) return s;
     e = cudaMemcpyAsync(ctx->h_pinned + 2, &ctrl->flips, 8, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 3, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "emc emit");
 }
@@ -434,7 +436,7 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
     }
     if (s != ISO_OK) return s;
     const uint64_t nv = ctx->h_pinned[1] & 0xFFFFFFFFu, nt = ctx->h_pinned[1] >> 32, nflips = ctx->h_pinned[2];
-    if ((s = read_device_errors(ctx)) != ISO_OK) return s;
+    if ((uint32_t)ctx->h_pinned[3] && (s = read_device_errors(ctx)) != ISO_OK) return s;
     ctx->last.num_vertices = nv;
     ctx->last.num_triangles = nt;
     ctx->last.num_cells = cells;

@@ -1096,7 +1096,8 @@ CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n) {
 // indices from its own first vertex) and their extents.  sync_sizes: the
 // counts are read back and size the context's mesh buffers before the emit;
 // otherwise it writes into out_v and out_i with the given capacities (no
-// host synchronisation: a graph capture).  ctx->edges holds the edge map.
+// host synchronisation: a graph capture).  ctx->edges holds the edge map; the
+// totals and the error flags also go to ctx->h_pinned[0 .. 2].
 iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, uint64_t cap_t, float* out_v,
                             uint32_t* out_i, uint32_t* extents, uint64_t* totals, bool sync_sizes) {
     CellArgs a = t->a;
@@ -1132,8 +1133,8 @@ iso_status mc_extract_table(iso_ctx* ctx, const CellTable* t, uint64_t cap_v, ui
         if (e == cudaSuccess)
             e = launch_pdl(mc_resolve_ids, dim3(resolve_blocks(cap_t)), dim3(256), 0, ctx->stream, out_i,
                            (const uint64_t*)totals, cap_t, (const uint32_t*)ctx->edges.p, t->nedges,
-                           (uint32_t*)nullptr, (uint64_t)0, (uint64_t)0, cap_v, (uint64_t*)nullptr,
-                           (const uint32_t*)nullptr);
+                           (uint32_t*)nullptr, (uint64_t)0, (uint64_t)0, cap_v, ctx->h_pinned,
+                           (const uint32_t*)ctx->d_err);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch emit");
         mc_cell_extents<<<(t->ngrids + 7) / 8, 256, 0, ctx->stream>>>(a, t->ngrids, (uint4*)extents);
     }
