@@ -296,6 +296,7 @@ struct OctArgs {
     uint32_t* tiles;           // refined nodes of every tile, of every super tile: generation g's from
     uint32_t* supers;          // off / TILE + g and off / (TILE * SUPER) + g
     Ctl* c;
+    Ctl* host;  // page-locked: the size, when it is known
     uint32_t* err;
 };
 
@@ -391,6 +392,7 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
         }
     }
     uint32_t off = 9, cnt = 64;
+    unsigned long long need = 0;
     for (uint32_t g = 2; g < last; ++g) {
         grid_barrier(A.c, g - 1, A.err);
         const uint32_t next = off + cnt;
@@ -455,11 +457,14 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
         off = next;
         cnt = fits ? (uint32_t)children : 0u;
         if (cnt == 0) {
-            if (blockIdx.x == 0 && tid == 0 && !fits) A.c->need = next + children;
+            if (!fits) need = next + children;
             break;
         }
     }
-    if (blockIdx.x == 0 && tid == 0) A.c->nodes = off + cnt;
+    if (blockIdx.x == 0 && tid == 0) {
+        A.c->nodes = A.host->nodes = off + cnt;
+        A.c->need = A.host->need = need;
+    }
 }
 
 // ---------------------------------------------------------------- dual cubes ---
@@ -488,6 +493,8 @@ struct CubeArgs {
     uint64_t* out_k;
     uint32_t cap_v, cap_t;
     uint32_t* err;
+    Ctl* host;           // page-locked: the counters and the error flags at the end
+    uint64_t* host_err;
 };
 
 // What a warp knows of family f (first child 8 f + 1) and its surroundings:
@@ -760,6 +767,10 @@ __global__ void __launch_bounds__(256) cube_offsets(CubeArgs A) {
 }
 
 __global__ void __launch_bounds__(128) cube_emit(CubeArgs A) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // all final by now
+        *A.host = *A.c;
+        *A.host_err = *A.err;
+    }
     const uint32_t n = (uint32_t)A.c->work;
     for (uint32_t p = blockIdx.x * 128 + threadIdx.x; p < n; p += gridDim.x * 128) {
         const uint2 q = A.list[p];
@@ -859,9 +870,8 @@ unsigned blocks_for(const iso_ctx* ctx, uint64_t items, unsigned per_block, unsi
 
 // The counts an extraction discovered: its nodes, dual cubes, triangles and
 // vertices.  An eager run fills one; a run recorded into a CUDA graph replays
-// one (queueing everything, synchronising nowhere) and copies each count it
-// computes to pinned memory, so that the replay can be checked against the
-// trace.
+// one (queueing everything, synchronising nowhere); its kernels store each
+// count in pinned memory, so that the replay can be checked against the trace.
 struct LhmcTrace {
     uint32_t nodes = 0, ncubes = 0, nt = 0, nv = 0;
 };
@@ -939,6 +949,7 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         oa.cap = (uint32_t)node_cap;
         oa.max_depth = max_depth;
         oa.c = (Ctl*)head;
+        oa.host = h;
         oa.err = ctx->d_err;
         oa.tiles = (uint32_t*)(oa.c + 1);
         oa.supers = oa.tiles + node_cap / TILE + MAX_GENS;
@@ -957,8 +968,7 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
             nodes = replay->nodes;
             break;
         }
-        e = cudaMemcpyAsync(h, oa.c, sizeof(Ctl), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "read octree size");
         if (h->need == 0) {
             nodes = h->nodes;
@@ -1008,6 +1018,8 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
     ca.vbase = a3.take<uint32_t>(bound);
     ca.tbase = a3.take<uint32_t>(bound);
     ca.err = ctx->d_err;
+    ca.host = h;
+    ca.host_err = ctx->h_pinned + 3;
     e = cudaMemsetAsync(ca.sums, 0, 8ull * cblocks, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "clear sums");
     family_count<<<fblocks, 256, 0, ctx->stream>>>(ca);
@@ -1032,10 +1044,8 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         cube_emit<<<pblocks, 128, 0, ctx->stream>>>(ca);
         ctx->launches++;
         if ((s = check_launch(ctx, "cube_emit")) != ISO_OK) return s;
-        e = cudaMemcpyAsync(h, oa.c, sizeof(Ctl), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_pinned + 3, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        if (rec) return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, "copy counts");
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (rec) return ISO_OK;
+        e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "read counts");
         if ((uint32_t)ctx->h_pinned[3] && (s = read_device_errors(ctx)) != ISO_OK) return s;
         t = counts_of(ctx);
