@@ -95,11 +95,15 @@ __device__ __forceinline__ BrickLattice lattice_of(const SampleGrid& sg) {
 // chunk: 495 us for 1024 chunks of 16^3 to 64^3 cells; now 39 and 139 for
 // batch_rows, which issues in 73 % of its slots.)
 __global__ void __launch_bounds__(256) batch_classify(const Task* tasks, const SampleGrid* grids, uint32_t ntasks,
-                                                      Mixed* list, uint32_t* count) {
+                                                      uint32_t ngrids, Mixed* list, uint32_t* count, uint32_t* err) {
     __shared__ float s_held[HELD][256];
     const uint32_t lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (t >= ntasks) return;
     const Task k = tasks[t];
+    if (k.grid >= ngrids) {  // warp-uniform
+        if (lane == 0) atomicOr(err, DERR_TABLE);
+        return;
+    }
     const SampleGrid sg = grids[k.grid];
     const BrickLattice g = lattice_of(sg);
     const VmEval ev{sg.pv};
@@ -208,10 +212,10 @@ namespace {
 size_t list_at(size_t n) { return (sizeof(Task) * n + 255) & ~(size_t)255; }
 
 // Device copy of `tasks`, with room for every sub-brick of theirs behind it.
-cudaError_t upload_tasks(const std::vector<Task>& tasks, Task** d_tasks) {
+cudaError_t upload_tasks(iso_ctx* ctx, const std::vector<Task>& tasks, Task** d_tasks) {
     const size_t n = tasks.size();
     cudaError_t e = cudaMalloc((void**)d_tasks, list_at(n) + 32 * sizeof(Mixed) * std::max<size_t>(n, 1));
-    if (e == cudaSuccess && n) e = cudaMemcpy(*d_tasks, tasks.data(), sizeof(Task) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && n) e = upload(ctx, *d_tasks, tasks.data(), sizeof(Task) * n);
     return e;
 }
 
@@ -222,7 +226,7 @@ iso_status build_tasks(iso_batch* b) {
     if (b->d_tasks) cudaFree(b->d_tasks);
     b->d_tasks = nullptr;
     b->ntasks = (uint32_t)tasks.size();
-    cudaError_t e = upload_tasks(tasks, &b->d_tasks);
+    cudaError_t e = upload_tasks(b->ctx, tasks, &b->d_tasks);
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;
@@ -241,13 +245,14 @@ unsigned rows_blocks(int sms) {
 }
 
 // the culled sampler over `ntasks` tasks
-cudaError_t launch_sampler(iso_ctx* ctx, const Task* d_tasks, uint32_t ntasks, const SampleGrid* d_sgrids,
-                           uint32_t* count) {
-    cudaError_t e = cudaMemsetAsync(count, 0, 4, ctx->stream);
+cudaError_t launch_sampler(const iso_batch* b, const Task* d_tasks, uint32_t ntasks) {
+    const cudaStream_t stream = b->ctx->stream;
+    cudaError_t e = cudaMemsetAsync(b->d_next, 0, 4, stream);
     if (e != cudaSuccess) return e;
     Mixed* list = (Mixed*)((char*)d_tasks + list_at(ntasks));
-    batch_classify<<<(ntasks + 7) / 8, 256, 0, ctx->stream>>>(d_tasks, d_sgrids, ntasks, list, count);
-    batch_rows<<<rows_blocks(ctx->sms), 256, 0, ctx->stream>>>(d_sgrids, list, count);
+    batch_classify<<<(ntasks + 7) / 8, 256, 0, stream>>>(d_tasks, b->d_sgrids, ntasks, (uint32_t)b->chunks.size(), list,
+                                                         b->d_next, b->ctx->d_err);
+    batch_rows<<<rows_blocks(b->ctx->sms), 256, 0, stream>>>(b->d_sgrids, list, b->d_next);
     return cudaGetLastError();
 }
 
@@ -266,7 +271,7 @@ iso_status enqueue(iso_batch* b, bool cells, bool sync_sizes) {
     iso_ctx* ctx = b->ctx;
     {
         StageTimer timer(ctx, ISO_STAGE_SAMPLE);
-        cudaError_t e = launch_sampler(ctx, b->d_tasks, b->ntasks, b->d_sgrids, b->d_next);
+        cudaError_t e = launch_sampler(b, b->d_tasks, b->ntasks);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch sampler");
     }
     ctx->launches += 2;
@@ -387,10 +392,9 @@ iso_status iso_batch_create(iso_ctx* ctx, const iso_program* const* programs, ui
         mc_fill_grid(grids.data() + mc_grid_bytes() * i, L, b->grid_chunk0[i], &nch, &cw);
         for (uint32_t r = b->grid_chunk0[i] / 256; r < (b->grid_chunk0[i] + nch + 255) / 256; ++r) range_grid[r] = i;
     }
-    e = cudaMemcpy(b->d_sgrids, b->sgrids.data(), sizeof(SampleGrid) * nchunks, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_grids, grids.data(), grids.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && nranges)
-        e = cudaMemcpy(b->d_range_grid, range_grid.data(), 4ull * nranges, cudaMemcpyHostToDevice);
+    e = upload(ctx, b->d_sgrids, b->sgrids.data(), sizeof(SampleGrid) * nchunks);
+    if (e == cudaSuccess) e = upload(ctx, b->d_grids, grids.data(), grids.size());
+    if (e == cudaSuccess && nranges) e = upload(ctx, b->d_range_grid, range_grid.data(), 4ull * nranges);
     if (e != cudaSuccess) {
         iso_batch_destroy(b);
         return cuda_fail(ctx, e, "batch tables");
@@ -568,7 +572,7 @@ iso_status iso_batch_run_per_chunk_async(iso_batch* b, iso_mesh_info* info) {
             mc_fill_grid(grids.data() + mc_grid_bytes() * i, L, 0, &b->solo_chunks[i], &b->solo_cw[i]);
         }
         cudaError_t e = cudaMalloc(&b->d_solo_grids, grids.size());
-        if (e == cudaSuccess) e = cudaMemcpy(b->d_solo_grids, grids.data(), grids.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(ctx, b->d_solo_grids, grids.data(), grids.size());
         if (e != cudaSuccess) return cuda_fail(ctx, e, "per-chunk grids");
     }
     // each chunk's output place and size, from the last run of the batch
@@ -660,7 +664,7 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
                 chunk_tasks(i, cl.first, d, [&](const Task& t) { tasks.push_back(t); });
             }
             Task* d_t = nullptr;
-            if (upload_tasks(tasks, &d_t) != cudaSuccess) {
+            if (upload_tasks(ctx, tasks, &d_t) != cudaSuccess) {
                 if (d_t) cudaFree(d_t);
                 cudaGetLastError();
                 return fail(ctx, ISO_ERR_OUT_OF_MEMORY, "autotune tasks");
@@ -668,7 +672,7 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
             float ms = 1e30f;
             for (int rep = 0; rep < 4; ++rep) {
                 cudaEventRecord(e0, ctx->stream);
-                launch_sampler(ctx, d_t, (uint32_t)tasks.size(), b->d_sgrids, b->d_next);
+                launch_sampler(b, d_t, (uint32_t)tasks.size());
                 cudaEventRecord(e1, ctx->stream);
                 cudaEventSynchronize(e1);
                 float t_ms = 0.0f;

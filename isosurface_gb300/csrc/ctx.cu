@@ -88,14 +88,24 @@ iso_status check_launch(iso_ctx* ctx, const char* what) {
     return e == cudaSuccess ? ISO_OK : cuda_fail(ctx, e, what);
 }
 
+cudaError_t upload(iso_ctx* ctx, void* to, const void* from, size_t bytes) {
+    return cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, ctx->stream);
+}
+
+cudaError_t download(iso_ctx* ctx, void* to, const void* from, size_t bytes) {
+    const cudaError_t e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
+}
+
 iso_status read_device_errors(iso_ctx* ctx) {
     uint32_t h = 0;
-    cudaError_t e = cudaMemcpy(&h, ctx->d_err, 4, cudaMemcpyDeviceToHost);
+    cudaError_t e = download(ctx, &h, ctx->d_err, 4);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "read error flags");
     if (h == 0) return ISO_OK;
-    cudaMemset(ctx->d_err, 0, 4);
+    cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream);
     if (h & DERR_SCAN_TIMEOUT) return fail(ctx, ISO_ERR_TIMEOUT, "scan look-back wait gave up");
     if (h & DERR_QUEUE_TIMEOUT) return fail(ctx, ISO_ERR_TIMEOUT, "work-queue wait gave up");
+    if (h & DERR_TABLE) return fail(ctx, ISO_ERR_CUDA, "a device table's entry names nothing");
     if (h & DERR_SVD_ITER) return fail(ctx, ISO_ERR_TIMEOUT, "QR iteration bound reached");
     return fail(ctx, ISO_ERR_CAPACITY, "device output capacity exceeded");
 }
@@ -481,7 +491,7 @@ iso_status iso_ctx_create(int device, iso_ctx** out) {
     if (s == ISO_OK) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (s == ISO_OK && e == cudaSuccess) e = cudaMallocHost(&ctx->h_pinned, 4096);
     if (s == ISO_OK && e == cudaSuccess) e = cudaMalloc(&ctx->d_err, 256);
-    if (s == ISO_OK && e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, 256);
+    if (s == ISO_OK && e == cudaSuccess) e = cudaMemsetAsync(ctx->d_err, 0, 256, ctx->own_stream);
     if (s != ISO_OK || e != cudaSuccess) {
         iso_status r = s != ISO_OK ? s : cuda_fail(ctx, e, "context setup");
         iso_ctx_destroy(ctx);
@@ -658,8 +668,7 @@ iso_status iso_program_create(iso_ctx* ctx, const uint8_t* bytes, size_t len, is
         p->d_jump = (int32_t*)(block + o_jump);
         if (set_bytes) p->d_set = (float*)(block + o_set);
         if (!p->prims.empty()) p->d_prims = (float4*)(block + o_prims);
-        // from pageable memory: returns once the bytes are staged
-        e = cudaMemcpyAsync(block, staged.data(), total, cudaMemcpyHostToDevice, ctx->stream);
+        e = upload(ctx, block, staged.data(), total);
     }
     if (e != cudaSuccess) {
         iso_status r = cuda_fail(ctx, e, "program upload");

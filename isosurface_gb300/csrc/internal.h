@@ -28,6 +28,7 @@ enum : uint32_t {
     DERR_CAPACITY = 2u,          // a kernel found its output buffer too small
     DERR_SVD_ITER = 4u,          // QR sweeps hit their bound
     DERR_QUEUE_TIMEOUT = 8u,     // work-queue wait gave up
+    DERR_TABLE = 16u,            // an entry of a device table names nothing
 };
 
 // Program kinds with a dedicated sampler.
@@ -204,6 +205,13 @@ iso_status ensure(iso_ctx* ctx, DevBuf& b, size_t bytes);
 iso_status check_launch(iso_ctx* ctx, const char* what);
 iso_status read_device_errors(iso_ctx* ctx);
 iso_status set_device(iso_ctx* ctx);
+// Copies between pageable host memory and the device on the context's
+// stream, which is non-blocking: a plain cudaMemcpy (or cudaMemset) runs on
+// the legacy default stream, may return before its bytes are in device
+// memory, and nothing orders a kernel on the context's stream after it.
+// upload returns once the bytes are staged, download once they are there.
+cudaError_t upload(iso_ctx* ctx, void* to, const void* from, size_t bytes);
+cudaError_t download(iso_ctx* ctx, void* to, const void* from, size_t bytes);
 // Work queued on *side after fork_side starts after the work queued on the
 // context's stream so far; join_side makes the context's stream wait for
 // the side stream's work so far.

@@ -1073,9 +1073,9 @@ CellTable* mc_table_create(iso_ctx* ctx, const Lattice* L, uint32_t n) {
                  l_at = take(16 * (nsegs + (uint64_t)a.group * a.nblocks)), c_at = take(64);
     cudaError_t e = cudaMalloc(&t->arena, off);
     char* base = (char*)t->arena;
-    if (e == cudaSuccess) e = cudaMemcpy(base + g_at, grids.data(), sizeof(Grid) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + t_at, tasks.data(), 16 * tasks.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + sg_at, seg_grid.data(), 4 * nsegs, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(ctx, base + g_at, grids.data(), sizeof(Grid) * n);
+    if (e == cudaSuccess) e = upload(ctx, base + t_at, tasks.data(), 16 * tasks.size());
+    if (e == cudaSuccess) e = upload(ctx, base + sg_at, seg_grid.data(), 4 * nsegs);
     if (e != cudaSuccess) {
         cudaGetLastError();
         mc_table_destroy(t);

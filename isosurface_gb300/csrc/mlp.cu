@@ -581,8 +581,8 @@ iso_status iso_mlp_create(iso_ctx* ctx, uint64_t seed, iso_mlp** out) {
         for (size_t k = 0; k < (size_t)fin * fout; ++k)
             h[off + k] = a * (2.0f * unit_float(splitmix(seed * 1000003ull + off + k)) - 1.0f);
     }
-    e = cudaMemcpy(net->params, h.data(), 4ull * NPARAMS, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(net->m, 0, 8ull * NPARAMS);
+    e = upload(ctx, net->params, h.data(), 4ull * NPARAMS);
+    if (e == cudaSuccess) e = cudaMemsetAsync(net->m, 0, 8ull * NPARAMS, ctx->stream);
     if (e != cudaSuccess) {
         iso_mlp_destroy(net);
         return cuda_fail(ctx, e, "mlp init");
@@ -607,13 +607,14 @@ uint64_t iso_mlp_num_params(void) { return NPARAMS; }
 
 iso_status iso_mlp_get_params(iso_mlp* net, float* host) {
     if (!net || !host) return ISO_ERR_INVALID_ARG;
-    cudaError_t e = cudaMemcpy(host, net->params, 4ull * NPARAMS, cudaMemcpyDeviceToHost);
+    cudaError_t e = download(net->ctx, host, net->params, 4ull * NPARAMS);
     return e == cudaSuccess ? ISO_OK : cuda_fail(net->ctx, e, "get params");
 }
 
 iso_status iso_mlp_set_params(iso_mlp* net, const float* host) {
     if (!net || !host) return ISO_ERR_INVALID_ARG;
-    cudaError_t e = cudaMemcpy(net->params, host, 4ull * NPARAMS, cudaMemcpyHostToDevice);
+    cudaError_t e = upload(net->ctx, net->params, host, 4ull * NPARAMS);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(net->ctx->stream);  // the caller's memory may be page-locked
     mlp_infer_invalidate(net, e == cudaSuccess ? host : nullptr);
     return e == cudaSuccess ? ISO_OK : cuda_fail(net->ctx, e, "set params");
 }
@@ -773,8 +774,8 @@ iso_status iso_mlp_save(iso_mlp* net, const char* path) {
     iso_status s = set_device(net->ctx);
     if (s != ISO_OK) return s;
     std::vector<float> host(3 * NPARAMS);
-    cudaError_t e = cudaMemcpy(host.data(), net->params, 4ull * NPARAMS, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(host.data() + NPARAMS, net->m, 8ull * NPARAMS, cudaMemcpyDeviceToHost);
+    cudaError_t e = download(net->ctx, host.data(), net->params, 4ull * NPARAMS);
+    if (e == cudaSuccess) e = download(net->ctx, host.data() + NPARAMS, net->m, 8ull * NPARAMS);
     if (e != cudaSuccess) return cuda_fail(net->ctx, e, "checkpoint read");
     CkptHeader h{};
     std::memcpy(h.magic, CKPT_MAGIC, 8);
@@ -803,8 +804,8 @@ iso_status iso_mlp_load(iso_mlp* net, const char* path) {
     std::fclose(f);
     if (!ok) return fail(net->ctx, ISO_ERR_INVALID_ARG, std::string("cannot read ") + path);
     // parameters | gradients | first moments | second moments, one allocation
-    cudaError_t e = cudaMemcpy(net->params, host.data(), 4ull * NPARAMS, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(net->m, host.data() + NPARAMS, 8ull * NPARAMS, cudaMemcpyHostToDevice);
+    cudaError_t e = upload(net->ctx, net->params, host.data(), 4ull * NPARAMS);
+    if (e == cudaSuccess) e = upload(net->ctx, net->m, host.data() + NPARAMS, 8ull * NPARAMS);
     if (e != cudaSuccess) return cuda_fail(net->ctx, e, "checkpoint load");
     net->step = h.step;
     mlp_infer_invalidate(net, host.data());
