@@ -256,6 +256,33 @@ cudaError_t launch_sampler(const iso_batch* b, const Task* d_tasks, uint32_t nta
     return cudaGetLastError();
 }
 
+// the sampler's best time of three over `tasks`, after a first run
+cudaError_t time_sampler(const iso_batch* b, const std::vector<Task>& tasks, cudaEvent_t begin, cudaEvent_t end,
+                         float* best) {
+    Task* d_tasks = nullptr;
+    cudaError_t e = upload_tasks(b->ctx, tasks, &d_tasks);
+    *best = 1e30f;
+    for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {
+        float ms = 0.0f;
+        e = cudaEventRecord(begin, b->ctx->stream);
+        if (e == cudaSuccess) e = launch_sampler(b, d_tasks, (uint32_t)tasks.size());
+        if (e == cudaSuccess) e = cudaEventRecord(end, b->ctx->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(end);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, begin, end);
+        if (rep > 0) *best = std::min(*best, ms);
+    }
+    if (d_tasks) cudaFree(d_tasks);
+    return e;
+}
+
+struct EventPair {
+    cudaEvent_t begin = nullptr, end = nullptr;
+    ~EventPair() {
+        if (begin) cudaEventDestroy(begin);
+        if (end) cudaEventDestroy(end);
+    }
+};
+
 // whether the cell passes can run: the table exists and the edge map is there
 bool edge_map_ready(iso_batch* b) {
     if (!b->table) return false;
@@ -647,10 +674,10 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
         }
     }
     const uint32_t candidates[] = {4, 8, 16, 0};
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    std::vector<uint32_t> saved = b->slab;
+    EventPair events;
+    cudaError_t e = cudaEventCreate(&events.begin);
+    if (e == cudaSuccess) e = cudaEventCreate(&events.end);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "autotune events");
     bool wrote = false;
     for (auto& cl : classes) {
         if (best.count(cl.first)) continue;
@@ -663,23 +690,12 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
                 if (b->chunks[i].size != cl.first) continue;
                 chunk_tasks(i, cl.first, d, [&](const Task& t) { tasks.push_back(t); });
             }
-            Task* d_t = nullptr;
-            if (upload_tasks(ctx, tasks, &d_t) != cudaSuccess) {
-                if (d_t) cudaFree(d_t);
+            float ms;
+            e = time_sampler(b, tasks, events.begin, events.end, &ms);
+            if (e != cudaSuccess) {
                 cudaGetLastError();
-                return fail(ctx, ISO_ERR_OUT_OF_MEMORY, "autotune tasks");
+                return cuda_fail(ctx, e, "autotune");
             }
-            float ms = 1e30f;
-            for (int rep = 0; rep < 4; ++rep) {
-                cudaEventRecord(e0, ctx->stream);
-                launch_sampler(b, d_t, (uint32_t)tasks.size());
-                cudaEventRecord(e1, ctx->stream);
-                cudaEventSynchronize(e1);
-                float t_ms = 0.0f;
-                cudaEventElapsedTime(&t_ms, e0, e1);
-                if (rep > 0) ms = std::min(ms, t_ms);
-            }
-            cudaFree(d_t);
             if (ms < best_ms) {
                 best_ms = ms;
                 best_depth = d;
@@ -688,10 +704,7 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
         best[cl.first] = best_depth;
         wrote = true;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "autotune");
+    if (wrote && (s = read_device_errors(ctx)) != ISO_OK) return s;
     if (cache_path && wrote) {
         if (FILE* f = std::fopen(cache_path, "a")) {
             for (auto& kv : best) std::fprintf(f, "%s|%u|%u\n", gpu.c_str(), kv.first, kv.second);
@@ -707,7 +720,6 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
             ++k;
         }
     }
-    (void)saved;
     return build_tasks(b);
 }
 

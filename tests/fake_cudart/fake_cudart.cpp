@@ -18,7 +18,7 @@ namespace {
 std::string g_log;
 std::map<const void*, std::string> g_kernels;
 void (*g_on_event)(const char*) = nullptr;
-char g_fail[128];         // kernels whose name holds this fail to launch
+char g_fail[128];         // kernels whose name holds this fail to launch ("cudaMalloc": that call)
 int g_device = 0;
 cudaError_t g_last = cudaSuccess;
 uintptr_t g_next = 1;
@@ -99,6 +99,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* ke
 }
 
 cudaError_t cudaMalloc(void** p, size_t bytes) {
+    if (!strcmp(g_fail, "cudaMalloc")) {
+        *p = nullptr;
+        return g_last = cudaErrorMemoryAllocation;
+    }
     *p = calloc(bytes ? bytes : 1, 1);
     note("malloc %p %zu", *p, bytes);
     return cudaSuccess;
