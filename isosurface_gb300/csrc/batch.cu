@@ -664,11 +664,11 @@ iso_status iso_batch_autotune(iso_batch* b, const char* cache_path, uint32_t* ch
         if (FILE* f = std::fopen(cache_path, "r")) {
             char line[512];
             while (std::fgets(line, sizeof(line), f)) {
-                std::string l(line);
-                size_t a = l.find('|'), c = l.rfind('|');
-                if (a == std::string::npos || c == a) continue;
-                if (l.substr(0, a) != gpu) continue;
-                best[(uint32_t)std::stoul(l.substr(a + 1, c - a - 1))] = (uint32_t)std::stoul(l.substr(c + 1));
+                // (a line without both numbers is passed over)
+                unsigned size = 0, depth = 0;
+                if (std::strncmp(line, gpu.c_str(), gpu.size()) == 0 &&
+                    std::sscanf(line + gpu.size(), "|%u|%u", &size, &depth) == 2)
+                    best[size] = depth;
             }
             std::fclose(f);
         }

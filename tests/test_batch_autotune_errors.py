@@ -28,3 +28,15 @@ b.run(graph=False)
 @pytest.mark.parametrize("what,status", [(b"batch_classify", 3), (b"batch_rows", 3), (b"cudaMalloc", 7)])
 def test_autotune_reports_what_failed(what, status):
     assert fake_cudart.run(SCRIPT % what).split("\n")[:3] == ["status %d" % status, "events 0", "blocks 0"]
+
+
+def test_autotune_passes_over_lines_without_numbers(tmp_path):
+    """A cache file cut short, or with other lines in it, ends no program."""
+    cache = tmp_path / "depths.txt"
+    cache.write_text("no device brick list|x|4\nno device brick list||\n\n|\nno device brick list|17|8\n"
+                     "no device brick list|33|")
+    out = fake_cudart.run("""
+from isosurface_gb300.api import Batch
+print(Batch(Context(0), [(17, scenes.sphere()), (33, scenes.sphere())]).autotune(%r))
+""" % str(cache))
+    assert out.strip() == "{17: 8, 33: 4}"  # 33 is timed: the first candidate of equals
