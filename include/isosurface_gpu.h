@@ -92,9 +92,11 @@ ISO_API iso_status iso_debug_fail_allocation(iso_ctx* ctx, int64_t after);
  * decoupled look-back scan of iso_mc_extract_field_noalloc runs with its
  * first block never publishing its status and the other blocks giving up
  * after 256 polls of a predecessor, so the call returns ISO_ERR_TIMEOUT
- * instead of waiting; the next call after disabling it extracts normally.
- * Process-wide (that entry point takes no context).  Nothing faults or
- * hangs: every wait is bounded either way. */
+ * instead of waiting; likewise one block of iso_lhmc_extract's octree build
+ * never comes to its barriers, where the others give up after 256 polls.
+ * The next call after disabling it extracts normally.  Process-wide (the
+ * first entry point takes no context).  Nothing faults or hangs: every wait is
+ * bounded either way. */
 ISO_API iso_status iso_debug_scan_timeout(int enable);
 
 /* Per-stage device timing: when enabled, every kernel the context launches is
@@ -367,7 +369,11 @@ ISO_API iso_status iso_dc_extract_slab(iso_ctx* ctx, const iso_program* prog, ui
  * the node's half-diagonal, then marching cubes on the dual cubes of its
  * leaves (traversal/implicit_octree.rs) with MortonKey dedup.  max_depth <= 10.
  * The reference emits the mesh in HashMap order, so only the triangle set is
- * defined; keys (ISO_FLAG_KEYS) are the MortonKey pair of each vertex. */
+ * defined; keys (ISO_FLAG_KEYS) are the MortonKey pair of each vertex.
+ * Programs of up to 64 ops and spheres build the octree in one launch whose
+ * blocks wait for one another between generations: ISO_ERR_TIMEOUT if that
+ * takes some seconds (no such program does on a device that runs it).  Longer
+ * programs take a launch per generation and have no such limit. */
 ISO_API iso_status iso_lhmc_extract(iso_ctx* ctx, const iso_program* prog, uint32_t max_depth, uint32_t flags,
                                     iso_mesh_info* info);
 

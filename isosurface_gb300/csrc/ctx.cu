@@ -612,6 +612,7 @@ iso_status parse_program(const uint8_t* bytes, size_t len, iso_program* p, std::
     if (!validate(p, err)) return ISO_ERR_BAD_PROGRAM;
     classify(p);
     cull_bounds(p);
+    for (uint32_t w : p->ops) p->cost += 1 + ((w & 0xFFu) == OP_SPHERE_SET ? (uint64_t)p->consts[w >> 8] : 0);
     for (float c : p->consts) p->tiny = p->tiny || (c != 0.0f && std::fabs(c) < 1e-18f);
     uint64_t hash = 0xCBF29CE484222325ull;  // FNV-1a 64
     for (size_t i = 0; i < len; ++i) hash = (hash ^ bytes[i]) * 0x100000001B3ull;

@@ -188,6 +188,7 @@ struct iso_program {
     // out next to zero by a few units of f32's smallest step (differences of
     // ordinary numbers are multiples of their own last places)
     bool tiny = false;
+    uint64_t cost = 0;  // ops and spheres that one evaluation goes through
     size_t block_bytes = 0;          // capacity of d_block
     uint64_t content_hash = 0;       // FNV-1a of the program bytes
     uint64_t uid = 0;  // unique per program created in this process
@@ -204,6 +205,7 @@ iso_status cuda_fail(iso_ctx* ctx, cudaError_t e, const char* what);
 iso_status ensure(iso_ctx* ctx, DevBuf& b, size_t bytes);
 iso_status check_launch(iso_ctx* ctx, const char* what);
 iso_status read_device_errors(iso_ctx* ctx);
+bool debug_waits_run_out();  // iso_debug_scan_timeout
 iso_status set_device(iso_ctx* ctx);
 // Copies between pageable host memory and the device on the context's
 // stream, which is non-blocking: a plain cudaMemcpy (or cudaMemset) runs on

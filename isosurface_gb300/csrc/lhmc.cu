@@ -4,8 +4,8 @@
 // (src/linear_hashed_octree.rs:30-51), with Morton keys (src/morton.rs).
 //
 // GPU form:
-// 1. Octree build in one cooperative launch (oct_build), generation by
-//    generation: evaluate the source
+// 1. Octree build in one cooperative launch (oct_build; a launch per
+//    generation for long programs), generation by generation: evaluate the source
 //    at the centres of the children of every refined node, apply
 //    should_refine (level < 2 || (level < max_depth && |d| < size * sqrt 3)),
 //    and append them in order.  Where a refined node's children go follows
@@ -273,16 +273,32 @@ constexpr uint32_t BLOCK_CUBES = 256;    // cubes with one sum of vertices and t
 
 // what the passes find out, read back by the host in one copy
 struct Ctl {
-    uint32_t nodes;
+    uint32_t nodes;                         // 0: the build was abandoned
     uint32_t arrived;                       // blocks at the barriers of oct_build
     uint32_t pad[30];
-    uint32_t released, pad2;                // turns of the barrier that are over (a cache line of its own)
-    unsigned long long need;                // nodes the arena had no room for (0: all fit)
+    uint32_t released, pad2;                // turns of the barrier that are over, or ABANDONED (a cache line of its own)
+    unsigned long long need;                // nodes the arena had no room for (0: all fit; NO_OCTREE: abandoned)
     unsigned long long work;                // crossing edges of the listed cubes << 32 | listed cubes
     unsigned long long stale;
     uint2 cubes;                            // dual cubes, 0
     uint2 mesh;                             // vertices, triangles
 };
+
+constexpr uint32_t ABANDONED = 0xFFFFFFFFu;
+constexpr unsigned long long NO_OCTREE = ~0ull;
+
+// One cooperative launch with barriers for programs up to this many ops and
+// spheres, a launch per generation beyond.  What a block waits for at a
+// barrier is the other blocks' evaluations, which have no limit of their own
+// (sets of up to 2^24 spheres), while the wait needs one: it ends after some
+// seconds, and at the line a generation of 10^9 nodes takes about a tenth of
+// one.  A launch is also the faster way for long programs, whose slowest block
+// the barriers wait for: a hard set at depth 8, a launch per generation
+// against one for all, recorded: 16 spheres 123 and 128 us, 64 237 and 250,
+// 256 1115 and 1186, 1023 5673 and 6390; called without a recording the
+// launches cost 9 us more (csg at depth 8: 206 and 197 us), which they are
+// worth from about 64 spheres on.
+constexpr uint64_t BARRIER_COST = 64;
 
 struct OctArgs {
     ProgView pv;
@@ -295,6 +311,9 @@ struct OctArgs {
     uint32_t max_depth;
     uint32_t* tiles;           // refined nodes of every tile, of every super tile: generation g's from
     uint32_t* supers;          // off / TILE + g and off / (TILE * SUPER) + g
+    uint2* gens;               // a launch per generation (else null): first node and nodes of generation g
+    uint32_t polls;            // limit of a wait
+    bool withhold;             // test hook: a block that never comes to the barriers
     Ctl* c;
     Ctl* host;  // page-locked: the size, when it is known
     uint32_t* err;
@@ -337,33 +356,43 @@ __device__ __forceinline__ uint32_t find_family(const unsigned long long* famili
 
 // All blocks of the (cooperative) launch have come here `turn` times; the
 // last one to come releases the others, which wait on a word of its own.
-// Bounded, and reported when the bound is reached.
-constexpr uint32_t BARRIER_SPINS = 1u << 22;
-__device__ __forceinline__ void grid_barrier(Ctl* c, uint32_t turn, uint32_t* err) {
+// Bounded: a block whose polls run out abandons the turn for all blocks, unless
+// it was released meanwhile (the word changes once for a turn).  False, in
+// every thread of every block, once a turn was abandoned.
+constexpr uint32_t BARRIER_POLLS = 1u << 22;
+__device__ __forceinline__ bool grid_barrier(const OctArgs& A, uint32_t turn) {
+    __shared__ uint32_t s_released;
     __syncthreads();
     if (threadIdx.x == 0) {
+        Ctl* c = A.c;
+        const volatile uint32_t* released = &c->released;
+        const bool comes = !(A.withhold && blockIdx.x + 1 == gridDim.x);
         __threadfence();
-        if (atomicAdd(&c->arrived, 1u) + 1 == turn * gridDim.x) {
+        if (comes && atomicAdd(&c->arrived, 1u) + 1 == turn * gridDim.x) {
             __threadfence();
-            *(volatile uint32_t*)&c->released = turn;
+            atomicCAS(&c->released, turn - 1, turn);
         } else {
-            uint32_t spins = 0;
-            while (*(volatile uint32_t*)&c->released < turn && ++spins < BARRIER_SPINS) __nanosleep(20);
-            if (spins == BARRIER_SPINS) atomicOr(err, DERR_QUEUE_TIMEOUT);
+            uint32_t polls = 0;
+            while (*released < turn && ++polls < A.polls) __nanosleep(20);
+            if (polls == A.polls && atomicCAS(&c->released, turn - 1, ABANDONED) == turn - 1)
+                atomicOr(A.err, DERR_QUEUE_TIMEOUT);
         }
         __threadfence();
+        s_released = *released;
     }
     __syncthreads();
+    return s_released != ABANDONED;
 }
 
-// The whole octree in one cooperative launch, a grid barrier between
-// generations.  Bound by one evaluation's chain per generation: launched
+// Generations first + 1 .. last: the whole octree in one cooperative launch
+// (first = 1), a grid barrier between generations, or a launch for each
+// generation (A.gens).  Bound by one evaluation's chain per generation: launched
 // generation by generation the interpreter's code and the program came from
 // L2 again each time (10-18 us each; 95 us for csg at depth 8).
 // Generations 0 to 2 (nodes 0, 1-8 and 9-72) every octree has; after that a
 // block takes the refined nodes of a tile and evaluates their children.
 // What other blocks wrote is read past L1.
-__global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t last) {
+__global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t first, uint32_t last) {
     __shared__ unsigned long long s_key[OCT_THREADS];
     __shared__ uint32_t s_sum[OCT_THREADS / 32], s_n[OCT_THREADS / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31;
@@ -376,7 +405,7 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
         for (int k = 0; k < OCT_THREADS / 32; ++k) all += s_sum[k];
         return all;
     };
-    if (blockIdx.x == 0 && tid < 96) {
+    if (first == 1 && blockIdx.x == 0 && tid < 96) {
         // nodes 1-72 to threads 0-71, so that families are eights of lanes
         const uint32_t at = tid == 72 ? 0 : tid + 1;
         bool r = false;
@@ -393,8 +422,20 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
     }
     uint32_t off = 9, cnt = 64;
     unsigned long long need = 0;
-    for (uint32_t g = 2; g < last; ++g) {
-        grid_barrier(A.c, g - 1, A.err);
+    if (first > 2) {
+        const uint2 gen = A.gens[first];
+        off = gen.x;
+        cnt = gen.y;
+        if (cnt == 0) return;  // the build is over
+    }
+    for (uint32_t g = max(first, 2u); g < last; ++g) {
+        if (!A.gens && !grid_barrier(A, g - 1)) {
+            if (blockIdx.x == 0 && tid == 0) {
+                A.c->nodes = A.host->nodes = 0;
+                A.c->need = A.host->need = NO_OCTREE;
+            }
+            return;
+        }
         const uint32_t next = off + cnt;
         const uint32_t ntiles = (cnt + TILE - 1) / TILE, nsupers = (ntiles + SUPER - 1) / SUPER;
         const uint32_t* tiles = A.tiles + off / TILE + g;
@@ -464,6 +505,7 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
     if (blockIdx.x == 0 && tid == 0) {
         A.c->nodes = A.host->nodes = off + cnt;
         A.c->need = A.host->need = need;
+        if (A.gens) A.gens[last] = make_uint2(off, cnt);
     }
 }
 
@@ -565,10 +607,11 @@ __device__ __forceinline__ Around look_around(const CubeArgs& A, uint32_t f) {
 __global__ void __launch_bounds__(256) family_count(CubeArgs A) {
     __shared__ uint32_t s_n[8];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t families = A.c->nodes ? A.nfamilies : 0;  // none of an abandoned octree (a replay comes here)
     uint32_t n = 0;
     for (uint32_t k = warp; k < BLOCK_FAMILIES; k += 8) {
         const uint32_t f = blockIdx.x * BLOCK_FAMILIES + k;
-        if (f >= A.nfamilies) break;
+        if (f >= families) break;
         const Around q = look_around(A, f);
         const uint32_t own = __popc(q.lo) + __popc(q.hi);
         if (lane == 0) A.fcount[f] = (uint8_t)own;
@@ -924,8 +967,8 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
             if (max_nodes > (1ull << 28)) break;
         }
     }
-    // counters, tile counts and the table of families | keys | values | refine flags
-    auto tile_words = [](size_t cap) { return cap / TILE + cap / (TILE * SUPER) + 3 * MAX_GENS; };
+    // counters, generations, tile counts and the table of families | keys | values | refine flags
+    auto tile_words = [](size_t cap) { return 2 * MAX_GENS + cap / TILE + cap / (TILE * SUPER) + 3 * MAX_GENS; };
     auto table_at = [&](size_t cap) { return (sizeof(Ctl) + 4 * tile_words(cap) + 255) & ~(size_t)255; };
     auto head_bytes = [&](size_t cap) { return table_at(cap) + 8 * (size_t)pow2_at_least(cap / 4); };
     auto node_bytes = [&](size_t cap) { return head_bytes(cap) + 12 * cap + cap / 8 + 4096; };
@@ -951,18 +994,29 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         oa.c = (Ctl*)head;
         oa.host = h;
         oa.err = ctx->d_err;
-        oa.tiles = (uint32_t*)(oa.c + 1);
+        uint2* gens = (uint2*)(oa.c + 1);
+        oa.tiles = (uint32_t*)(gens + MAX_GENS);
         oa.supers = oa.tiles + node_cap / TILE + MAX_GENS;
         e = cudaMemsetAsync(head, 0, head_bytes(node_cap), ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "octree counters");
         // blocks beyond the widest generation's tiles would only come to the barriers
         const uint64_t most = std::min<uint64_t>(1ull << std::min(3 * (last - 1), 32u), node_cap);
         const unsigned blocks = (unsigned)std::min<uint64_t>(oct_blocks(ctx), (most + TILE - 1) / TILE);
-        uint32_t last_arg = last;
-        void* args[] = {&oa, &last_arg};
-        e = cudaLaunchCooperativeKernel(oct_build, dim3(blocks), dim3(OCT_THREADS), args, 0, ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "octree launch");
-        ctx->launches++;
+        if (prog->cost <= BARRIER_COST) {
+            oa.withhold = debug_waits_run_out();
+            oa.polls = oa.withhold ? 256 : BARRIER_POLLS;
+            uint32_t first_arg = 1, last_arg = last;
+            void* args[] = {&oa, &first_arg, &last_arg};
+            e = cudaLaunchCooperativeKernel(oct_build, dim3(blocks), dim3(OCT_THREADS), args, 0, ctx->stream);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "octree launch");
+            ctx->launches++;
+        } else {
+            oa.gens = gens;
+            for (uint32_t g = 1; g < last; ++g) {
+                oct_build<<<g == 1 ? 1 : blocks, OCT_THREADS, 0, ctx->stream>>>(oa, g, g + 1);
+                ctx->launches++;
+            }
+        }
         if ((s = check_launch(ctx, "octree")) != ISO_OK) return s;
         if (rec) {
             nodes = replay->nodes;
@@ -970,6 +1024,10 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         }
         e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "read octree size");
+        if (h->need == NO_OCTREE) {
+            s = read_device_errors(ctx);
+            return s != ISO_OK ? s : fail(ctx, ISO_ERR_TIMEOUT, "octree barrier gave up");
+        }
         if (h->need == 0) {
             nodes = h->nodes;
             ctx->lhmc_room = std::max<uint64_t>(ctx->lhmc_room, node_cap);
@@ -1087,7 +1145,7 @@ static iso_status lhmc_planned(iso_ctx* ctx, const iso_program* prog, uint32_t d
     iso_ctx::LhmcPlan& P = ctx->lhmc_plan;
     void* bufs[6];
     lhmc_buffers(ctx, bufs);
-    if (P.exec && !ctx->timing && P.prog == prog && P.prog_uid == prog->uid && P.depth == depth && P.flags == flags &&
+    if (P.exec && !ctx->timing && !debug_waits_run_out() && P.prog == prog && P.prog_uid == prog->uid && P.depth == depth && P.flags == flags &&
         std::memcmp(P.bufs, bufs, sizeof(bufs)) == 0 && set_device(ctx) == ISO_OK) {
         cudaError_t e = cudaGraphLaunch(P.exec, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1113,7 +1171,7 @@ static iso_status lhmc_planned(iso_ctx* ctx, const iso_program* prog, uint32_t d
     const uint64_t key[3] = {prog->uid, depth, flags};
     const bool repeat = std::memcmp(key, ctx->lhmc_last_key, sizeof(key)) == 0;
     std::memcpy(ctx->lhmc_last_key, key, sizeof(key));
-    if (ctx->timing || !repeat) return ISO_OK;
+    if (ctx->timing || debug_waits_run_out() || !repeat) return ISO_OK;
     // record the same extraction with the counts just found
     lhmc_plan_release(ctx);
     const uint64_t launches0 = ctx->launches;

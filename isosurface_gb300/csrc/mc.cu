@@ -1343,10 +1343,12 @@ iso_status noalloc_scratch(unsigned char** out) {
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // iso_debug_scan_timeout: the look-back scan's first block withholds its
-// status and the others give up after a few polls
+// status and the others give up after a few polls; so at the octree's barriers
 std::atomic<int> g_debug_scan_timeout{0};
 
 }  // namespace
+
+bool iso::debug_waits_run_out() { return g_debug_scan_timeout.load() != 0; }
 
 extern "C" ISO_API iso_status iso_debug_scan_timeout(int enable) {
     g_debug_scan_timeout.store(enable ? 1 : 0);
@@ -1394,7 +1396,7 @@ extern "C" ISO_API iso_status iso_mc_extract_field_noalloc(const float* field, u
     cudaError_t e = cudaMemsetAsync(s, 0, off_status + 8 * nblocks, cs);
     if (e == cudaSuccess) e = launch_sign_bits_on(cs, field, nx, ny, nz, pitch, bits);
     if (e != cudaSuccess) return ISO_ERR_CUDA;
-    const bool withhold = g_debug_scan_timeout.load() != 0;
+    const bool withhold = iso::debug_waits_run_out();
     CountArgs ca{bits,   W,      nx,  ny, nz, (uint32_t)rows, rowtri, rowvert, status, ticket, totals, err,
                  withhold ? 256u : SPIN_LIMIT, withhold ? 1u : 0u};
     mc_count_scan<<<(unsigned)nblocks, WARPS * 32, 0, cs>>>(ca);
