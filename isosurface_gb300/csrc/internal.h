@@ -145,7 +145,14 @@ struct iso_ctx {
         uint64_t launches = 0;
     } lhmc_plan;
     uint64_t lhmc_last_key[3] = {};
-    uint64_t lhmc_room = 0;  // nodes the largest octree so far was given room for
+    // the nodes of the last octrees that outgrew a first guess of their room
+    // (more would be found again by another build)
+    struct OctreeRoom {
+        uint64_t program = 0;  // iso_program::content_hash
+        uint32_t depth = 0;
+        uint64_t nodes = 0;
+    } lhmc_rooms[8];
+    uint32_t lhmc_next_room = 0;
 };
 
 namespace iso {

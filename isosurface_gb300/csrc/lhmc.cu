@@ -972,8 +972,12 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
     auto table_at = [&](size_t cap) { return (sizeof(Ctl) + 4 * tile_words(cap) + 255) & ~(size_t)255; };
     auto head_bytes = [&](size_t cap) { return table_at(cap) + 8 * (size_t)pow2_at_least(cap / 4); };
     auto node_bytes = [&](size_t cap) { return head_bytes(cap) + 12 * cap + cap / 8 + 4096; };
-    // a first guess, or the room an earlier octree needed
-    size_t node_cap = (size_t)std::min<uint64_t>(max_nodes, std::max<uint64_t>(1ull << 20, ctx->lhmc_room));
+    // a first guess, or what this octree had last time: the arena may be larger
+    // from other ones, but the table in it is cleared for each build
+    uint64_t guess = 1ull << 20;
+    for (const auto& r : ctx->lhmc_rooms)
+        if (r.program == prog->content_hash && r.depth == max_depth) guess = std::max(guess, r.nodes);
+    size_t node_cap = (size_t)std::min(max_nodes, guess);
     const uint32_t last = std::max(2u, max_depth) + 1;  // the last generation there can be: see morton::level
     Ctl* const h = (Ctl*)(ctx->h_pinned + LHMC_PIN_CTL);
     cudaError_t e;
@@ -1030,7 +1034,8 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         }
         if (h->need == 0) {
             nodes = h->nodes;
-            ctx->lhmc_room = std::max<uint64_t>(ctx->lhmc_room, node_cap);
+            if (nodes > guess)
+                ctx->lhmc_rooms[ctx->lhmc_next_room++ % 8] = iso_ctx::OctreeRoom{prog->content_hash, max_depth, nodes};
             break;
         }
         // a generation did not fit: again in a larger arena
