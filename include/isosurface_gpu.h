@@ -102,7 +102,9 @@ ISO_API iso_status iso_debug_scan_timeout(int enable);
 /* Per-stage device timing: when enabled, every kernel the context launches is
  * bracketed by CUDA events on its stream.  iso_ctx_stage_times synchronises,
  * writes the accumulated milliseconds and launch counts of each stage
- * (ISO_STAGE_COUNT entries each) and resets them. */
+ * (ISO_STAGE_COUNT entries each) and resets them.  DualContouring's placement
+ * and ExtendedMarchingCubes' feature points run beside other passes, so the
+ * stages of those calls may add up to more than the call. */
 #define ISO_STAGE_SAMPLE 0      /* grid sampler (field + sign bits)            */
 #define ISO_STAGE_CLASSIFY 1    /* cell classification + count + scan          */
 #define ISO_STAGE_EMIT 2        /* vertex / index emission                     */

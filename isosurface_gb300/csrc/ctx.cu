@@ -124,11 +124,11 @@ static cudaEvent_t take_event(iso_ctx* ctx) {
     return e;
 }
 
-StageTimer::StageTimer(iso_ctx* c, int s) : ctx(c), stage(s) {
+StageTimer::StageTimer(iso_ctx* c, int s, cudaStream_t on) : ctx(c), stage(s), stream(on) {
     ctx->stage_launches[stage]++;
     if (!ctx->timing) return;
     a = take_event(ctx);
-    if (a) cudaEventRecord(a, ctx->stream);
+    if (a) cudaEventRecord(a, stream);
 }
 
 StageTimer::~StageTimer() {
@@ -138,7 +138,7 @@ StageTimer::~StageTimer() {
         ctx->event_pool.push_back(a);
         return;
     }
-    cudaEventRecord(b, ctx->stream);
+    cudaEventRecord(b, stream);
     ctx->pending.push_back({stage, a, b});
 }
 

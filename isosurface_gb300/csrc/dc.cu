@@ -477,6 +477,7 @@ static iso_status dc_lattice(iso_ctx* ctx, const iso_program* prog, uint32_t n, 
     // (count and scan of a 256^3 lattice, 17 us, run beside it)
     cudaStream_t side;
     if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
+    timer.ends_on(side);
     const VmHermite ev{prog->view()};
     const uint64_t place_blocks = std::min<uint64_t>((ndual + 127) / 128, 152 * 64);
     cudaError_t je = cudaSuccess;

@@ -330,8 +330,11 @@ static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t n
                            const unsigned long long* sums) {
     iso_status s;
     cudaError_t e = cudaMemcpyAsync(ctx->h_pinned, ctrl, 16, cudaMemcpyDeviceToHost, ctx->stream);
-    emc_offsets<<<nblocks, 256, 0, ctx->stream>>>(A, (uint32_t)cells, sums);
-    ctx->launches++;
+    {
+        StageTimer timer(ctx, ISO_STAGE_CLASSIFY);
+        emc_offsets<<<nblocks, 256, 0, ctx->stream>>>(A, (uint32_t)cells, sums);
+        ctx->launches++;
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "emc counts");
     const Ctrl* h = (const Ctrl*)ctx->h_pinned;
@@ -343,16 +346,20 @@ static iso_status emc_emit(iso_ctx* ctx, emc::Args A, uint64_t cells, uint32_t n
     A.cap_v = h->totals.x;
     A.cap_t = h->totals.y;
     if (nactive) {
-        StageTimer timer(ctx, ISO_STAGE_EMIT);
+        StageTimer timer(ctx, ISO_STAGE_EMIT);  // (without the wait for the side stream)
         emc_vertices<<<grid_for(ctx, nactive, 128, 32), 128, 0, ctx->stream>>>(A, active, ctrl);
         emc_triangles<<<grid_for(ctx, nactive, 256, 16), 256, 0, ctx->stream>>>(A, active, ctrl);
         ctx->launches += 2;
         if (nfeat) {
             emc_flips<<<grid_for(ctx, nfeat, 64, 32), 64, 0, ctx->stream>>>(A, features, nfeat, ctrl);
-            if ((s = join_side(ctx)) != ISO_OK) return s;
-            emc_points<<<grid_for(ctx, nfeat, 32, 32), 32, 0, ctx->stream>>>(A, features, kept, cap, nfeat);
-            ctx->launches += 2;
+            ctx->launches++;
         }
+    }
+    if (nfeat) {
+        if ((s = join_side(ctx)) != ISO_OK) return s;
+        StageTimer timer(ctx, ISO_STAGE_EMIT);
+        emc_points<<<grid_for(ctx, nfeat, 32, 32), 32, 0, ctx->stream>>>(A, features, kept, cap, nfeat);
+        ctx->launches++;
     }
     if ((s = check_launch(ctx, "emc emit")) != ISO_OK) return s;
     e = cudaMemcpyAsync(ctx->h_pinned + 2, &ctrl->flips, 8, cudaMemcpyDeviceToHost, ctx->stream);
@@ -425,7 +432,10 @@ static iso_status emc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint32
         // the feature points on a side stream: the passes below neither read
         // nor wait for them
         if ((s = fork_side(ctx, &side)) != ISO_OK) return s;
-        emc_features<<<ROW_WARPS * (unsigned)std::max(ctx->sms, 1), 32, 0, side>>>(A, kept, cap, ctrl);
+        {
+            StageTimer features_timer(ctx, ISO_STAGE_EMIT, side);
+            emc_features<<<ROW_WARPS * (unsigned)std::max(ctx->sms, 1), 32, 0, side>>>(A, kept, cap, ctrl);
+        }
         scan_block_sums<<<1, 1024, 0, ctx->stream>>>(sums, nblocks, &ctrl->totals);
         ctx->launches += 2;
     }

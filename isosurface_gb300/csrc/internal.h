@@ -156,12 +156,17 @@ struct iso_ctx {
 };
 
 namespace iso {
-// Brackets the kernels launched in its scope with events when timing is on.
+// Brackets the kernels launched in its scope with events when timing is on, on
+// the context's stream unless told otherwise; ends_on: the last of them are on
+// another one (forked from it).
 struct StageTimer {
     iso_ctx* ctx;
     int stage;
+    cudaStream_t stream;
     cudaEvent_t a = nullptr;
-    StageTimer(iso_ctx* c, int s);
+    StageTimer(iso_ctx* c, int s, cudaStream_t on);
+    StageTimer(iso_ctx* c, int s) : StageTimer(c, s, c->stream) {}
+    void ends_on(cudaStream_t on) { stream = on; }
     ~StageTimer();
 };
 }  // namespace iso
