@@ -675,14 +675,20 @@ static iso_status mc_lattice_passes(iso_ctx* ctx, const Lattice& L, uint32_t fla
     // when the edge indices fit 32 bits; otherwise the block emit resolves
     // owners itself
     const uint64_t nedges = 3ull * L.nx * L.ny * L.nz;
-    const bool cells = nedges < (1ull << 32);
+    bool cells = nedges < (1ull << 32);
+    iso_status s;
+    if (cells && L.positions && ensure(ctx, ctx->edges, 4 * nedges) != ISO_OK) {
+        // a dual lattice without room for the map (as the chunk batch)
+        cudaGetLastError();
+        ctx->last_error.clear();
+        cells = false;
+    }
     const Grid grid = make_grid(L, 0, segment_shift(ctx, L));
     const uint32_t nranges = (uint32_t)((chunks + RANGE - 1) / RANGE);
     const uint64_t nsegs = (uint64_t)grid.SL * (L.nz - 1);
     const uint32_t nblocks = (uint32_t)((nsegs + SCAN_BLOCK_SEGS - 1) / SCAN_BLOCK_SEGS);
     const size_t smem = block_emit_smem(CW);
     if (smem > 220 * 1024) return fail(ctx, ISO_ERR_INVALID_ARG, "rows too long for the emit pass");
-    iso_status s;
     const uint32_t group = emit_group(ctx, nsegs);
     // cell passes: per segment its counts, active chunks and list entry (and
     // the padding of each scan block's part); block emit: per-chunk prefixes
