@@ -738,16 +738,25 @@ iso_status launch_sample_grid(iso_ctx* ctx, const iso_program* prog, uint32_t nx
                               float* field, uint64_t pitch, uint32_t* bits, bool near_only, uint32_t zoff,
                               float reach_steps) {
     const uint32_t W = words_per_row(nx);
-    const bool smooth = near_only && smooth_culled(prog, nx, ny, nz);
+    bool smooth = near_only && smooth_culled(prog, nx, ny, nz);
+    if (smooth) {
+        const iso_status s = launch_smooth_set(
+            ctx, prog, brick_lattice(prog, nx, ny, nz, inv, field, pitch, bits, W, zoff, reach_steps));
+        if (s != ISO_OK && s != ISO_ERR_OUT_OF_MEMORY) return s;
+        if (s != ISO_OK) {
+            // no room for the boxes' lists: the samplers below need less
+            cudaGetLastError();
+            ctx->last_error.clear();
+            smooth = false;
+        }
+    }
     // the culled sampler (bricks.cuh) for the extractors on general
     // programs; hard sphere unions have their own culling below
     const bool bricks = near_only && !smooth && prog->lip > 0.0f && 4 * W <= BRICK_MAX &&
                         brick_tiles(W, ny, nz) >= (uint64_t)ctx->sms && brick_tiles(W, ny, nz) < (1ull << 22) &&
                         !(prog->kind == PK_SPHERE_SET_HARD && prog->set_n <= 8192);
     if (smooth) {
-        iso_status s = launch_smooth_set(
-            ctx, prog, brick_lattice(prog, nx, ny, nz, inv, field, pitch, bits, W, zoff, reach_steps));
-        if (s != ISO_OK) return s;
+        // launched above
     } else if (bricks) {
         // values only where marching cubes can read them (bricks.cuh): tiles
         // of 4 layers x up to 32 rows, one block each, then the mixed
