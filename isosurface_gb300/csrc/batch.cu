@@ -238,12 +238,6 @@ iso_status build_tasks(iso_batch* b) {
     return e == cudaSuccess ? ISO_OK : cuda_fail(b->ctx, e, "tasks");
 }
 
-// blocks of batch_rows that fill every SM (looked up once per process)
-unsigned rows_blocks(int sms) {
-    static std::atomic<int> per_sm{0};
-    return persistent_blocks((const void*)batch_rows, per_sm, sms);
-}
-
 // the culled sampler over `ntasks` tasks
 cudaError_t launch_sampler(const iso_batch* b, const Task* d_tasks, uint32_t ntasks) {
     const cudaStream_t stream = b->ctx->stream;
@@ -252,7 +246,7 @@ cudaError_t launch_sampler(const iso_batch* b, const Task* d_tasks, uint32_t nta
     Mixed* list = (Mixed*)((char*)d_tasks + list_at(ntasks));
     batch_classify<<<(ntasks + 7) / 8, 256, 0, stream>>>(d_tasks, b->d_sgrids, ntasks, (uint32_t)b->chunks.size(), list,
                                                          b->d_next, b->ctx->d_err);
-    batch_rows<<<rows_blocks(b->ctx->sms), 256, 0, stream>>>(b->d_sgrids, list, b->d_next);
+    batch_rows<<<persistent_blocks(b->ctx, (const void*)batch_rows), 256, 0, stream>>>(b->d_sgrids, list, b->d_next);
     return cudaGetLastError();
 }
 

@@ -4,7 +4,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <atomic>
 
 #include "internal.h"
 #include "vm.cuh"
@@ -101,18 +100,10 @@ __global__ void __launch_bounds__(256) brick_rows(VmEval ev, Tiles tiles, const 
     brick_rows_body(ev, tiles, list, count, cap);
 }
 
-// Blocks of a persistent kernel that fill every SM (its occupancy at 256
-// threads, looked up once per process and kernel).
-inline unsigned persistent_blocks(const void* kernel, std::atomic<int>& per_sm, int sms) {
-    int b = per_sm.load(std::memory_order_relaxed);
-    if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 256, 0) != cudaSuccess || b < 1) {
-            cudaGetLastError();
-            b = 4;
-        }
-        per_sm.store(b, std::memory_order_relaxed);
-    }
-    return (unsigned)(b * (sms > 0 ? sms : 1));
+// Blocks of a persistent kernel of 256 threads that fill every SM.
+inline unsigned persistent_blocks(iso_ctx* ctx, const void* kernel) {
+    const int b = resident_blocks(ctx, kernel);
+    return (unsigned)((b ? b : 4) * (ctx->sms > 0 ? ctx->sms : 1));
 }
 
 // jit.cu: the culled sampler over one lattice with the program's compiled
@@ -125,11 +116,5 @@ bool jit_sample_bricks(iso_ctx* ctx, const iso_program* prog, const GridTiles& t
 // program has none
 bool jit_sample_field(iso_ctx* ctx, const iso_program* prog, const BrickLattice& g, uint64_t blocks,
                       cudaError_t* err);
-
-template <class Tiles>
-inline unsigned brick_rows_blocks(int sms) {
-    static std::atomic<int> per_sm{0};
-    return persistent_blocks((const void*)brick_rows<Tiles>, per_sm, sms);
-}
 
 }  // namespace iso

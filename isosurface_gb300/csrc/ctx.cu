@@ -97,6 +97,18 @@ cudaError_t download(iso_ctx* ctx, void* to, const void* from, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
+int resident_blocks(iso_ctx* ctx, const void* kernel) {
+    for (const auto& r : ctx->resident)
+        if (r.first == kernel) return r.second;
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 256, 0) != cudaSuccess || b < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    ctx->resident.push_back({kernel, b});
+    return b;
+}
+
 iso_status read_device_errors(iso_ctx* ctx) {
     uint32_t h = 0;
     cudaError_t e = download(ctx, &h, ctx->d_err, 4);

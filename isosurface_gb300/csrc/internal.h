@@ -97,6 +97,8 @@ struct iso_ctx {
     // steady-state MarchingCubes: the whole extraction recorded as one CUDA
     // graph, replayed while the program, size, flags and buffers stay the same
     bool capturing = false;  // no allocation while a stream capture records
+    // resident blocks per SM of the kernels asked for so far (resident_blocks)
+    std::vector<std::pair<const void*, int>> resident;
     // a second stream for work that overlaps the context's stream (created on
     // first use) and the events that fork it from and join it to that stream
     cudaStream_t side = nullptr;
@@ -219,6 +221,9 @@ iso_status check_launch(iso_ctx* ctx, const char* what);
 iso_status read_device_errors(iso_ctx* ctx);
 bool debug_waits_run_out();  // iso_debug_scan_timeout
 iso_status set_device(iso_ctx* ctx);
+// How many blocks of 256 threads of `kernel` an SM of the context's device
+// holds (0: the lookup failed), looked up once per context.
+int resident_blocks(iso_ctx* ctx, const void* kernel);
 // Copies between pageable host memory and the device on the context's
 // stream, which is non-blocking: a plain cudaMemcpy (or cudaMemset) runs on
 // the legacy default stream, may return before its bytes are in device

@@ -319,7 +319,6 @@ struct Module {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t classify = nullptr, rows = nullptr, field = nullptr;
     cudaKernel_t dc_place = nullptr;  // only for a program whose normals are compiled too
-    std::atomic<int> rows_per_sm{0};
 };
 
 std::mutex g_jit_mutex;
@@ -430,7 +429,7 @@ bool jit_sample_bricks(iso_ctx* ctx, const iso_program* prog, const GridTiles& t
         const BrickTask* clist = list;
         const uint32_t* ccount = count;
         void* a2[] = {&t, &clist, &ccount, &c};
-        const unsigned blocks = persistent_blocks((const void*)m->rows, m->rows_per_sm, ctx->sms);
+        const unsigned blocks = persistent_blocks(ctx, (const void*)m->rows);
         e = cudaLaunchKernel((const void*)m->rows, dim3(blocks), dim3(256), a2, 0, ctx->stream);
     }
     *err = e;

@@ -55,7 +55,6 @@
 #include <cstring>
 
 #include <algorithm>
-#include <atomic>
 #include <vector>
 
 #include "block_sums.cuh"
@@ -927,18 +926,10 @@ static LhmcTrace counts_of(const iso_ctx* ctx) {
     return LhmcTrace{c->nodes, c->cubes.x, c->mesh.y, c->mesh.x};
 }
 
-// blocks of oct_build, all of which are resident at once (looked up once per process)
-static unsigned oct_blocks(const iso_ctx* ctx) {
-    static std::atomic<int> per_sm{0};
-    int b = per_sm.load(std::memory_order_relaxed);
-    if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, oct_build, OCT_THREADS, 0) != cudaSuccess || b < 1) {
-            cudaGetLastError();
-            b = 1;
-        }
-        b = std::min(b, 4);
-        per_sm.store(b, std::memory_order_relaxed);
-    }
+// blocks of oct_build, all of which are resident at once
+static unsigned oct_blocks(iso_ctx* ctx) {
+    static_assert(OCT_THREADS == 256, "resident_blocks");
+    const int b = std::max(1, std::min(resident_blocks(ctx, (const void*)oct_build), 4));
     return (unsigned)(b * std::max(ctx->sms, 1));
 }
 

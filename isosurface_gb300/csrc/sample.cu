@@ -782,7 +782,7 @@ iso_status launch_sample_grid(iso_ctx* ctx, const iso_program* prog, uint32_t nx
             const VmEval ev{prog->view()};
             brick_classify<GridTiles><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(ev, gt, list, count,
                                                                                   (uint32_t)cap, ctx->d_err);
-            brick_rows<GridTiles><<<brick_rows_blocks<GridTiles>(ctx->sms), 256, 0, ctx->stream>>>(
+            brick_rows<GridTiles><<<persistent_blocks(ctx, (const void*)brick_rows<GridTiles>), 256, 0, ctx->stream>>>(
                 ev, gt, list, count, (uint32_t)cap);
         }
         ctx->launches++;

@@ -437,13 +437,12 @@ static iso_status launch_smooth_set(iso_ctx* ctx, const iso_program* prog, const
     A.tasks = (uint2*)(base + o_tasks);
     cudaError_t e = cudaMemsetAsync(A.ntasks, 0, 4, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "smooth set task count");
-    static std::atomic<int> per_sm{0};
     StageTimer timer(ctx, ISO_STAGE_SAMPLE);
     smooth_boxes<<<(unsigned)nb, 256, 0, ctx->stream>>>(A);
     if (A.rk != 0.0f) smooth_classify<true><<<(unsigned)nb, 64, 0, ctx->stream>>>(A);
     else smooth_classify<false><<<(unsigned)nb, 64, 0, ctx->stream>>>(A);
     auto* const rows = A.rk != 0.0f ? smooth_rows<true> : smooth_rows<false>;
-    rows<<<persistent_blocks((const void*)rows, per_sm, ctx->sms), 256, 0, ctx->stream>>>(A);
+    rows<<<persistent_blocks(ctx, (const void*)rows), 256, 0, ctx->stream>>>(A);
     ctx->launches += 2;
     return ISO_OK;
 }

@@ -223,9 +223,11 @@ cudaError_t cudaDeviceGetStreamPriorityRange(int* least, int* greatest) {
     *least = *greatest = 0;
     return cudaSuccess;
 }
-// resident blocks by kernel and device: a name's length stands for its needs
+// resident blocks by kernel and device
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* blocks, const void* kernel, int, size_t, unsigned) {
-    *blocks = 1 + (int)(strlen(name_of(kernel)) % 2) + 2 * g_device;
+    int sum = 0;
+    for (const char* c = name_of(kernel); *c; ++c) sum += *c;
+    *blocks = 1 + sum % 3 + 3 * g_device;
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* blocks, const void* kernel, int threads, size_t shared) {
