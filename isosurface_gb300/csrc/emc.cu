@@ -1,8 +1,8 @@
 // ExtendedMarchingCubes::new(size).extract (src/extended_marching_cubes.rs:
 // 51-93) on the device.  The work of each lattice point and cell is in
 // emc.cuh; here each pass is one grid-stride launch over its items, the
-// counts are scanned with scan_u32, and the host reads the two totals once
-// to size the mesh.
+// counts are scanned over blocks of cells (block_sums.cuh), and the host reads
+// the two totals once to size the mesh.
 //
 //   emc_sample     Directed value of every lattice point (float4 per point)
 //                  and one sign bit per point
@@ -44,7 +44,10 @@ namespace {
 
 constexpr uint32_t BLOCK_CELLS = 1024;  // cells with one entry in the scan
 // feature cells whose tangent planes and points are kept, per lattice line:
-// sharp edges are curves, so their cells grow with the size, not its square
+// sharp edges are curves, so their cells grow with the size, not its square (a
+// box with a sphere and a torus at 128: 2200 cells, 17 per line; at 48 the room
+// is 11 KB per line).  Cells beyond it are solved after the scan, by
+// emc_points.
 constexpr uint32_t FEATURES_PER_LINE = 48;
 
 // emc_count's result for a feature cell, and emc_features'

@@ -12,7 +12,8 @@
 //    from how many nodes before it are refined, which the previous generation
 //    left as sums over tiles of nodes; the generations' sizes stay on the
 //    device.  Generation g holds keys with 3g+1 bits in ascending order.
-// 2. Primal vertices: every leaf emits primal_vertex(level, i) for i < 8; the
+// 2. Primal vertices: in the reference every leaf emits primal_vertex(level, i)
+//    (morton.rs:120-136) for i < 8; the
 //    reference keeps, per vertex, the deepest level (its max-level map).  Of
 //    the leaves of that level the one with the smallest key owns the vertex
 //    here, which gives a deterministic order (leaf order, then i) for the walk
@@ -21,8 +22,9 @@
 //    have it), leaves (the smaller key has it) or part of a coarser leaf.
 //    That takes the families around: a warp per family of eight children
 //    looks up the 27 families around it and tests the family's 27 vertices.
-// 3. Dual cubes: for each primal vertex and corner i, dual_vertex(level,
-//    REMAP_CUBE[i]) walks parent() until a node exists; the corner is that
+// 3. Dual cubes: for each primal vertex and corner i, the cell dual_vertex(level,
+//    REMAP_CUBE[i]) (morton.rs:140-144), or the first of its parents that is a
+//    node; the corner is that
 //    node's centre and value.  A corner with no ancestor keeps the previous
 //    corner's data in the reference (an order-dependent case); it is counted
 //    and reported through iso_lhmc_stale_corners.  No input reaches it: all
@@ -79,7 +81,6 @@ constexpr uint64_t DILATE_TX = 0x9249249249249249ull;
 constexpr uint64_t DILATE_T1 = 0xB6DB6DB6DB6DB6DBull;
 constexpr uint64_t DILATE_T2 = 0xDB6DB6DB6DB6DB6Dull;
 constexpr uint64_t DILATE_T3 = 0x6DB6DB6DB6DB6DB6ull;
-constexpr int MAX_LEVEL = 21;
 
 // morton.rs:54-59 computes floor(ln(k) * 0.48089834696); the constant sits
 // just below 1/(3 ln 2), so the result is floor(log2(k) / 3) except at exact
@@ -132,17 +133,6 @@ __device__ inline V3 center(uint64_t k) {  // morton.rs:78-116
     const float s = 1.0f / (float)(2u << lv);
     const float s2 = s * 2.0f;
     return v3((float)(uint32_t)bx * s2 + s, (float)(uint32_t)by * s2 + s, (float)(uint32_t)bz * s2 + s);
-}
-__device__ inline uint64_t primal_vertex(uint64_t self, int lv, uint64_t which) {  // morton.rs:120-136
-    const uint64_t k = 1ull << (3 * lv);
-    const uint64_t k1 = k << 1;
-    const uint64_t vk = add(self, which);
-    const uint64_t dk = sub(vk, k);
-    if (vk >= k1 || (dk & DILATE_TX) == 0 || (dk & DILATE_TY) == 0 || (dk & DILATE_TZ) == 0) return 0;
-    return vk << (3 * (MAX_LEVEL - lv));
-}
-__device__ inline uint64_t dual_vertex(uint64_t self, int lv, uint64_t which) {  // morton.rs:140-144
-    return sub(self >> (3 * (MAX_LEVEL - lv)), which);
 }
 }  // namespace morton
 
@@ -567,7 +557,7 @@ __device__ __forceinline__ Around look_around(const CubeArgs& A, uint32_t f) {
                                                        (vz & 1) << 2 | (vz >> 1) << 5));
     q.first = n == 13 ? 8 * f + 1 : find_family(A.families, A.fmask, q.key);
     q.refine = q.first ? __ldg(A.refine + (q.first >> 3)) : 0u;
-    // strictly inside the domain (primal_vertex, morton.rs:120-136)
+    // strictly inside the domain (morton.rs:120-136)
     const uint64_t lead = 1ull << (3 * L), low = P ^ lead;
     auto inside = [&](uint32_t v, uint64_t axis) {
         const uint64_t all = axis & (lead - 1), at = low & axis;

@@ -21,8 +21,8 @@
 //   segments with active cells, and mc_cell_emit writes those segments'
 //   vertices, records each owned vertex's id in a dense per-edge map and
 //   writes the triangles as map keys, which mc_resolve_ids turns into vertex
-//   ids.  Chunk batches and grids whose edge count exceeds 32 bits use the
-//   passes of mc_chunk.cuh, whose mc_block_emit finds each owner's id from
+//   ids.  Grids and batches whose edge count exceeds 32 bits, and dual lattices
+//   and batches without room for the edge map, use the passes of mc_chunk.cuh, whose mc_block_emit finds each owner's id from
 //   per-chunk prefixes in shared memory.
 // * The allocation-free entry point (iso_mc_extract_field_noalloc) keeps the
 //   row passes below: mc_count_scan classifies every cell and scans, per
@@ -67,10 +67,8 @@ __device__ __constant__ uint8_t c_edge_axis[12] = {0, 1, 0, 1, 0, 1, 0, 1, 2, 2,
 // Local edge by axis and the lower endpoint's two off-axis offsets (d1 + 2*d2):
 // x: (dy, dz), y: (dx, dz), z: (dx, dy).
 __device__ __constant__ uint8_t c_local_edge[3][4] = {{0, 2, 4, 6}, {3, 1, 7, 5}, {8, 9, 11, 10}};
-// the same two tables in global memory, for lanes that index them divergently
+// the axes again in global memory, for lanes that index them divergently
 // (constant memory serialises distinct addresses within a warp)
-static __device__ const uint8_t g_edge_lo[12][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {0, 0, 1}, {1, 0, 1},
-                                                    {0, 1, 1}, {0, 0, 1}, {0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
 static __device__ const uint8_t g_edge_axis[12] = {0, 1, 0, 1, 0, 1, 0, 1, 2, 2, 2, 2};
 
 // Owned-edge masks by boundary class (x==0) | (y==0)<<1 | (z==0)<<2.  An edge
@@ -622,8 +620,12 @@ cudaError_t emit_smem_attribute(size_t smem) {
 // log2 of a segment's chunks: eight for a lattice with few segments of 32
 // (128^3 and below), where a segment's chain of rounds in one emitting warp
 // is the emission's time (128^3 torus: 23 us with 32 chunks, 11 with eight;
-// 65^3 sphere: 16 and 11), else 32, whose cells fill the rounds (257^3 csg:
-// 27 us with 32 chunks, 44 with eight)
+// 65^3 sphere: 16 and 11), else 32, whose cells fill the rounds.  Whole
+// extractions, eight against 32 chunks (us): csg 33 and 40 at 65 samples, 48
+// and 52 at 97, 46 and 47 at 129, 51 and 50 at 144, 61 and 57 at 192; 64
+// spheres 46 and 52, 46 and 49, 58 and 57, 63 and 60, 76 and 72; a torus, with
+// fewer cells per segment, 24 and 27, 29 and 30, 33 and 35, 33 and 35, 34 and
+// 38, and equal at 257.
 static uint32_t segment_shift(const iso_ctx* ctx, const Lattice& L) {
     const uint64_t segs = ((uint64_t)((L.nx - 1 + 31) / 32) * (L.ny - 1) + 31) / 32 * (L.nz - 1);
     return segs <= 16 * (uint64_t)std::max(ctx->sms, 1) ? 3 : 5;
@@ -638,7 +640,9 @@ static uint32_t emit_group(const iso_ctx* ctx, uint64_t nsegs) {
 
 // layers per counting warp: long runs share the sign words between layers;
 // short ones keep the warps many (a step is one round trip to memory) and
-// their ends even
+// their ends even.  Whole extractions of 64 spheres at 513 samples with 80,
+// 160 and 320 warps per SM: 222, 220 and 225 us; at 385 145, 146 and 149; no
+// difference at 257 and below.
 static uint32_t count_run(const iso_ctx* ctx, uint64_t nsegs) {
     return (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(1, nsegs / (160 * (uint64_t)std::max(ctx->sms, 1))));
 }

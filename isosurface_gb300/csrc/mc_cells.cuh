@@ -24,7 +24,7 @@
 // triangle count up: count and scan 55, emit 79.  401 x 401 x 301 samples of
 // a dense field: 18 + 8 + 114 against 48 + 126.  A dual lattice of 256^3: 9 +
 // 8 + 28 against 19 + 4 + 50 with the block emit.  A table of 1024 lattices
-// of 16^3 to 64^3 cells: 23 + 8 + 150 and 44 for the ids against 55 + 9 + 305
+// of 16^3 to 64^3 cells: 25 + 9 + 116 and 46 for the ids against 55 + 9 + 305
 // with the block emit.
 constexpr uint32_t SCAN_BLOCK_SEGS = 4096;  // segments per block of mc_cell_scan (512 threads x 8)
 

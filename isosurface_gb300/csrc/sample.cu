@@ -235,8 +235,6 @@ __device__ __forceinline__ void sphere_column(const SetArgs& A, const float4* ke
     }
 }
 
-// The samples of column (x, y), layers z0..z1, from the nk kept spheres;
-// sign words go to word wx of each row.
 // The fold over nk spheres (sphere(i), in order) at 32 points of a row and
 // z0 .. z1: a sphere at a time over up to FOLD_Z layers, so that it is read
 // and its x and y terms computed once for them, and their chains overlap.
@@ -270,6 +268,8 @@ __device__ __forceinline__ void fold_column(const SetArgs& A, F&& sphere, uint32
     }
 }
 
+// The samples of column (x, y), layers z0..z1, from the nk kept spheres;
+// sign words go to word wx of each row.
 __device__ __forceinline__ void sample_column(const SetArgs& A, const float4* keep, const float4* thr, uint32_t nk,
                                               float px, float py, uint32_t x, uint32_t y, uint32_t z0, uint32_t z1,
                                               bool valid, int lane, uint32_t wx) {

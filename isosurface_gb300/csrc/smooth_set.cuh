@@ -393,7 +393,8 @@ __global__ void __launch_bounds__(256) smooth_rows(SmoothArgs A) {
 // union.  Below 16 spheres a box list saves nothing over the general culled
 // sampler; without a Lipschitz bound there is nothing to cull by; beyond
 // magnitudes of about 10^13 squared distances near f32's range, where the
-// bounds above would no longer be finite.
+// bounds above would no longer be finite.  (The slack is 2^-13 of the largest
+// magnitude, the width's included, so this also ends the widths, near 2^43.)
 static bool smooth_culled(const iso_program* prog, uint32_t nx, uint32_t ny, uint32_t nz) {
     return prog->smooth_set && prog->lip > 0.0f && prog->slack < 1e9f && prog->set_n >= 16 && prog->set_n <= SMOOTH_MAX && nx > 1 &&
            (uint64_t)words_per_row(nx) * ((ny + 3) / 4) * ((nz + 3) / 4) < (1ull << 26);
@@ -405,7 +406,7 @@ static iso_status launch_smooth_set(iso_ctx* ctx, const iso_program* prog, const
     A.n = prog->set_n;
     A.k = prog->set_k;
     A.kpad = prog->set_k * (1.0f + 1.0f / 1024.0f) + prog->slack;
-    A.rk = A.k >= 0x1p-60f && A.k <= 0x1p60f ? 1.0f / A.k : 0.0f;
+    A.rk = A.k >= 0x1p-60f ? 1.0f / A.k : 0.0f;  // (smooth_culled ends the widths far below 2^60)
     A.domain = prog->has_domain;
     A.sx = prog->domain[0]; A.sy = prog->domain[1]; A.sz = prog->domain[2];
     A.ox = prog->domain[3]; A.oy = prog->domain[4]; A.oz = prog->domain[5];
