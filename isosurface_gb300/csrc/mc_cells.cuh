@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256, 5) mc_cell_emit(CellEmitArgs A) {
             }
             const Grid& g = TABLE ? A.c.grids[gi] : A.c.grid;
             uint32_t grid_v0 = 0;  // first vertex of this lattice's mesh
-            if (TABLE) grid_v0 = __ldg(&A.c.segs[g.seg0]).x + blocks_before(A.c, g.seg0 / SCAN_BLOCK_SEGS, lane).x;
+            if (TABLE) grid_v0 = __ldcg(&A.c.segs[g.seg0]).x + blocks_before(A.c, g.seg0 / SCAN_BLOCK_SEGS, lane).x;
             __syncwarp();  // the previous chunks are used
             uint32_t act = 0;
             {
