@@ -375,7 +375,8 @@ ISO_API iso_status iso_dc_extract_slab(iso_ctx* ctx, const iso_program* prog, ui
  * Programs of up to 64 ops and spheres build the octree in one launch whose
  * blocks wait for one another between generations: ISO_ERR_TIMEOUT if that
  * takes some seconds (no such program does on a device that runs it).  Longer
- * programs take a launch per generation and have no such limit. */
+ * programs, and calls served by a recorded graph, take a launch per generation
+ * and have no such limit. */
 ISO_API iso_status iso_lhmc_extract(iso_ctx* ctx, const iso_program* prog, uint32_t max_depth, uint32_t flags,
                                     iso_mesh_info* info);
 

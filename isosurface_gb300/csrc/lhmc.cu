@@ -5,7 +5,8 @@
 //
 // GPU form:
 // 1. Octree build in one cooperative launch (oct_build; a launch per
-//    generation for long programs), generation by generation: evaluate the source
+//    generation for long programs and in recordings), generation by
+//    generation: evaluate the source
 //    at the centres of the children of every refined node, apply
 //    should_refine (level < 2 || (level < max_depth && |d| < size * sqrt 3)),
 //    and append them in order.  Where a refined node's children go follows
@@ -262,7 +263,7 @@ constexpr uint32_t BLOCK_CUBES = 256;    // cubes with one sum of vertices and t
 
 // what the passes find out, read back by the host in one copy
 struct Ctl {
-    uint32_t nodes;                         // 0: the build was abandoned
+    uint32_t nodes;
     uint32_t arrived;                       // blocks at the barriers of oct_build
     uint32_t pad[30];
     uint32_t released, pad2;                // turns of the barrier that are over, or ABANDONED (a cache line of its own)
@@ -277,16 +278,16 @@ constexpr uint32_t ABANDONED = 0xFFFFFFFFu;
 constexpr unsigned long long NO_OCTREE = ~0ull;
 
 // One cooperative launch with barriers for programs up to this many ops and
-// spheres, a launch per generation beyond.  What a block waits for at a
-// barrier is the other blocks' evaluations, which have no limit of their own
-// (sets of up to 2^24 spheres), while the wait needs one: it ends after some
-// seconds, and at the line a generation of 10^9 nodes takes about a tenth of
-// one.  A launch is also the faster way for long programs, whose slowest block
-// the barriers wait for: a hard set at depth 8, a launch per generation
-// against one for all, recorded: 16 spheres 123 and 128 us, 64 237 and 250,
-// 256 1115 and 1186, 1023 5673 and 6390; called without a recording the
-// launches cost 9 us more (csg at depth 8: 206 and 197 us), which they are
-// worth from about 64 spheres on.
+// spheres, a launch per generation beyond and in recordings.  What a block
+// waits for at a barrier is the other blocks' evaluations, which have no limit
+// of their own (sets of up to 2^24 spheres), while the wait needs one: it ends
+// after some seconds, and at the line a generation of 10^9 nodes takes about a
+// tenth of one.  A launch is also the faster way where the host's part of it costs
+// nothing, as the barriers wait for the slowest block: recorded, a launch per
+// generation against one for all, at depth 8: csg 216 and 222 us, a hard set of
+// 16 spheres 123 and 128, 64 237 and 250, 256 1115 and 1186, 1023 5673 and
+// 6390.  Called without a recording the launches cost 9 us more (csg: 206 and
+// 197 us), which they are worth from about 64 spheres on.
 constexpr uint64_t BARRIER_COST = 64;
 
 struct OctArgs {
@@ -345,32 +346,42 @@ __device__ __forceinline__ uint32_t find_family(const unsigned long long* famili
 
 // All blocks of the (cooperative) launch have come here `turn` times; the
 // last one to come releases the others, which wait on a word of its own.
-// Bounded: a block whose polls run out abandons the turn for all blocks, unless
-// it was released meanwhile (the word changes once for a turn).  False, in
-// every thread of every block, once a turn was abandoned.
+// Bounded: a block whose polls run out marks the count of arrivals.  If the
+// turn was not complete then, it is abandoned for all blocks, the last one to
+// come among them, which finds the mark; if it was, the mark ends the next
+// one.  False, in every thread of every block, once a turn was abandoned.
 constexpr uint32_t BARRIER_POLLS = 1u << 22;
+constexpr uint32_t GAVE_UP = 1u << 31;
 __device__ __forceinline__ bool grid_barrier(const OctArgs& A, uint32_t turn) {
-    __shared__ uint32_t s_released;
+    __shared__ bool s_go;
     __syncthreads();
     if (threadIdx.x == 0) {
         Ctl* c = A.c;
-        const volatile uint32_t* released = &c->released;
+        volatile uint32_t* released = &c->released;
+        const uint32_t all = turn * gridDim.x;
         const bool comes = !(A.withhold && blockIdx.x + 1 == gridDim.x);
+        uint32_t seen = 0;
         __threadfence();
-        if (comes && atomicAdd(&c->arrived, 1u) + 1 == turn * gridDim.x) {
+        const uint32_t before = comes ? atomicAdd(&c->arrived, 1u) : 0u;
+        if (before & GAVE_UP) {
+            seen = ABANDONED;
+        } else if (before + 1 == all) {
             __threadfence();
-            atomicCAS(&c->released, turn - 1, turn);
+            *released = seen = turn;
         } else {
             uint32_t polls = 0;
-            while (*released < turn && ++polls < A.polls) __nanosleep(20);
-            if (polls == A.polls && atomicCAS(&c->released, turn - 1, ABANDONED) == turn - 1)
-                atomicOr(A.err, DERR_QUEUE_TIMEOUT);
+            while ((seen = *released) < turn && ++polls < A.polls) __nanosleep(20);
+            if (seen < turn) seen = (atomicOr(&c->arrived, GAVE_UP) & ~GAVE_UP) < all ? ABANDONED : turn;
+        }
+        if (seen == ABANDONED) {
+            *released = ABANDONED;
+            atomicOr(A.err, DERR_QUEUE_TIMEOUT);
         }
         __threadfence();
-        s_released = *released;
+        s_go = seen != ABANDONED;
     }
     __syncthreads();
-    return s_released != ABANDONED;
+    return s_go;
 }
 
 // Generations first + 1 .. last: the whole octree in one cooperative launch
@@ -420,8 +431,7 @@ __global__ void __launch_bounds__(OCT_THREADS, 4) oct_build(OctArgs A, uint32_t 
     for (uint32_t g = max(first, 2u); g < last; ++g) {
         if (!A.gens && !grid_barrier(A, g - 1)) {
             if (blockIdx.x == 0 && tid == 0) {
-                A.c->nodes = A.host->nodes = 0;
-                A.c->need = A.host->need = NO_OCTREE;
+                A.host->need = NO_OCTREE;
             }
             return;
         }
@@ -596,11 +606,10 @@ __device__ __forceinline__ Around look_around(const CubeArgs& A, uint32_t f) {
 __global__ void __launch_bounds__(256) family_count(CubeArgs A) {
     __shared__ uint32_t s_n[8];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t families = A.c->nodes ? A.nfamilies : 0;  // none of an abandoned octree (a replay comes here)
     uint32_t n = 0;
     for (uint32_t k = warp; k < BLOCK_FAMILIES; k += 8) {
         const uint32_t f = blockIdx.x * BLOCK_FAMILIES + k;
-        if (f >= families) break;
+        if (f >= A.nfamilies) break;
         const Around q = look_around(A, f);
         const uint32_t own = __popc(q.lo) + __popc(q.hi);
         if (lane == 0) A.fcount[f] = (uint8_t)own;
@@ -987,7 +996,7 @@ static iso_status lhmc_extract_impl(iso_ctx* ctx, const iso_program* prog, uint3
         // blocks beyond the widest generation's tiles would only come to the barriers
         const uint64_t most = std::min<uint64_t>(1ull << std::min(3 * (last - 1), 32u), node_cap);
         const unsigned blocks = (unsigned)std::min<uint64_t>(oct_blocks(ctx), (most + TILE - 1) / TILE);
-        if (prog->cost <= BARRIER_COST) {
+        if (prog->cost <= BARRIER_COST && !rec) {
             oa.withhold = debug_waits_run_out();
             oa.polls = oa.withhold ? 256 : BARRIER_POLLS;
             uint32_t first_arg = 1, last_arg = last;
